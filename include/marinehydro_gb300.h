@@ -405,7 +405,9 @@ int mh_surrogate_judge_read(mh_context* ctx, int64_t count, double* estimates, i
 int mh_wu_wave_terms(mh_context* ctx, int64_t m, const double* hh, const double* vv, double* out, int mem);
 /* _dimless_wave_term and _d_dimless_wave_term_dr (exact_Guevel_Delhommeau.jl:15-46)
    for m points: out 2 complex per point; rtol/atol: adaptive Gauss-Kronrod
-   tolerances (the reference's Integrals.jl call uses its defaults). */
+   tolerances (the reference's Integrals.jl call uses its defaults), used at points
+   with z > 0 (or r = z = 0); at and below the surface the integrals are evaluated in
+   closed form up to a smooth finite integral, to rounding. */
 int mh_exact_wave_terms(mh_context* ctx, int64_t m, const double* r, const double* z, double rtol, double atol,
                         double* out, int mem);
 /* J0, J1, Y0, Y1 at m points x >= 0, as the Wu kernels evaluate them: out 4 doubles
@@ -413,7 +415,8 @@ int mh_exact_wave_terms(mh_context* ctx, int64_t m, const double* r, const doubl
    reference calls SpecialFunctions.jl besselj0/besselj1/bessely0/bessely1 at the same
    argument (wu.jl:203, 335, 396, 431). */
 int mh_bessel01_points(mh_context* ctx, int64_t m, const double* x, double* out, int mem);
-/* Tolerances used by assembly with MH_GF_EXACT_DELHOMMEAU (default 1e-12, 1e-14). */
+/* Tolerances used by assembly with MH_GF_EXACT_DELHOMMEAU (default 1e-12, 1e-14) where a
+   pair's z is above the surface (see mh_exact_wave_terms). */
 int mh_set_quadrature_tolerance(mh_context* ctx, double rtol, double atol);
 
 /* ---- diagnostics (no counterpart in the reference) ---------------------- */

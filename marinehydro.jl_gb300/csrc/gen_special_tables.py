@@ -30,6 +30,14 @@ mpmath at 40 digits):
   are rounded from the 40-digit values; the integer evaluation, emulated here bit for bit,
   is checked against mpmath below.
 
+* Exact Guevel-Delhommeau term (namespace egdq, mh_egd.cuh): below x = 8 the entire parts of
+  pi (H0 + Y0) and pi (H0' + Y0') left when Y's logarithm and pole are split off,
+      F0 = pi H0 + pi Y0 - 2 lam J0,   F1 = -pi H1 - pi Y1 - 2/x + 2 lam J1,
+      lam = log(x/2) + gamma,
+  as fixed-point rows like the Bessel ones (v 2^-60, |values| < 8); above it
+  x pi (H0 - Y0) / 2 and 2 - pi (H1 - Y1) as polynomials of u = (8/x)^2 in z = u - 1/2; and Gauss-Legendre nodes on [0, 1] (distance from the right end) and weights,
+  Newton's method on Legendre's recurrence at 40 digits.
+
 Wu fits: the polynomials A-D and dA-dC of Liang, Wu & Noblesse (wu.jl:131-197, 235-329) in
 rho in [0, 1] have monomial coefficients up to 2e5 of alternating sign, so evaluated in FP32
 their rounding is amplified ~1e5-fold.  The same polynomials written exactly in the
@@ -278,6 +286,70 @@ def bessel_tables(deg_low, deg_hankel, single):
     return tabs, exact, worst_low, worst_hk
 
 
+# ---- exact Guevel-Delhommeau term (mh_egd.cuh) ---------------------------------------------
+EGD_QF = 60      # fraction bits (|values| < 8)
+DEG_STRUVE = 22  # in u = (8/x)^2
+GL_SIZES = (18, 24)
+
+
+def egd_low(which, x):
+    """F0 (which = 0) or F1 (which = 1) of the module's notes."""
+    lam = mp.log(x / 2) + mp.euler
+    if which == 0:
+        return mp.pi * (mp.struveh(0, x) + mp.bessely(0, x)) - 2 * lam * mp.besselj(0, x)
+    return -mp.pi * (mp.struveh(1, x) + mp.bessely(1, x)) - 2 / x + 2 * lam * mp.besselj(1, x)
+
+
+def egd_high(which, u):
+    x = 8 / mp.sqrt(u)
+    if which == 0:
+        return mp.pi * x / 2 * (mp.struveh(0, x) - mp.bessely(0, x))
+    return 2 - mp.pi * (mp.struveh(1, x) - mp.bessely(1, x))
+
+
+def egd_tables():
+    """Fixed-point rows of F0, F1 (degree DEG_LOW per half-unit interval) and the two
+    polynomials above x = 8; worst absolute errors of their emulated evaluation."""
+    tabs, worst = {}, mp.mpf(0)
+    for w in (0, 1):
+        rows = []
+        for q in range(16):
+            a = mp.mpf(q) / 2
+            c = cheb_monomials(lambda x, w=w: egd_low(w, x), a, a + mp.mpf(1) / 2, DEG_LOW)
+            row = [q_int(v / mp.mpf(2) ** i, EGD_QF) for i, v in enumerate(c)]
+            for k in range(1, 17):
+                x = float(a + (mp.mpf(k) - mp.mpf(1) / 3) / 32)
+                z = (int(mp.floor(mp.mpf(x) * 2 ** 60)) - (q << 59) - (1 << 58)) << 5
+                worst = max(worst, abs(mp.mpf(fx_horner(row, z)) / 2 ** EGD_QF - egd_low(w, mp.mpf(x))))
+            rows += row
+        tabs[f"F{w}"] = rows
+        c = cheb_monomials(lambda u, w=w: egd_high(w, u), mp.mpf(0), mp.mpf(1), DEG_STRUVE)
+        co = [q_int(v, EGD_QF) for v in c]
+        assert max(abs(v) for v in co) < 2 ** 62
+        for k in range(1, 65):
+            u = float(mp.mpf(k) / 64)
+            z = min(int(mp.floor(mp.mpf(u - 0.5) * 2 ** 64)), 2 ** 63 - 2 ** 10)
+            worst = max(worst, abs(mp.mpf(fx_horner(co, z)) / 2 ** EGD_QF - egd_high(w, mp.mpf(u))))
+        tabs[f"S{w}"] = co
+    return tabs, worst
+
+
+def gauss_legendre(n):
+    """Nodes as distances from the right end of [0, 1], ascending, and weights of sum 1."""
+    out = []
+    for k in range(n):
+        x = mp.cos(mp.pi * (k + mp.mpf(3) / 4) / (n + mp.mpf(1) / 2))
+        for _ in range(8):
+            p0, p1 = mp.mpf(1), x
+            for j in range(2, n + 1):
+                p0, p1 = p1, ((2 * j - 1) * x * p1 - (j - 1) * p0) / j
+            dp = n * (x * p1 - p0) / (x * x - 1)
+            x -= p1 / dp
+        out.append(((1 - x) / 2, 1 / ((1 - x * x) * dp * dp)))
+    assert abs(mp.fsum(w for _, w in out) - 1) < mp.mpf(10) ** -35
+    return [c for c, _ in out], [w for _, w in out]
+
+
 def wu_fit_chebyshev(mono):
     """Exact Chebyshev coefficients (basis T_j(2 rho - 1)) of a monomial polynomial in rho."""
     n = len(mono) - 1
@@ -336,6 +408,9 @@ def main():
     assert worst_e < 5e-17 and worst_l < 4e-17
     tabf, _, wlf, whf = bessel_tables(DEG_LOW_F, DEG_HANKEL_F, True)
     print("FP32 Bessel: worst abs error low region", mp.nstr(wlf, 3), "Hankel P, Q/s", mp.nstr(whf, 3))
+    tabe, we = egd_tables()
+    print("exact term, fixed point: worst abs error", mp.nstr(we, 3))
+    assert we < 1e-16
     wu = {}
     for key, mono in WU_FITS.items():
         ch = wu_fit_chebyshev(mono)
@@ -392,6 +467,21 @@ def main():
         fh.write(f"__device__ const long long kLogTab[32 * kLogTerms] = {{\n    {fmt_int(ltab)}}};\n")
         fh.write(f"constexpr unsigned long long kLn2Q64 = {ln2}ULL;\n\n")
         fh.write("}  // namespace fxq\n\n")
+        fh.write("namespace egdq {\n\n")
+        fh.write(f"constexpr int kFrac = {EGD_QF};  // integers v 2^-kFrac\n")
+        fh.write(f"constexpr int kStruveTerms = {DEG_STRUVE + 1};\n\n")
+        for key, what in (("F0", "pi H0 + pi Y0 - 2 lam J0"), ("F1", "-pi H1 - pi Y1 - 2/x + 2 lam J1")):
+            fh.write(f"// {what} on [q/2, q/2 + 1/2), q = 0..15, in z = 2 (x - q/2 - 1/4)\n")
+            fh.write(f"__device__ const long long k{key}[16 * bes::kLowTerms] = {{\n    {fmt_int(tabe[key])}}};\n\n")
+        for key, what in (("S0", "x pi (H0 - Y0) / 2"), ("S1", "2 - pi (H1 - Y1)")):
+            fh.write(f"// {what} for x >= 8, in z = u - 1/2\n")
+            fh.write(f"__constant__ long long k{key}[kStruveTerms] = {{\n    {fmt_int(tabe[key])}}};\n\n")
+        for n in GL_SIZES:
+            c, w = gauss_legendre(n)
+            fh.write(f"// Gauss-Legendre, {n} nodes on [0, 1]: distance from the right end, weight\n")
+            fh.write(f"__constant__ double kGl{n}[{n}][2] = {{\n    ")
+            fh.write(",\n    ".join(f"{{{float(a):.17e}, {float(b):.17e}}}" for a, b in zip(c, w)) + "};\n\n")
+        fh.write("}  // namespace egdq\n\n")
         fh.write("namespace wuf {\n\n")
         fh.write("// Wu fits (wu.jl:131-197, 235-329) as sum_j c_j T_j(2 rho - 1), FP32\n")
         for key in WU_FITS:

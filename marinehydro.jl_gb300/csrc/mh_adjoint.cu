@@ -22,7 +22,7 @@
 #include <cuda_runtime.h>
 
 #include "mh_dual.cuh"
-#include "mh_greens.cuh"
+#include "mh_egd.cuh"
 #include "mh_internal.cuh"
 
 namespace mh {
@@ -613,15 +613,12 @@ __global__ void __launch_bounds__(kRows) wave_adjoint_kernel(AssemblyParams p, d
 }
 
 // G and dG/dr of the exact term for every unordered pair (i <= j) at wavenumber k, packed
-// (pair q = j (j + 1)/2 + i at out[2q], out[2q + 1]), one warp per pair, with the primal's
-// rules: the adaptive quadrature at the assembly's tolerance, the closed form at r = 0.
-constexpr int kEgdWarps = 4;
-__global__ void __launch_bounds__(32 * kEgdWarps) egd_pair_values_kernel(AssemblyParams p, double k, int64_t npairs,
-                                                                         double2* __restrict__ out) {
-  __shared__ double sw[kEgdWarps][8 * kGKWarpStack];
-  const int warp = threadIdx.x >> 5;
-  const int64_t q = blockIdx.x * (int64_t)kEgdWarps + warp;
-  if (q >= npairs) return;  // warp-uniform
+// (pair q = j (j + 1)/2 + i at out[2q], out[2q + 1]), one thread per pair, as in the primal.
+constexpr int kEgdThreads = 128;
+__global__ void __launch_bounds__(kEgdThreads) egd_pair_values_kernel(AssemblyParams p, double k, int64_t npairs,
+                                                                      double2* __restrict__ out) {
+  const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (q >= npairs) return;
   int64_t j = (int64_t)((sqrt(8.0 * (double)q + 1.0) - 1.0) * 0.5);
   while (j * (j + 1) / 2 > q) --j;
   while ((j + 1) * (j + 2) / 2 <= q) ++j;
@@ -629,15 +626,7 @@ __global__ void __launch_bounds__(32 * kEgdWarps) egd_pair_values_kernel(Assembl
   double r, z;
   reduced_coords(p.P[i].c, p.P[j].c, k, r, z);
   double2 G, Gr;
-  if (r == 0.0) {
-    if ((threadIdx.x & 31) != 0) return;
-    const double2 f = egd_integrand<false>(0.0, 0.0, z);
-    G = make_double2(2.0 * kPi * f.x, 2.0 * kPi * f.y);
-    Gr = make_double2(0.0, 0.0);
-  } else {
-    egd_warp(r, z, p.quad_rtol, p.quad_atol, sw[warp], G, Gr);
-    if ((threadIdx.x & 31) != 0) return;
-  }
+  egd_values(r, z, p.quad_rtol, p.quad_atol, G, Gr);
   out[2 * q] = G;
   out[2 * q + 1] = Gr;
 }
@@ -950,7 +939,7 @@ void launch_egd_pair_values(cudaStream_t st, LaunchCounter lc, const AssemblyPar
   const int64_t m = egd_packed_pairs(p.n);
   if (m <= 0) return;
   MH_LAUNCH(lc, st, "egd_pair_values",
-            egd_pair_values_kernel<<<(unsigned)((m + kEgdWarps - 1) / kEgdWarps), 32 * kEgdWarps, 0, st>>>(p, k, m, out));
+            egd_pair_values_kernel<<<(unsigned)((m + kEgdThreads - 1) / kEgdThreads), kEgdThreads, 0, st>>>(p, k, m, out));
 }
 
 void launch_egd_dk(cudaStream_t st, LaunchCounter lc, const AssemblyParams& p, double k, const double2* values,

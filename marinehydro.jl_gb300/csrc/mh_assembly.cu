@@ -17,6 +17,7 @@
 
 #include <algorithm>
 
+#include "mh_egd.cuh"
 #include "mh_greens.cuh"
 #include "mh_internal.cuh"
 #include "mh_mlp.cuh"
@@ -252,8 +253,9 @@ __device__ __forceinline__ void wave_terms(const AssemblyParams& p, const double
   if (WMODE & 2) {  // both_greens_and_gradient_greens(::ExactGuevelDelhommeau)
     double r, z;
     reduced_coords(ci, cj, k, r, z);
-    const WaveTerms e = egd_wave_terms(r, z, k, egd_adaptive<false>(r, z, p.quad_rtol, p.quad_atol),
-                                       egd_adaptive<true>(r, z, p.quad_rtol, p.quad_atol));
+    double2 G, Gr;
+    egd_values(r, z, p.quad_rtol, p.quad_atol, G, Gr);
+    const WaveTerms e = egd_wave_terms(r, z, k, G, Gr);
     w.I = zadd(w.I, e.I);
     w.Gh = zadd(w.Gh, e.Gh);
     w.Gz = zadd(w.Gz, e.Gz);
@@ -613,85 +615,39 @@ __global__ void __launch_bounds__(kTcRows) wave_kernel_tc(AssemblyParams p, cons
   if (warp == 0) tc::tmem_dealloc(tmem, kTcCols);
 }
 
-// The exact Delhommeau terms of one unordered pair {i, j} at wavenumber k, computed by the
-// whole warp (egd_warp); lane 0 writes both S/D entries.
-template <bool DIRECT>
-__device__ __forceinline__ void exact_pair_warp(const AssemblyParams& p, int64_t i, int64_t j, double k, double* sw,
-                                                const double* __restrict__ SR, const double* __restrict__ DR,
-                                                double2* __restrict__ Sb, double2* __restrict__ Db, int wave_identity) {
-  const PanelRec& Pi = p.P[i];
-  const PanelRec& Pj = p.P[j];
-  const double ci[3] = {Pi.c[0], Pi.c[1], Pi.c[2]};
-  double r, z;
-  reduced_coords(ci, Pj.c, k, r, z);
-  double2 GF, dGdr;
-  if (r == 0.0) {
-    // self pairs and vertically stacked centres: at r = 0 the integrand does not depend on
-    // theta (zeta = z), so 4 times its integral over [0, pi/2] is 2 pi times its value; the
-    // r-derivative is not needed (the horizontal gradient vanishes for r <= 1e-6)
-    if ((threadIdx.x & 31) != 0) return;
-    const double2 f = egd_integrand<false>(0.0, 0.0, z);
-    GF = make_double2(2.0 * kPi * f.x, 2.0 * kPi * f.y);
-    dGdr = make_double2(0.0, 0.0);
-  } else {
-    egd_warp(r, z, p.quad_rtol, p.quad_atol, sw, GF, dGdr);
-    if ((threadIdx.x & 31) != 0) return;
-  }
-  // both_greens_and_gradient_greens + with_reduced_coordinates_derivative, as wave_terms<., 2>
-  const double dx1 = DIRECT ? Pj.c[0] - ci[0] : ci[0] - Pj.c[0];
-  const double dx2 = DIRECT ? Pj.c[1] - ci[1] : ci[1] - Pj.c[1];
-  const WaveTerms w = egd_wave_terms(r, z, k, GF, dGdr);
-  const double ni[3] = {Pi.n[0], Pi.n[1], Pi.n[2]};
-  const double ani[3] = {Pi.area * ni[0], Pi.area * ni[1], Pi.area * ni[2]};
-  const double anj[3] = {Pj.area * Pj.n[0], Pj.area * Pj.n[1], Pj.area * Pj.n[2]};
-  store_pair<DIRECT>(p, w, i, j, ni, Pi.area, ani, Pj, anj, dx1, dx2, SR, DR, Sb, Db, wave_identity);
-}
+constexpr int kPairThreads = 128;  // threads per CTA of the kernels with one thread per pair or point
 
-constexpr int kExactWarps = 4;  // warps per CTA of the warp-per-pair exact kernels
-
-// Exact Delhommeau wave part: one warp per unordered pair {i <= j}, pairs in column-major
-// upper-triangle order q = j (j + 1) / 2 + i, grid-strided; blockIdx.y = wavenumber.
+// Exact Delhommeau terms for the pairs the surrogate queued (one thread per pair).
 template <bool DIRECT>
-__global__ void __launch_bounds__(32 * kExactWarps) exact_wave_warp_kernel(AssemblyParams p,
-                                                                            const double* __restrict__ SR,
-                                                                            const double* __restrict__ DR,
-                                                                            const double* __restrict__ ks,
-                                                                            double2* __restrict__ S,
-                                                                            double2* __restrict__ D, int64_t sstride,
-                                                                            int wave_identity) {
-  __shared__ double sw[kExactWarps][8 * kGKWarpStack];
-  const int warp = threadIdx.x >> 5;
-  const int64_t npairs = p.n * (p.n + 1) / 2;
-  const double k = ks[blockIdx.y];
-  double2* Sb = S + blockIdx.y * sstride;
-  double2* Db = D + blockIdx.y * sstride;
-  for (int64_t q = blockIdx.x * (int64_t)kExactWarps + warp; q < npairs; q += (int64_t)gridDim.x * kExactWarps) {
-    int64_t j = (int64_t)((sqrt(8.0 * (double)q + 1.0) - 1.0) * 0.5);
-    while (j * (j + 1) / 2 > q) --j;
-    while ((j + 1) * (j + 2) / 2 <= q) ++j;
-    const int64_t i = q - j * (j + 1) / 2;
-    exact_pair_warp<DIRECT>(p, i, j, k, sw[warp], SR, DR, Sb, Db, wave_identity);
-  }
-}
-
-// Exact Delhommeau terms for the pairs the surrogate queued (one warp per pair).
-template <bool DIRECT>
-__global__ void __launch_bounds__(32 * kExactWarps) surrogate_fallback_kernel(AssemblyParams p,
-                                                                               const double* __restrict__ SR,
-                                                                               const double* __restrict__ DR,
-                                                                               const double* __restrict__ ks,
-                                                                               double2* __restrict__ S,
-                                                                               double2* __restrict__ D,
-                                                                               int64_t sstride, int wave_identity) {
-  __shared__ double sw[kExactWarps][8 * kGKWarpStack];
-  const int warp = threadIdx.x >> 5;
+__global__ void __launch_bounds__(kPairThreads) surrogate_fallback_kernel(AssemblyParams p,
+                                                                          const double* __restrict__ SR,
+                                                                          const double* __restrict__ DR,
+                                                                          const double* __restrict__ ks,
+                                                                          double2* __restrict__ S,
+                                                                          double2* __restrict__ D,
+                                                                          int64_t sstride, int wave_identity) {
   const unsigned long long queued = p.fb_state[0];
   if (blockIdx.x == 0 && threadIdx.x == 0 && (int64_t)queued > p.fb_cap) p.fb_state[1] = 1ull;  // sticky overflow
   const int64_t count = (int64_t)queued < p.fb_cap ? (int64_t)queued : p.fb_cap;
-  for (int64_t q = blockIdx.x * (int64_t)kExactWarps + warp; q < count; q += (int64_t)gridDim.x * kExactWarps) {
+  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < count; q += (int64_t)gridDim.x * blockDim.x) {
     const int4 e = p.fb_list[q];
-    exact_pair_warp<DIRECT>(p, e.x, e.y, ks[e.z], sw[warp], SR, DR, S + e.z * sstride, D + e.z * sstride,
-                            wave_identity);
+    const PanelRec& Pi = p.P[e.x];
+    const PanelRec& Pj = p.P[e.y];
+    const double k = ks[e.z];
+    const double ci[3] = {Pi.c[0], Pi.c[1], Pi.c[2]};
+    double r, z;
+    reduced_coords(ci, Pj.c, k, r, z);
+    double2 G, Gr;
+    egd_values(r, z, p.quad_rtol, p.quad_atol, G, Gr);
+    // both_greens_and_gradient_greens + with_reduced_coordinates_derivative, as wave_terms<., 2>
+    const double dx1 = DIRECT ? Pj.c[0] - ci[0] : ci[0] - Pj.c[0];
+    const double dx2 = DIRECT ? Pj.c[1] - ci[1] : ci[1] - Pj.c[1];
+    const WaveTerms w = egd_wave_terms(r, z, k, G, Gr);
+    const double ni[3] = {Pi.n[0], Pi.n[1], Pi.n[2]};
+    const double ani[3] = {Pi.area * ni[0], Pi.area * ni[1], Pi.area * ni[2]};
+    const double anj[3] = {Pj.area * Pj.n[0], Pj.area * Pj.n[1], Pj.area * Pj.n[2]};
+    store_pair<DIRECT>(p, w, e.x, e.y, ni, Pi.area, ani, Pj, anj, dx1, dx2, SR, DR, S + e.z * sstride,
+                       D + e.z * sstride, wave_identity);
   }
 }
 
@@ -736,27 +692,21 @@ __global__ void bessel01_points_kernel(int64_t m, const double* __restrict__ x, 
   out[4 * q + 3] = y_defined ? Y1 : __longlong_as_double(0x7FF8000000000000LL);
 }
 
-// one warp per point
-__global__ void __launch_bounds__(32 * kExactWarps) exact_points_kernel(int64_t m, const double* __restrict__ r,
-                                                                         const double* __restrict__ z, double rtol,
-                                                                         double atol, double2* __restrict__ out) {
-  __shared__ double sw[kExactWarps][8 * kGKWarpStack];
-  const int warp = threadIdx.x >> 5;
-  const int64_t q = blockIdx.x * (int64_t)kExactWarps + warp;
-  if (q >= m) return;  // warp-uniform
+__global__ void __launch_bounds__(kPairThreads) exact_points_kernel(int64_t m, const double* __restrict__ r,
+                                                                    const double* __restrict__ z, double rtol,
+                                                                    double atol, double2* __restrict__ out) {
+  const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (q >= m) return;
   double2 G, Gr;
-  egd_warp(r[q], z[q], rtol, atol, sw[warp], G, Gr);
-  if ((threadIdx.x & 31) == 0) {
-    out[2 * q] = G;
-    out[2 * q + 1] = Gr;
-  }
+  egd_values(r[q], z[q], rtol, atol, G, Gr);
+  out[2 * q] = G;
+  out[2 * q + 1] = Gr;
 }
 
 // The exact path's check of a surrogate-assembled matrix (the learned term approximates
-// exact_Guevel_Delhommeau.jl:15-46): one warp per sampled ordered pair (i, j), drawn from a
+// exact_Guevel_Delhommeau.jl:15-46): one thread per sampled ordered pair (i, j), drawn from a
 // counter-based SplitMix64 stream of (seed, matrix, sample), recomputes the pair's S and D
-// entries with the exact term (the adaptive quadrature at the assembly's tolerance; the
-// closed form at r = 0), adds the static part as the assembly does, and accumulates the
+// entries with the exact term, adds the static part as the assembly does, and accumulates the
 // squared differences to the assembled entries and the squared assembled entries per matrix:
 // acc[2 b] += |dS|^2 + |dD|^2, acc[2 b + 1] += |S|^2 + |D|^2.
 __device__ __forceinline__ uint64_t judge_mix(uint64_t x) {
@@ -767,15 +717,13 @@ __device__ __forceinline__ uint64_t judge_mix(uint64_t x) {
 }
 
 template <bool DIRECT>
-__global__ void __launch_bounds__(32 * kExactWarps) surrogate_judge_kernel(
+__global__ void __launch_bounds__(kPairThreads) surrogate_judge_kernel(
     AssemblyParams p, const double* __restrict__ SR, const double* __restrict__ DR, const double* __restrict__ ks,
     const double2* __restrict__ S, const double2* __restrict__ D, int64_t sstride, int64_t n_samples, uint64_t seed,
     int64_t first_matrix, int wave_identity, double* __restrict__ acc) {
-  __shared__ double sw[kExactWarps][8 * kGKWarpStack];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t q = blockIdx.x * (int64_t)kExactWarps + warp;
+  const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int b = blockIdx.y;
-  if (q >= n_samples) return;  // warp-uniform
+  if (q >= n_samples) return;
   const int64_t n = p.n;
   const uint64_t h = judge_mix(seed ^ judge_mix(((uint64_t)(first_matrix + b) << 32) ^ (uint64_t)q));
   const int64_t i = (int64_t)((h & 0xFFFFFFFFULL) % (uint64_t)n);
@@ -787,16 +735,8 @@ __global__ void __launch_bounds__(32 * kExactWarps) surrogate_judge_kernel(
   double r, z;
   reduced_coords(ci, Pj.c, k, r, z);
   double2 GF, dGdr;
-  if (r == 0.0) {
-    if (lane != 0) return;
-    const double2 f = egd_integrand<false>(0.0, 0.0, z);
-    GF = make_double2(2.0 * kPi * f.x, 2.0 * kPi * f.y);
-    dGdr = make_double2(0.0, 0.0);
-  } else {
-    egd_warp(r, z, p.quad_rtol, p.quad_atol, sw[warp], GF, dGdr);
-    if (lane != 0) return;
-  }
-  // the (i, j) entries as exact_pair_warp and store_pair form them
+  egd_values(r, z, p.quad_rtol, p.quad_atol, GF, dGdr);
+  // the (i, j) entries as store_pair forms them
   const double dx1 = DIRECT ? Pj.c[0] - ci[0] : ci[0] - Pj.c[0];
   const double dx2 = DIRECT ? Pj.c[1] - ci[1] : ci[1] - Pj.c[1];
   const WaveTerms w = egd_wave_terms(r, z, k, GF, dGdr);
@@ -877,20 +817,9 @@ void launch_assemble_wave(cudaStream_t st, LaunchCounter lc, const AssemblyParam
     lc.post(st, "assemble_wave_surrogate");
     lc.pre(st);
     const int fbg = 8 * 152;
-    if (p.direct) surrogate_fallback_kernel<true><<<fbg, 32 * kExactWarps, 0, st>>>(p, SR, DR, ks_dev, S, D, sstride, wave_identity);
-    else surrogate_fallback_kernel<false><<<fbg, 32 * kExactWarps, 0, st>>>(p, SR, DR, ks_dev, S, D, sstride, wave_identity);
+    if (p.direct) surrogate_fallback_kernel<true><<<fbg, kPairThreads, 0, st>>>(p, SR, DR, ks_dev, S, D, sstride, wave_identity);
+    else surrogate_fallback_kernel<false><<<fbg, kPairThreads, 0, st>>>(p, SR, DR, ks_dev, S, D, sstride, wave_identity);
     lc.post(st, "assemble_wave_fallback");
-    return;
-  }
-  if (wv == MH_GF_EXACT_DELHOMMEAU) {
-    // one warp per unordered pair; enough CTAs for several resident per SM
-    const int64_t npairs = p.n * (p.n + 1) / 2;
-    const int64_t want = (npairs + kExactWarps - 1) / kExactWarps;
-    dim3 g((unsigned)std::min<int64_t>(want, 152 * 16), (unsigned)nk);
-    lc.pre(st);
-    if (p.direct) exact_wave_warp_kernel<true><<<g, 32 * kExactWarps, 0, st>>>(p, SR, DR, ks_dev, S, D, sstride, wave_identity);
-    else exact_wave_warp_kernel<false><<<g, 32 * kExactWarps, 0, st>>>(p, SR, DR, ks_dev, S, D, sstride, wave_identity);
-    lc.post(st, "assemble_wave_exact");
     return;
   }
   const int mode = (wv == MH_GF_WU) ? 1 : (wv == MH_GF_EXACT_DELHOMMEAU ? 2 : 3);
@@ -910,14 +839,14 @@ void launch_surrogate_judge(cudaStream_t st, LaunchCounter lc, const AssemblyPar
                             int64_t sstride, int64_t n_samples, uint64_t seed, int64_t first_matrix,
                             int wave_identity, double* acc) {
   if (p.n <= 0 || nk <= 0 || n_samples <= 0) return;
-  dim3 g((unsigned)((n_samples + kExactWarps - 1) / kExactWarps), (unsigned)nk);
+  dim3 g((unsigned)((n_samples + kPairThreads - 1) / kPairThreads), (unsigned)nk);
   if (p.direct)
     MH_LAUNCH(lc, st, "surrogate_judge",
-              surrogate_judge_kernel<true><<<g, 32 * kExactWarps, 0, st>>>(p, SR, DR, ks_dev, S, D, sstride, n_samples,
+              surrogate_judge_kernel<true><<<g, kPairThreads, 0, st>>>(p, SR, DR, ks_dev, S, D, sstride, n_samples,
                                                                          seed, first_matrix, wave_identity, acc));
   else
     MH_LAUNCH(lc, st, "surrogate_judge",
-              surrogate_judge_kernel<false><<<g, 32 * kExactWarps, 0, st>>>(p, SR, DR, ks_dev, S, D, sstride, n_samples,
+              surrogate_judge_kernel<false><<<g, kPairThreads, 0, st>>>(p, SR, DR, ks_dev, S, D, sstride, n_samples,
                                                                           seed, first_matrix, wave_identity, acc));
 }
 
@@ -938,7 +867,7 @@ void launch_exact_points(cudaStream_t st, LaunchCounter lc, int64_t m, const dou
                          double atol, double2* out) {
   if (m <= 0) return;
   MH_LAUNCH(lc, st, "exact_points",
-            exact_points_kernel<<<(unsigned)((m + kExactWarps - 1) / kExactWarps), 32 * kExactWarps, 0, st>>>(
+            exact_points_kernel<<<(unsigned)((m + kPairThreads - 1) / kPairThreads), kPairThreads, 0, st>>>(
                 m, r, z, rtol, atol, out));
 }
 

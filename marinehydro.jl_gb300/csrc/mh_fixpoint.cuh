@@ -208,6 +208,37 @@ __device__ __forceinline__ double sqrt_pos(double x) {
   return __longlong_as_double((long long)(((unsigned long long)ex << 52) | (mant & 0x000FFFFFFFFFFFFFull)));
 }
 
+// 1/sqrt(x) for a normal x > 0 on the integer pipe (+inf for x below the normal range): the
+// seed and the two Newton steps of sqrt_pos, y = 1/sqrt(m) in (1/2, 1] as y 2^63, rounded to
+// 53 bits: within one ulp of the correctly rounded value, without the FP64 pipe.
+__device__ __forceinline__ double rsqrt_pos(double x) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  const int e = (int)((b >> 52) & 0x7FF);
+  if (e == 0) return __longlong_as_double(0x7FF0000000000000ll);
+  const unsigned long long frac = b & 0x000FFFFFFFFFFFFFull;
+  const int odd = (e - 1023) & 1;
+  const unsigned long long M62 = ((frac | (1ull << 52)) << 10) << odd;  // m 2^62
+  float yf;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(__int_as_float(((127 + odd) << 23) | (int)(frac >> 29))));
+  const unsigned int yb = __float_as_uint(yf);
+  unsigned long long Y = yb >= 0x3F800000u
+                             ? (1ull << 63)
+                             : (unsigned long long)((yb & 0x7FFFFFu) | 0x800000u) << (40 + (int)(yb >> 23) - 126 - 1);
+#pragma unroll
+  for (int it = 0; it < 2; ++it) {
+    const unsigned long long Y2 = __umul64hi(Y, Y);       // y^2 2^62
+    const unsigned long long T = __umul64hi(M62, Y2);     // m y^2 2^60
+    const unsigned long long E = 3ull * (1ull << 60) - T;  // (3 - m y^2) 2^60
+    Y = __umul64hi(Y, E) << 3;                            // y (3 - m y^2) / 2  2^63
+  }
+  const int p = 63 - __clzll(Y);  // 62 or 63
+  const int sh = p - 52;
+  unsigned long long mant = (Y >> sh) + ((Y >> (sh - 1)) & 1ull);
+  int ex = p - 63 + 1023 - ((e - 1023 - odd) >> 1);  // 1/sqrt(x) = (Y 2^-63) 2^-h, x = m 2^(2h)
+  if (mant >> 53) { mant >>= 1; ++ex; }
+  return __longlong_as_double((long long)(((unsigned long long)ex << 52) | (mant & 0x000FFFFFFFFFFFFFull)));
+}
+
 // sum_i c[i] t^i for t in [0, 1) as unit_q64(t); coefficients and result v 2^-F
 template <int N>
 __device__ __forceinline__ long long horner_u(const long long (&c)[N], unsigned long long t) {

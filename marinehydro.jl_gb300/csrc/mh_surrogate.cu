@@ -6,7 +6,7 @@
 // [1e-3, 1e3]) and z uniform in [-50, 0], drawn from a counter-based generator (SplitMix64, Steele, Lea & Flood,
 // "Fast splittable pseudorandom number generators", OOPSLA 2014) so that sample q of
 // a seed is the same on every device and launch shape.  Targets come from the exact
-// kernel (egd_adaptive, the device restatement of exact_Guevel_Delhommeau.jl:15-46)
+// kernel (egd_values, the device restatement of exact_Guevel_Delhommeau.jl:15-46)
 // and the Wu fits (wu_wave_term_and_derivs).
 //
 // Training step (batch B, one thread per sample):
@@ -20,7 +20,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
-#include "mh_greens.cuh"
+#include "mh_egd.cuh"
 #include "mh_internal.cuh"
 #include "mh_mlp.cuh"
 #include "mh_wu_f32.cuh"
@@ -52,25 +52,22 @@ __device__ __forceinline__ void sample_point(uint64_t seed, uint64_t q, uint64_t
   z = -50.0 * u01(h2);
 }
 
-constexpr int kSampleWarps = 4;
+constexpr int kPointThreads = 128;
 
-// one warp per sample (the exact kernel's warp-cooperative quadrature); lane 0 writes
-__global__ void __launch_bounds__(32 * kSampleWarps) surrogate_samples_kernel(uint64_t seed, int64_t M,
-                                                                               int64_t offset, int64_t count,
-                                                                               double rtol, double atol,
-                                                                               float2* __restrict__ X,
-                                                                               float* __restrict__ Y8,
-                                                                               double* __restrict__ R2) {
-  __shared__ double sw[kSampleWarps][8 * kGKWarpStack];
-  const int warp = threadIdx.x >> 5;
-  const int64_t t = blockIdx.x * (int64_t)kSampleWarps + warp;
-  if (t >= count) return;  // warp-uniform
+// one thread per sample
+__global__ void __launch_bounds__(kPointThreads) surrogate_samples_kernel(uint64_t seed, int64_t M,
+                                                                          int64_t offset, int64_t count,
+                                                                          double rtol, double atol,
+                                                                          float2* __restrict__ X,
+                                                                          float* __restrict__ Y8,
+                                                                          double* __restrict__ R2) {
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (t >= count) return;
   const int64_t q = offset + t;
   double r, z;
   sample_point(seed, (uint64_t)q, (uint64_t)M, r, z);
   double2 G, Gr;
-  egd_warp(r, z, rtol, atol, sw[warp], G, Gr);
-  if ((threadIdx.x & 31) != 0) return;
+  egd_values(r, z, rtol, atol, G, Gr);
   double2 GF, Gh, Gv;
   wu_wave_term_and_derivs(r, z, GF, Gh, Gv);
   const double d = sqrt(r * r + z * z);
@@ -286,26 +283,23 @@ __global__ void round_bf16_kernel(const float* __restrict__ in, float* __restric
   out[p] = p < count ? __bfloat162float(__float2bfloat16_rn(in[p])) : 0.0f;
 }
 
-// surrogate GF, Gh, Gv at points (r, z) (the layout of the Wu point evaluator), one warp per
-// point; points outside the training box take the exact kernel (warp-cooperative, as in
-// assembly), inside it lane 0 evaluates the Wu terms and the network
-__global__ void __launch_bounds__(32 * kSampleWarps) surrogate_points_kernel(const float* __restrict__ mlp, int64_t m,
+// surrogate GF, Gh, Gv at points (r, z) (the layout of the Wu point evaluator), one thread per
+// point; points outside the training box take the exact term, as in assembly, inside it the
+// Wu terms and the network
+__global__ void __launch_bounds__(kPointThreads) surrogate_points_kernel(const float* __restrict__ mlp, int64_t m,
                                                                               const double* __restrict__ r,
                                                                               const double* __restrict__ z,
                                                                               double rtol, double atol,
                                                                               double2* __restrict__ out) {
   extern __shared__ float4 spp4[];
-  __shared__ double sw[kSampleWarps][8 * kGKWarpStack];
   load_params(spp4, mlp);
   __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t q = blockIdx.x * (int64_t)kSampleWarps + warp;
-  if (q >= m) return;  // warp-uniform
+  const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (q >= m) return;
   const double rq = r[q], zq = z[q];
   double2 GF, Gh, Gv;
   if (surrogate_in_box((float)rq, (float)zq)) {
     // FP32 throughout, as the tensor-core assembly (wave_kernel_tc)
-    if (lane != 0) return;
     const float rf = (float)rq, zf = (float)zq;
     float2 g, gh, gv, dG, dGr, dGz;
     wu_wave_term_and_derivs_f32(rf, zf, g, gh, gv);
@@ -314,8 +308,7 @@ __global__ void __launch_bounds__(32 * kSampleWarps) surrogate_points_kernel(con
     Gh = make_double2(gh.x + dGr.x, gh.y + dGr.y);
     Gv = make_double2(gv.x + dGz.x, gv.y + dGz.y);
   } else {
-    egd_warp(rq, zq, rtol, atol, sw[warp], GF, Gh);
-    if (lane != 0) return;
+    egd_values(rq, zq, rtol, atol, GF, Gh);
     Gv = make_double2(GF.x + 2.0 / hypot(rq, zq), GF.y);
   }
   out[3 * q] = GF;
@@ -331,8 +324,7 @@ void launch_surrogate_samples(cudaStream_t st, LaunchCounter lc, uint64_t seed, 
                               int64_t count, double rtol, double atol, float2* X, float* Y8, double* R2) {
   if (count <= 0) return;
   MH_LAUNCH(lc, st, "surrogate_samples",
-            surrogate_samples_kernel<<<(unsigned)((count + kSampleWarps - 1) / kSampleWarps), 32 * kSampleWarps, 0,
-                                       st>>>(seed, M, offset, count, rtol, atol, X, Y8, R2));
+            surrogate_samples_kernel<<<(unsigned)((count + kPointThreads - 1) / kPointThreads), kPointThreads, 0, st>>>(seed, M, offset, count, rtol, atol, X, Y8, R2));
 }
 
 void launch_mlp_loss_grad(cudaStream_t st, LaunchCounter lc, const float* qparams, const float2* X, const float* Y8,
@@ -368,8 +360,7 @@ void launch_surrogate_points(cudaStream_t st, LaunchCounter lc, const float* mlp
   if (m <= 0) return;
   const size_t psmem = sizeof(float) * kMlpParamsPadded;
   MH_LAUNCH(lc, st, "surrogate_points",
-            surrogate_points_kernel<<<(unsigned)((m + kSampleWarps - 1) / kSampleWarps), 32 * kSampleWarps, psmem,
-                                      st>>>(mlp, m, r, z, rtol, atol, out));
+            surrogate_points_kernel<<<(unsigned)((m + kPointThreads - 1) / kPointThreads), kPointThreads, psmem, st>>>(mlp, m, r, z, rtol, atol, out));
 }
 
 }  // namespace mh
