@@ -253,8 +253,8 @@ int mh_batch_release(mh_context* ctx);
      choices[4q+0]  reserved (the FP64 tensor-core update, MH_PREC_FP64_TC, is a persistent
                     kernel over equal slices of its tiles; the value is kept and ignored)
      choices[4q+1]  128-column tiles per CTA of the BF16x3 FP32 update (MH_PREC_MIXED)
-     choices[4q+2]  largest thread-block cluster of the FP64 LU panel
-     choices[4q+3]  largest thread-block cluster of the FP32 LU panel
+     choices[4q+2]  largest thread-block cluster of the FP64 LU panel (8: up to 16 CTAs)
+     choices[4q+3]  largest thread-block cluster of the FP32 LU panel (8: up to 16 CTAs)
    n_entries = 0 restores the defaults (8, 4, 8, 8).  The table applies to every later
    factorization of the context, including the captured batch graph (a changed table
    re-captures it).  The shapes change only the schedule: each output entry is computed

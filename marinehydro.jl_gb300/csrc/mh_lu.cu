@@ -9,15 +9,16 @@
 // Work split per panel step k (nb = 32 columns):
 //   panel_cluster_kernel  a thread-block cluster of P CTAs per matrix: the panel's
 //                  rows are split over the P CTAs and held in shared memory; pivot
-//                  candidates and the pivot row travel through distributed shared
-//                  memory with two cluster barriers per column, so the panel's FP64
+//                  candidates and their rows are pushed through distributed shared
+//                  memory with one cluster barrier per column, so the panel's FP64
 //                  rank-1 updates run on P SMs instead of one
 //   panel_kernel   the same on one CTA straight from global memory, for panels too
 //                  tall for the cluster's shared memory
 //   laswp_kernel   the panel's row interchanges applied to every column outside it,
 //                  as one permutation of at most 64 rows (a warp per column)
-//   trsm_kernel    U12 = L11^-1 A12, one thread per column, L11 in shared memory
-//   gemm_kernel    A22 -= L21 U12, 64x64 tiles, 4x4 complex outputs per thread
+//   trsm8_kernel, trsm_kernel   U12 = L11^-1 A12 with L11 in shared memory: eight lanes
+//                  per column in FP64, one thread per column in FP32
+//   gemm3m_kernel, gemm_kernel  A22 -= L21 U12 on the CUDA cores (FP64, FP32)
 // Templated on the real type: double (the plain FP64 path) and float (the factor
 // used by mixed-precision iterative refinement).
 #include <cooperative_groups.h>
@@ -79,6 +80,15 @@ template <> __device__ __forceinline__ double2 crecip<double2>(double2 a) {
   const double sx = a.x * f, sy = a.y * f;
   const double rf = fx::recip(fma(sx, sx, sy * sy)) * f;
   return make_double2(sx * rf, -sy * rf);
+}
+// FP32: the same scaling with one division
+template <> __device__ __forceinline__ float2 crecip<float2>(float2 a) {
+  const int ex = (__float_as_int(a.x) >> 23) & 0xFF, ey = (__float_as_int(a.y) >> 23) & 0xFF;
+  const int e = ex > ey ? ex : ey;
+  const float f = __int_as_float((254 - e) << 23);
+  const float sx = a.x * f, sy = a.y * f;
+  const float rf = __fdividef(1.0f, fmaf(sx, sx, sy * sy)) * f;
+  return make_float2(sx * rf, -sy * rf);
 }
 template <typename C> __device__ __forceinline__ C cdiv(C a, C b) { return cmul(a, crecip(b)); }
 template <typename C> __device__ __forceinline__ C czero() { C r; r.x = 0; r.y = 0; return r; }
@@ -168,32 +178,53 @@ __global__ void __launch_bounds__(512) panel_kernel(BatchDesc d, typename cplx_t
 
 // ---------------------------- panel on a cluster -------------------------------
 constexpr int kPanelThreads = 512;
-// panel rows one CTA holds in shared memory (32 complex columns each, < 227 KB)
-template <typename T> struct PanelRows;
-template <> struct PanelRows<double> { static constexpr int value = 432; };
-template <> struct PanelRows<float> { static constexpr int value = 864; };
+constexpr int kPanelMaxCtas = 16;  // largest cluster (above 8 CTAs it is a non-portable size)
+// panel rows one CTA of a cluster of P holds in shared memory: 32 complex columns each, and the
+// candidate rows of two columns and P CTAs, below 227 KB
+template <typename T> __host__ __device__ constexpr int panel_rows(int P) {
+  return sizeof(T) == 8 ? (P <= 8 ? 430 : 414) : 864;
+}
+// rows per CTA of a panel of m rows on P CTAs: a multiple of 32 where `cap` allows
+__host__ __device__ inline int panel_chunk(int64_t m, int P, int cap) {
+  const int64_t c = ((m + P - 1) / P + 31) / 32 * 32;
+  return (int)(c < cap ? c : cap);
+}
+// dynamic shared memory of the panel kernel: the chunk (odd leading dimension) and the slots
+template <typename T> constexpr size_t panel_smem_bytes(int chunk, int width, int P) {
+  return 2 * sizeof(T) * ((size_t)(chunk | 1) * width + 2 * (size_t)P * kNB);
+}
 
 // Pivot candidates compare |re| + |im| through the bit pattern of the (non-negative) value as
-// a signed integer, which orders like the value: FP64 comparisons run on GB300's narrow FP64
-// pipe, integer ones do not.  -1 stands below every candidate.
+// an unsigned integer, which orders like the value (and puts a NaN above every number): FP64
+// comparisons run on GB300's narrow FP64 pipe, integer ones do not.  "No candidate" is key 0
+// with row INT_MAX, which loses against any row (a zero column is recognised by the key 0).
 template <typename T> struct PivotKey;
 template <> struct PivotKey<double> {
-  using type = long long;
-  __device__ static __forceinline__ long long of(double v) { return __double_as_longlong(v); }
+  using type = unsigned long long;
+  __device__ static __forceinline__ type of(double v) { return (type)__double_as_longlong(v); }
 };
 template <> struct PivotKey<float> {
-  using type = int;
-  __device__ static __forceinline__ int of(float v) { return __float_as_int(v); }
+  using type = unsigned;
+  __device__ static __forceinline__ type of(float v) { return __float_as_uint(v); }
 };
 
-// (value, row) of the larger |re| + |im|; ties go to the smaller row (izamax's first maximum)
-template <typename T> __device__ __forceinline__ void argmax_merge(T& v, int& i, T ov, int oi) {
+// (key, row) of the larger |re| + |im|; ties go to the smaller row (izamax's first maximum)
+template <typename K> __device__ __forceinline__ void argmax_merge(K& v, int& i, K ov, int oi) {
   if (ov > v || (ov == v && oi < i)) { v = ov; i = oi; }
 }
-template <typename T> __device__ __forceinline__ void warp_argmax(T& v, int& i) {
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) argmax_merge(v, i, __shfl_xor_sync(0xffffffffu, v, off),
-                                                       __shfl_xor_sync(0xffffffffu, i, off));
+// over the warp, by the warp-wide integer reductions (three for a 64-bit key, two for a 32-bit
+// one, against five rounds of three shuffles)
+__device__ __forceinline__ void warp_argmax(unsigned long long& v, int& i) {
+  const unsigned hi = (unsigned)(v >> 32), lo = (unsigned)v;
+  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+  i = (int)__reduce_min_sync(0xffffffffu, (unsigned)((hi == mh && lo == ml) ? i : INT_MAX));
+  v = ((unsigned long long)mh << 32) | ml;
+}
+__device__ __forceinline__ void warp_argmax(unsigned& v, int& i) {
+  const unsigned m = __reduce_max_sync(0xffffffffu, v);
+  i = (int)__reduce_min_sync(0xffffffffu, (unsigned)(v == m ? i : INT_MAX));
+  v = m;
 }
 
 // split cluster barrier: arrive (releasing this thread's writes), later wait (acquiring
@@ -202,22 +233,27 @@ __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 
 // Rows k .. n-1 of the panel (m = n - k panel rows, panel row r = matrix row k + r) are
-// split into chunks of `chunk` rows, chunk >= kb, so CTA 0 holds the kb diagonal rows.
-// Thread t of a CTA owns its chunk's rows t, t + 512, ...: it alone writes them in shared
-// memory.  Rows cross CTAs only through double-buffered publication slots, so one cluster
-// barrier per column suffices.  Per column j:
-//   every CTA posts its best candidate (value, row) and a copy of that row; CTA 0 also
-//   posts a copy of row j;  cluster barrier
-//   warp 0 of every CTA reduces the P candidates and fetches the pivot row (and, in the
-//   CTA that owns the pivot row, row j) from the winners' slots through distributed
-//   shared memory;  CTA barrier
-//   the owners write the interchanged rows, then every thread scales its rows' entry j and
-//   applies the rank-1 update to columns j+1 .. kb-1, searching column j+1 as it goes.
-// Slots of parity j are rewritten at column j + 2, after every CTA has passed the barrier
-// of column j + 1 and so finished its reads of column j.  (Posting column j+1 before the
-// rest of the update and overlapping that update with a split barrier was measured slower:
-// the extra CTA barriers cost more than the overlap saves.)  Same arithmetic, in the same
-// order, as panel_kernel.
+// split into chunks of `chunk` rows (a multiple of 32, so that no warp of the update is left
+// part empty; CTA 0 holds the kb <= 32 diagonal rows), one per CTA, in its shared memory with
+// an odd leading dimension (a row's entries then sit in different banks).  Per column j:
+//   every CTA finds its best candidate and pushes it, with a copy of its row, into a slot of
+//   every CTA of the cluster (distributed shared memory stores); CTA 0 pushes row j;
+//   cluster barrier; warp 0 of every CTA picks the winner among the P slots, now local, and
+//   takes the pivot's reciprocal; CTA barrier
+//   a thread per row forms the multipliers l (the interchanged row's from the copy of row j);
+//   CTA barrier
+//   the rank-1 update, in items of 32 rows by a few columns dealt to all 16 warps, column
+//   j + 1 first, which is searched as it is updated.
+// What bounds it: for few rows the chain of barriers and reductions, for many the FP64 pipe
+// (124 FMAs per row at j = 0, two per clock and SM).  A warp issues to one of the SM's four
+// FP64 pipes, so the update goes by items and not by one thread per row (that left three pipes
+// idle for 32 rows, and a fifth of the time at 400); pushing saves the two remote reads of
+// the pull form, warp-wide integer reductions the shuffles.  Per 32-column panel on a GB300,
+// launch included: 200 rows 142 -> 82 us, five matrices of 1000 rows 165 -> 105 us, one of 3000
+// rows (16 CTAs instead of 8) 210 -> 146 us.
+// Slots of parity j are written again at column j + 2, after the barrier of column j + 1, which
+// every CTA reaches only when it is done reading column j's.
+template <typename T> struct PanelItem { static constexpr int cols = sizeof(T) == 8 ? 4 : 8; };
 template <typename T>
 __global__ void __launch_bounds__(kPanelThreads) panel_cluster_kernel(BatchDesc d, typename cplx_t<T>::type* __restrict__ Aall,
                                                                      int32_t* __restrict__ ipiv_all,
@@ -225,74 +261,89 @@ __global__ void __launch_bounds__(kPanelThreads) panel_cluster_kernel(BatchDesc 
                                                                      int chunk_cap, int width) {
   using C = typename cplx_t<T>::type;
   using K = typename PivotKey<T>::type;
+  constexpr int kWarps = kPanelThreads / 32, GC = PanelItem<T>::cols;
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   extern __shared__ __align__(16) unsigned char panel_smem[];
-  C* sp = reinterpret_cast<C*>(panel_smem);  // chunk x kb, column-major (leading dimension chunk)
-  __shared__ C pub_row[2][kNB];               // this CTA's candidate row, by column parity
-  __shared__ C pub_j[2][kNB];                 // CTA 0: row j
-  __shared__ K cand_v[2];
-  __shared__ int cand_i[2];
+  C* sp = reinterpret_cast<C*>(panel_smem);            // chunk x kb, column-major (leading dimension ld)
+  C* slots = sp + (size_t)(chunk_cap | 1) * width;     // candidate rows [parity][CTA][kNB]
+  __shared__ C pub_j[2][kNB];                          // row j
+  __shared__ K cand_v[2][kPanelMaxCtas];
+  __shared__ int cand_i[2][kPanelMaxCtas];
   __shared__ C urow[kNB], jrow[kNB];
-  __shared__ K red_v[kPanelThreads / 32];
-  __shared__ int red_i[kPanelThreads / 32];
+  __shared__ K red_v[kWarps];
+  __shared__ int red_i[kWarps];
   __shared__ int s_piv;
   __shared__ C s_inv;
   const int P = (int)cl.num_blocks(), rank = (int)cl.block_rank();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t bmat = blockIdx.y, n = d.order(bmat);
   if (k >= n) return;  // a grouped batch: this matrix is factored (the whole cluster leaves)
+  cluster_arrive();    // every CTA of the cluster runs before the first push
   C* A = Aall + d.offset(bmat);
   const int64_t m = n - k;
   const int kb = (int)(m < width ? m : width);  // panel width: 32, or 16 for a half of a two-level panel
-  // rows per CTA for this matrix: at most the launch's capacity, at least the diagonal block
-  const int chunk = (int)max((int64_t)kb, min((int64_t)chunk_cap, (m + P - 1) / P));
+  const int chunk = panel_chunk(m, P, chunk_cap);
+  const int ld = chunk | 1;
   const int r0 = rank * chunk;  // first panel row of this CTA
   const int rows = (int)((m - r0) < chunk ? ((m - r0) > 0 ? (m - r0) : 0) : chunk);
+  const int nrb = (rows + 31) >> 5;
+  C* Ap = A + (k + r0) + k * n;
 
-  for (int c = 0; c < kb; ++c)
-    for (int i = tid; i < rows; i += kPanelThreads) sp[c * chunk + i] = A[(k + r0 + i) + (k + c) * n];
-  // candidate for column 0 (each thread reads only its own rows)
-  K best = -1;
-  int bi = INT_MAX;
-  for (int i = tid; i < rows; i += kPanelThreads) {
-    const C a = sp[i];
-    argmax_merge(best, bi, PivotKey<T>::of(fabs(a.x) + fabs(a.y)), r0 + i);
+#pragma unroll 4
+  for (int q = warp; q < nrb * kb; q += kWarps) {
+    const int c = q / nrb, i = (q - c * nrb) * 32 + lane;
+    if (i < rows) sp[c * ld + i] = Ap[i + c * n];
   }
+  // candidate for column 0 (the rows that this thread loaded)
+  K best = 0;
+  int bi = INT_MAX;
+  for (int q = warp; q < nrb; q += kWarps) {
+    const int i = q * 32 + lane;
+    if (i < rows) {
+      const C a = sp[i];
+      argmax_merge(best, bi, PivotKey<T>::of(fabs(a.x) + fabs(a.y)), r0 + i);
+    }
+  }
+  cluster_wait();
   for (int j = 0; j < kb; ++j) {
     const int par = j & 1;
-    // post this CTA's candidate for column j with a copy of its row, and (CTA 0) row j
     warp_argmax(best, bi);
     if (lane == 0) { red_v[warp] = best; red_i[warp] = bi; }
     __syncthreads();
     if (warp == 0) {
-      best = lane < kPanelThreads / 32 ? red_v[lane] : (K)-1;
-      bi = lane < kPanelThreads / 32 ? red_i[lane] : INT_MAX;
+      best = lane < kWarps ? red_v[lane] : (K)0;
+      bi = lane < kWarps ? red_i[lane] : INT_MAX;
       warp_argmax(best, bi);
-      if (lane == 0) { cand_v[par] = best; cand_i[par] = bi; }
-      if (bi != INT_MAX && lane < kb) pub_row[par][lane] = sp[lane * chunk + (bi - r0)];
-      if (rank == 0 && lane < kb) pub_j[par][lane] = sp[lane * chunk + j];
-    }
-    cl.sync();  // candidates and rows posted
-    if (warp == 0) {
-      K v = -1;
-      int vi = INT_MAX;
-      if (lane < P) {
-        v = *cl.map_shared_rank(&cand_v[par], (unsigned)lane);
-        vi = *cl.map_shared_rank(&cand_i[par], (unsigned)lane);
+      const bool have = bi != INT_MAX;
+      C row = czero<C>(), rj = czero<C>();
+      if (have && lane < kb) row = sp[lane * ld + (bi - r0)];
+      if (rank == 0 && lane < kb) rj = sp[lane * ld + j];
+      C* slot = slots + (par * P + rank) * kNB + lane;
+      for (int q = 0; q < P; ++q) {
+        if (have && lane < kb) *cl.map_shared_rank(slot, (unsigned)q) = row;
+        if (rank == 0 && lane < kb) *cl.map_shared_rank(&pub_j[par][lane], (unsigned)q) = rj;
       }
+      if (lane < P) {
+        *cl.map_shared_rank(&cand_v[par][rank], (unsigned)lane) = best;
+        *cl.map_shared_rank(&cand_i[par][rank], (unsigned)lane) = bi;
+      }
+    }
+    cluster_arrive();
+    cluster_wait();
+    if (warp == 0) {
+      K v = lane < P ? cand_v[par][lane] : (K)0;
+      int vi = lane < P ? cand_i[par][lane] : INT_MAX;
       warp_argmax(v, vi);
-      const bool zero = !(v > 0);
+      const bool zero = v == 0;
       const int p = zero ? j : vi;  // panel row of the pivot
-      const int owner = p / chunk;
-      C u = czero<C>(), rj = czero<C>();
       if (lane < kb) {
-        rj = cl.map_shared_rank(&pub_j[par][0], 0u)[lane];
-        u = (p == j) ? rj : cl.map_shared_rank(&pub_row[par][0], (unsigned)owner)[lane];
+        const C rj = pub_j[par][lane];
+        const C u = (p == j) ? rj : slots[(par * P + p / chunk) * kNB + lane];
         urow[lane] = u;
         jrow[lane] = rj;
+        if (lane == j) s_inv = zero ? czero<C>() : crecip(u);
       }
-      if (lane == j) s_inv = zero ? czero<C>() : crecip(u);
       if (lane == 0) {
         s_piv = p;
         if (rank == 0) {
@@ -303,32 +354,42 @@ __global__ void __launch_bounds__(kPanelThreads) panel_cluster_kernel(BatchDesc 
     }
     __syncthreads();
     const int p = s_piv;
-    if (p != j) {
-      if (rank == 0 && tid == j)
-        for (int c = 0; c < kb; ++c) sp[c * chunk + j] = urow[c];
-      const int owner = p / chunk, lp = p - owner * chunk;
-      if (rank == owner && tid == lp % kPanelThreads)
-        for (int c = 0; c < kb; ++c) sp[c * chunk + lp] = jrow[c];
-    }
+    const int lp = (p != j && rank == p / chunk) ? p - r0 : -1;  // this CTA's row that takes row j
     const C inv = s_inv;
-    best = -1;
+    for (int i = tid; i < rows; i += kPanelThreads)
+      if (r0 + i > j) sp[j * ld + i] = cmul(i == lp ? jrow[j] : sp[j * ld + i], inv);
+    if (warp == kWarps - 1 && p != j) {  // the interchanged rows' entries that the update leaves alone
+      if (rank == 0 && lane < kb) sp[lane * ld + j] = urow[lane];
+      if (lp >= 0 && lane < j) sp[lane * ld + lp] = jrow[lane];
+    }
+    __syncthreads();
+    best = 0;
     bi = INT_MAX;
-    for (int i = tid; i < rows; i += kPanelThreads) {
-      const int pr = r0 + i;
-      if (pr <= j) continue;
-      const C l = cmul(sp[j * chunk + i], inv);
-      sp[j * chunk + i] = l;
-      for (int c = j + 1; c < kb; ++c) {
-        const C v = cfms(sp[c * chunk + i], l, urow[c]);
-        sp[c * chunk + i] = v;
-        if (c == j + 1) argmax_merge(best, bi, PivotKey<T>::of(fabs(v.x) + fabs(v.y)), pr);
-      }
+    const int items = nrb * ((kb - 1 - j + GC - 1) / GC);
+    for (int q = warp; q < items; q += kWarps) {
+      const int g = q / nrb, i = (q - g * nrb) * 32 + lane;
+      if (i >= rows || r0 + i <= j) continue;
+      const C l = sp[j * ld + i];
+      const int c0 = j + 1 + g * GC;
+      C v[GC];
+#pragma unroll
+      for (int t = 0; t < GC; ++t)
+        if (c0 + t < kb) v[t] = i == lp ? jrow[c0 + t] : sp[(c0 + t) * ld + i];
+#pragma unroll
+      for (int t = 0; t < GC; ++t)
+        if (c0 + t < kb) {
+          v[t] = cfms(v[t], l, urow[c0 + t]);
+          sp[(c0 + t) * ld + i] = v[t];
+        }
+      if (g == 0) argmax_merge(best, bi, PivotKey<T>::of(fabs(v[0].x) + fabs(v[0].y)), r0 + i);
     }
   }
-  // other CTAs may still read this CTA's slots of the last column: wait for them
-  cl.sync();
-  for (int c = 0; c < kb; ++c)
-    for (int i = tid; i < rows; i += kPanelThreads) A[(k + r0 + i) + (k + c) * n] = sp[c * chunk + i];
+  __syncthreads();
+#pragma unroll 4
+  for (int q = warp; q < nrb * kb; q += kWarps) {
+    const int c = q / nrb, i = (q - c * nrb) * 32 + lane;
+    if (i < rows) Ap[i + c * n] = sp[c * ld + i];
+  }
 }
 
 // The interchanges of panel step k as one permutation: final row dst = original row src for
@@ -488,6 +549,45 @@ __global__ void __launch_bounds__(128) trsm_kernel(BatchDesc d, typename cplx_t<
     if (r < kb) A[(k + r) + c * n] = x[r];
 }
 
+// FP64: eight lanes per column, lane r8 holding rows r8, r8 + 8, ..; the column-oriented
+// substitution broadcasts x_q within the eight and every lane updates its rows below q.  One
+// thread per column (trsm_kernel) runs 1984 FP64 FMAs in a row, each a 64-cycle issue of one of
+// the SM's four FP64 pipes, on a few warps in all: 74 us whatever the width; here the same
+// columns spread over eight times the warps with 320 FMAs each: 25 us at up to five matrices
+// of order 1000.
+constexpr int kTrsmCols = 32;  // columns per CTA of 256 threads
+__global__ void __launch_bounds__(8 * kTrsmCols) trsm8_kernel(BatchDesc d, double2* __restrict__ Aall, int64_t k) {
+  __shared__ double2 sL[kNB][kNB + 1];
+  const int64_t n = d.order(blockIdx.y), ncols = n + d.extra;
+  if (k >= n) return;  // this matrix is factored (grouped batches)
+  double2* A = Aall + d.offset(blockIdx.y);
+  const int kb = (int)((k + kNB < n) ? kNB : n - k);
+  if (k + kb >= ncols) return;  // nothing right of the panel
+  for (int idx = threadIdx.x; idx < kNB * kNB; idx += blockDim.x) {
+    const int r = idx & (kNB - 1), q = idx / kNB;
+    sL[r][q] = (r < kb && q < kb) ? A[(k + r) + (k + q) * n] : make_double2(0.0, 0.0);
+  }
+  __syncthreads();
+  const int64_t c = k + kb + blockIdx.x * (int64_t)kTrsmCols + (threadIdx.x >> 3);
+  const bool live = c < ncols;
+  const int r8 = threadIdx.x & 7, base = threadIdx.x & 24;  // first lane of this column's eight
+  double2 x[4];
+#pragma unroll
+  for (int t = 0; t < 4; ++t) x[t] = (live && r8 + 8 * t < kb) ? A[(k + r8 + 8 * t) + c * n] : make_double2(0.0, 0.0);
+#pragma unroll
+  for (int q = 0; q < kNB - 1; ++q) {
+    const double2 xq = shfl_c(x[q >> 3], base | (q & 7));
+#pragma unroll
+    for (int t = q >> 3; t < 4; ++t) {
+      const int r = r8 + 8 * t;
+      if (r > q) x[t] = cfms(x[t], sL[r][q], xq);
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < 4; ++t)
+    if (live && r8 + 8 * t < kb) A[(k + r8 + 8 * t) + c * n] = x[t];
+}
+
 // ------------------------------ trailing update -------------------------------
 // Tile shapes per precision: FP64 is FP64-pipe bound already with 64x64 CTA tiles
 // and 4x4 complex outputs per thread; FP32 needs 8x8 outputs per thread (128x128
@@ -571,17 +671,17 @@ __global__ void __launch_bounds__(256) gemm_kernel(BatchDesc d, typename cplx_t<
 // a small multiple of the unit roundoff times |L21| |U12|), which is the property the LU's
 // backward stability rests on; componentwise the imaginary parts can differ from the
 // four-multiplication product in the last digits.
-constexpr int kG3TM = 64, kG3RM = 4, kG3KC = 16;
-constexpr size_t kG3Smem = 6 * sizeof(double) * kG3KC * (kG3TM + 1);
-
+// Tile: 16 RM x 16 RM outputs per CTA of 256 threads.  The FP64 pipe bounds it at every tile size
+// (98 % busy; an RM = 4 tile keeps an SM for 95 us, RM = 2 24 us, RM = 1 6 us), so the tile only
+// has to be small enough that the launch's tiles fill the SMs evenly: RM = 2 from 8 tiles per
+// SM, RM = 1 below.  Per panel step: order 200 110 -> 12 us, 450 111 -> 21 us, five of 1000
+// 374 -> 300 us.
+constexpr int kG3KC = 16;
+template <int RM>
 __global__ void __launch_bounds__(256) gemm3m_kernel(BatchDesc d, double2* __restrict__ Aall, int64_t k) {
-  extern __shared__ unsigned char gemm_smem[];
-  double (*sAr)[kG3TM + 1] = reinterpret_cast<double (*)[kG3TM + 1]>(gemm_smem);
-  double (*sAi)[kG3TM + 1] = sAr + kG3KC;
-  double (*sAs)[kG3TM + 1] = sAi + kG3KC;
-  double (*sBr)[kG3TM + 1] = sAs + kG3KC;
-  double (*sBi)[kG3TM + 1] = sBr + kG3KC;
-  double (*sBs)[kG3TM + 1] = sBi + kG3KC;
+  constexpr int kG3RM = RM, kG3TM = 16 * RM;
+  __shared__ double sAr[kG3KC][kG3TM + 1], sAi[kG3KC][kG3TM + 1], sAs[kG3KC][kG3TM + 1];
+  __shared__ double sBr[kG3KC][kG3TM + 1], sBi[kG3KC][kG3TM + 1], sBs[kG3KC][kG3TM + 1];
   const int64_t n = d.order(blockIdx.z);
   if (k + kNB >= n) return;  // no trailing block for this matrix (grouped batches)
   double2* A = Aall + d.offset(blockIdx.z);
@@ -1165,31 +1265,24 @@ void convert_with_norms(cudaStream_t st, LaunchCounter lc, const BatchDesc& d, c
 }
 
 
-// CTAs per cluster for a panel of m rows in a batch of `batch` matrices: enough to hold
-// the panel in shared memory, and more (up to 8) while all `batch` clusters still fit on
-// the GPU at once (clusters are placed within one GPC, so this is taken from the
-// occupancy query, not from the SM count), at most `cap` beyond the minimum (the
-// launch-shape table's cluster bound); 0 when the panel does not fit the largest cluster
-// the GPU can schedule (panel_kernel then runs).
+// Clusters of p CTAs of the panel kernel resident on the GPU at once, by p (clusters are placed
+// within one GPC, so this is the occupancy query's answer, not the SM count's); `width` 32 at the
+// largest chunk (a full-width panel fills one SM's shared memory), 16 half of it.
 template <typename T>
-int panel_cluster_size(int64_t m, int64_t batch, int cap_ctas, int width = kNB) {
-  using C = typename cplx_t<T>::type;
-  constexpr int cap = PanelRows<T>::value;
-  struct Table { int resident[17]; };
-  // clusters resident at once at the largest chunk: a full-width panel fills one SM's shared
-  // memory, a half-width one (two-level panels) half of it
+const int* panel_residency(int width) {
+  struct Table { int resident[kPanelMaxCtas + 1]; };
   auto make_table = [](int w) {
     Table t{};
     // the attribute always allows the full-width panel; the query uses this width's size
-    cudaFuncSetAttribute(panel_cluster_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         cap * kNB * (int)sizeof(C));
+    int most = 0;
+    for (int p = 1; p <= kPanelMaxCtas; ++p) most = std::max(most, (int)panel_smem_bytes<T>(panel_rows<T>(p), kNB, p));
+    cudaFuncSetAttribute(panel_cluster_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
     cudaFuncSetAttribute(panel_cluster_kernel<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    const int smem = cap * w * (int)sizeof(C);
-    for (int p = 1; p <= 16; ++p) {
+    for (int p = 1; p <= kPanelMaxCtas; ++p) {
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3((unsigned)p, 1, 1);
       cfg.blockDim = dim3(kPanelThreads, 1, 1);
-      cfg.dynamicSmemBytes = (size_t)smem;
+      cfg.dynamicSmemBytes = panel_smem_bytes<T>(panel_rows<T>(p), w, p);
       cudaLaunchAttribute attr[1];
       attr[0].id = cudaLaunchAttributeClusterDimension;
       attr[0].val.clusterDim.x = (unsigned)p;
@@ -1202,29 +1295,48 @@ int panel_cluster_size(int64_t m, int64_t batch, int cap_ctas, int width = kNB) 
         cudaGetLastError();
         num = 0;
       }
-      t.resident[p] = num;  // clusters of p CTAs resident at once, at the largest chunk
+      t.resident[p] = num;
     }
     return t;
   };
   static const Table tab_full = make_table(kNB);
   static const Table tab_half = make_table(kNB / 2);
+  return width < kNB ? tab_half.resident : tab_full.resident;
+}
+
+// the fewest CTAs whose shared memory holds a panel of m rows (0: no cluster does)
+template <typename T>
+int panel_least_ctas(int64_t m) {
+  for (int p = 1; p <= kPanelMaxCtas; ++p)
+    if (m <= (int64_t)p * panel_rows<T>(p)) return p;
+  return 0;
+}
+
+// CTAs per cluster for a panel of m rows in a batch of `batch` matrices: enough to hold the
+// panel in shared memory, and more while all `batch` clusters still fit on the GPU at once,
+// every CTA has an SM of its own (the panel is FP64-bound per SM) and rows of its own (32 or
+// more), up to `cap_ctas` beyond the minimum (the launch-shape table's cluster bound; its
+// largest value, 8, stands for the largest cluster of 16); 0 when the panel does not fit the
+// largest cluster the GPU can schedule (panel_kernel then runs).
+template <typename T>
+int panel_cluster_size(int64_t m, int64_t batch, int cap_ctas, int width = kNB) {
   static const int sms = [] {
     int dev = 0, v = 152;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
     return v;
   }();
-  const Table& tab = width < kNB ? tab_half : tab_full;
-  int64_t need = (m + cap - 1) / cap;
-  if (need < 1) need = 1;
-  if (need > 16 || tab.resident[need] <= 0) return 0;
-  const int64_t lim = m / kNB > 1 ? m / kNB : 1;  // keeps every chunk >= 32 rows (CTA 0 holds the diagonal block)
-  int64_t p = need;
-  // more CTAs per matrix while all clusters stay resident and every CTA keeps an SM of its own
-  // (the panel is FP64-bound per SM)
-  for (int64_t q = need + 1; q <= 8 && q <= lim && q <= cap_ctas; ++q)
-    if (tab.resident[q] >= batch && q * batch <= sms) p = q;
-  return (int)p;
+  const int* resident = panel_residency<T>(width);
+  const int need = panel_least_ctas<T>(m);
+  if (need == 0 || resident[need] <= 0) return 0;
+  const int most = cap_ctas >= 8 ? kPanelMaxCtas : cap_ctas;
+  int p = need;
+  for (int q = need + 1; q <= most; ++q) {
+    const int chunk = panel_chunk(m, q, panel_rows<T>(q));
+    if ((m + chunk - 1) / chunk != q) continue;  // a CTA would be without rows
+    if (resident[q] >= batch && q * batch <= sms) p = q;
+  }
+  return p;
 }
 
 // true when the full-width panel of m rows runs its clusters for all `batch` matrices at once
@@ -1232,35 +1344,8 @@ int panel_cluster_size(int64_t m, int64_t batch, int cap_ctas, int width = kNB) 
 // does not fit runs in waves, and the FP64 tensor-core path factors it in two halves instead
 template <typename T>
 bool panel_fits_one_wave(int64_t m, int64_t batch) {
-  constexpr int cap = PanelRows<T>::value;
-  const int64_t need = (m + cap - 1) / cap;
-  static int resident[17] = {-1};
-  if (resident[0] < 0) {
-    using C = typename cplx_t<T>::type;
-    cudaFuncSetAttribute(panel_cluster_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap * kNB * (int)sizeof(C));
-    cudaFuncSetAttribute(panel_cluster_kernel<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    for (int p = 1; p <= 16; ++p) {
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3((unsigned)p, 1, 1);
-      cfg.blockDim = dim3(kPanelThreads, 1, 1);
-      cfg.dynamicSmemBytes = (size_t)cap * kNB * sizeof(C);
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = (unsigned)p;
-      attr[0].val.clusterDim.y = 1;
-      attr[0].val.clusterDim.z = 1;
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      int num = 0;
-      if (cudaOccupancyMaxActiveClusters(&num, panel_cluster_kernel<T>, &cfg) != cudaSuccess) {
-        cudaGetLastError();
-        num = 0;
-      }
-      resident[p] = num;
-    }
-    resident[0] = 0;
-  }
-  return need <= 16 && resident[need] >= batch;
+  const int need = panel_least_ctas<T>(m);
+  return need > 0 && panel_residency<T>(kNB)[need] >= batch;
 }
 
 template <typename T>
@@ -1275,17 +1360,15 @@ int lu_factor_batched(cudaStream_t st, LaunchCounter lc, const BatchDesc& d, typ
     constexpr int TM = GemmTile<T>::TM;
     constexpr size_t gsmem = 2 * sizeof(typename cplx_t<T>::type) * GemmTile<T>::KC * (TM + 1);
     cudaFuncSetAttribute(gemm_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gsmem);
-    if (sizeof(T) == 8)
-      cudaFuncSetAttribute(gemm3m_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kG3Smem);
   }
   const int cap_ctas = sizeof(T) == 8 ? lc.tile(n).cluster_f64 : lc.tile(n).cluster_f32;
   // the panel at k0 of `width` columns on a cluster of P CTAs
   auto cluster_panel = [&](int64_t k0, int width, int P) {
-    const int chunk = (int)((n - k0 + P - 1) / P);
+    const int chunk = panel_chunk(n - k0, P, panel_rows<T>(P));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)P, (unsigned)d.batch, 1);
     cfg.blockDim = dim3(kPanelThreads, 1, 1);
-    cfg.dynamicSmemBytes = (size_t)chunk * width * sizeof(typename cplx_t<T>::type);
+    cfg.dynamicSmemBytes = panel_smem_bytes<T>(chunk, width, P);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1345,8 +1428,13 @@ int lu_factor_batched(cudaStream_t st, LaunchCounter lc, const BatchDesc& d, typ
       }
     }
     if (!trsm_done) {
-      dim3 tg((unsigned)((rest_c + 127) / 128), (unsigned)d.batch);
-      MH_LAUNCH(lc, st, sizeof(T) == 8 ? "lu_trsm_f64" : "lu_trsm_f32", trsm_kernel<T><<<tg, 128, 0, st>>>(d, A, k));
+      if constexpr (sizeof(T) == 8) {
+        dim3 tg((unsigned)((rest_c + kTrsmCols - 1) / kTrsmCols), (unsigned)d.batch);
+        MH_LAUNCH(lc, st, "lu_trsm_f64", trsm8_kernel<<<tg, 8 * kTrsmCols, 0, st>>>(d, A, k));
+      } else {
+        dim3 tg((unsigned)((rest_c + 127) / 128), (unsigned)d.batch);
+        MH_LAUNCH(lc, st, "lu_trsm_f32", trsm_kernel<T><<<tg, 128, 0, st>>>(d, A, k));
+      }
     }
     if (rest <= 0) continue;
     if (emu_ws) {
@@ -1358,8 +1446,11 @@ int lu_factor_batched(cudaStream_t st, LaunchCounter lc, const BatchDesc& d, typ
       continue;
     }
     if constexpr (sizeof(T) == 8) {  // FP64: three real products per complex multiply-add
-      dim3 gg((unsigned)((rest + kG3TM - 1) / kG3TM), (unsigned)((rest + kG3TM - 1) / kG3TM), (unsigned)d.batch);
-      MH_LAUNCH(lc, st, "lu_gemm_f64", gemm3m_kernel<<<gg, 256, kG3Smem, st>>>(d, A, k));
+      const int64_t t2 = (rest + 31) / 32, t1 = (rest + 15) / 16;
+      const bool wide = t2 * t2 * d.batch >= 8 * 152;
+      dim3 gg((unsigned)(wide ? t2 : t1), (unsigned)(wide ? t2 : t1), (unsigned)d.batch);
+      if (wide) MH_LAUNCH(lc, st, "lu_gemm_f64", gemm3m_kernel<2><<<gg, 256, 0, st>>>(d, A, k));
+      else MH_LAUNCH(lc, st, "lu_gemm_f64", gemm3m_kernel<1><<<gg, 256, 0, st>>>(d, A, k));
     } else {
       constexpr int TM = GemmTile<T>::TM;
       dim3 gg((unsigned)((rest + TM - 1) / TM), (unsigned)((rest + TM - 1) / TM), (unsigned)d.batch);

@@ -1,0 +1,54 @@
+"""The dense LU at the sizes where its kernels change shape: panels of 1 to 16 CTAs and their
+32-row chunks, ragged last panels, the tile choice of the FP64 update, in every precision."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+EPS = 2.0 ** -53
+
+
+def _solve_ok(mh, ctx, n, rhs, precision, adjoint=False, scale=False):
+    rng = np.random.default_rng(1000 * n + rhs)
+    A = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    if scale:  # rows of very different size, so that the pivot search decides every column
+        A *= 10.0 ** rng.uniform(-6, 6, n)[:, None]
+    b = rng.standard_normal((n, rhs)) + 1j * rng.standard_normal((n, rhs))
+    x = (mh.linsolve_adjoint if adjoint else mh.linsolve)(A, b, precision=precision, ctx=ctx)
+    M = A.conj().T if adjoint else A
+    # normwise backward error of Gaussian elimination with partial pivoting: a modest multiple
+    # of n eps (the growth of random matrices is of order n^(2/3))
+    r = np.abs(b - M @ x).max(axis=0)
+    bound = 20 * n * EPS * (np.abs(M).sum(axis=1).max() * np.abs(x).max(axis=0) + np.abs(b).max(axis=0))
+    assert (r <= bound).all(), (n, precision, (r / bound).max())
+
+
+SIZES = [1, 2, 15, 16, 17, 31, 32, 33, 48, 63, 64, 65, 97, 129, 200, 255, 257, 415, 429, 431, 513, 700, 861]
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed", "fp64_tc"])
+@pytest.mark.parametrize("n", SIZES)
+def test_linsolve_sizes(mh, ctx, n, precision):
+    _solve_ok(mh, ctx, n, 3, precision)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp64_tc"])
+@pytest.mark.parametrize("n", [33, 200, 431])
+def test_linsolve_pivoting(mh, ctx, n, precision):
+    _solve_ok(mh, ctx, n, 2, precision, scale=True)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed", "fp64_tc"])
+@pytest.mark.parametrize("n", [33, 97, 431])
+def test_linsolve_adjoint_sizes(mh, ctx, n, precision):
+    _solve_ok(mh, ctx, n, 2, precision, adjoint=True)
+
+
+@pytest.mark.parametrize("n", [40, 65])
+def test_zero_column_is_reported(mh, ctx, n):
+    rng = np.random.default_rng(n)
+    A = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    A[:, n // 2] = 0.0
+    for precision in ("fp64", "fp64_tc"):
+        with pytest.raises(np.linalg.LinAlgError):
+            mh.linsolve(A, np.ones(n, complex), precision=precision, ctx=ctx)
