@@ -194,7 +194,7 @@ int factor_mixed(mh_context* ctx, const BatchDesc& d, const double2* Adev, float
   const int64_t n = d.n, nn = n * n;
   int32_t *ipiv, *info;
   float2* LU32;
-  MH_TRY(ws_get_t(ctx, kSlotIpiv, (size_t)(n * d.batch), &ipiv));
+  MH_TRY(ws_get_t(ctx, kSlotIpiv, (size_t)(ipiv_stride(n) * d.batch), &ipiv));
   MH_TRY(ws_get_t(ctx, kSlotInfo, (size_t)d.batch, &info));
   MH_TRY(ws_get_t(ctx, kSlotLU32, (size_t)(nn * d.batch), &LU32));
   double* anrm;
@@ -229,7 +229,7 @@ int refine_mixed(mh_context* ctx, const BatchDesc& d, const double2* Adev, const
   const int64_t n = d.n, nn = n * n;
   int32_t* ipiv;
   float2* X32;
-  MH_TRY(ws_get_t(ctx, kSlotIpiv, (size_t)(n * d.batch), &ipiv));
+  MH_TRY(ws_get_t(ctx, kSlotIpiv, (size_t)(ipiv_stride(n) * d.batch), &ipiv));
   MH_TRY(ws_get_t(ctx, kSlotX32, (size_t)(xstride * d.batch), &X32));
   BatchDesc d32 = d;
   d32.stride = nn;
@@ -307,7 +307,7 @@ int solve_core(mh_context* ctx, const BatchDesc& d, double2* Adev, double2* X, i
                int precision, bool adjoint) {
   const int64_t n = d.n;
   int32_t *ipiv, *info;
-  MH_TRY(ws_get_t(ctx, kSlotIpiv, (size_t)(n * d.batch), &ipiv));
+  MH_TRY(ws_get_t(ctx, kSlotIpiv, (size_t)(ipiv_stride(n) * d.batch), &ipiv));
   MH_TRY(ws_get_t(ctx, kSlotInfo, (size_t)d.batch, &info));
   if (precision == MH_PREC_FP64) {
     lu_factor_batched<double>(ctx->stream, ctx->lc(), d, Adev, ipiv, info);
@@ -352,7 +352,7 @@ int solve_core(mh_context* ctx, const BatchDesc& d, double2* Adev, double2* X, i
 int solve_core_appended(mh_context* ctx, const BatchDesc& d, double2* Adev) {
   const int64_t n = d.n;
   int32_t *ipiv, *info;
-  MH_TRY(ws_get_t(ctx, kSlotIpiv, (size_t)(n * d.batch), &ipiv));
+  MH_TRY(ws_get_t(ctx, kSlotIpiv, (size_t)(ipiv_stride(n) * d.batch), &ipiv));
   MH_TRY(ws_get_t(ctx, kSlotInfo, (size_t)d.batch, &info));
   unsigned char* ws;
   const size_t wsb = ozaki_workspace_bytes(n, d.batch, d.extra);

@@ -95,7 +95,7 @@ size_t layout_grouped(BatchCache& c, const BatchOpts& o, char* base) {
     c.X32_all = (float2*)take(xn * 8);
     c.anorm_all = (double*)take(M * 8);
   }
-  c.ipiv_all = (int32_t*)take(M * (size_t)c.n_max * 4);
+  c.ipiv_all = (int32_t*)take(M * (size_t)ipiv_stride(c.n_max) * 4);
   c.info_all = (int32_t*)take(M * 4);
   c.orders = (int64_t*)take(M * 8);
   c.offsets = (int64_t*)take(M * 8);
@@ -130,7 +130,7 @@ BatchDesc grouped_desc(const BatchCache& c, const BatchCache::SizeClass& k, int6
   return d;
 }
 int32_t* grouped_ipiv(const BatchCache& c, const BatchCache::SizeClass& k, int64_t m0) {
-  return c.ipiv_all + k.m_start * c.n_max + (m0 - k.m_start) * k.n_max;
+  return c.ipiv_all + k.m_start * ipiv_stride(c.n_max) + (m0 - k.m_start) * ipiv_stride(k.n_max);
 }
 
 // The body's work before the factorization, enqueued on `st` with no host synchronisation:

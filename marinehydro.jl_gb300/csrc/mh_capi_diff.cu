@@ -76,7 +76,7 @@ int hydro_vjp_core(mh_context* ctx, mh_mesh* m, int64_t n_omega, const double* o
   MH_TRY(ws_get_t(ctx, kSlotF, (size_t)(ni * ncol * n_omega), &F));
   MH_TRY(ws_get_t(ctx, kSlotFK, (size_t)(ni * std::max<int64_t>(nb, 1) * n_omega), &FK));
   MH_TRY(ws_get_t(ctx, kSlotCw, (size_t)(ni * ncol * n_omega), &cw));  // not kSlotNorm: the refinement owns it
-  MH_TRY(ws_get_t(ctx, kSlotIpiv, (size_t)(n * chunk), &ipiv));
+  MH_TRY(ws_get_t(ctx, kSlotIpiv, (size_t)(ipiv_stride(n) * chunk), &ipiv));
   MH_TRY(ws_get_t(ctx, kSlotInfo, (size_t)chunk, &info));
   MH_TRY(ws_get_t(ctx, kSlotGrad, (size_t)((19 + 3 * n_dofs) * n), &grad));
   void* oz_ws = nullptr;  // FP64 LU update on the tensor cores (MH_PREC_FP64_TC)
@@ -354,7 +354,7 @@ int mh_hydro_frequency_derivative(mh_context* ctx, mh_mesh* m, int64_t n_omega, 
   MH_TRY(ws_get_t(ctx, kSlotFK, (size_t)(n_omega * ninf1 * nb1), &FK));
   MH_TRY(ws_get_t(ctx, kSlotGrad, (size_t)(n_omega * ninf1 * nrhs), &dF));
   MH_TRY(ws_get_t(ctx, kSlotWork, zgemm_work_elems(n, nrhs, 1), &work));
-  MH_TRY(ws_get_t(ctx, kSlotIpiv, (size_t)n, &ipiv));
+  MH_TRY(ws_get_t(ctx, kSlotIpiv, (size_t)ipiv_stride(n), &ipiv));
 
   EpilogueGeom eg{n, nh, m->C, m->N, m->A, dofs_d};
   AssemblyParams p = make_params(ctx, m, gfs, direct, 1, nullptr);
@@ -388,7 +388,7 @@ int mh_hydro_frequency_derivative(mh_context* ctx, mh_mesh* m, int64_t n_omega, 
       // phi = D^-1 S b;  dphi = D^-1 (dS b + S db - dD phi)
       times(S, B, X);
       MH_TRY(solve_core(ctx, d, D, X, nrhs, bstride, MH_PREC_FP64, false));
-      MH_TRY(ws_get_t(ctx, kSlotIpiv, (size_t)n, &ipiv));
+      MH_TRY(ws_get_t(ctx, kSlotIpiv, (size_t)ipiv_stride(n), &ipiv));
       times(dS, B, R);
       MH_CUDA(ctx, cudaMemsetAsync(P2, 0, sizeof(double2) * bstride, s0));
       launch_zaxpy(s0, lc, bstride, dk, R, P2);
@@ -402,7 +402,7 @@ int mh_hydro_frequency_derivative(mh_context* ctx, mh_mesh* m, int64_t n_omega, 
       // sigma = D^-1 b, phi = S sigma;  dsigma = D^-1 (db - dD sigma), dphi = dS sigma + S dsigma
       MH_CUDA(ctx, cudaMemcpyAsync(X, B, sizeof(double2) * bstride, cudaMemcpyDeviceToDevice, s0));
       MH_TRY(solve_core(ctx, d, D, X, nrhs, bstride, MH_PREC_FP64, false));
-      MH_TRY(ws_get_t(ctx, kSlotIpiv, (size_t)n, &ipiv));
+      MH_TRY(ws_get_t(ctx, kSlotIpiv, (size_t)ipiv_stride(n), &ipiv));
       MH_CUDA(ctx, cudaMemcpyAsync(R, dB, sizeof(double2) * bstride, cudaMemcpyDeviceToDevice, s0));
       times(dD, X, T);
       launch_zaxpy(s0, lc, bstride, -dk, T, R);
@@ -586,7 +586,7 @@ int mh_solve_pullback(mh_context* ctx, int64_t n, int64_t nrhs, const double* D,
       return solve_core(ctx, d, Ad, rhs, nrhs, (int64_t)nx, precision, true);
     }
     int32_t* ipiv;
-    MH_TRY(ws_get_t(ctx, kSlotIpiv, (size_t)n, &ipiv));
+    MH_TRY(ws_get_t(ctx, kSlotIpiv, (size_t)ipiv_stride(n), &ipiv));
     lu_solve_batched<double>(st, lc, d, Ad, ipiv, rhs, nrhs, (int64_t)nx, true);
     return check_launch(ctx, "adjoint solve");
   };

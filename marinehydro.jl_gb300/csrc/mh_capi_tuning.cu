@@ -122,7 +122,7 @@ int mh_autotune(mh_context* ctx, int precision, int64_t n_sizes, const int64_t* 
     TileChoice base = saved.lookup(n);
     const BatchDesc d{n, batch, nn};
     int32_t *ipiv = nullptr, *info = nullptr;
-    rc = ws_get_t(ctx, kSlotIpiv, (size_t)(n * batch), &ipiv);
+    rc = ws_get_t(ctx, kSlotIpiv, (size_t)(ipiv_stride(n) * batch), &ipiv);
     if (!rc) rc = ws_get_t(ctx, kSlotInfo, (size_t)batch, &info);
     double2* A64 = nullptr;
     float2* A32 = nullptr;

@@ -158,6 +158,9 @@ void launch_exact_points(cudaStream_t st, LaunchCounter lc, int64_t m, const dou
                          double atol, double2* out);
 
 // dense linear algebra (mh_lu.cu)
+// int32 entries per matrix of order n in the pivot array: the pivots (after the factorization
+// the row permutation), then one flag word per 32 x 32 diagonal block (lu_finish_kernel)
+__host__ __device__ inline int64_t ipiv_stride(int64_t n) { return n + (n + 31) / 32; }
 struct BatchDesc {
   int64_t n;        // order (a grouped batch: the largest order)
   int64_t batch;    // number of matrices
@@ -165,7 +168,7 @@ struct BatchDesc {
   // A grouped batch holds matrices of different orders (the many-body batch factors every
   // body's matrices in one launch per panel step): device arrays of each matrix's order,
   // the element offset of the matrix and of its block of right-hand sides.  Null for a
-  // uniform batch.  Pivot indices keep the stride n per matrix either way.
+  // uniform batch.  Pivot indices keep the stride ipiv_stride(n) per matrix either way.
   const int64_t* orders = nullptr;
   const int64_t* offsets = nullptr;
   const int64_t* xoffsets = nullptr;

@@ -26,6 +26,8 @@
 
 #include <algorithm>
 #include <climits>
+#include <cmath>
+#include <initializer_list>
 
 #include "mh_fixpoint.cuh"
 #include "mh_internal.cuh"
@@ -90,7 +92,6 @@ template <> __device__ __forceinline__ float2 crecip<float2>(float2 a) {
   const float rf = __fdividef(1.0f, fmaf(sx, sx, sy * sy)) * f;
   return make_float2(sx * rf, -sy * rf);
 }
-template <typename C> __device__ __forceinline__ C cdiv(C a, C b) { return cmul(a, crecip(b)); }
 template <typename C> __device__ __forceinline__ C czero() { C r; r.x = 0; r.y = 0; return r; }
 
 __device__ __forceinline__ double2 shfl_c(double2 v, int src) {
@@ -113,7 +114,7 @@ __global__ void __launch_bounds__(512) panel_kernel(BatchDesc d, typename cplx_t
   const int64_t n = d.order(blockIdx.x);
   if (k >= n) return;  // a grouped batch: this matrix is factored
   C* A = Aall + d.offset(blockIdx.x);
-  int32_t* ipiv = ipiv_all + blockIdx.x * d.n;
+  int32_t* ipiv = ipiv_all + blockIdx.x * ipiv_stride(d.n);
   const int64_t kend = (k + kNB < n) ? k + kNB : n;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = blockDim.x >> 5;
   for (int64_t j = k; j < kend; ++j) {
@@ -347,7 +348,7 @@ __global__ void __launch_bounds__(kPanelThreads) panel_cluster_kernel(BatchDesc 
       if (lane == 0) {
         s_piv = p;
         if (rank == 0) {
-          ipiv_all[bmat * d.n + k + j] = (int32_t)(k + p);
+          ipiv_all[bmat * ipiv_stride(d.n) + k + j] = (int32_t)(k + p);
           if (zero && info_all[bmat] == 0) info_all[bmat] = (int32_t)(k + j + 1);
         }
       }
@@ -439,7 +440,7 @@ __global__ void __launch_bounds__(256) laswp_kernel(BatchDesc d, typename cplx_t
   const int64_t bmat = blockIdx.y, n = d.order(bmat);
   if (k >= n) return;  // a grouped batch: this matrix is factored
   kb = (int)((k + kNB < n) ? kNB : n - k);
-  if (threadIdx.x < 32) panel_permutation(ipiv_all + bmat * d.n, k, kb, s_slot, s_content, s_dst, s_src);
+  if (threadIdx.x < 32) panel_permutation(ipiv_all + bmat * ipiv_stride(d.n), k, kb, s_slot, s_content, s_dst, s_src);
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int d0 = s_dst[lane], s0 = s_src[lane], d1 = s_dst[lane + 32], s1 = s_src[lane + 32];
@@ -468,7 +469,7 @@ __global__ void __launch_bounds__(256) laswp_cols_kernel(BatchDesc d, typename c
   __shared__ int s_slot[32], s_content[64], s_dst[64], s_src[64];
   const int64_t bmat = blockIdx.y, n = d.order(bmat);
   if (k + kb > n) return;
-  if (threadIdx.x < 32) panel_permutation(ipiv_all + bmat * d.n, k, kb, s_slot, s_content, s_dst, s_src);
+  if (threadIdx.x < 32) panel_permutation(ipiv_all + bmat * ipiv_stride(d.n), k, kb, s_slot, s_content, s_dst, s_src);
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int d0 = s_dst[lane], s0 = s_src[lane], d1 = s_dst[lane + 32], s1 = s_src[lane + 32];
@@ -756,366 +757,416 @@ __global__ void __launch_bounds__(256) gemm3m_kernel(BatchDesc d, double2* __res
 }
 
 // ------------------------------ substitution ---------------------------------
-// x_r[i] -= sum_{j in [jb, je)} M[i, j] x_r[j] for the g right-hand sides of the
-// group (M = the stored factor, or its conjugate transpose when CT); every matrix
-// element is loaded once and applied to up to kSG vectors held in registers.
-constexpr int kSG = 8;
-
-
-// Diagonal 32x32 block solves done by one warp: the block sits in shared memory
-// (blk, 32 x 33 padded, blk[l*33+q] = M[jb+l, jb+q] as stored), lane l owns
-// entry jb+l of the solution, and solved entries travel by shuffle.
-// KIND 0: unit lower L; 1: upper U; 2: lower U^H; 3: unit upper L^H.
-template <typename C>
-__device__ __forceinline__ void load_diag_block(const C* __restrict__ LU, int64_t n, int64_t jb, int bw, C* blk) {
-  for (int idx = threadIdx.x; idx < bw * bw; idx += blockDim.x) {
-    int r = idx % bw, q = idx / bw;
-    blk[r * 33 + q] = LU[(jb + r) + (jb + q) * n];
-  }
+// After the last panel step lu_finish_kernel turns the factors into what the substitutions read:
+// the 32 x 32 diagonal blocks of L and U are replaced by their inverses (each in its own
+// triangle, L's unit diagonal implied) and the pivot sequence by the row permutation it
+// composes to (x = b[sigma] applies the interchanges).  Block substitution with inverted
+// diagonal blocks turns the 64-step dependent chain of each block into a product (Higham,
+// Accuracy and Stability of Numerical Algorithms, 2nd ed., sec. 14.2; 14.3 for its error), and
+// both are done once per factorization, whatever the number of solves.
+// The product's residual exceeds the substitution's by up to k = | |T| |T^-1| |_inf of the block,
+// so in FP64 a triangle with k above 512 stays as it is and is solved by substitution (its bit
+// in the block's flag word: 1 for L, 2 for U).  Second-kind boundary operators have k of 1 to 20,
+// random matrices 100 to 300, a Hilbert-like matrix millions.  FP32 factors are refined.
+// |x| to FP32 precision from the bits (a conversion instruction would run on the FP64 pipe): 0
+// below FP32's normal range, a NaN pattern above it
+__device__ __forceinline__ float magnitude_f32(double x) {
+  const unsigned hi = (unsigned)(__double_as_longlong(x) >> 32) & 0x7FFFFFFFu;
+  const int e = (int)(hi >> 20) - 896;  // biased exponent in FP32
+  return e <= 0 ? 0.0f : (e >= 255 ? __uint_as_float(0x7FFFFFFFu) : __uint_as_float((unsigned)e << 23 | (hi & 0xFFFFFu) << 3));
 }
-
-template <typename C, int KIND>
-__device__ __forceinline__ void diag_block_solve(const C* blk, int64_t n, int64_t jb, int bw, C* xs, int g,
-                                                 int lane) {
-  for (int r = 0; r < g; ++r) {
-    C* x = xs + (int64_t)r * n;
-    C xl = lane < bw ? x[jb + lane] : czero<C>();
-    if (KIND == 0 || KIND == 2) {
-#pragma unroll 4
-      for (int q = 0; q < bw; ++q) {
-        C m = (KIND == 0) ? blk[lane * 33 + q] : cconj(blk[q * 33 + lane]);
-        if (KIND == 2 && lane == q) xl = cdiv(xl, m);
-        C xq = shfl_c(xl, q);
-        if (lane > q && lane < bw) xl = cfms(xl, m, xq);
-      }
-    } else {
-#pragma unroll 4
-      for (int q = bw - 1; q >= 0; --q) {
-        C m = (KIND == 1) ? blk[lane * 33 + q] : cconj(blk[q * 33 + lane]);
-        if (KIND == 1 && lane == q) xl = cdiv(xl, m);
-        C xq = shfl_c(xl, q);
-        if (lane < q) xl = cfms(xl, m, xq);
-      }
-    }
-    if (lane < bw) x[jb + lane] = xl;
-  }
-}
-
-template <typename C, bool CT>
-__device__ __forceinline__ void update_row(const C* __restrict__ LU, int64_t n, int64_t i, int64_t jb, int64_t je,
-                                           C* xs, int g) {
-  for (int r0 = 0; r0 < g; r0 += kSG) {
-    C acc[kSG];
-#pragma unroll
-    for (int r = 0; r < kSG; ++r) acc[r] = czero<C>();
-    const int gr = (g - r0 < kSG) ? g - r0 : kSG;
-    if (je - jb == 32) {
-#pragma unroll 8
-      for (int jj = 0; jj < 32; ++jj) {
-        const int64_t j = jb + jj;
-        C m = CT ? cconj(LU[j + i * n]) : LU[i + j * n];
-#pragma unroll
-        for (int r = 0; r < kSG; ++r)
-          if (r < gr) acc[r] = cfma(acc[r], m, xs[(r0 + r) * n + j]);
-      }
-    } else {
-      for (int64_t j = jb; j < je; ++j) {
-        C m = CT ? cconj(LU[j + i * n]) : LU[i + j * n];
-#pragma unroll
-        for (int r = 0; r < kSG; ++r)
-          if (r < gr) acc[r] = cfma(acc[r], m, xs[(r0 + r) * n + j]);
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < kSG; ++r)
-      if (r < gr) xs[(r0 + r) * n + i] = csub(xs[(r0 + r) * n + i], acc[r]);
-  }
-}
-
-// One CTA per (group of right-hand sides, matrix); the group's vectors live in
-// shared memory.  Forward: unit lower L; backward: upper U; both in 32-column
-// blocks (warp 0 solves the diagonal block, all threads update the rest).
-// ADJ: solves A^H x = b = U^H L^H P^T x.
-template <typename T, bool ADJ>
-__global__ void __launch_bounds__(512) solve_kernel(BatchDesc d, const typename cplx_t<T>::type* __restrict__ LUall,
-                                                    const int32_t* __restrict__ ipiv_all,
-                                                    typename cplx_t<T>::type* __restrict__ Xall, int64_t nrhs,
-                                                    int64_t xstride, int group, int upper_only) {
+__device__ __forceinline__ float magnitude_f32(float x) { return fabsf(x); }
+constexpr int kFinishThreads = 256;
+constexpr int kFinishMaxSmem = 2 * 4 * 12288;  // the permutation of the largest order the library takes
+constexpr float kFinishGrowth = 512.0f;
+template <typename T>
+__global__ void __launch_bounds__(kFinishThreads) lu_finish_kernel(BatchDesc d, typename cplx_t<T>::type* __restrict__ Aall,
+                                                                  int32_t* __restrict__ ipiv_all, int nblk) {
   using C = typename cplx_t<T>::type;
-  extern __shared__ unsigned char smem_raw[];
-  C* blk = reinterpret_cast<C*>(smem_raw);
-  C* xs = blk + 32 * 33;
+  __shared__ C sM[kNB][kNB + 1], sX[kNB][kNB + 1];
+  __shared__ C rd[kNB];
+  __shared__ float ssum[2][kNB];
+  extern __shared__ int finish_smem[];
   const int64_t n = d.order(blockIdx.y);
-  const C* LU = LUall + d.offset(blockIdx.y);
-  const int32_t* ipiv = ipiv_all + blockIdx.y * d.n;
-  C* X = Xall + d.xoffset(blockIdx.y, xstride);
-  const int64_t r0 = blockIdx.x * (int64_t)group;
-  const int g = (int)((r0 + group <= nrhs) ? group : nrhs - r0);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int64_t idx = tid; idx < g * n; idx += blockDim.x) {
-    int64_t r = idx / n, i = idx % n;
-    xs[r * n + i] = X[i + (r0 + r) * n];
+  int32_t* ipiv = ipiv_all + blockIdx.y * ipiv_stride(d.n);
+  const int tid = threadIdx.x;
+  const bool upper_only = d.extra > 0;  // the right-hand sides went through the factorization: only U is solved
+  if ((int)blockIdx.x == nblk) {
+    if (upper_only) return;
+    // the permutation: sequential in the pivots, one thread, from shared memory
+    int* sig = finish_smem;
+    int* piv = finish_smem + d.n;
+    for (int64_t i = tid; i < n; i += kFinishThreads) { sig[i] = (int)i; piv[i] = ipiv[i]; }
+    __syncthreads();
+    if (tid == 0) {
+      int next = piv[0];
+      for (int j = 0; j < (int)n; ++j) {
+        const int q = next;
+        next = j + 1 < (int)n ? piv[j + 1] : 0;  // off the exchange's chain
+        const int a = sig[j], b = sig[q];
+        sig[j] = b;
+        sig[q] = a;
+      }
+    }
+    __syncthreads();
+    for (int64_t i = tid; i < n; i += kFinishThreads) ipiv[i] = sig[i];
+    return;
+  }
+  const int64_t jb = (int64_t)blockIdx.x * kNB;
+  if (jb >= n) return;
+  const int bw = (int)(n - jb < kNB ? n - jb : kNB);
+  C* A = Aall + d.offset(blockIdx.y) + jb + jb * n;
+  // the block and the identity: L X = I runs on the strict lower triangles of sM and sX, U X = I
+  // on the upper ones, at the same time (their steps touch different entries)
+  for (int e = tid; e < kNB * kNB; e += kFinishThreads) {
+    const int r = e & (kNB - 1), c = e / kNB;
+    sM[r][c] = (r < bw && c < bw) ? A[r + c * n] : czero<C>();
+    C x = czero<C>();
+    if (r == c) x.x = 1;
+    sX[r][c] = x;
   }
   __syncthreads();
-  if (!ADJ) {
-    if (tid < g && !upper_only) {  // apply the row interchanges in order (zgetrs / zlaswp)
-      C* x = xs + tid * n;
-      for (int64_t j = 0; j < n; ++j) {
-        int64_t p = ipiv[j];
-        if (p != j) { C t = x[j]; x[j] = x[p]; x[p] = t; }
-      }
-    }
-    __syncthreads();
-    // L y = b
-    for (int64_t jb = 0; jb < (upper_only ? 0 : n); jb += 32) {
-      const int64_t je = (jb + 32 < n) ? jb + 32 : n;
-      load_diag_block(LU, n, jb, (int)(je - jb), blk);
-      __syncthreads();
-      if (warp == 0) diag_block_solve<C, 0>(blk, n, jb, (int)(je - jb), xs, g, lane);
-      __syncthreads();
-      for (int64_t i = je + tid; i < n; i += blockDim.x) update_row<C, false>(LU, n, i, jb, je, xs, g);
-      __syncthreads();
-    }
-    // U x = y
-    const int64_t nblk = (n + 31) / 32;
-    for (int64_t bI = nblk - 1; bI >= 0; --bI) {
-      const int64_t jb = bI * 32, je = (jb + 32 < n) ? jb + 32 : n;
-      load_diag_block(LU, n, jb, (int)(je - jb), blk);
-      __syncthreads();
-      if (warp == 0) diag_block_solve<C, 1>(blk, n, jb, (int)(je - jb), xs, g, lane);
-      __syncthreads();
-      for (int64_t i = tid; i < jb; i += blockDim.x) update_row<C, false>(LU, n, i, jb, je, xs, g);
-      __syncthreads();
-    }
-  } else {
-    // U^H w = b (lower triangular, conj(U) transposed)
-    for (int64_t jb = 0; jb < n; jb += 32) {
-      const int64_t je = (jb + 32 < n) ? jb + 32 : n;
-      load_diag_block(LU, n, jb, (int)(je - jb), blk);
-      __syncthreads();
-      if (warp == 0) diag_block_solve<C, 2>(blk, n, jb, (int)(je - jb), xs, g, lane);
-      __syncthreads();
-      for (int64_t i = je + tid; i < n; i += blockDim.x) update_row<C, true>(LU, n, i, jb, je, xs, g);
-      __syncthreads();
-    }
-    // L^H v = w (upper, unit diagonal)
-    const int64_t nblk = (n + 31) / 32;
-    for (int64_t bI = nblk - 1; bI >= 0; --bI) {
-      const int64_t jb = bI * 32, je = (jb + 32 < n) ? jb + 32 : n;
-      load_diag_block(LU, n, jb, (int)(je - jb), blk);
-      __syncthreads();
-      if (warp == 0) diag_block_solve<C, 3>(blk, n, jb, (int)(je - jb), xs, g, lane);
-      __syncthreads();
-      for (int64_t i = tid; i < jb; i += blockDim.x) update_row<C, true>(LU, n, i, jb, je, xs, g);
-      __syncthreads();
-    }
-    if (tid < g) {  // x = P v: undo the interchanges in reverse order
-      C* x = xs + tid * n;
-      for (int64_t j = n - 1; j >= 0; --j) {
-        int64_t p = ipiv[j];
-        if (p != j) { C t = x[j]; x[j] = x[p]; x[p] = t; }
+  if (tid < bw) {
+    rd[tid] = crecip(sM[tid][tid]);
+    sX[tid][tid] = rd[tid];  // the diagonal of U^-1 (L^-1's is 1)
+  }
+  __syncthreads();
+  for (int s = 0; s < bw - 1; ++s) {
+    // L: column oriented, once row s of X is final rows q > s take -L[q][s] X[s][c], c <= s
+    // U: from the bottom, once row t of X is final rows q < t take -U[q][t] X[t][c], c >= t, and row
+    // t - 1 is then scaled by 1 / U[t-1][t-1]
+    const int t = bw - 1 - s, w = s + 1, ne = (bw - 1 - s) * w;
+    for (int e = tid + (upper_only ? ne : 0); e < 2 * ne; e += kFinishThreads) {
+      if (e < ne) {
+        const int q = s + 1 + e / w, c = e % w;
+        C x = c == s ? czero<C>() : sX[s][c];
+        if (c == s) x.x = 1;
+        sX[q][c] = cfms(sX[q][c], sM[q][s], x);
+      } else {
+        const int q = (e - ne) / w, c = t + (e - ne) % w;
+        const C v = cfms(sX[q][c], sM[q][t], sX[t][c]);
+        sX[q][c] = q == t - 1 ? cmul(v, rd[q]) : v;
       }
     }
     __syncthreads();
   }
-  for (int64_t idx = tid; idx < g * n; idx += blockDim.x) {
-    int64_t r = idx / n, i = idx % n;
-    X[i + (r0 + r) * n] = xs[r * n + i];
+  bool keep_l = false, keep_u = false;
+  if (sizeof(T) == 8) {
+    // k of both triangles, in FP32: row sums of |X|, then |T| times them
+    const int r = tid & (kNB - 1), part = tid >> 5;
+    auto mag = [](C v) { return magnitude_f32(v.x) + magnitude_f32(v.y); };
+    if (part < 2) {
+      float sum = 0.0f;
+      for (int c = 0; c < bw; ++c) {
+        if (part == 0) sum += c < r ? mag(sX[r][c]) : (c == r ? 1.0f : 0.0f);
+        else if (c >= r) sum += mag(sX[r][c]);
+      }
+      ssum[part][r] = sum;
+    }
+    __syncthreads();
+    float k = 0.0f;
+    if (part < 2 && r < bw)
+      for (int c = 0; c < bw; ++c) {
+        if (part == 0) k += c < r ? mag(sM[r][c]) * ssum[0][c] : (c == r ? ssum[0][c] : 0.0f);
+        else if (c >= r) k += mag(sM[r][c]) * ssum[1][c];
+      }
+    const bool big = !(k <= kFinishGrowth);  // also for NaN
+    keep_l = __syncthreads_or(part == 0 && big);
+    keep_u = __syncthreads_or(part == 1 && big);
+  }
+  if (tid == 0) ipiv[d.n + blockIdx.x] = (keep_l ? 1 : 0) | (keep_u ? 2 : 0);
+  for (int e = tid; e < kNB * kNB; e += kFinishThreads) {
+    const int r = e & (kNB - 1), c = e / kNB;
+    if (r < bw && c < bw && !(r > c ? keep_l || upper_only : keep_u)) A[r + c * n] = sX[r][c];
   }
 }
 
-// ---------------------------- solve on a cluster --------------------------------
-// One cluster of P CTAs per (group of g <= kSG right-hand sides, matrix).  The 32-row
-// blocks of the solution are dealt out cyclically (block b to CTA b % P), each CTA keeps
-// its blocks' entries of the g vectors in shared memory.  The solve is a sequence of
-// 2 nblk block steps (L then U, or U^H then L^H).  At step s the owner of block s has
-// already solved it and posted its entries in a double-buffered slot; every CTA copies
-// the slot through distributed shared memory and subtracts the block's contribution from
-// its own rows.  The owner of block s + 1 first updates that block's rows, solves it (one
-// warp per vector, reciprocals of the diagonal precomputed), posts it and arrives at the
-// split cluster barrier, and only then updates the rest of its rows; every other CTA
-// arrives as soon as it has its copy.  So the barrier waits only for the next block, not
-// for the whole update.  The permutation of the right-hand sides (the LU's row
-// interchanges) is composed once per CTA into an index map: x = b[sigma] before L
-// (forward), x[sigma] = v after L^H (adjoint).
+// One cluster of P CTAs per (group of g <= kSG right-hand sides, matrix).  The 32-row blocks of
+// the solution are dealt out cyclically (block b to CTA b % P); each CTA keeps its blocks'
+// entries of the g vectors in shared memory.  The solve is a sequence of 2 nblk block steps (L
+// then U, or U^H then L^H for A^H x = b = U^H L^H P^T x).  At step s every CTA has x_s, the
+// block solved last, in a slot of its own.  The owner of block s + 1 takes x_s into that block's
+// rows, multiplies by the inverted diagonal block and pushes the result into the slots of all
+// P CTAs (four warps, one per FP64 pipe; both 32 x 32 operands were brought into shared
+// memory a step ahead); all arrive at the split cluster barrier, take x_s into the rest of
+// their rows, and wait.  Three slots: a CTA may still read x_(s-1) while x_(s+1) arrives.
+//
+// Bound: the chain of 2 nblk steps (two 32 x 32 products by g vectors on one SM, 2300 g cycles
+// each in FP64, and a barrier), or for many right-hand sides the FP64 pipes of the SMs in use;
+// solve_shape trades the two; in FP32 the latency of a step's loads, which prefetch_rows brings
+// into L2 a step ahead.  With the diagonal blocks solved by substitution and always eight
+// vectors on up to 8 CTAs -> now, on a GB300: FP64 order 200, 2 vectors 215 -> 65 us; five of
+// 1000, 7 vectors 1.78 -> 0.52 ms; 2999, 9 vectors 10.9 -> 1.7 ms; FP32 four of 8000, 4 vectors
+// 11.0 -> 2.3 ms.  lu_finish_kernel adds 45 us at order 200, 70 us at 2999.
+constexpr int kSG = 8;
+constexpr int kSolveThreads = 512;
+constexpr int kSolveMaxCtas = 16;
+constexpr int kSolveMaxSmem = 220 * 1024;
+constexpr int kBlkLd = kNB + 1;
 
-// kind of block step s (KIND of diag_block_solve) and its block index
+// kind of block step s and its block index.  KIND 0: unit lower L; 1: upper U; 2: lower U^H; 3:
+// unit upper L^H.
 template <bool ADJ> __device__ __forceinline__ void solve_step(int s, int nblk, int& kind, int& bI) {
   if (s < nblk) { kind = ADJ ? 2 : 0; bI = s; }
   else { kind = ADJ ? 3 : 1; bI = 2 * nblk - 1 - s; }
 }
-
-// one warp solves the block entries x[0 .. bw) of one vector in place; rd: reciprocals of
-// the diagonal (KIND 1, 2)
-template <typename C, int KIND>
-__device__ __forceinline__ void block_solve_slot(const C* blk, const C* rd, int bw, C* x, int lane) {
-  C xl = lane < bw ? x[lane] : czero<C>();
-  if (KIND == 0 || KIND == 2) {
-#pragma unroll 4
-    for (int q = 0; q < bw; ++q) {
-      C m = (KIND == 0) ? blk[lane * 33 + q] : cconj(blk[q * 33 + lane]);
-      if (KIND == 2 && lane == q) xl = cmul(xl, rd[q]);
-      C xq = shfl_c(xl, q);
-      if (lane > q && lane < bw) xl = cfms(xl, m, xq);
-    }
-  } else {
-#pragma unroll 4
-    for (int q = bw - 1; q >= 0; --q) {
-      C m = (KIND == 1) ? blk[lane * 33 + q] : cconj(blk[q * 33 + lane]);
-      if (KIND == 1 && lane == q) xl = cmul(xl, rd[q]);
-      C xq = shfl_c(xl, q);
-      if (lane < q) xl = cfms(xl, m, xq);
-    }
-  }
-  if (lane < bw) x[lane] = xl;
-}
-
-constexpr int kXbStride = 33;  // padded: the g vectors of one row read different banks
 
 // rows of block b2 take the contribution of block bI at this step?
 __device__ __forceinline__ bool step_updates(int kind, int bI, int b2) {
   return (kind == 0 || kind == 2) ? (b2 > bI) : (b2 < bI);
 }
 
-// x_i -= sum_jj M(i, jb + jj) xb[q][jj] for the local rows li in [l0, l1) that step (kind,
-// bI) updates, skipping local block `skip`; work item = (row, vector) so that one block's
-// 32 rows still spread over the CTA
+// entry (i, j) of the triangular factor of this kind, off its diagonal blocks
 template <typename C>
-__device__ __forceinline__ void cluster_update_rows(const C* __restrict__ LU, int64_t n, int kind, int bI, int bw,
-                                                    int P, int rank, int g, int ln, C* xl, const C* xb, int l0, int l1,
-                                                    int skip) {
-  const bool ct = (kind >= 2);
-  const int64_t jb = (int64_t)bI * 32;
-  const int rows = l1 - l0;
-  for (int w = threadIdx.x; w < rows * g; w += blockDim.x) {
-    const int li = l0 + w / g, q = w % g;  // the g vectors of a row on neighbouring threads
-    const int lb = li >> 5;
-    if (lb == skip) continue;
-    const int b2 = rank + lb * P;
-    if (!step_updates(kind, bI, b2)) continue;
-    const int64_t i = (int64_t)b2 * 32 + (li & 31);
-    if (i >= n) continue;
-    C acc = czero<C>();
-    const C* xq = xb + q * kXbStride;
-    if (ct) {
-      const C* col = LU + i * n + jb;  // M(i, j) = conj(LU[j, i]): row i of LU^H is column i of LU
-#pragma unroll 8
-      for (int jj = 0; jj < bw; ++jj) acc = cfma(acc, cconj(col[jj]), xq[jj]);
-    } else {
-      const C* row = LU + i + jb * n;
-#pragma unroll 8
-      for (int jj = 0; jj < bw; ++jj) acc = cfma(acc, row[(int64_t)jj * n], xq[jj]);
-    }
-    xl[(int64_t)q * ln + li] = csub(xl[(int64_t)q * ln + li], acc);
-  }
+__device__ __forceinline__ C factor_entry(const C* __restrict__ LU, int64_t n, int kind, int64_t i, int64_t j) {
+  return kind >= 2 ? cconj(__ldg(LU + j + i * n)) : __ldg(LU + i + j * n);
 }
 
-template <typename C, bool ADJ>
-__device__ __forceinline__ void cluster_solve_block(const C* __restrict__ LU, int64_t n, int kind, int bI, int P,
-                                                    int g, int ln, C* xl, C* blk, C* rd, C* post) {
+// entry (r, c) of what stands in diagonal block jb (bw x bw) of this kind: the inverse, or the
+// block itself where it was left
+template <typename C>
+__device__ __forceinline__ C inverse_entry(const C* __restrict__ LU, int64_t n, int kind, int64_t jb, int bw, int r,
+                                           int c) {
+  C v = czero<C>();
+  if (r >= bw || c >= bw) return v;
+  const bool unit = kind == 0 || kind == 3, low = kind == 0 || kind == 2;
+  if (unit && r == c) { v.x = 1; return v; }
+  if (low ? c > r : c < r) return v;
+  return factor_entry(LU, n, kind, jb + r, jb + c);
+}
+
+// sum over the lanes that share a row of an RW-row group (lanes RW apart)
+template <int RW, typename C> __device__ __forceinline__ C row_sum(C v) {
+#pragma unroll
+  for (int off = 16; off >= RW; off >>= 1) {
+    v.x += __shfl_xor_sync(0xffffffffu, v.x, off);
+    v.y += __shfl_xor_sync(0xffffffffu, v.y, off);
+  }
+  return v;
+}
+
+// x_i -= M(i, block bI) x_s for the local rows that step (kind, bI) updates, skipping local block
+// `skip`: a warp takes RW rows, its 32 / RW lanes per row every (32 / RW)-th column
+template <int RW, typename C>
+__device__ __forceinline__ void solve_update_rows(const C* __restrict__ LU, int64_t n, int kind, int bI, int P, int rank,
+                                                  int g, int ln, C* xl, const C* xs, int nloc, int skip) {
+  constexpr int CG = 32 / RW, NC = 32 / CG;  // lanes per row, columns per lane
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t jb = (int64_t)bI * 32;
   const int bw = (int)((jb + 32 < n) ? 32 : n - jb);
-  load_diag_block(LU, n, jb, bw, blk);
-  __syncthreads();
-  if (warp == 0 && lane < bw) {
-    const C dgl = blk[lane * 33 + lane];
-    rd[lane] = crecip(kind == 2 ? cconj(dgl) : dgl);
-  }
-  __syncthreads();
-  if (warp < g) {
-    C* x = xl + (int64_t)warp * ln + (bI / P) * 32;
-    switch (kind) {
-      case 0: block_solve_slot<C, 0>(blk, rd, bw, x, lane); break;
-      case 1: block_solve_slot<C, 1>(blk, rd, bw, x, lane); break;
-      case 2: block_solve_slot<C, 2>(blk, rd, bw, x, lane); break;
-      default: block_solve_slot<C, 3>(blk, rd, bw, x, lane); break;
+  const int cg = lane / RW;
+  for (int li0 = warp * RW; li0 < nloc; li0 += (kSolveThreads / 32) * RW) {
+    const int lb = li0 >> 5, b2 = rank + lb * P;
+    if (lb == skip || !step_updates(kind, bI, b2)) continue;
+    const int li = li0 + (lane & (RW - 1));
+    const int64_t i = (int64_t)b2 * 32 + (li & 31);
+    C mrow[NC];
+#pragma unroll
+    for (int t = 0; t < NC; ++t) {
+      const int c = cg + CG * t;
+      mrow[t] = (i < n && c < bw) ? factor_entry(LU, n, kind, i, jb + c) : czero<C>();
     }
-    __syncwarp();
-    post[warp * 32 + lane] = lane < bw ? x[lane] : czero<C>();
+    for (int q = 0; q < g; ++q) {
+      C acc = czero<C>();
+#pragma unroll
+      for (int t = 0; t < NC; ++t) acc = cfma(acc, mrow[t], xs[q * kBlkLd + cg + CG * t]);
+      acc = row_sum<RW>(acc);
+      if (cg == 0) xl[(int64_t)q * ln + li] = csub(xl[(int64_t)q * ln + li], acc);
+    }
   }
 }
 
+// this CTA's rows of the factor's block column bI (the operand of the update of its step) into L2:
+// a step's loads are short of one another's latency, so they should not wait for HBM
+template <typename C>
+__device__ __forceinline__ void prefetch_rows(const C* __restrict__ LU, int64_t n, int kind, int bI, int P, int rank,
+                                              int nlb) {
+  constexpr int lines = 32 * (int)sizeof(C) / 128;  // 128-byte lines of 32 entries
+  const int64_t jb = (int64_t)bI * 32;
+  for (int e = threadIdx.x; e < nlb * 32 * lines; e += kSolveThreads) {
+    const int part = e % lines, c = (e / lines) & 31, b2 = rank + e / (32 * lines) * P;
+    if (!step_updates(kind, bI, b2)) continue;
+    const int64_t i = (int64_t)b2 * 32;
+    // the line's entries run along the rows (L, U) or along the columns (their adjoints)
+    const int64_t off = part * (128 / (int)sizeof(C));
+    const int64_t row = kind >= 2 ? jb + off : i + off, col = kind >= 2 ? i + c : jb + c;
+    if (row < n && col < n) asm volatile("prefetch.global.L2 [%0];" ::"l"(LU + row + col * n));
+  }
+}
+
+// out[r] = sum_c blk[r][c] x[c] for row r = 8 warp + (lane & 7) of a 32 x 32 block, on every lane
+// of the row (warps 0 to 3)
+template <typename C>
+__device__ __forceinline__ C block_times(const C* blk, const C* x) {
+  const int lane = threadIdx.x & 31, r = (threadIdx.x >> 5) * 8 + (lane & 7), cg = lane >> 3;
+  C a0 = czero<C>(), a1 = czero<C>();
+#pragma unroll
+  for (int t = 0; t < 8; t += 2) {
+    a0 = cfma(a0, blk[r * kBlkLd + cg + 4 * t], x[cg + 4 * t]);
+    a1 = cfma(a1, blk[r * kBlkLd + cg + 4 * t + 4], x[cg + 4 * t + 4]);
+  }
+  return row_sum<8>(cadd(a0, a1));
+}
+
+template <typename T> constexpr size_t solve_smem_bytes(int group, int ln) {
+  return 2 * sizeof(T) * ((size_t)group * ln + 4 * kNB * kBlkLd + 4 * (size_t)group * kBlkLd);
+}
+
 template <typename T, bool ADJ>
-__global__ void __launch_bounds__(512) solve_cluster_kernel(BatchDesc d, const typename cplx_t<T>::type* __restrict__ LUall,
-                                                            const int32_t* __restrict__ ipiv_all,
-                                                            typename cplx_t<T>::type* __restrict__ Xall, int64_t nrhs,
-                                                            int64_t xstride, int group, int ln, int upper_only) {
+__global__ void __launch_bounds__(kSolveThreads, 2) solve_cluster_kernel(BatchDesc d, const typename cplx_t<T>::type* __restrict__ LUall,
+                                                                     const int32_t* __restrict__ sigma_all,
+                                                                     typename cplx_t<T>::type* __restrict__ Xall,
+                                                                     int64_t nrhs, int64_t xstride, int group, int ln,
+                                                                     int upper_only) {
   using C = typename cplx_t<T>::type;
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   extern __shared__ __align__(16) unsigned char solve_smem[];
-  C* xl = reinterpret_cast<C*>(solve_smem);                          // g x ln, vector-major
-  int* sig = reinterpret_cast<int*>(xl + (int64_t)group * ln);       // n
-  int* spv = sig + d.n;                                              // n: the pivots
-  __shared__ C blk[32 * 33];
-  __shared__ C rd[32];
-  __shared__ C pub[2][32 * kSG];
-  __shared__ C xb[2][kXbStride * kSG];
+  __shared__ int kept[2];                        // flag words of the staged diagonal blocks
+  C* xl = reinterpret_cast<C*>(solve_smem);      // group x ln, vector-major
+  C* blk = xl + (int64_t)group * ln;             // [2][M(next, current), inverse(next)] 32 x kBlkLd
+  C* slots = blk + 4 * kNB * kBlkLd;             // [3] group x kBlkLd: solved blocks
+  C* rb = slots + 3 * group * kBlkLd;            // group x kBlkLd: the next block's right-hand sides
   const int P = (int)cl.num_blocks(), rank = (int)cl.block_rank();
   const int64_t n = d.order(blockIdx.z);
   const int nblk = (int)((n + 31) / 32);
   const C* LU = LUall + d.offset(blockIdx.z);
-  const int32_t* ipiv = ipiv_all + blockIdx.z * d.n;
+  const int32_t* sig = sigma_all + blockIdx.z * ipiv_stride(d.n);
+  const int32_t* flags = sig + d.n;
   C* X = Xall + d.xoffset(blockIdx.z, xstride);
   const int64_t r0 = blockIdx.y * (int64_t)group;
   const int g = (int)((r0 + group <= nrhs) ? group : nrhs - r0);
-  const int tid = threadIdx.x;
-  // sigma: the row interchanges composed in order (x = b[sigma] applies them to b); the
-  // identity when the right-hand sides went through the factorization (upper_only)
-  for (int64_t i = tid; i < n; i += blockDim.x) { sig[i] = (int)i; spv[i] = upper_only ? (int)i : ipiv[i]; }
-  __syncthreads();
-  if (tid == 0 && !upper_only)
-    for (int64_t j = 0; j < n; ++j) {
-      const int p = spv[j];
-      if (p != j) { const int t = sig[j]; sig[j] = sig[p]; sig[p] = t; }
-    }
-  __syncthreads();
-  const int nlb = (nblk - rank + P - 1) / P;
-  const int nloc = nlb * 32;
-  for (int w = tid; w < nloc * g; w += blockDim.x) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nlb = (nblk - rank + P - 1) / P;  // blocks of this CTA (may be 0)
+  const int nloc = nlb > 0 ? nlb * 32 : 0;
+  for (int w = tid; w < nloc * g; w += kSolveThreads) {
     const int li = w % nloc, q = w / nloc;
     const int64_t i = (int64_t)(rank + (li >> 5) * P) * 32 + (li & 31);
-    if (i < n) xl[(int64_t)q * ln + li] = X[(ADJ ? i : sig[i]) + (r0 + q) * n];
+    C v = czero<C>();
+    if (i < n) v = X[((ADJ || upper_only) ? i : (int64_t)sig[i]) + (r0 + q) * n];
+    xl[(int64_t)q * ln + li] = v;
   }
-  __syncthreads();
   const int nsteps = 2 * nblk;
   const int s0 = upper_only ? nblk : 0;  // upper_only: the U steps alone
-  int kind, bI;
-  solve_step<ADJ>(s0, nblk, kind, bI);
-  if (bI % P == rank) cluster_solve_block<C, ADJ>(LU, n, kind, bI, P, g, ln, xl, blk, rd, pub[s0 & 1]);
+  constexpr int kPer = kNB * kNB / kSolveThreads;  // entries of a block per thread
+  // the operands of step s into registers / from registers into buffer s & 1
+  auto fetch = [&](int s, C (&va)[kPer], C (&vi)[kPer]) {
+    int kind, bI, pkind, pI;
+    solve_step<ADJ>(s, nblk, kind, bI);
+    if (tid == 0) kept[s & 1] = flags[bI];
+    solve_step<ADJ>(s - 1, nblk, pkind, pI);
+    const int64_t jb = (int64_t)bI * 32, jp = (int64_t)pI * 32;
+    const int bw = (int)((jb + 32 < n) ? 32 : n - jb), pw = (int)((jp + 32 < n) ? 32 : n - jp);
+    const bool upd = s > s0 && step_updates(pkind, pI, bI);
+#pragma unroll
+    for (int e = 0; e < kPer; ++e) {
+      // consecutive threads along the memory-contiguous direction of this kind
+      const int x = (tid + e * kSolveThreads) & 31, y = (tid + e * kSolveThreads) >> 5;
+      const int r = kind >= 2 ? y : x, c = kind >= 2 ? x : y;
+      va[e] = (upd && r < bw && c < pw) ? factor_entry(LU, n, pkind, jb + r, jp + c) : czero<C>();
+      vi[e] = inverse_entry(LU, n, kind, jb, bw, r, c);
+    }
+  };
+  auto stash = [&](int s, const C (&va)[kPer], const C (&vi)[kPer]) {
+    int kind, bI;
+    solve_step<ADJ>(s, nblk, kind, bI);
+    C* b = blk + (s & 1) * 2 * kNB * kBlkLd;
+#pragma unroll
+    for (int e = 0; e < kPer; ++e) {
+      const int x = (tid + e * kSolveThreads) & 31, y = (tid + e * kSolveThreads) >> 5;
+      const int r = kind >= 2 ? y : x, c = kind >= 2 ? x : y;
+      b[r * kBlkLd + c] = va[e];
+      b[kNB * kBlkLd + r * kBlkLd + c] = vi[e];
+    }
+  };
+  auto owner = [&](int s) {
+    int kind, bI;
+    solve_step<ADJ>(s, nblk, kind, bI);
+    return bI % P;
+  };
+  // warps 0 to 3 of the owner of step s: x_s = inverse (b_s - M x_(s-1)), pushed to every CTA
+  auto solve_block = [&](int s) {
+    int kind, bI;
+    solve_step<ADJ>(s, nblk, kind, bI);
+    const C* b = blk + (s & 1) * 2 * kNB * kBlkLd;
+    const C* xp = slots + ((s + 2) % 3) * group * kBlkLd;  // x_(s-1)
+    const int r = warp * 8 + (lane & 7), cgi = lane >> 3;
+    C* xb = xl + (bI / P) * 32 + r;
+    for (int q = 0; q < g; ++q) {
+      C v = xb[(int64_t)q * ln];
+      if (s > s0) v = csub(v, block_times(b, xp + q * kBlkLd));
+      if (cgi == 0) rb[q * kBlkLd + r] = v;
+    }
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+    if (kept[s & 1] & ((kind == 0 || kind == 3) ? 1 : 2)) {
+      // this block was left as it is: substitution, one warp per vector, then the push
+      const C* m = b + kNB * kBlkLd;
+      const bool low = kind == 0 || kind == 2;
+      for (int q = warp; q < g; q += 4) {
+        const int bw = (int)((int64_t)bI * 32 + 32 < n ? 32 : n - (int64_t)bI * 32);
+        C x = rb[q * kBlkLd + lane];
+        C rdl = czero<C>();
+        if (lane < bw) rdl = crecip(m[lane * kBlkLd + lane]);
+        for (int e = 0; e < bw; ++e) {
+          const int c = low ? e : bw - 1 - e;
+          if (lane == c) x = cmul(x, rdl);
+          const C xc = shfl_c(x, c);
+          if (low ? lane > c : lane < c) x = cfms(x, m[lane * kBlkLd + c], xc);
+        }
+        if (lane >= bw) x = czero<C>();
+        xl[(int64_t)q * ln + (bI / P) * 32 + lane] = x;
+        C* slot = slots + (s % 3) * group * kBlkLd + q * kBlkLd + lane;
+        for (int t = 0; t < P; ++t) *cl.map_shared_rank(slot, (unsigned)t) = x;
+      }
+      return;
+    }
+    for (int q = 0; q < g; ++q) {
+      const C v = block_times(b + kNB * kBlkLd, rb + q * kBlkLd);
+      if (cgi == 0) xb[(int64_t)q * ln] = v;
+      C* slot = slots + (s % 3) * group * kBlkLd + q * kBlkLd + r;
+      for (int t = cgi; t < P; t += 4) *cl.map_shared_rank(slot, (unsigned)t) = v;
+    }
+  };
+  C va[kPer], vi[kPer];
+  cluster_arrive();  // every CTA of the cluster runs before the first push
+  for (int s = s0; s < s0 + 2 && s < nsteps; ++s)
+    if (owner(s) == rank) {
+      fetch(s, va, vi);
+      stash(s, va, vi);
+    }
+  cluster_wait();
+  __syncthreads();
+  if (owner(s0) == rank && warp < 4) solve_block(s0);
   cluster_arrive();
   cluster_wait();
   for (int s = s0; s < nsteps; ++s) {
+    int kind, bI, skip = -1;
     solve_step<ADJ>(s, nblk, kind, bI);
-    const int bw = (int)(((int64_t)bI * 32 + 32 < n) ? 32 : n - (int64_t)bI * 32);
-    C* xs = xb[s & 1];
-    const C* src = cl.map_shared_rank(&pub[s & 1][0], (unsigned)(bI % P));
-    for (int e = tid; e < 32 * g; e += blockDim.x) xs[(e >> 5) * kXbStride + (e & 31)] = src[e];
-    __syncthreads();
-    const bool last = (s + 1 == nsteps);
-    int nkind = 0, nbI = 0, skip = -1;
-    if (!last) {
+    const bool last = s + 1 == nsteps;
+    if (!last && owner(s + 1) == rank) {
+      int nkind, nbI;
       solve_step<ADJ>(s + 1, nblk, nkind, nbI);
-      if (nbI % P == rank) {
-        // the next block first: its rows, its solve, its slot
-        const int lb = nbI / P;
-        if (step_updates(kind, bI, nbI))
-          cluster_update_rows<C>(LU, n, kind, bI, bw, P, rank, g, ln, xl, xs, lb * 32, lb * 32 + 32, -1);
-        __syncthreads();
-        cluster_solve_block<C, ADJ>(LU, n, nkind, nbI, P, g, ln, xl, blk, rd, pub[(s + 1) & 1]);
-        skip = lb;
-      }
+      skip = nbI / P;
+      if (warp < 4) solve_block(s + 1);
     }
-    cluster_arrive();  // step s + 1 posted (or nothing to post)
-    cluster_update_rows<C>(LU, n, kind, bI, bw, P, rank, g, ln, xl, xs, 0, nloc, skip);
-    cluster_wait();
+    if (!last) cluster_arrive();  // x_(s+1) pushed
+    const bool ahead = s + 2 < nsteps && owner(s + 2) == rank;
+    if (ahead) fetch(s + 2, va, vi);
+    if (!last) {
+      int nkind, nbI;
+      solve_step<ADJ>(s + 1, nblk, nkind, nbI);
+      prefetch_rows<C>(LU, n, nkind, nbI, P, rank, nlb);
+    }
+    const C* xs = slots + (s % 3) * group * kBlkLd;
+    solve_update_rows<8, C>(LU, n, kind, bI, P, rank, g, ln, xl, xs, nloc, skip);
+    if (ahead) stash(s + 2, va, vi);
+    __syncthreads();
+    if (!last) cluster_wait();
   }
-  __syncthreads();
-  for (int w = tid; w < nloc * g; w += blockDim.x) {
+  for (int w = tid; w < nloc * g; w += kSolveThreads) {
     const int li = w % nloc, q = w / nloc;
     const int64_t i = (int64_t)(rank + (li >> 5) * P) * 32 + (li & 31);
-    if (i < n) X[(ADJ ? sig[i] : i) + (r0 + q) * n] = xl[(int64_t)q * ln + li];
+    if (i < n) X[(ADJ ? (int64_t)sig[i] : i) + (r0 + q) * n] = xl[(int64_t)q * ln + li];
   }
 }
 
@@ -1458,103 +1509,111 @@ int lu_factor_batched(cudaStream_t st, LaunchCounter lc, const BatchDesc& d, typ
       MH_LAUNCH(lc, st, "lu_gemm_f32", gemm_kernel<T><<<gg, 256, gsmem, st>>>(d, A, k));
     }
   }
+  const int nblk = (int)((n + kNB - 1) / kNB);
+  const size_t fsmem = 2 * sizeof(int) * (size_t)n;
+  cudaFuncSetAttribute(lu_finish_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFinishMaxSmem);
+  MH_LAUNCH(lc, st, sizeof(T) == 8 ? "lu_finish_f64" : "lu_finish_f32",
+            lu_finish_kernel<T><<<dim3((unsigned)(nblk + 1), (unsigned)d.batch), kFinishThreads, fsmem, st>>>(
+                d, A, ipiv, nblk));
   return 0;
 }
 
-// Cluster size for the solve: the fewest CTAs whose shares of the vectors fit in shared
-// memory, raised (up to 8) while every (matrix, group) cluster is still resident at once.
-// Returns false when even 8 CTAs cannot hold the vectors (the one-CTA kernel then runs).
+// The solve's shape: CTAs per cluster and right-hand sides per cluster, by an estimate of its
+// time in SM cycles.  A step's chain is two 32 x 32 products by the g vectors on one SM (2300 g
+// cycles each on the FP64 pipes; latency in FP32) and a cluster barrier; its bulk the update of
+// half the rows, by the cluster's SMs.  More CTAs shorten the bulk, fewer vectors per cluster
+// both, as long as the clusters stay resident and have SMs of their own.
+struct SolveShape { int P, g; };
 template <typename T>
-bool solve_on_cluster(cudaStream_t st, LaunchCounter lc, const BatchDesc& d, const typename cplx_t<T>::type* LU,
-                      const int32_t* ipiv, typename cplx_t<T>::type* X, int64_t nrhs, int64_t xstride, bool adjoint,
-                      bool upper_only) {
-  using C = typename cplx_t<T>::type;
-  const int64_t n = d.n;
-  const int g = (int)(nrhs < kSG ? nrhs : kSG);
-  const int64_t ngroups = (nrhs + g - 1) / g;
-  const int64_t nblk = (n + 31) / 32;
-  const size_t max_dyn = 190 * 1024;
-  auto dyn_bytes = [&](int p) {
-    const int64_t ln = (nblk + p - 1) / p * 32;
-    return (size_t)ln * g * sizeof(C) + 2 * sizeof(int) * (size_t)n;
-  };
-  const void* fn = adjoint ? (const void*)solve_cluster_kernel<T, true> : (const void*)solve_cluster_kernel<T, false>;
-  static const bool attr_set = [] {
-    cudaFuncSetAttribute(solve_cluster_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 190 * 1024);
-    cudaFuncSetAttribute(solve_cluster_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 190 * 1024);
-    return true;
+SolveShape solve_shape(int64_t n, int64_t nrhs, int64_t batch, bool upper_only) {
+  struct Table { int one[kSolveMaxCtas + 1]; };
+  // clusters of P CTAs resident at once with one CTA per SM; also sets the kernels' attributes
+  static const Table tab = [] {
+    Table t{};
+    for (const void* fn : {(const void*)solve_cluster_kernel<T, false>, (const void*)solve_cluster_kernel<T, true>}) {
+      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolveMaxSmem);
+      cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    }
+    for (int p = 1; p <= kSolveMaxCtas; ++p) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3((unsigned)p, 1, 1);
+      cfg.blockDim = dim3(kSolveThreads, 1, 1);
+      cfg.dynamicSmemBytes = kSolveMaxSmem;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = (unsigned)p;
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      int num = 0;
+      if (cudaOccupancyMaxActiveClusters(&num, solve_cluster_kernel<T, false>, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        num = 0;
+      }
+      t.one[p] = num;
+    }
+    return t;
   }();
-  (void)attr_set;
-  auto make_cfg = [&](int p, cudaLaunchAttribute* attr) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)p, (unsigned)ngroups, (unsigned)d.batch);
-    cfg.blockDim = dim3(512, 1, 1);
-    cfg.dynamicSmemBytes = dyn_bytes(p);
-    cfg.stream = st;
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)p;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cfg;
-  };
-  int need = 0;
-  for (int p = 1; p <= 8 && p <= nblk; ++p)
-    if (dyn_bytes(p) <= max_dyn) { need = p; break; }
-  if (need == 0) return false;
-  int P = need;
-  const int64_t clusters = ngroups * d.batch;
-  for (int p = need + 1; p <= 8 && p <= nblk; ++p) {
-    cudaLaunchAttribute attr[1];
-    cudaLaunchConfig_t cfg = make_cfg(p, attr);
-    int num = 0;
-    if (cudaOccupancyMaxActiveClusters(&num, fn, &cfg) != cudaSuccess) { cudaGetLastError(); break; }
-    if (num >= clusters) P = p;
+  const int64_t nblk = (n + 31) / 32;
+  const double steps = (double)(upper_only ? nblk : 2 * nblk);
+  SolveShape best{0, 0};
+  double best_t = 0.0;
+  for (int p = 1; p <= kSolveMaxCtas && p <= nblk; ++p) {
+    const int ln = (int)((nblk + p - 1) / p * 32);
+    for (int g = 1; g <= kSG && g <= nrhs; ++g) {
+      const size_t smem = solve_smem_bytes<T>(g, ln);
+      if (smem > kSolveMaxSmem || tab.one[p] <= 0) continue;
+      const double clusters = (double)((nrhs + g - 1) / g * batch);
+      // a second CTA fits an SM when the shared memory does, and shares its pipes
+      const int per_sm = smem <= 110 * 1024 ? 2 : 1;
+      const double waves = std::ceil(clusters / ((double)tab.one[p] * per_sm));
+      const double share = std::min(std::ceil(clusters / (double)tab.one[p]), (double)per_sm);
+      const double rows = 0.5 * (double)n / p;
+      double chain, bulk;
+      if (sizeof(T) == 8) {
+        chain = (4600.0 * g + 1000.0) * share;
+        bulk = (rows * 32 * g * 2.4 + 4600.0 * g / p + 1000.0) * share;
+      } else {
+        chain = 1500.0 + 200.0 * g;
+        bulk = 1500.0 + rows * 32 * (0.2 + 0.08 * g) * share;
+      }
+      const double sync = p == 1 ? 0.0 : 800.0 + 50.0 * p;
+      const double t = waves * steps * (std::max(chain, bulk) + sync);
+      if (best.P == 0 || t < best_t) {
+        best = SolveShape{p, g};
+        best_t = t;
+      }
+    }
   }
-  cudaLaunchAttribute attr[1];
-  cudaLaunchConfig_t cfg = make_cfg(P, attr);
-  const int ln = (int)((nblk + P - 1) / P * 32);
-  lc.pre(st);
-  if (adjoint) cudaLaunchKernelEx(&cfg, solve_cluster_kernel<T, true>, d, LU, ipiv, X, nrhs, xstride, g, ln, 0);
-  else cudaLaunchKernelEx(&cfg, solve_cluster_kernel<T, false>, d, LU, ipiv, X, nrhs, xstride, g, ln, (int)upper_only);
-  lc.post(st, sizeof(T) == 8 ? "lu_solve_f64" : "lu_solve_f32");
-  return true;
+  return best;
 }
 
 template <typename T>
 void lu_solve_batched(cudaStream_t st, LaunchCounter lc, const BatchDesc& d, const typename cplx_t<T>::type* LU,
                       const int32_t* ipiv, typename cplx_t<T>::type* X, int64_t nrhs, int64_t xstride,
                       bool adjoint, bool upper_only) {
-  using C = typename cplx_t<T>::type;
   const int64_t n = d.n;
   if (n <= 0 || nrhs <= 0 || d.batch <= 0) return;
   upper_only = upper_only && !adjoint;
-  if (solve_on_cluster<T>(st, lc, d, LU, ipiv, X, nrhs, xstride, adjoint, upper_only)) return;
-  const size_t max_smem = 200 * 1024;
-  const size_t blk_bytes = sizeof(C) * 32 * 33;
-  int64_t group = (int64_t)((max_smem - blk_bytes) / (sizeof(C) * n));
-  // Enough CTAs to occupy every SM twice: each CTA streams the factor once for
-  // its group of right-hand sides, so fewer RHS per CTA trades factor re-reads
-  // (from L2 / HBM) for parallelism.
-  int dev = 0, sms = 152;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int64_t want_ctas = 2 * (int64_t)sms;
-  const int64_t g_par = (nrhs * d.batch + want_ctas - 1) / want_ctas;
-  if (group > g_par) group = g_par;
-  if (group < 1) group = 1;
-  if (group > nrhs) group = nrhs;
-  const size_t smem = blk_bytes + sizeof(C) * n * group;
-  dim3 grid((unsigned)((nrhs + group - 1) / group), (unsigned)d.batch);
+  const SolveShape sh = solve_shape<T>(n, nrhs, d.batch, upper_only);
+  const int64_t nblk = (n + 31) / 32;
+  const int ln = (int)((nblk + sh.P - 1) / sh.P * 32);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)sh.P, (unsigned)((nrhs + sh.g - 1) / sh.g), (unsigned)d.batch);
+  cfg.blockDim = dim3(kSolveThreads, 1, 1);
+  cfg.dynamicSmemBytes = solve_smem_bytes<T>(sh.g, ln);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)sh.P;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
   lc.pre(st);
-  if (adjoint) {
-    cudaFuncSetAttribute(solve_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem);
-    solve_kernel<T, true><<<grid, 512, smem, st>>>(d, LU, ipiv, X, nrhs, xstride, (int)group, 0);
-  } else {
-    cudaFuncSetAttribute(solve_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem);
-    solve_kernel<T, false><<<grid, 512, smem, st>>>(d, LU, ipiv, X, nrhs, xstride, (int)group, (int)upper_only);
-  }
+  if (adjoint) cudaLaunchKernelEx(&cfg, solve_cluster_kernel<T, true>, d, LU, ipiv, X, nrhs, xstride, sh.g, ln, 0);
+  else cudaLaunchKernelEx(&cfg, solve_cluster_kernel<T, false>, d, LU, ipiv, X, nrhs, xstride, sh.g, ln, (int)upper_only);
   lc.post(st, sizeof(T) == 8 ? "lu_solve_f64" : "lu_solve_f32");
 }
 

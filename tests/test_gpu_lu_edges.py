@@ -52,3 +52,26 @@ def test_zero_column_is_reported(mh, ctx, n):
     for precision in ("fp64", "fp64_tc"):
         with pytest.raises(np.linalg.LinAlgError):
             mh.linsolve(A, np.ones(n, complex), precision=precision, ctx=ctx)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed", "fp64_tc"])
+@pytest.mark.parametrize("n, rhs", [(33, 1), (64, 9), (200, 2), (300, 17), (545, 8), (1000, 33), (1537, 5), (2999, 3)])
+def test_substitution_shapes(mh, ctx, n, rhs, precision):
+    # cluster sizes 1 to 16 and groups of 1 to 8 right-hand sides, whole and ragged
+    _solve_ok(mh, ctx, n, rhs, precision)
+    _solve_ok(mh, ctx, n, rhs, precision, adjoint=True)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp64_tc"])
+@pytest.mark.parametrize("decades", [4, 8, 11])
+def test_ill_conditioned_backward_error(mh, ctx, precision, decades):
+    # singular values spread over `decades`: the inverted diagonal blocks keep the residual at
+    # the size elimination itself leaves
+    n = 320
+    rng = np.random.default_rng(decades)
+    q = [np.linalg.qr(rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n)))[0] for _ in range(2)]
+    A = (q[0] * np.logspace(0, -decades, n)) @ q[1]
+    b = rng.standard_normal((n, 2)) + 1j * rng.standard_normal((n, 2))
+    x = mh.linsolve(A, b, precision=precision, ctx=ctx)
+    r = np.abs(b - A @ x).max(axis=0)
+    assert (r <= 20 * n * EPS * np.abs(A).sum(axis=1).max() * np.abs(x).max(axis=0)).all()
