@@ -19,7 +19,8 @@ mpmath at 40 digits):
   inverting the two relations.  Worst absolute error of P, Q/s: 3e-17.
 * FP32 tables: the same construction at degree 6 (half-unit intervals) and 6 (Hankel), for
   errors below FP32 rounding.
-* exp and log on the integer pipe (namespace fxq): 2^(j/32) and the degree-7 series of
+* exp, log and atan on the integer pipe (namespace fxq; atan by degree-9 Chebyshev interpolants
+  on the 32 intervals of [0, 1)): 2^(j/32) and the degree-7 series of
   2^(g/32) for exp, degree-10 Chebyshev interpolants of log on the 32 intervals of [1, 2)
   for log, all as integers c 2^62; the integer evaluation is emulated bit for bit below.
 * Fixed-point tables (namespace besq) of the same FP64 polynomials for the integer-pipe
@@ -180,6 +181,7 @@ def fx_bessel_errors(fq):
 
 # ---- exp and log on the integer pipe (mh_fixpoint.cuh) ------------------------------------
 EXP_DEG = 7   # 2^(g/32), g in [0, 1)
+ATAN_DEG = 9   # atan(j/32 + u/32), u in [0, 1), per interval j = 0..31
 LOG_DEG = 10  # log(1 + j/32 + u/32), u in [0, 1), per interval j = 0..31
 
 
@@ -206,6 +208,30 @@ def fx_log_tables():
         rows += [q_int(c, 62) for c in cu]
     ln2 = int(mp.nint(mp.log(2) * mp.mpf(2) ** 64))
     return rows, ln2
+
+
+def fx_atan_table():
+    rows = []
+    for j in range(32):
+        c = cheb_monomials(lambda u, j=j: mp.atan((j + u) / mp.mpf(32)), mp.mpf(0), mp.mpf(1), ATAN_DEG)
+        # from powers of u - 1/2 to powers of u
+        p = [mp.mpf(0)] * (ATAN_DEG + 1)
+        for i, v in enumerate(c):
+            for k in range(i + 1):
+                p[k] += v * mp.binomial(i, k) * mp.mpf(-0.5) ** (i - k)
+        rows += [q_int(v, 62) for v in p]
+    return rows
+
+
+def emu_atan(x, rows):
+    """The device's atan of a double x in [0, 1): U = x 2^64, interval U >> 59."""
+    U = int(mp.floor(mp.mpf(x) * 2 ** 64))
+    j, G = U >> 59, (U << 5) & (2 ** 64 - 1)
+    r = rows[j * (ATAN_DEG + 1):(j + 1) * (ATAN_DEG + 1)]
+    v = r[-1]
+    for c in reversed(r[:-1]):
+        v = c + mulhi_su(v, G)
+    return mp.mpf(v) / 2 ** 62
 
 
 def mulhi_su(v, t):
@@ -406,6 +432,10 @@ def main():
     worst_l = max(abs(emu_log(w, ltab, ln2) - mp.log(w)) for w in ws)
     print("fixed-point exp: worst relative error", mp.nstr(worst_e, 3), "; log: worst absolute error", mp.nstr(worst_l, 3))
     assert worst_e < 5e-17 and worst_l < 4e-17
+    atab = fx_atan_table()
+    worst_a = max(abs(emu_atan(x, atab) - mp.atan(x)) for x in [rng.random() for _ in range(600)] + [0.0, 0.5, 1 - 2.0 ** -53])
+    print("fixed-point atan: worst absolute error", mp.nstr(worst_a, 3))
+    assert worst_a < 2e-17
     tabf, _, wlf, whf = bessel_tables(DEG_LOW_F, DEG_HANKEL_F, True)
     print("FP32 Bessel: worst abs error low region", mp.nstr(wlf, 3), "Hankel P, Q/s", mp.nstr(whf, 3))
     tabe, we = egd_tables()
@@ -466,6 +496,9 @@ def main():
         fh.write(f"constexpr int kLogTerms = {LOG_DEG + 1};\n")
         fh.write(f"__device__ const long long kLogTab[32 * kLogTerms] = {{\n    {fmt_int(ltab)}}};\n")
         fh.write(f"constexpr unsigned long long kLn2Q64 = {ln2}ULL;\n\n")
+        fh.write("// atan on the integer pipe: atan(j/32 + u/32) = sum_k c_k u^k on u in [0, 1), c_k 2^62, row\n// j = 0..31\n")
+        fh.write(f"constexpr int kAtanTerms = {ATAN_DEG + 1};\n")
+        fh.write(f"__device__ const long long kAtanTab[32 * kAtanTerms] = {{\n    {fmt_int(atab)}}};\n\n")
         fh.write("}  // namespace fxq\n\n")
         fh.write("namespace egdq {\n\n")
         fh.write(f"constexpr int kFrac = {EGD_QF};  // integers v 2^-kFrac\n")

@@ -125,9 +125,120 @@ __device__ __forceinline__ double identity_jump(const AssemblyParams& p, const d
   return 0.5;
 }
 
-// Static (Rankine-family) part.  BIRK: assemble_birk_rankine (matrix_assembly.jl:274-331);
-// otherwise the broadcasting sum over the static tuple (matrix_assembly.jl:70-88).
-template <bool DIRECT, bool BIRK>
+// entry idx of a real n x n array held with `step` doubles per entry: 1 (a real array) or 2 (the
+// real parts of a complex one, whose imaginary parts are then 0)
+__device__ __forceinline__ void store_static(double* __restrict__ M, int64_t idx, int step, double v) {
+  if (step == 2) reinterpret_cast<double2*>(M)[idx] = make_double2(v, 0.0);
+  else M[idx] = v;
+}
+
+// Birk Rankine part: assemble_birk_rankine (matrix_assembly.jl:274-331).  A pair's two terms
+// (direct and image) are the point-source form beyond 7 panel radii, ~12 FP64 instructions
+// each with the reciprocal root on the integer pipe, and the 4-edge Birk integral nearer, ~200.
+// A warp's 32 rows nearly always hold a near pair somewhere, so the CTA takes its tile (128 rows
+// by `cols` columns) in two passes: the far terms, thread by thread into a tile in shared
+// memory, listing the near ones; then the listed ones, densely.  Bound: the FP64 pipe; few
+// columns per CTA where the mesh is small (launch_assemble_static).  Measured on a GB300, one
+// launch, before (both forms in one divergent pass, all on the FP64 pipe) and now: 200 panels
+// 460 -> 34 us, 2000 panels 1.5 -> 0.33 ms, 8000 panels 10.0 -> 3.4 ms.
+template <bool DIRECT>
+__global__ void __launch_bounds__(kRowsPerCta) static_birk_kernel(AssemblyParams p, double* __restrict__ SR,
+                                                                  double* __restrict__ DR, int step, int cols) {
+  __shared__ PanelRec sp[kColsPerCta];
+  __shared__ double near2[kColsPerCta][2];       // (7 radius)^2 less / more four roundings
+  __shared__ double tS[2][kColsPerCta][kRowsPerCta], tD[2][kColsPerCta][kRowsPerCta];  // [direct, image]
+  __shared__ unsigned short todo[2 * kColsPerCta * kRowsPerCta];  // image << 10 | column << 7 | row
+  __shared__ int count;
+  const int64_t n = p.n;
+  const int64_t i0 = blockIdx.x * (int64_t)kRowsPerCta, i = i0 + threadIdx.x;
+  const int64_t j0 = blockIdx.y * (int64_t)cols;
+  const int jmax = (int)((n - j0) < cols ? (n - j0) : cols);
+  {
+    const double2* src = reinterpret_cast<const double2*>(p.P + j0);
+    double2* dst = reinterpret_cast<double2*>(sp);
+    for (int q = threadIdx.x; q < jmax * 16; q += kRowsPerCta) dst[q] = __ldg(src + q);
+  }
+  if (threadIdx.x == 0) count = 0;
+  __syncthreads();
+  if (threadIdx.x < jmax) {
+    const double t = 7 * sp[threadIdx.x].radius, t2 = t * t;
+    near2[threadIdx.x][0] = t2 * (1.0 - 0x1p-50);
+    near2[threadIdx.x][1] = t2 * (1.0 + 0x1p-50);
+  }
+  __syncthreads();
+  const bool need_R = (p.gfs & MH_GF_RANKINE) != 0;
+  const bool need_I = (p.gfs & MH_GF_RANKINE_REFLECTED) != 0;
+  const bool need_N = (p.gfs & MH_GF_RANKINE_REFLECTED_NEGATIVE) != 0;
+  const bool row_ok = i < n;
+  double ci[3] = {0, 0, 0}, ni[3] = {0, 0, 1};
+  if (row_ok)
+    for (int c = 0; c < 3; ++c) { ci[c] = __ldg(&p.P[i].c[c]); ni[c] = __ldg(&p.P[i].n[c]); }
+  if (row_ok) {
+    for (int jj = 0; jj < jmax; ++jj) {
+      const PanelRec& Pj = sp[jj];
+      double nv[3];
+      pick_normal<DIRECT>(p, Pj, ni, nv);
+      const double dx = ci[0] - Pj.c[0], dy = ci[1] - Pj.c[1];
+      const double h2 = dx * dx + dy * dy, nh = nv[0] * dx + nv[1] * dy;
+#pragma unroll
+      for (int image = 0; image < 2; ++image) {
+        double s = 0.0, d = 0.0;
+        if (image ? (need_I || need_N) : need_R) {
+          const double dz = image ? -ci[2] - Pj.c[2] : ci[2] - Pj.c[2];
+          const double r2 = h2 + dz * dz;
+          // r > 7 radius (rankine_vectorized.jl:273-287); the root itself only where rounding decides
+          bool far = r2 > near2[jj][1];
+          if (!far && r2 >= near2[jj][0]) far = sqrt(r2) > 7 * Pj.radius;
+          if (far) {
+            const double ir = fx::rsqrt_pos(r2);
+            s = Pj.area * ir;
+            const double q = s * ir * ir;
+            // gradient in the source; indirect: in the field point, reflected back for the image
+            if (DIRECT) d = q * (nh + nv[2] * dz);
+            else d = image ? q * (nv[2] * dz - nh) : -q * (nh + nv[2] * dz);
+          } else {
+            todo[atomicAdd(&count, 1)] = (unsigned short)(image << 10 | jj << 7 | (int)threadIdx.x);
+          }
+        }
+        tS[image][jj][threadIdx.x] = s;
+        tD[image][jj][threadIdx.x] = d;
+      }
+    }
+  }
+  __syncthreads();
+  for (int q = threadIdx.x; q < count; q += kRowsPerCta) {
+    const int e = todo[q], image = e >> 10, jj = (e >> 7) & 7, row = e & 127;
+    const PanelRec& Pi = p.P[i0 + row];
+    const PanelRec& Pj = sp[jj];
+    const double pt[3] = {__ldg(&Pi.c[0]), __ldg(&Pi.c[1]), image ? -__ldg(&Pi.c[2]) : __ldg(&Pi.c[2])};
+    const double nr[3] = {__ldg(&Pi.n[0]), __ldg(&Pi.n[1]), __ldg(&Pi.n[2])};
+    double nv[3], phi, g[3];
+    pick_normal<DIRECT>(p, Pj, nr, nv);
+    vrankine_near(pt, Pj, phi, g);
+    if (!DIRECT) {
+      g[0] = -g[0];
+      g[1] = -g[1];
+      if (!image) g[2] = -g[2];  // vertical_reflection(-g) keeps the image's
+    }
+    tS[image][jj][row] = phi;
+    tD[image][jj][row] = nv[0] * g[0] + nv[1] * g[1] + nv[2] * g[2];
+  }
+  __syncthreads();
+  if (!row_ok) return;
+  const double image_sign = (need_I ? 1.0 : 0.0) + (need_N ? -1.0 : 0.0);
+  for (int jj = 0; jj < jmax; ++jj) {
+    const int64_t j = j0 + jj;
+    const double sv = kMinusInv4Pi * (tS[0][jj][threadIdx.x] + image_sign * tS[1][jj][threadIdx.x]);
+    double dv = kMinusInv4Pi * (tD[0][jj][threadIdx.x] + image_sign * tD[1][jj][threadIdx.x]);
+    if (p.include_identity && i == j) dv += identity_jump(p, ni);
+    store_static(SR, i + j * n, step, sv);
+    store_static(DR, i + j * n, step, dv);
+  }
+}
+
+// Sets with Delhommeau Rankine kinds: the broadcasting sum over the static tuple
+// (matrix_assembly.jl:70-88).
+template <bool DIRECT>
 __global__ void __launch_bounds__(kRowsPerCta) static_kernel(AssemblyParams p, double* __restrict__ SR,
                                                              double* __restrict__ DR) {
   __shared__ PanelRec sp[kColsPerCta];
@@ -139,10 +250,6 @@ __global__ void __launch_bounds__(kRowsPerCta) static_kernel(AssemblyParams p, d
   if (i >= n) return;
   double ci[3], ni[3];
   for (int c = 0; c < 3; ++c) { ci[c] = __ldg(&p.P[i].c[c]); ni[c] = __ldg(&p.P[i].n[c]); }
-  const bool need_R = (p.gfs & MH_GF_RANKINE) != 0;
-  const bool need_I = (p.gfs & MH_GF_RANKINE_REFLECTED) != 0;
-  const bool need_N = (p.gfs & MH_GF_RANKINE_REFLECTED_NEGATIVE) != 0;
-  const double image_sign = (need_I ? 1.0 : 0.0) + (need_N ? -1.0 : 0.0);
   const int jmax = (int)((n - j0) < kColsPerCta ? (n - j0) : kColsPerCta);
   for (int jj = 0; jj < jmax; ++jj) {
     const int64_t j = j0 + jj;
@@ -150,50 +257,33 @@ __global__ void __launch_bounds__(kRowsPerCta) static_kernel(AssemblyParams p, d
     double nv[3];
     pick_normal<DIRECT>(p, Pj, ni, nv);
     double s = 0.0, d = 0.0;
-    if (BIRK) {
-      double phi, g[3];
-      if (need_R) {
-        vrankine_from_geom(ci, Pj, phi, g);
+    // canonical tuple order: Rankine, RankineReflected, RankineReflectedNegative,
+    // DelhommeauRankine, DelhommeauRankineReflected
+    const double* vj = p.V + 12 * j;
+    double v12[12];
+    for (int q = 0; q < 12; ++q) v12[q] = __ldg(vj + q);
+    double gs[3] = {0.0, 0.0, 0.0};
+    const uint32_t kinds[5] = {MH_GF_RANKINE, MH_GF_RANKINE_REFLECTED, MH_GF_RANKINE_REFLECTED_NEGATIVE,
+                               MH_GF_DELHOMMEAU_RANKINE, MH_GF_DELHOMMEAU_RANKINE_REFLECTED};
+    for (int q = 0; q < 5; ++q) {
+      const uint32_t kd = kinds[q];
+      if (!(p.gfs & kd)) continue;
+      const bool refl = kd == MH_GF_RANKINE_REFLECTED || kd == MH_GF_RANKINE_REFLECTED_NEGATIVE ||
+                        kd == MH_GF_DELHOMMEAU_RANKINE_REFLECTED;
+      double pt[3] = {ci[0], ci[1], refl ? -ci[2] : ci[2]};
+      double I, g[3];
+      if (kd & kBirkKinds) {
+        vrankine_from_geom(pt, Pj, I, g);
         if (!DIRECT) { g[0] = -g[0]; g[1] = -g[1]; g[2] = -g[2]; }
-        s += phi;
-        d += nv[0] * g[0] + nv[1] * g[1] + nv[2] * g[2];
+      } else {
+        delhommeau_rankine(pt, Pj, v12, !DIRECT, I, g);
       }
-      if (need_I || need_N) {
-        double cr[3] = {ci[0], ci[1], -ci[2]};
-        vrankine_from_geom(cr, Pj, phi, g);
-        if (!DIRECT) { g[0] = -g[0]; g[1] = -g[1]; }  // vertical_reflection(-g)
-        s += image_sign * phi;
-        d += image_sign * (nv[0] * g[0] + nv[1] * g[1] + nv[2] * g[2]);
-      }
-    } else {
-      // canonical tuple order: Rankine, RankineReflected, RankineReflectedNegative,
-      // DelhommeauRankine, DelhommeauRankineReflected
-      const double* vj = p.V + 12 * j;
-      double v12[12];
-      for (int q = 0; q < 12; ++q) v12[q] = __ldg(vj + q);
-      double gs[3] = {0.0, 0.0, 0.0};
-      const uint32_t kinds[5] = {MH_GF_RANKINE, MH_GF_RANKINE_REFLECTED, MH_GF_RANKINE_REFLECTED_NEGATIVE,
-                                 MH_GF_DELHOMMEAU_RANKINE, MH_GF_DELHOMMEAU_RANKINE_REFLECTED};
-      for (int q = 0; q < 5; ++q) {
-        const uint32_t kd = kinds[q];
-        if (!(p.gfs & kd)) continue;
-        const bool refl = kd == MH_GF_RANKINE_REFLECTED || kd == MH_GF_RANKINE_REFLECTED_NEGATIVE ||
-                          kd == MH_GF_DELHOMMEAU_RANKINE_REFLECTED;
-        double pt[3] = {ci[0], ci[1], refl ? -ci[2] : ci[2]};
-        double I, g[3];
-        if (kd & kBirkKinds) {
-          vrankine_from_geom(pt, Pj, I, g);
-          if (!DIRECT) { g[0] = -g[0]; g[1] = -g[1]; g[2] = -g[2]; }
-        } else {
-          delhommeau_rankine(pt, Pj, v12, !DIRECT, I, g);
-        }
-        if (refl && !DIRECT) g[2] = -g[2];
-        if (kd == MH_GF_RANKINE_REFLECTED_NEGATIVE) { I = -I; g[0] = -g[0]; g[1] = -g[1]; g[2] = -g[2]; }
-        s += I;
-        gs[0] += g[0]; gs[1] += g[1]; gs[2] += g[2];
-      }
-      d = nv[0] * gs[0] + nv[1] * gs[1] + nv[2] * gs[2];
+      if (refl && !DIRECT) g[2] = -g[2];
+      if (kd == MH_GF_RANKINE_REFLECTED_NEGATIVE) { I = -I; g[0] = -g[0]; g[1] = -g[1]; g[2] = -g[2]; }
+      s += I;
+      gs[0] += g[0]; gs[1] += g[1]; gs[2] += g[2];
     }
+    d = nv[0] * gs[0] + nv[1] * gs[1] + nv[2] * gs[2];
     double sv = kMinusInv4Pi * s, dv = kMinusInv4Pi * d;
     if (p.include_identity && i == j) dv += identity_jump(p, ni);
     SR[i + j * n] = sv;
@@ -274,13 +364,14 @@ __device__ __forceinline__ void wave_entry(const WaveTerms& w, double dx1, doubl
 
 // writes the (i, j) entry and, for i != j, the mirrored (j, i) entry of one unordered pair;
 // ani, anj: area-weighted normals of panels i and j (used as the entries' normals in the
-// direct formulation with panel normals)
+// direct formulation with panel normals); `step`: doubles per entry of SR and DR (2: they are
+// the real parts of S and D themselves)
 template <bool DIRECT>
 __device__ __forceinline__ void store_pair(const AssemblyParams& p, const WaveTerms& w, int64_t i, int64_t j,
                                            const double ni[3], double ai, const double ani[3], const PanelRec& Pj,
                                            const double anj[3], double dx1, double dx2,
-                                           const double* __restrict__ SR, const double* __restrict__ DR,
-                                           double2* __restrict__ Sb, double2* __restrict__ Db, int wave_identity) {
+                                           const double* SR, const double* DR, double2* Sb, double2* Db,
+                                           int wave_identity, int step = 1) {
   const int64_t n = p.n;
   const bool own = DIRECT && !p.has_fixed;  // entry normals are the source panels' own
   // (i, j): source j
@@ -297,8 +388,8 @@ __device__ __forceinline__ void store_pair(const AssemblyParams& p, const WaveTe
   if (wave_identity && i == j) dv.x += identity_jump(p, ni);
   const int64_t idx = i + j * n;
   if (SR) {
-    sv.x = SR[idx] + sv.x;
-    dv.x = DR[idx] + dv.x;
+    sv.x = SR[idx * step] + sv.x;
+    dv.x = DR[idx * step] + dv.x;
   }
   Sb[idx] = sv;
   Db[idx] = dv;
@@ -317,33 +408,35 @@ __device__ __forceinline__ void store_pair(const AssemblyParams& p, const WaveTe
   wave_entry(w, dx1, dx2, -1.0, ai, an, sm, dm);
   const int64_t mdx = j + i * n;
   if (SR) {
-    sm.x = SR[mdx] + sm.x;
-    dm.x = DR[mdx] + dm.x;
+    sm.x = SR[mdx * step] + sm.x;
+    dm.x = DR[mdx * step] + dm.x;
   }
   Sb[mdx] = sm;
   Db[mdx] = dm;
 }
 
 template <bool DIRECT, int WMODE>  // WMODE 1 = Wu only, 2 = exact Delhommeau, 3 = both
-__global__ void __launch_bounds__(kRowsPerCta) wave_kernel(AssemblyParams p, const double* __restrict__ SR,
-                                                           const double* __restrict__ DR,
-                                                           const double* __restrict__ ks, double2* __restrict__ S,
-                                                           double2* __restrict__ D, int64_t sstride,
-                                                           int wave_identity) {
+__global__ void __launch_bounds__(kRowsPerCta) wave_kernel(AssemblyParams p, const double* SR, const double* DR,
+                                                           const double* __restrict__ ks, double2* S, double2* D,
+                                                           int64_t sstride, int wave_identity, int step, int cols) {
   __shared__ PanelRec sp[kColsPerCta];
   __shared__ double san[kColsPerCta][3];  // area-weighted normals of the staged panels
   const int64_t n = p.n;
   const int64_t i0 = blockIdx.x * (int64_t)kRowsPerCta;
-  const int64_t j0 = blockIdx.y * (int64_t)kColsPerCta;
-  if (i0 > j0 + kColsPerCta - 1) return;  // tile strictly below the diagonal
+  const int64_t j0 = blockIdx.y * (int64_t)cols;
+  if (i0 > j0 + cols - 1) return;  // tile strictly below the diagonal
   const int64_t i = i0 + threadIdx.x;
-  const double k = ks[blockIdx.z];
+  const double k = ks ? ks[blockIdx.z] : p.k;
   const double kc[4] = {0.0, kMinusInv4Pi * k, kMinusInv4Pi * k * k, kMinusInv4Pi * k * k * k};
   double2* Sb = S + blockIdx.z * sstride;
   double2* Db = D + blockIdx.z * sstride;
-  stage_panels(sp, p.P, j0, n);
+  const int jmax = (int)((n - j0) < cols ? (n - j0) : cols);
+  {
+    const double2* src = reinterpret_cast<const double2*>(p.P + j0);
+    double2* dst = reinterpret_cast<double2*>(sp);
+    for (int q = threadIdx.x; q < jmax * 16; q += kRowsPerCta) dst[q] = __ldg(src + q);
+  }
   __syncthreads();
-  const int jmax = (int)((n - j0) < kColsPerCta ? (n - j0) : kColsPerCta);
   for (int q = threadIdx.x; q < 3 * jmax; q += blockDim.x) san[q / 3][q % 3] = sp[q / 3].area * sp[q / 3].n[q % 3];
   __syncthreads();
   if (i >= n) return;
@@ -360,7 +453,7 @@ __global__ void __launch_bounds__(kRowsPerCta) wave_kernel(AssemblyParams p, con
     // (i, j) orientation: gradient w.r.t. the source (direct) or the field point (indirect)
     const double dx1 = DIRECT ? Pj.c[0] - ci[0] : ci[0] - Pj.c[0];
     const double dx2 = DIRECT ? Pj.c[1] - ci[1] : ci[1] - Pj.c[1];
-    store_pair<DIRECT>(p, w, i, j, ni, ai, ani, Pj, san[jj], dx1, dx2, SR, DR, Sb, Db, wave_identity);
+    store_pair<DIRECT>(p, w, i, j, ni, ai, ani, Pj, san[jj], dx1, dx2, SR, DR, Sb, Db, wave_identity, step);
   }
 }
 
@@ -769,29 +862,44 @@ void launch_panel_geometry(cudaStream_t st, LaunchCounter lc, int64_t n, const d
             panel_geometry_kernel<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(n, V, C, N, A, R, out));
 }
 
-cudaError_t load_panel_geometry_kernel() {
-  cudaFuncAttributes attr;
-  return cudaFuncGetAttributes(&attr, panel_geometry_kernel);
+// columns per CTA of the pair kernels: 8, fewer where the launch (`tiles` CTAs of one column each)
+// would not give every SM 16 CTAs (about four rounds of the resident ones, so that a last round
+// that is partly empty costs little)
+static int columns_per_cta(int64_t tiles) {
+  return (int)std::max<int64_t>(1, std::min<int64_t>(kColsPerCta, tiles / (16 * 152)));
 }
 
-void launch_assemble_static(cudaStream_t st, LaunchCounter lc, const AssemblyParams& p, double* SR, double* DR) {
+void launch_assemble_static(cudaStream_t st, LaunchCounter lc, const AssemblyParams& p, double* SR, double* DR,
+                            int step) {
   if (p.n <= 0) return;
-  dim3 grid((unsigned)((p.n + kRowsPerCta - 1) / kRowsPerCta), (unsigned)((p.n + kColsPerCta - 1) / kColsPerCta));
-  const bool birk = (p.gfs & kDelhKinds) == 0;
-  lc.pre(st);
-  if (p.direct) {
-    if (birk) static_kernel<true, true><<<grid, kRowsPerCta, 0, st>>>(p, SR, DR);
-    else static_kernel<true, false><<<grid, kRowsPerCta, 0, st>>>(p, SR, DR);
-  } else {
-    if (birk) static_kernel<false, true><<<grid, kRowsPerCta, 0, st>>>(p, SR, DR);
-    else static_kernel<false, false><<<grid, kRowsPerCta, 0, st>>>(p, SR, DR);
+  const int64_t rt = (p.n + kRowsPerCta - 1) / kRowsPerCta;
+  if ((p.gfs & kDelhKinds) == 0) {
+    const int cols = columns_per_cta(rt * p.n);
+    dim3 grid((unsigned)rt, (unsigned)((p.n + cols - 1) / cols));
+    if (p.direct)
+      MH_LAUNCH(lc, st, "assemble_static", static_birk_kernel<true><<<grid, kRowsPerCta, 0, st>>>(p, SR, DR, step, cols));
+    else
+      MH_LAUNCH(lc, st, "assemble_static", static_birk_kernel<false><<<grid, kRowsPerCta, 0, st>>>(p, SR, DR, step, cols));
+    return;
   }
-  lc.post(st, "assemble_static");
+  dim3 grid((unsigned)rt, (unsigned)((p.n + kColsPerCta - 1) / kColsPerCta));
+  if (p.direct) MH_LAUNCH(lc, st, "assemble_static", static_kernel<true><<<grid, kRowsPerCta, 0, st>>>(p, SR, DR));
+  else MH_LAUNCH(lc, st, "assemble_static", static_kernel<false><<<grid, kRowsPerCta, 0, st>>>(p, SR, DR));
+}
+
+cudaError_t load_pair_kernels() {
+  cudaFuncAttributes attr;
+  cudaError_t e = cudaFuncGetAttributes(&attr, panel_geometry_kernel);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&attr, static_birk_kernel<true>);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&attr, static_birk_kernel<false>);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&attr, wave_kernel<true, 1>);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&attr, wave_kernel<false, 1>);
+  return e;
 }
 
 void launch_assemble_wave(cudaStream_t st, LaunchCounter lc, const AssemblyParams& p, const double* SR,
                           const double* DR, int nk, const double* ks_dev, double2* S, double2* D, int64_t sstride,
-                          int wave_identity) {
+                          int wave_identity, int step) {
   if (p.n <= 0 || nk <= 0) return;
   const uint32_t wv = p.gfs & (MH_GF_WU | MH_GF_EXACT_DELHOMMEAU | MH_GF_SURROGATE);
   if (!wv) {
@@ -824,7 +932,10 @@ void launch_assemble_wave(cudaStream_t st, LaunchCounter lc, const AssemblyParam
   }
   const int mode = (wv == MH_GF_WU) ? 1 : (wv == MH_GF_EXACT_DELHOMMEAU ? 2 : 3);
   lc.pre(st);
-#define MH_WAVE(DIR, MODE) wave_kernel<DIR, MODE><<<grid, kRowsPerCta, 0, st>>>(p, SR, DR, ks_dev, S, D, sstride, wave_identity)
+  const int cols = columns_per_cta((int64_t)grid.x * p.n * nk / 2);
+  grid.y = (unsigned)((p.n + cols - 1) / cols);
+#define MH_WAVE(DIR, MODE) \
+  wave_kernel<DIR, MODE><<<grid, kRowsPerCta, 0, st>>>(p, SR, DR, ks_dev, S, D, sstride, wave_identity, step, cols)
   if (p.direct) {
     if (mode == 1) MH_WAVE(true, 1); else if (mode == 2) MH_WAVE(true, 2); else MH_WAVE(true, 3);
   } else {

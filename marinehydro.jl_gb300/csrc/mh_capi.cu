@@ -580,14 +580,17 @@ int mh_assemble_matrices(mh_context* ctx, mh_mesh* m, double k, uint32_t gfs, in
     MH_TRY(ws_get_t(ctx, kSlotS, nn, &Sd));
     MH_TRY(ws_get_t(ctx, kSlotD, nn, &Dd));
   }
-  double* kd;
-  MH_TRY(ws_get_t(ctx, kSlotSmall, 4, &kd));
-  double* hk;
-  MH_TRY(pinned_get(ctx, 64, &hk));
-  hk[0] = k;
-  MH_CUDA(ctx, cudaMemcpyAsync(kd, hk, sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
   AssemblyParams p = make_params(ctx, m, gfs, direct, include_identity, fixed_normal);
+  p.k = k;
   MH_TRY(prepare_surrogate(ctx, p, 1));
+  double* kd = nullptr;  // the surrogate kernels read the wavenumber from device memory
+  if (gfs & MH_GF_SURROGATE) {
+    MH_TRY(ws_get_t(ctx, kSlotSmall, 4, &kd));
+    double* hk;
+    MH_TRY(pinned_get(ctx, 64, &hk));
+    hk[0] = k;
+    MH_CUDA(ctx, cudaMemcpyAsync(kd, hk, sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+  }
   launch_assemble_wave(ctx->stream, ctx->lc(), p, st ? m->SR : nullptr, st ? m->DR : nullptr, 1, kd, Sd, Dd,
                        (int64_t)nn, (!st && include_identity) ? 1 : 0);
   MH_TRY(check_launch(ctx, "wave assembly"));

@@ -174,6 +174,37 @@ __device__ __forceinline__ double log_pos(double w) {
   return to_double(q, 53);
 }
 
+// atan2(y, x) with its quotient, table and octant on the integer pipe but for four FP64
+// operations: the smaller over the larger magnitude (fx::recip, two roundings), a degree-9
+// interpolant on the 1/32-interval of the quotient (table fxq::kAtanTab), absolute error below
+// 1e-17 before the final roundings.  atan2(0, 0) = 0 as in C.
+__device__ __forceinline__ double atan2_int(double y, double x) {
+  const unsigned long long kSign = 0x8000000000000000ull;
+  const unsigned long long by = (unsigned long long)__double_as_longlong(y), bx = (unsigned long long)__double_as_longlong(x);
+  const unsigned long long ay = by & ~kSign, ax = bx & ~kSign;
+  const bool swap = ay > ax;
+  const unsigned long long mx = swap ? ay : ax, mn = swap ? ax : ay;
+  double a = 0.0;
+  if (mn != 0) {
+    const double q = __longlong_as_double((long long)mn) * recip(__longlong_as_double((long long)mx));
+    if (__double_as_longlong(q) >= 0x3FF0000000000000ll) {
+      a = 0.78539816339744830962;
+    } else {
+      const unsigned long long U = unit_q64(q);
+      const long long* __restrict__ row = fxq::kAtanTab + (int)(U >> 59) * fxq::kAtanTerms;
+      const unsigned long long G = U << 5;
+      long long v = __ldg(row + fxq::kAtanTerms - 1);
+#pragma unroll
+      for (int i = fxq::kAtanTerms - 2; i >= 0; --i) v = __ldg(row + i) + mulhi_su(v, G);
+      // below 2^-9 the fixed point holds too few bits of the result: atan q = q - q^3/3 + q^5/5
+      a = __double_as_longlong(q) < 0x3F60000000000000ll ? q - q * q * q * (1.0 / 3.0 - q * q * 0.2) : to_double(v, 62);
+    }
+  }
+  if (swap) a = 1.57079632679489661923 - a;
+  if (bx & kSign) a = 3.14159265358979323846 - a;
+  return __longlong_as_double((long long)((unsigned long long)__double_as_longlong(a) | (by & kSign)));
+}
+
 // sqrt(x) for x >= 0 on the integer pipe (0 for x below the normal range): x = m 2^(2h),
 // m in [1, 4); the FP32 reciprocal square root (one MUFU operation) of m's leading bits as
 // the seed, two Newton steps y <- y (3 - m y^2) / 2 in 64-bit fixed point (m 2^62, y 2^63),

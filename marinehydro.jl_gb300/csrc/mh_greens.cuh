@@ -23,24 +23,12 @@ __device__ __forceinline__ double2 zmul(double2 a, double2 b) {
   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 __device__ __forceinline__ double2 zscale(double s, double2 a) { return make_double2(s * a.x, s * a.y); }
-__device__ __forceinline__ double zabs(double2 a) { return hypot(a.x, a.y); }
-__device__ __forceinline__ double2 zdiv(double2 a, double2 b) {
-  // Smith's algorithm (scaled) for a / b
-  if (fabs(b.x) >= fabs(b.y)) {
-    double r = b.y / b.x, den = b.x + b.y * r;
-    return make_double2((a.x + a.y * r) / den, (a.y - a.x * r) / den);
-  } else {
-    double r = b.x / b.y, den = b.y + b.x * r;
-    return make_double2((a.x * r + a.y) / den, (a.y * r - a.x) / den);
-  }
-}
 __device__ __forceinline__ double2 zexp(double2 a) {
   double s, c;
   sincos(a.y, &s, &c);
   double e = exp(a.x);
   return make_double2(e * c, e * s);
 }
-__device__ __forceinline__ double2 zlog(double2 a) { return make_double2(log(hypot(a.x, a.y)), atan2(a.y, a.x)); }
 
 // ------------------------------- Birk Rankine -------------------------------
 constexpr double kBirkZTol = 1e-14;   // rankine_vectorized.jl:24
@@ -48,23 +36,23 @@ constexpr double kBirkDkTol = 1e-14;  // rankine_vectorized.jl:25
 
 // _abs_ad (rankine_vectorized.jl:30): -0.0 stays -0.0
 __device__ __forceinline__ double abs_ad(double x) { return x < 0.0 ? -x : x; }
-// _atan_ratio (rankine_vectorized.jl:42-45)
-__device__ __forceinline__ double atan_ratio(double num, double den) {
-  double flipped = den < 0.0 ? -num : num;
-  return atan2(flipped, abs_ad(den));
-}
 
 // birk_phi_and_velocity (rankine_vectorized.jl:241-267); lc = 4 local corners (x, y),
-// edge = their 4 edge lengths (per panel, precomputed; the same hypot of the corner offsets)
+// edge = their 4 edge lengths (per panel, precomputed; the same hypot of the corner offsets).
+// Square roots, reciprocals, logarithms and arc tangents run on the integer pipe
+// (mh_fixpoint.cuh), and an edge's two arc tangents (den >= 0, so each lies in [-pi/2, pi/2])
+// are taken as one: the argument of the product of one complex number with the other's
+// conjugate is their difference.  About 170 FP64 instructions are left of some 700.
 __device__ inline void birk_phi_and_velocity(double x, double y, double z, const double* lc, const double* edge,
                                              double& phi, double v[3]) {
   double sx[4], sy[4], r[4], e[4], h[4];
+  const double z2 = z * z;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     sx[k] = x - lc[2 * k];
     sy[k] = y - lc[2 * k + 1];
-    r[k] = sqrt(sx[k] * sx[k] + sy[k] * sy[k] + z * z);
-    e[k] = sx[k] * sx[k] + z * z;
+    e[k] = sx[k] * sx[k] + z2;
+    r[k] = fx::sqrt_pos(sy[k] * sy[k] + e[k]);
     h[k] = sx[k] * sy[k];
   }
   const bool inplane = fabs(z) <= kBirkZTol;  // _inplane_atan (:49-54)
@@ -72,26 +60,46 @@ __device__ inline void birk_phi_and_velocity(double x, double y, double z, const
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     const int kn = (k + 1) & 3;
-    double dx = lc[2 * kn] - lc[2 * k];
-    double dy = lc[2 * kn + 1] - lc[2 * k + 1];
     const double dk = edge[k];
-    if (!(dk <= kBirkDkTol)) {
-      double rsum = r[k] + r[kn];
-      double log_term = log((rsum - dk) / (rsum + dk));
-      double lt_dk = log_term / dk;
-      double vzk = 0.0;
-      if (!inplane)
-        vzk = atan_ratio(dy * e[k] - dx * h[k], dx * z * r[k]) - atan_ratio(dy * e[kn] - dx * h[kn], dx * z * r[kn]);
-      s0 += (sx[k] * dy - sy[k] * dx) * lt_dk + z * vzk;
-      s1 += dy * lt_dk;
-      s2 += -dx * lt_dk;
-      s3 += vzk;
+    if (dk <= kBirkDkTol) continue;
+    const double dx = lc[2 * kn] - lc[2 * k];
+    const double dy = lc[2 * kn + 1] - lc[2 * k + 1];
+    const double rsum = r[k] + r[kn];
+    const double num = rsum - dk;
+    const double w = num * fx::recip(rsum + dk);
+    // on the edge itself num vanishes or rounds below zero: log's own answer
+    const double log_term = num > 0.0 ? fx::log_pos(w) : log(w);
+    const double lt_dk = log_term * fx::recip(dk);
+    if (!inplane) {
+      const double dxz = dx * z;
+      double n1 = dy * e[k] - dx * h[k], d1 = dxz * r[k];
+      double n2 = dy * e[kn] - dx * h[kn], d2 = dxz * r[kn];
+      if (d1 < 0.0) { n1 = -n1; d1 = -d1; }  // _atan_ratio (:42-45): den's sign moved to num
+      if (d2 < 0.0) { n2 = -n2; d2 = -d2; }
+      s3 += fx::atan2_int(n1 * d2 - n2 * d1, d1 * d2 + n1 * n2);
     }
+    s0 += (sx[k] * dy - sy[k] * dx) * lt_dk;
+    s1 += dy * lt_dk;
+    s2 -= dx * lt_dk;
   }
+  s0 += z * s3;
   phi = kMinusInv4Pi * s0;
   v[0] = kMinusInv4Pi * s1;
   v[1] = kMinusInv4Pi * s2;
   v[2] = kMinusInv4Pi * s3;
+}
+
+// the near-field form of vrankine_from_geom (pt within 7 radii of the panel's centre)
+__device__ inline void vrankine_near(const double pt[3], const PanelRec& P, double& phi, double g[3]) {
+  double d0 = pt[0] - P.qgc[0], d1 = pt[1] - P.qgc[1], d2 = pt[2] - P.qgc[2];
+  double fx_ = P.T[0] * d0 + P.T[1] * d1 + P.T[2] * d2;
+  double fy_ = P.T[3] * d0 + P.T[4] * d1 + P.T[5] * d2;
+  double fz_ = P.T[6] * d0 + P.T[7] * d1 + P.T[8] * d2;
+  double phb, vl[3];
+  birk_phi_and_velocity(fx_, fy_, fz_, P.lc, P.edge, phb, vl);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) g[i] = kFourPi * (P.T[i] * vl[0] + P.T[3 + i] * vl[1] + P.T[6 + i] * vl[2]);
+  phi = -kFourPi * phb;
 }
 
 // _vrankine_from_geom (rankine_vectorized.jl:273-287): integral of 1/r over panel P
@@ -109,15 +117,7 @@ __device__ inline void vrankine_from_geom(const double pt[3], const PanelRec& P,
     g[2] = rb2 * s;
     return;
   }
-  double d0 = pt[0] - P.qgc[0], d1 = pt[1] - P.qgc[1], d2 = pt[2] - P.qgc[2];
-  double fx = P.T[0] * d0 + P.T[1] * d1 + P.T[2] * d2;
-  double fy = P.T[3] * d0 + P.T[4] * d1 + P.T[5] * d2;
-  double fz = P.T[6] * d0 + P.T[7] * d1 + P.T[8] * d2;
-  double phb, vl[3];
-  birk_phi_and_velocity(fx, fy, fz, P.lc, P.edge, phb, vl);
-#pragma unroll
-  for (int i = 0; i < 3; ++i) g[i] = kFourPi * (P.T[i] * vl[0] + P.T[3 + i] * vl[1] + P.T[6 + i] * vl[2]);
-  phi = -kFourPi * phb;
+  vrankine_near(pt, P, phi, g);
 }
 
 // ---------------------------- Delhommeau Rankine ----------------------------
@@ -338,25 +338,6 @@ __device__ __forceinline__ void reduced_coords(const double x[3], const double x
   double dis = (d2 == 0) ? sqrt(d2 + purt * purt) - purt : fx::sqrt_pos(d2);
   hh = k * dis;
   vv = k * (x[2] + xi[2]);
-}
-
-// _wu_sd (wu.jl:112-127): s, d for one pair before the -1/4pi scale
-__device__ inline void wu_sd(const double x[3], const double xi[3], const double nv[3], double area2, double k,
-                             double dx1, double dx2, double2& s, double2& d) {
-  double hh, vv;
-  reduced_coords(x, xi, k, hh, vv);
-  double2 GF, Gh, Gv;
-  wu_wave_term_and_derivs(hh, vv, GF, Gh, Gv);
-  double dr1 = 0.0, dr2 = 0.0;
-  if (fabs(hh) > 1e-6) {
-    dr1 = k * k / hh * dx1;
-    dr2 = k * k / hh * dx2;
-  }
-  double g0r = k * (dr1 * Gh.x), g0i = k * (dr1 * Gh.y);
-  double g1r = k * (dr2 * Gh.x), g1i = k * (dr2 * Gh.y);
-  double g2r = k * (k * Gv.x), g2i = k * (k * Gv.y);
-  s = make_double2((k * GF.x) * area2, (k * GF.y) * area2);
-  d = make_double2((nv[0] * g0r + nv[1] * g1r + nv[2] * g2r) * area2, (nv[0] * g0i + nv[1] * g1i + nv[2] * g2i) * area2);
 }
 
 // ------------------------- exact Guevel-Delhommeau --------------------------

@@ -90,9 +90,9 @@ struct LaunchCounter {
 // assembly (mh_assembly.cu)
 void launch_panel_geometry(cudaStream_t st, LaunchCounter lc, int64_t n, const double* V, const double* C,
                            const double* N, const double* A, const double* R, PanelRec* out);
-// loads panel_geometry_kernel's module on the current device now (lazy loading would do it
-// at the first launch)
-cudaError_t load_panel_geometry_kernel();
+// loads the panel-geometry, Birk and Wu kernels on the current device now (lazy loading would do
+// it at their first launch)
+cudaError_t load_pair_kernels();
 
 struct AssemblyParams {
   int64_t n;
@@ -115,12 +115,15 @@ struct AssemblyParams {
 };
 
 // Static (wavenumber-independent) part into real n x n arrays SR, DR (identity included when asked).
-void launch_assemble_static(cudaStream_t st, LaunchCounter lc, const AssemblyParams& p, double* SR, double* DR);
+// step 2 (Birk kinds only): into the real parts of complex arrays, the imaginary parts zeroed
+void launch_assemble_static(cudaStream_t st, LaunchCounter lc, const AssemblyParams& p, double* SR, double* DR,
+                            int step = 1);
 // S = SR + S_wave(k), D = DR + D_wave(k) (complex); SR/DR may be null (no static part).
-// batch: `nk` wavenumbers ks[b], output b at S + b*sstride (complex elements).
+// batch: `nk` wavenumbers ks[b], output b at S + b*sstride (complex elements).  ks_dev null: the
+// one wavenumber p.k.  step 2 (Wu and exact kinds): SR and DR are the real parts of S and D.
 void launch_assemble_wave(cudaStream_t st, LaunchCounter lc, const AssemblyParams& p, const double* SR,
                           const double* DR, int nk, const double* ks_dev, double2* S, double2* D, int64_t sstride,
-                          int wave_identity);
+                          int wave_identity, int step = 1);
 // The exact term's check of surrogate-assembled matrices: n_samples pairs per matrix drawn from
 // (seed, first_matrix + b, sample); acc[2 b] += sum |assembled - exact|^2 over S and D entries,
 // acc[2 b + 1] += sum |assembled|^2 (acc zeroed by the caller)

@@ -1,0 +1,48 @@
+"""The Birk Rankine assembly (far terms per thread, near terms from a list) at ragged row and
+column tiles, both formulations, image signs and the no-allocation entry point's in-place static
+part, against the oracle."""
+import ctypes
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+KINDS = {"direct_only": (1, 0), "image": (1, 2), "negative": (1, 4), "image_only": (0, 2)}
+
+
+@pytest.mark.parametrize("n_lat, n_lon", [(1, 3), (3, 5), (7, 18), (8, 16), (9, 15), (16, 41)])
+@pytest.mark.parametrize("kinds", list(KINDS))
+@pytest.mark.parametrize("direct", [True, False])
+def test_static_tiles(mh, oracle, ctx, n_lat, n_lon, kinds, direct):
+    mesh = mh.hemisphere_mesh(1.3, n_lat, n_lon)
+    gfs = sum(KINDS[kinds])
+    names = {1: mh.Rankine, 2: mh.RankineReflected, 4: mh.RankineReflectedNegative}
+    S, D = mh.assemble_matrices(tuple(names[b]() for b in (1, 2, 4) if gfs & b), mesh, 1.0, direct=direct, ctx=ctx)
+    So, Do = oracle.assemble_matrices(mesh, 1.0, gfs=gfs, direct=direct)
+    # entries differ by a few roundings of the terms they sum (at most 2 pi and 1/r^2 of them)
+    assert np.abs(S - So).max() <= 64 * 2.0 ** -53 * np.abs(So).max()
+    assert np.abs(D - Do).max() <= 64 * 2.0 ** -53 * max(1.0, np.abs(Do).max())
+
+
+@pytest.mark.parametrize("n_lat, n_lon", [(1, 3), (8, 16), (16, 41)])
+@pytest.mark.parametrize("direct", [True, False])
+@pytest.mark.parametrize("fixed", [None, (1.0, 0.0, 0.0)])
+def test_noalloc_equals_allocating(mh, ctx, n_lat, n_lon, direct, fixed):
+    torch = pytest.importorskip("torch")
+    mesh = mh.hemisphere_mesh(1.3, n_lat, n_lon)
+    n, L = mesh.nfaces, mh.load_library()
+    dev = [torch.from_numpy(np.ascontiguousarray(a, dtype=np.float64)).cuda()
+           for a in (mesh.panel_vertices, mesh.centers, mesh.normals, mesh.areas, mesh.radii)]
+    for greens in ((mh.Rankine(), mh.RankineReflected(), mh.GFWu()), (mh.Rankine(),), (mh.GFWu(),)):
+        S = torch.full((n, n), float("nan"), dtype=torch.complex128, device="cuda")
+        D = torch.full_like(S, float("nan"))
+        fx = None if fixed is None else np.asarray(fixed)
+        rc = L.mh_assemble_matrices_noalloc(torch.cuda.current_stream().cuda_stream, n, *[t.data_ptr() for t in dev],
+                                            0.8, mh.gf_flags(greens), int(direct), 1,
+                                            None if fx is None else fx.ctypes.data_as(ctypes.c_void_p), S.data_ptr(),
+                                            D.data_ptr())
+        assert rc == 0
+        torch.cuda.synchronize()
+        S0, D0 = mh.assemble_matrices(greens, mesh, 0.8, direct=direct, all_normals=fixed, ctx=ctx)
+        assert np.array_equal(S.cpu().numpy().T, S0) and np.array_equal(D.cpu().numpy().T, D0)
