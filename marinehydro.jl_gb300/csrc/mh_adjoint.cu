@@ -45,46 +45,65 @@ template <typename R> struct CR { R x, y; };
 // ---------------------------------------------------------------------------
 // Wu wave term on a generic scalar (the same operations as wu_wave_term_and_derivs)
 // ---------------------------------------------------------------------------
-template <typename R> __device__ R pA(R t) {
-  R v = (21859.0 + -4838.6 * t) * t;
-  v = (-41592.9 + v) * t; v = (42002.57 + v) * t; v = (-24314.21 + v) * t; v = (8418.94 + v) * t;
-  v = (-1763.96 + v) * t; v = (215.896 + v) * t; v = (-13.328 + v) * t;
-  return 1.21 + v;
+// The seven fits (wu.jl:131-197, 235-329) and their derivatives in rho.  The terms from rho^2 up run
+// in 64-bit fixed point (mh_fixpoint.cuh) with the fraction bits that the largest partial sum on
+// [0, 1] leaves, the last two steps in FP64.  The differentiated coefficients are integer
+// multiples of the fixed-point ones: as doubles (7 * 205690.43 ..) they would round by up to
+// 1e-10, the same way in every pair, and the added mass' frequency derivative would be off by
+// 2e-14 instead of 8e-15.
+template <int F, int N>
+__device__ __forceinline__ double wu_fit(double c0, double c1, const long long (&c)[N], double rho, unsigned long long t) {
+  return fma(fma(fx::to_double(fx::horner_u_mid(c, t), F), rho, c1), rho, c0);
 }
-template <typename R> __device__ R pB(R t) {
-  R v = (-29030.24 + 7671.22 * t) * t;
-  v = (44894.06 + v) * t; v = (-36618.81 + v) * t; v = (17137.74 + v) * t; v = (-4780.77 + v) * t;
-  v = (796.534 + v) * t; v = (-67.92 + v) * t; v = (5.737 + v) * t;
-  return 0.938 + v;
-}
-template <typename R> __device__ R pC(R t) {
-  R v = (9136.4 + -3272.62 * t) * t;
-  v = (-9844.35 + v) * t; v = (5155.67 + v) * t; v = (-1397.89 + v) * t; v = (209.653 + v) * t;
-  v = (-9.747 + v) * t;
-  return 1.268 + v;
-}
-template <typename R> __device__ R pD(R t) {
-  R v = (128170.2 + -33744.6 * t) * t;
-  v = (-205690.43 + v) * t; v = (181856.75 + v) * t; v = (-96293.05 + v) * t; v = (31127.39 + v) * t;
-  v = (-6072.07 + v) * t; v = (667.16 + v) * t; v = (-40.97 + v) * t;
-  return 0.632 + v;
-}
-template <typename R> __device__ R pdA(R t) {
-  R v = (-46688.0 + 12622.25 * t) * t;
-  v = (68220.87 + v) * t; v = (-48811.41 + v) * t; v = (16370.75 + v) * t; v = (-1187.71 + v) * t;
-  v = (-754.85 + v) * t; v = (249.69 + v) * t; v = (-24.53 + v) * t;
-  return 2.948 + v;
-}
-template <typename R> __device__ R pdB(R t) {
-  R v = (-76209.82 + 19923.28 * t) * t;
-  v = (118879.26 + v) * t; v = (-97014.11 + v) * t; v = (44270.15 + v) * t; v = (-11336.19 + v) * t;
-  v = (1565.35 + v) * t; v = (-76.765 + v) * t; v = (2.894 + v) * t;
-  return 1.11 + v;
-}
-template <typename R> __device__ R pdC(R t) {
-  R v = (3168.35 + -1590.27 * t) * t;
-  v = (-2318.58 + v) * t; v = (847.8 + v) * t; v = (-148.24 + v) * t;
-  return 14.19 + v;
+__device__ __forceinline__ void wu_fits_and_derivatives(double rho, WuFits& f, WuFits& d) {
+  constexpr long long k0A[8] = {fx::q(215.896, 47), fx::q(-1763.96, 47), fx::q(8418.94, 47), fx::q(-24314.21, 47),
+                                fx::q(42002.57, 47), fx::q(-41592.9, 47), fx::q(21859.0, 47), fx::q(-4838.6, 47)};
+  constexpr long long k1A[7] = {3 * fx::q(-1763.96, 44), 4 * fx::q(8418.94, 44), 5 * fx::q(-24314.21, 44),
+                                6 * fx::q(42002.57, 44), 7 * fx::q(-41592.9, 44), 8 * fx::q(21859.0, 44),
+                                9 * fx::q(-4838.6, 44)};
+  constexpr long long k0B[8] = {fx::q(-67.92, 47), fx::q(796.534, 47), fx::q(-4780.77, 47), fx::q(17137.74, 47),
+                                fx::q(-36618.81, 47), fx::q(44894.06, 47), fx::q(-29030.24, 47), fx::q(7671.22, 47)};
+  constexpr long long k1B[7] = {3 * fx::q(796.534, 44), 4 * fx::q(-4780.77, 44), 5 * fx::q(17137.74, 44),
+                                6 * fx::q(-36618.81, 44), 7 * fx::q(44894.06, 44), 8 * fx::q(-29030.24, 44),
+                                9 * fx::q(7671.22, 44)};
+  constexpr long long k0C[6] = {fx::q(209.653, 49), fx::q(-1397.89, 49), fx::q(5155.67, 49), fx::q(-9844.35, 49),
+                                fx::q(9136.4, 49), fx::q(-3272.62, 49)};
+  constexpr long long k1C[5] = {3 * fx::q(-1397.89, 47), 4 * fx::q(5155.67, 47), 5 * fx::q(-9844.35, 47),
+                                6 * fx::q(9136.4, 47), 7 * fx::q(-3272.62, 47)};
+  constexpr long long k0D[8] = {fx::q(667.16, 45), fx::q(-6072.07, 45), fx::q(31127.39, 45), fx::q(-96293.05, 45),
+                                fx::q(181856.75, 45), fx::q(-205690.43, 45), fx::q(128170.2, 45),
+                                fx::q(-33744.6, 45)};
+  constexpr long long k1D[7] = {3 * fx::q(-6072.07, 42), 4 * fx::q(31127.39, 42), 5 * fx::q(-96293.05, 42),
+                                6 * fx::q(181856.75, 42), 7 * fx::q(-205690.43, 42), 8 * fx::q(128170.2, 42),
+                                9 * fx::q(-33744.6, 42)};
+  constexpr long long k0dA[8] = {fx::q(249.69, 46), fx::q(-754.85, 46), fx::q(-1187.71, 46), fx::q(16370.75, 46),
+                                 fx::q(-48811.41, 46), fx::q(68220.87, 46), fx::q(-46688.0, 46), fx::q(12622.25, 46)};
+  constexpr long long k1dA[7] = {3 * fx::q(-754.85, 44), 4 * fx::q(-1187.71, 44), 5 * fx::q(16370.75, 44),
+                                 6 * fx::q(-48811.41, 44), 7 * fx::q(68220.87, 44), 8 * fx::q(-46688.0, 44),
+                                 9 * fx::q(12622.25, 44)};
+  constexpr long long k0dB[8] = {fx::q(-76.765, 46), fx::q(1565.35, 46), fx::q(-11336.19, 46), fx::q(44270.15, 46),
+                                 fx::q(-97014.11, 46), fx::q(118879.26, 46), fx::q(-76209.82, 46),
+                                 fx::q(19923.28, 46)};
+  constexpr long long k1dB[7] = {3 * fx::q(1565.35, 43), 4 * fx::q(-11336.19, 43), 5 * fx::q(44270.15, 43),
+                                 6 * fx::q(-97014.11, 43), 7 * fx::q(118879.26, 43), 8 * fx::q(-76209.82, 43),
+                                 9 * fx::q(19923.28, 43)};
+  constexpr long long k0dC[4] = {fx::q(847.8, 51), fx::q(-2318.58, 51), fx::q(3168.35, 51), fx::q(-1590.27, 51)};
+  constexpr long long k1dC[3] = {3 * fx::q(-2318.58, 49), 4 * fx::q(3168.35, 49), 5 * fx::q(-1590.27, 49)};
+  const unsigned long long t = fx::unit_q64(rho);
+  f.A = wu_fit<47>(1.21, -13.328, k0A, rho, t);
+  f.B = wu_fit<47>(0.938, 5.737, k0B, rho, t);
+  f.C = wu_fit<49>(1.268, -9.747, k0C, rho, t);
+  f.D = wu_fit<45>(0.632, -40.97, k0D, rho, t);
+  f.dA = wu_fit<46>(2.948, -24.53, k0dA, rho, t);
+  f.dB = wu_fit<46>(1.11, 2.894, k0dB, rho, t);
+  f.dC = wu_fit<51>(14.19, -148.24, k0dC, rho, t);
+  d.A = wu_fit<44>(-13.328, 2 * 215.896, k1A, rho, t);
+  d.B = wu_fit<44>(5.737, 2 * -67.92, k1B, rho, t);
+  d.C = wu_fit<47>(-9.747, 2 * 209.653, k1C, rho, t);
+  d.D = wu_fit<42>(-40.97, 2 * 667.16, k1D, rho, t);
+  d.dA = wu_fit<44>(-24.53, 2 * 249.69, k1dA, rho, t);
+  d.dB = wu_fit<43>(2.894, 2 * -76.765, k1dB, rho, t);
+  d.dC = wu_fit<49>(-148.24, 2 * 847.8, k1dC, rho, t);
 }
 
 template <typename R>
@@ -93,7 +112,10 @@ __device__ void wu_terms_t(R hh, R vv, CR<R>& GF, CR<R>& Gh, CR<R>& Gv) {
   const R inv_dd = 1.0 / dd;
   R alpha = -vv * inv_dd;
   R beta = hh * inv_dd;
-  R rho = dd / (1.0 + dd);
+  const R opdd = 1.0 + dd;
+  R rho = dd / opdd;
+  // one residual correction, as in the primal: an ulp of rho moves the fits by up to 1e-13
+  rho.v = fma(fma(-rho.v, opdd.v, dd.v), fx::recip(opdd.v), rho.v);
   R dd2 = dd * dd, dd3 = dd * dd * dd;
   R omr = 1.0 - rho;
   R omr3 = omr * omr * omr;
@@ -114,10 +136,12 @@ __device__ void wu_terms_t(R hh, R vv, CR<R>& GF, CR<R>& Gh, CR<R>& Gv) {
     R d2 = kPi * (1.0 + (3.81095112 + (2.26216956 + 0.10885141 * yy) * yy) * yy);
     H1 = d1 / d2 + Y1;
   }
-  R RR = (1.0 - beta) * pA(rho);
-  RR -= beta * pB(rho);
-  RR -= alpha * pC(rho) / (1.0 + 6.0 * alpha * rho * (1.0 - rho));
-  RR += beta * (1.0 - beta) * pD(rho);
+  WuFits fit, der;
+  wu_fits_and_derivatives(val(rho), fit, der);
+  R RR = (1.0 - beta) * chain1(rho, fit.A, der.A);
+  RR -= beta * chain1(rho, fit.B, der.B);
+  RR -= alpha * chain1(rho, fit.C, der.C) / (1.0 + 6.0 * alpha * rho * (1.0 - rho));
+  RR += beta * (1.0 - beta) * chain1(rho, fit.D, der.D);
   R Lp = rho * omr3 * RR;
   const double gama = 0.5772156649;
   R PP = log(0.5 * (dd - vv)) + gama - 2.0 * dd2;
@@ -128,9 +152,9 @@ __device__ void wu_terms_t(R hh, R vv, CR<R>& GF, CR<R>& Gh, CR<R>& Gv) {
   const double twopi = 2 * kPi;
   GF.x = -L0 - (twopi * H0) * ev;
   GF.y = -((twopi * -J0) * ev);
-  R RS = beta * pdA(rho);
-  RS -= (1.0 - alpha) * pdB(rho);
-  RS += beta * (1.0 - beta) * rho * (1.0 - 2.0 * rho) * pdC(rho);
+  R RS = beta * chain1(rho, fit.dA, der.dA);
+  RS -= (1.0 - alpha) * chain1(rho, fit.dB, der.dB);
+  RS += beta * (1.0 - beta) * rho * (1.0 - 2.0 * rho) * chain1(rho, fit.dC, der.dC);
   R Lsp = rho * omr3 * RS;
   R PS = (beta + hh) / (dd - vv);
   PS = PS - 2.0 * beta + 2.0 * ev * dd - hh;
@@ -144,17 +168,11 @@ __device__ void wu_terms_t(R hh, R vv, CR<R>& GF, CR<R>& Gh, CR<R>& Gv) {
 }
 
 // ---------------------------------------------------------------------------
-// Birk panel pipeline on a generic scalar: geometry from the 4 corners and the
-// near-field panel integral (rankine_vectorized.jl:79-137, 241-287)
+// Birk panel frame on a generic scalar: T (s, t, n), area centroid and local corners from the
+// panel's 4 corners (rankine_vectorized.jl:79-137), as panel_geometry_kernel computes them
 // ---------------------------------------------------------------------------
-template <typename R> __device__ R abs_ad_t(R x) { return val(x) < 0.0 ? -x : x; }
-template <typename R> __device__ R atan_ratio_t(R num, R den) {
-  R flipped = val(den) < 0.0 ? -num : num;
-  return atan2(flipped, abs_ad_t(den));
-}
-
 template <typename R>
-__device__ void birk_near_t(const R p[3], const R v[12], R& phi, R g[3]) {
+__device__ void birk_geometry_t(const R v[12], R T[9], R qgc[3], R lc[8]) {
   R mid[4][3], mgc[3], s[3], tt[3], nn[3], t[3];
   for (int i = 0; i < 4; ++i) {
     int ip = (i + 1) & 3;
@@ -192,87 +210,139 @@ __device__ void birk_near_t(const R p[3], const R v[12], R& phi, R g[3]) {
     My = My + (yk1 - yk) * (xk * xk + xk * xk1 + xk1 * xk1) / 6.0;
   }
   R clx = My / Ar, cly = -Mx / Ar;
-  R qgc[3], lc[8];
   for (int c = 0; c < 3; ++c) qgc[c] = mgc[c] + clx * s[c] + cly * t[c];
   for (int k = 0; k < 4; ++k) {
     lc[2 * k] = tc[k][0] - clx;
     lc[2 * k + 1] = tc[k][1] - cly;
   }
-  // field point in the local frame
-  R d0 = p[0] - qgc[0], d1 = p[1] - qgc[1], d2 = p[2] - qgc[2];
-  R x = s[0] * d0 + s[1] * d1 + s[2] * d2;
-  R y = t[0] * d0 + t[1] * d1 + t[2] * d2;
-  R z = nn[0] * d0 + nn[1] * d1 + nn[2] * d2;
-  R sx[4], sy[4], r[4], e[4], h[4];
+  for (int c = 0; c < 3; ++c) {
+    T[c] = s[c];
+    T[3 + c] = t[c];
+    T[6 + c] = nn[c];
+  }
+}
+
+constexpr int kGeo = 20;  // a panel's geometry in the near-field adjoint: T (9), qgc (3), lc (8)
+
+// d/d corners from d/d (T, qgc, lc), once per panel: three forward sweeps of four corner
+// coordinates each
+__global__ void __launch_bounds__(64) birk_geometry_adjoint_kernel(int64_t n, const double* __restrict__ V,
+                                                                   const double* __restrict__ geo,
+                                                                   double* __restrict__ gv) {
+  const int64_t j = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / 3;
+  const int chunk = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) % 3);
+  if (j >= n) return;
+  Dn<4> v[12], T[9], q[3], lc[8];
+  for (int e = 0; e < 12; ++e) v[e] = Dn<4>::var(V[12 * j + e], e - 4 * chunk);
+  birk_geometry_t(v, T, q, lc);
+  const double* g = geo + kGeo * j;
+  for (int e = 0; e < 4; ++e) {
+    double a = 0.0;
+    for (int c = 0; c < 9; ++c) a = fma(g[c], T[c].d[e], a);
+    for (int c = 0; c < 3; ++c) a = fma(g[9 + c], q[c].d[e], a);
+    for (int c = 0; c < 8; ++c) a = fma(g[12 + c], lc[c].d[e], a);
+    gv[12 * j + 4 * chunk + e] += a;
+  }
+}
+
+// Reverse mode through birk_phi_and_velocity (mh_greens.cuh): L = A0 s0 + B1 s1 + B2 s2 + B3 s3 of
+// the edge sums s0 (4 pi times the potential) and s1..s3 (the velocity) at the local point
+// (x, y, z).  Returns s1..s3, and the derivatives of L in the point (gp) and the local corners
+// (gl; the edge lengths are functions of them).  In the panel's plane (|z| <= tol) the arc-tangent
+// terms are 0 as in the primal, with the tangent the reference keeps (_zero_primal_keep_tangent,
+// rankine_vectorized.jl:36-37): each moves only with z, at the rate d(vz)/dz of the Birk
+// Hessian (hzz = lambda rsum / (rk rk1 rho), velocity_hessian, rankine_vectorized.jl:200-235),
+// which stays finite where the arc tangent is 0/0 (field point on the line of an edge).
+__device__ inline void birk_reverse(double x, double y, double z, const double* lc, const double* edge, double A0,
+                                    double B1, double B2, double B3, double sum[3], double gp[3], double gl[8]) {
+  double sx[4], sy[4], r[4], e[4], h[4];
+  double gsx[4], gsy[4], gr[4], ge[4], gh[4];
+  const double z2 = z * z;
+#pragma unroll
   for (int k = 0; k < 4; ++k) {
     sx[k] = x - lc[2 * k];
     sy[k] = y - lc[2 * k + 1];
-    r[k] = sqrt(sx[k] * sx[k] + sy[k] * sy[k] + z * z);
-    e[k] = sx[k] * sx[k] + z * z;
+    e[k] = sx[k] * sx[k] + z2;
+    r[k] = fx::sqrt_pos(sy[k] * sy[k] + e[k]);
     h[k] = sx[k] * sy[k];
+    gsx[k] = gsy[k] = gr[k] = ge[k] = gh[k] = 0.0;
+    gl[2 * k] = gl[2 * k + 1] = 0.0;
   }
-  const bool inplane = fabs(val(z)) <= kBirkZTol;
-  R s0(0.0), s1(0.0), s2(0.0), s3(0.0);
+  const bool inplane = fabs(z) <= kBirkZTol;
+  const double W = fma(A0, z, B3);  // adjoint of every arc-tangent term (s0 holds z s3)
+  double s1 = 0.0, s2 = 0.0, s3 = 0.0, gz = 0.0;
+#pragma unroll
   for (int k = 0; k < 4; ++k) {
     const int kn = (k + 1) & 3;
-    R dx = lc[2 * kn] - lc[2 * k];
-    R dy = lc[2 * kn + 1] - lc[2 * k + 1];
-    R dk = hypot(dx, dy);
-    if (!(val(dk) <= kBirkDkTol)) {
-      R rsum = r[k] + r[kn];
-      R log_term = log((rsum - dk) / (rsum + dk));
-      R lt_dk = log_term / dk;
-      R vzk;
-      if (!inplane) {
-        vzk = atan_ratio_t(dy * e[k] - dx * h[k], dx * z * r[k]) - atan_ratio_t(dy * e[kn] - dx * h[kn], dx * z * r[kn]);
-      } else {
-        // In-plane field point (|z| <= tol): value 0 as in the primal, and the tangent the
-        // reference keeps (_zero_primal_keep_tangent, rankine_vectorized.jl:36-37): at z = 0
-        // the atan pair moves only with z, at the rate d(vz)/dz of the Birk Hessian
-        // (hzz = lambda rsum / (rk rk1 rho), velocity_hessian, rankine_vectorized.jl:200-235).
-        // Written this way it stays finite where the atan form is 0/0 (field point on the
-        // line of an edge).
-        const double sxk = val(sx[k]), syk = val(sy[k]), sxn = val(sx[kn]), syn = val(sy[kn]);
-        const double rk = val(r[k]), rn = val(r[kn]), zv = val(z);
-        const double lam = sxk * syn - sxn * syk;
-        const double rho = rk * rn + sxk * sxn + syk * syn + zv * zv;
-        const double rate = (rho > 0.0) ? lam * (rk + rn) / (rk * rn * rho) : 0.0;
-        vzk = (z - zv) * rate;
+    const double dk = edge[k];
+    if (dk <= kBirkDkTol) continue;
+    const double dx = lc[2 * kn] - lc[2 * k], dy = lc[2 * kn + 1] - lc[2 * k + 1];
+    const double rs = r[k] + r[kn], num = rs - dk, inv_sum = fx::recip(rs + dk), inv_d = fx::recip(dk);
+    const double w = num * inv_sum;
+    const double lt = (num > 0.0 ? fx::log_pos(w) : log(w)) * inv_d;
+    const double inv_num = num > 0.0 ? fx::recip(num) : 1.0 / num;
+    const double cl = fma(A0, sx[k] * dy - sy[k] * dx, fma(B1, dy, -(B2 * dx)));  // adjoint of lt
+    s1 = fma(dy, lt, s1);
+    s2 = fma(-dx, lt, s2);
+    gsx[k] = fma(A0 * dy, lt, gsx[k]);
+    gsy[k] = fma(-(A0 * dx), lt, gsy[k]);
+    double gdx = -lt * fma(A0, sy[k], B2), gdy = lt * fma(A0, sx[k], B1);
+    // lt = log((rs - d) / (rs + d)) / d
+    const double den2 = 2.0 * inv_num * inv_sum;
+    gr[k] = fma(cl, den2, gr[k]);
+    gr[kn] = fma(cl, den2, gr[kn]);
+    const double gd = -(cl * inv_d * inv_d) * fma(rs, den2, lt);
+    gdx = fma(gd, dx, gdx);
+    gdy = fma(gd, dy, gdy);
+    if (!inplane) {
+      const double dxz = dx * z;
+      const double N1 = dy * e[k] - dx * h[k], D1 = dxz * r[k];
+      const double N2 = dy * e[kn] - dx * h[kn], D2 = dxz * r[kn];
+      const double n1 = D1 < 0.0 ? -N1 : N1, d1 = fabs(D1), n2 = D2 < 0.0 ? -N2 : N2, d2 = fabs(D2);
+      s3 += fx::atan2_int(n1 * d2 - n2 * d1, d1 * d2 + n1 * n2);
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const int q = c ? kn : k;
+        const double N = c ? N2 : N1, D = c ? D2 : D1;
+        const double m2 = fma(N, N, D * D);
+        const double f = m2 > 0.0 ? (c ? -W : W) * fx::recip(m2) : 0.0;
+        const double gN = f * D, gD = -f * N;
+        gdy = fma(gN, e[q], gdy);
+        ge[q] = fma(gN, dy, ge[q]);
+        gh[q] = fma(-gN, dx, gh[q]);
+        gdx = fma(gD * z, r[q], fma(-gN, h[q], gdx));
+        gz = fma(gD * dx, r[q], gz);
+        gr[q] = fma(gD, dxz, gr[q]);
       }
-      s0 = s0 + ((sx[k] * dy - sy[k] * dx) * lt_dk + z * vzk);
-      s1 = s1 + dy * lt_dk;
-      s2 = s2 - dx * lt_dk;
-      s3 = s3 + vzk;
+    } else {
+      const double lam = sx[k] * sy[kn] - sx[kn] * sy[k];
+      const double rr = r[k] * r[kn], rho = rr + sx[k] * sx[kn] + sy[k] * sy[kn] + z2;
+      if (rho > 0.0) gz = fma(W, lam * rs / (rr * rho), gz);
     }
+    gl[2 * kn] += gdx;
+    gl[2 * k] -= gdx;
+    gl[2 * kn + 1] += gdy;
+    gl[2 * k + 1] -= gdy;
   }
-  R phb = kMinusInv4Pi * s0;
-  R vl0 = kMinusInv4Pi * s1, vl1 = kMinusInv4Pi * s2, vl2 = kMinusInv4Pi * s3;
-  g[0] = kFourPi * (s[0] * vl0 + t[0] * vl1 + nn[0] * vl2);
-  g[1] = kFourPi * (s[1] * vl0 + t[1] * vl1 + nn[1] * vl2);
-  g[2] = kFourPi * (s[2] * vl0 + t[2] * vl1 + nn[2] * vl2);
-  phi = -kFourPi * phb;
-}
-
-// near-field derivatives of (phi, g) w.r.t. the field point (3) and the corners (12):
-// four forward sweeps of 4 directions each
-__device__ void birk_near_jacobian(const double p[3], const double* v12, double dphi[15], double dg[3][15],
-                                   double& phi, double g[3]) {
-  for (int chunk = 0; chunk < 4; ++chunk) {
-    Dn<4> P[3], V[12], ph, G[3];
-    for (int c = 0; c < 3; ++c) P[c] = Dn<4>::var(p[c], c - 4 * chunk);
-    for (int q = 0; q < 12; ++q) V[q] = Dn<4>::var(v12[q], 3 + q - 4 * chunk);
-    birk_near_t(P, V, ph, G);
-    if (chunk == 0) {
-      phi = ph.v;
-      g[0] = G[0].v; g[1] = G[1].v; g[2] = G[2].v;
-    }
-    for (int q = 0; q < 4; ++q) {
-      int slot = 4 * chunk + q;
-      if (slot >= 15) break;
-      dphi[slot] = ph.d[q];
-      for (int c = 0; c < 3; ++c) dg[c][slot] = G[c].d[q];
-    }
+  gz = fma(A0, s3, gz);
+  double gx = 0.0, gy = 0.0;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const double t = r[k] > 0.0 ? gr[k] * fx::recip(r[k]) : 0.0;
+    const double u = fma(2.0, ge[k], t);
+    const double a = fma(gh[k], sy[k], fma(u, sx[k], gsx[k])), b = fma(gh[k], sx[k], fma(t, sy[k], gsy[k]));
+    gz = fma(u, z, gz);
+    gx += a;
+    gy += b;
+    gl[2 * k] -= a;
+    gl[2 * k + 1] -= b;
   }
+  sum[0] = s1;
+  sum[1] = s2;
+  sum[2] = s3;
+  gp[0] = gx;
+  gp[1] = gy;
+  gp[2] = gz;
 }
 
 // sum of NV values over the CTA's threads (thread 0 gets the total)
@@ -301,94 +371,192 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double* red /*NV * 4*
 // source gradient of the panel integral at the field point (or its image).  Indirect: the
 // field-point gradient of the same integral, -M g (M = diag(1, 1, -1) for the image point),
 // with the field panel's normal: D = a (nv . g), nv = -M n_i.
+//
+// A CTA takes 128 rows by kCols columns.  Far terms (beyond 7 radii) go thread by thread, their
+// column sums through a tile in shared memory.  Near terms are listed column by column and
+// taken densely, 128 at a time, in reverse mode: the derivative of one scalar in the 23
+// quantities of the panel's frame, centroid, local corners and normal, about 600 FP64
+// instructions.  The corners follow from the frame once per panel
+// (birk_geometry_adjoint_kernel).  Forward duals per pair (15 inputs in four sweeps of the whole
+// geometry, some 14000 FP64 instructions paid by every warp that holds one near pair) took
+// 21.6 ms for 1400 panels; now 0.5 ms.  Bound: the FP64 pipe.
 // ---------------------------------------------------------------------------
+constexpr int kNearVals = kGeo + 3;      // geometry and source normal
+constexpr int kTileLd = kRows + 1;       // odd: the column sums read down a column
+constexpr int kStaticAdjSmem = 8 * kTileLd * (7 * kCols > kNearVals ? 7 * kCols : kNearVals);
+
 template <bool DIRECT>
 __global__ void __launch_bounds__(kRows) static_adjoint_kernel(AssemblyParams p, const double* __restrict__ RS,
-                                                               const double* __restrict__ RD, GradPtrs gp) {
+                                                               const double* __restrict__ RD, GradPtrs gp,
+                                                               double* __restrict__ geo) {
+  extern __shared__ double tile[];       // far: [7 kCols][kTileLd]; near: [kNearVals][kTileLd]
   __shared__ PanelRec sp[kCols];
-  __shared__ double red[19 * 4];
+  __shared__ double near2[kCols][2];     // (7 radius)^2 less / more four roundings
+  __shared__ unsigned short todo[2 * kCols * kRows];  // image << 10 | column << 7 | row, by column
+  __shared__ int cnt[2 * kCols][kRows / 32];          // near terms per (column, image) and warp, then offsets
+  __shared__ int cstart[kCols + 1];
   const int64_t n = p.n;
   const int64_t i0 = blockIdx.x * (int64_t)kRows;
   const int64_t i = i0 + threadIdx.x;
   const int64_t j0 = blockIdx.y * (int64_t)kCols;
   const int ncol = (int)((n - j0) < kCols ? (n - j0) : kCols);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   {
     const double2* src = reinterpret_cast<const double2*>(p.P + j0);
     double2* dst = reinterpret_cast<double2*>(sp);
     for (int q = threadIdx.x; q < ncol * 16; q += blockDim.x) dst[q] = src[q];
   }
   __syncthreads();
+  if (threadIdx.x < ncol) {
+    const double t = 7 * sp[threadIdx.x].radius, t2 = t * t;
+    near2[threadIdx.x][0] = t2 * (1.0 - 0x1p-50);
+    near2[threadIdx.x][1] = t2 * (1.0 + 0x1p-50);
+  }
+  __syncthreads();
   const bool active = i < n;
   double ci[3] = {0, 0, 0}, ni[3] = {0, 0, 0};
   if (active)
     for (int c = 0; c < 3; ++c) { ci[c] = p.P[i].c[c]; ni[c] = p.P[i].n[c]; }
-  const bool need_R = (p.gfs & MH_GF_RANKINE) != 0;
-  const bool need_I = (p.gfs & (MH_GF_RANKINE_REFLECTED | MH_GF_RANKINE_REFLECTED_NEGATIVE)) != 0;
+  const bool need[2] = {(p.gfs & MH_GF_RANKINE) != 0,
+                        (p.gfs & (MH_GF_RANKINE_REFLECTED | MH_GF_RANKINE_REFLECTED_NEGATIVE)) != 0};
   const double image_sign = ((p.gfs & MH_GF_RANKINE_REFLECTED) ? 1.0 : 0.0) -
                             ((p.gfs & MH_GF_RANKINE_REFLECTED_NEGATIVE) ? 1.0 : 0.0);
   double gci[3] = {0, 0, 0}, gni[3] = {0, 0, 0};
+  unsigned near_mask = 0;  // bit 2 column + image
   for (int jj = 0; jj < ncol; ++jj) {
-    const int64_t j = j0 + jj;
     const PanelRec& Pj = sp[jj];
-    // column accumulators: gc_j (3), gn_j (3), ga_j (1), gv_j (12)
-    double col[19];
-#pragma unroll
-    for (int q = 0; q < 19; ++q) col[q] = 0.0;
+    // column terms: gc_j (3), gn_j (3), ga_j (1)
+    double col[7] = {0, 0, 0, 0, 0, 0, 0};
     if (active) {
-      const double ws = RS[i + j * n], wd = RD[i + j * n];
+      const double ws = RS[i + (j0 + jj) * n], wd = RD[i + (j0 + jj) * n];
+      const double rx = ci[0] - Pj.c[0], ry = ci[1] - Pj.c[1], h2 = rx * rx + ry * ry;
+#pragma unroll
       for (int img = 0; img < 2; ++img) {
-        if (img == 0 && !need_R) continue;
-        if (img == 1 && !need_I) continue;
-        const double sgn = img ? image_sign : 1.0;
-        const double pt[3] = {ci[0], ci[1], img ? -ci[2] : ci[2]};
+        if (!need[img]) continue;
         const double zf = img ? -1.0 : 1.0;  // d pt / d ci_z
-        const double a = kMinusInv4Pi * sgn;
+        const double rz = (img ? -ci[2] : ci[2]) - Pj.c[2];
+        const double r2 = h2 + rz * rz;
+        bool far = r2 > near2[jj][1];
+        if (!far && r2 >= near2[jj][0]) far = sqrt(r2) > 7 * Pj.radius;
+        if (!far) {
+          near_mask |= 1u << (2 * jj + img);
+          continue;
+        }
+        const double a = img ? kMinusInv4Pi * image_sign : kMinusInv4Pi;
         double nv[3];
         if (DIRECT) { nv[0] = Pj.n[0]; nv[1] = Pj.n[1]; nv[2] = Pj.n[2]; }
-        else { nv[0] = -ni[0]; nv[1] = -ni[1]; nv[2] = -zf * ni[2]; }
-        double rb[3] = {pt[0] - Pj.c[0], pt[1] - Pj.c[1], pt[2] - Pj.c[2]};
-        double r = sqrt(rb[0] * rb[0] + rb[1] * rb[1] + rb[2] * rb[2]);
-        double g[3];  // source gradient of the integral (far field: A rb / r^3)
-        if (r > 7 * Pj.radius) {
-          // S = a A/r ; D = a A (nv . rb)/r^3
-          const double r3 = r * r * r, r5 = r3 * r * r, A = Pj.area;
-          const double nr = nv[0] * rb[0] + nv[1] * rb[1] + nv[2] * rb[2];
-          for (int c = 0; c < 3; ++c) {
-            const double dS = a * A * (-rb[c] / r3);
-            const double dD = a * A * (nv[c] / r3 - 3.0 * nr * rb[c] / r5);
-            const double gtot = ws * dS + wd * dD;  // d/d pt_c
-            gci[c] += (c == 2 ? zf : 1.0) * gtot;
-            col[c] -= gtot;  // d/d c_j = - d/d pt
-            g[c] = A * rb[c] / r3;
-          }
-          col[6] += ws * a / r + wd * a * nr / r3;  // d/d A_j
-        } else {
-          double dphi[15], dg[3][15], phi;
-          birk_near_jacobian(pt, p.V + 12 * j, dphi, dg, phi, g);
-          for (int q = 0; q < 15; ++q) {
-            const double dS = a * dphi[q];
-            const double dD = a * (nv[0] * dg[0][q] + nv[1] * dg[1][q] + nv[2] * dg[2][q]);
-            const double gtot = ws * dS + wd * dD;
-            if (q < 3) gci[q] += (q == 2 ? zf : 1.0) * gtot;
-            else col[7 + (q - 3)] += gtot;
-          }
-        }
-        // d/d normal: the source's (direct) or the field panel's through nv = -M n_i (indirect)
+        else { nv[0] = -ni[0]; nv[1] = -ni[1]; nv[2] = img ? ni[2] : -ni[2]; }
+        // S = a A / r, D = a A (nv . rb) / r^3
+        const double rb[3] = {rx, ry, rz};
+        const double ir = fx::rsqrt_pos(r2), ir2 = ir * ir, q = a * Pj.area * ir * ir2;
+        const double nr = (nv[0] * rx + nv[1] * ry + nv[2] * rz) * ir2;
+        const double f = fma(3.0 * wd, nr, ws);
         for (int c = 0; c < 3; ++c) {
-          if (DIRECT) col[3 + c] += wd * a * g[c];
-          else gni[c] -= wd * a * (c == 2 ? zf : 1.0) * g[c];
+          const double gtot = q * (wd * nv[c] - f * rb[c]);  // d/d pt_c
+          gci[c] += (c == 2 ? zf : 1.0) * gtot;
+          col[c] -= gtot;
+        }
+        col[6] += a * ir * fma(wd, nr, ws);  // d/d A_j
+        const double wq = wd * q;
+        for (int c = 0; c < 3; ++c) {
+          if (DIRECT) col[3 + c] += wq * rb[c];
+          else gni[c] -= wq * (c == 2 ? zf : 1.0) * rb[c];
         }
       }
     }
-    block_sum<19>(col, red);
-    if (threadIdx.x == 0) {
-      for (int c = 0; c < 3; ++c) {
-        atomicAdd(gp.gc + 3 * j + c, col[c]);
-        atomicAdd(gp.gn + 3 * j + c, col[3 + c]);
-      }
-      atomicAdd(gp.ga + j, col[6]);
-      for (int q = 0; q < 12; ++q) atomicAdd(gp.gv + 12 * j + q, col[7 + q]);
+    for (int c = 0; c < 7; ++c) tile[(7 * jj + c) * kTileLd + threadIdx.x] = col[c];
+  }
+  // near terms per column, image and warp
+  for (int b = 0; b < 2 * kCols; ++b) {
+    const unsigned m = __ballot_sync(0xffffffffu, (near_mask >> b) & 1u);
+    if (lane == 0) cnt[b][warp] = __popc(m);
+  }
+  __syncthreads();
+  // column sums of the far terms, two threads each
+  for (int t = threadIdx.x; t < 2 * 7 * ncol; t += kRows) {
+    const int v = t >> 1;
+    const double* src = tile + v * kTileLd + (t & 1) * (kRows / 2);
+    double a = 0.0, b = 0.0;
+    for (int q = 0; q < kRows / 2; q += 2) {
+      a += src[q];
+      b += src[q + 1];
     }
+    a += b;
+    const int64_t j = j0 + v / 7;
+    const int c = v % 7;
+    atomicAdd(c < 3 ? gp.gc + 3 * j + c : (c < 6 ? gp.gn + 3 * j + c - 3 : gp.ga + j), a);
+  }
+  if (threadIdx.x == 0) {
+    int base = 0;
+    for (int b = 0; b < 2 * kCols; ++b) {
+      if ((b & 1) == 0) cstart[b >> 1] = base;
+      for (int w = 0; w < kRows / 32; ++w) {
+        const int c = cnt[b][w];
+        cnt[b][w] = base;
+        base += c;
+      }
+    }
+    cstart[kCols] = base;
+  }
+  __syncthreads();
+  for (int b = 0; b < 2 * kCols; ++b) {
+    const bool mine = (near_mask >> b) & 1u;
+    const unsigned m = __ballot_sync(0xffffffffu, mine);
+    if (mine)
+      todo[cnt[b][warp] + __popc(m & ((1u << lane) - 1u))] =
+          (unsigned short)((b & 1) << 10 | (b >> 1) << 7 | (int)threadIdx.x);
+  }
+  __syncthreads();
+  const int total = cstart[kCols];
+  for (int base = 0; base < total; base += kRows) {
+    const int q = base + threadIdx.x;
+    if (q < total) {
+      const int ent = todo[q], img = ent >> 10, jj = (ent >> 7) & 7, row = ent & 127;
+      const PanelRec& Pj = sp[jj];
+      const PanelRec& Pi = p.P[i0 + row];
+      const int64_t idx = i0 + row + (j0 + jj) * n;
+      const double zf = img ? -1.0 : 1.0, a = img ? kMinusInv4Pi * image_sign : kMinusInv4Pi;
+      const double ws = a * RS[idx], wd = a * RD[idx];
+      double nv[3];
+      for (int c = 0; c < 3; ++c) nv[c] = DIRECT ? Pj.n[c] : -(c == 2 ? zf : 1.0) * __ldg(&Pi.n[c]);
+      const double d[3] = {__ldg(&Pi.c[0]) - Pj.qgc[0], __ldg(&Pi.c[1]) - Pj.qgc[1],
+                           zf * __ldg(&Pi.c[2]) - Pj.qgc[2]};
+      const double* T = Pj.T;
+      double loc[3], nl[3];
+      for (int c = 0; c < 3; ++c) {
+        loc[c] = T[3 * c] * d[0] + T[3 * c + 1] * d[1] + T[3 * c + 2] * d[2];
+        nl[c] = T[3 * c] * nv[0] + T[3 * c + 1] * nv[1] + T[3 * c + 2] * nv[2];
+      }
+      // S = a s0, D = a (nv . g) with g = -(s s1 + t s2 + n s3)
+      double sum[3], gl3[3], gl[8];
+      birk_reverse(loc[0], loc[1], loc[2], Pj.lc, Pj.edge, ws, -wd * nl[0], -wd * nl[1], -wd * nl[2], sum, gl3, gl);
+      double* out = tile + threadIdx.x;
+      for (int c = 0; c < 3; ++c)
+        for (int x = 0; x < 3; ++x) out[(3 * c + x) * kTileLd] = fma(gl3[c], d[x], -(wd * sum[c]) * nv[x]);
+      for (int x = 0; x < 3; ++x) {
+        const double gx = T[x] * gl3[0] + T[3 + x] * gl3[1] + T[6 + x] * gl3[2];  // d/d pt
+        const double wg = -wd * (T[x] * sum[0] + T[3 + x] * sum[1] + T[6 + x] * sum[2]);  // d/d nv
+        out[(9 + x) * kTileLd] = -gx;
+        out[(kGeo + x) * kTileLd] = DIRECT ? wg : 0.0;
+        atomicAdd(gp.gc + 3 * (i0 + row) + x, x == 2 ? zf * gx : gx);
+        if (!DIRECT) atomicAdd(gp.gn + 3 * (i0 + row) + x, -(x == 2 ? zf : 1.0) * wg);
+      }
+      for (int c = 0; c < 8; ++c) out[(12 + c) * kTileLd] = gl[c];
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < kNearVals * ncol; t += kRows) {
+      const int v = t % kNearVals, jj = t / kNearVals;
+      const int q0 = max(cstart[jj], base) - base, q1 = min(cstart[jj + 1], base + kRows) - base;
+      if (q0 >= q1 || (!DIRECT && v >= kGeo)) continue;
+      double s0 = 0.0, s1 = 0.0;
+      for (int e = q0; e < q1; ++e) {
+        if (e & 1) s1 += tile[v * kTileLd + e];
+        else s0 += tile[v * kTileLd + e];
+      }
+      const int64_t j = j0 + jj;
+      atomicAdd(v < kGeo ? geo + kGeo * j + v : gp.gn + 3 * j + v - kGeo, s0 + s1);
+    }
+    __syncthreads();
   }
   if (active)
     for (int c = 0; c < 3; ++c) {
@@ -447,7 +615,7 @@ struct PairGrad {
   double gcf[3], gcs[3], gns[3], gas;
 };
 
-__device__ void wave_pair_grad(double k, double dx, double dy, double dis, double as, const double ns[3],
+__device__ void wave_pair_grad(double k, double dx, double dy, double dis, double inv_dis, double as, const double ns[3],
                                const CR<Dn<2>>& GF, const CR<Dn<2>>& Gh, const CR<Dn<2>>& Gv, double2 WS,
                                double2 WD, PairGrad& o) {
   const double sc = kMinusInv4Pi;
@@ -459,7 +627,7 @@ __device__ void wave_pair_grad(double k, double dx, double dy, double dis, doubl
   const double2 Ghx = make_double2(Gh.x.v, Gh.y.v), Gvx = make_double2(Gv.x.v, Gv.y.v);
   const double2 GFx = make_double2(GF.x.v, GF.y.v);
   const bool horiz = fabs(hh) > 1e-6;      // the primal zeroes the horizontal term below
-  const double ux = horiz ? dx / dis : 0.0, uy = horiz ? dy / dis : 0.0;
+  const double ux = horiz ? dx * inv_dis : 0.0, uy = horiz ? dy * inv_dis : 0.0;
   const double u = ns[0] * ux + ns[1] * uy;
   const double k2 = k * k;
   // S
@@ -478,8 +646,8 @@ __device__ void wave_pair_grad(double k, double dx, double dy, double dis, doubl
   // du / d(dx, dy)
   double du_dx = 0.0, du_dy = 0.0;
   if (horiz) {
-    du_dx = (ns[0] - u * ux) / dis;
-    du_dy = (ns[1] - u * uy) / dis;
+    du_dx = (ns[0] - u * ux) * inv_dis;
+    du_dy = (ns[1] - u * uy) * inv_dis;
   }
   // dhh / d(dx, dy).  hh = k |(dx, dy)| has a kink at dis = 0; inside the band where the
   // primal treats the pair as vertically aligned (hh <= 1e-6, which also catches centres
@@ -560,7 +728,8 @@ __global__ void __launch_bounds__(kRows) wave_adjoint_kernel(AssemblyParams p, d
         egd_terms_from_values(gv[2 * q], gv[2 * q + 1], hh, vv, GF, Gh, Gv);
       }
       const double dx = Pj.c[0] - ci[0], dy = Pj.c[1] - ci[1];
-      const double dis = sqrt(dx * dx + dy * dy);
+      const double dis = fx::sqrt_pos(dx * dx + dy * dy);
+      const double inv_dis = dis > 0.0 ? fx::recip(dis) : 0.0;
       // weights of (i, j) and (j, i)
       double2 WSij = make_double2(0, 0), WDij = WSij, WSji = WSij, WDji = WSij;
       for (int h = 0; h < w.nh; ++h) {
@@ -575,20 +744,20 @@ __global__ void __launch_bounds__(kRows) wave_adjoint_kernel(AssemblyParams p, d
       WDji = cmulz(cD, WDji);
       PairGrad g1;  // field i, source j
       if (DIRECT) {
-        wave_pair_grad(k, dx, dy, dis, Pj.area, Pj.n, GF, Gh, Gv, WSij, WDij, g1);
+        wave_pair_grad(k, dx, dy, dis, inv_dis, Pj.area, Pj.n, GF, Gh, Gv, WSij, WDij, g1);
         for (int c = 0; c < 3; ++c) { gci[c] += g1.gcf[c]; col[c] += g1.gcs[c]; col[3 + c] += g1.gns[c]; }
       } else {
-        wave_pair_grad(k, -dx, -dy, dis, Pj.area, ni, GF, Gh, Gv, WSij, WDij, g1);
+        wave_pair_grad(k, -dx, -dy, dis, inv_dis, Pj.area, ni, GF, Gh, Gv, WSij, WDij, g1);
         for (int c = 0; c < 3; ++c) { gci[c] += g1.gcs[c]; col[c] += g1.gcf[c]; gni[c] += g1.gns[c]; }
       }
       col[6] += g1.gas;
       if (i != j) {
         PairGrad g2;  // field j, source i
         if (DIRECT) {
-          wave_pair_grad(k, -dx, -dy, dis, ai, ni, GF, Gh, Gv, WSji, WDji, g2);
+          wave_pair_grad(k, -dx, -dy, dis, inv_dis, ai, ni, GF, Gh, Gv, WSji, WDji, g2);
           for (int c = 0; c < 3; ++c) { col[c] += g2.gcf[c]; gci[c] += g2.gcs[c]; gni[c] += g2.gns[c]; }
         } else {
-          wave_pair_grad(k, dx, dy, dis, ai, Pj.n, GF, Gh, Gv, WSji, WDji, g2);
+          wave_pair_grad(k, dx, dy, dis, inv_dis, ai, Pj.n, GF, Gh, Gv, WSji, WDji, g2);
           for (int c = 0; c < 3; ++c) { col[c] += g2.gcs[c]; gci[c] += g2.gcf[c]; col[3 + c] += g2.gns[c]; }
         }
         gai += g2.gas;
@@ -899,15 +1068,21 @@ __global__ void conj_kernel(int64_t count, double2* __restrict__ x) {
 
 }  // namespace
 
+int64_t static_adjoint_work(int64_t n) { return kGeo * n; }
+
 void launch_static_adjoint(cudaStream_t st, LaunchCounter lc, const AssemblyParams& p, const double* RS,
-                           const double* RD, double* gc, double* gn, double* ga, double* gv) {
+                           const double* RD, double* gc, double* gn, double* ga, double* gv, double* work) {
   dim3 grid((unsigned)((p.n + kRows - 1) / kRows), (unsigned)((p.n + kCols - 1) / kCols));
+  cudaMemsetAsync(work, 0, sizeof(double) * kGeo * p.n, st);
+  cudaFuncSetAttribute(static_adjoint_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStaticAdjSmem);
+  cudaFuncSetAttribute(static_adjoint_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStaticAdjSmem);
+  const GradPtrs gp{gc, gn, ga, gv};
   if (p.direct)
-    MH_LAUNCH(lc, st, "adjoint_static",
-              static_adjoint_kernel<true><<<grid, kRows, 0, st>>>(p, RS, RD, GradPtrs{gc, gn, ga, gv}));
+    MH_LAUNCH(lc, st, "adjoint_static", static_adjoint_kernel<true><<<grid, kRows, kStaticAdjSmem, st>>>(p, RS, RD, gp, work));
   else
-    MH_LAUNCH(lc, st, "adjoint_static",
-              static_adjoint_kernel<false><<<grid, kRows, 0, st>>>(p, RS, RD, GradPtrs{gc, gn, ga, gv}));
+    MH_LAUNCH(lc, st, "adjoint_static", static_adjoint_kernel<false><<<grid, kRows, kStaticAdjSmem, st>>>(p, RS, RD, gp, work));
+  MH_LAUNCH(lc, st, "adjoint_geometry",
+            birk_geometry_adjoint_kernel<<<(unsigned)((3 * p.n + 63) / 64), 64, 0, st>>>(p.n, p.V, work, gv));
 }
 
 void launch_wave_adjoint(cudaStream_t st, LaunchCounter lc, const AssemblyParams& p, double k, const double2* lS,

@@ -78,7 +78,7 @@ int hydro_vjp_core(mh_context* ctx, mh_mesh* m, int64_t n_omega, const double* o
   MH_TRY(ws_get_t(ctx, kSlotCw, (size_t)(ni * ncol * n_omega), &cw));  // not kSlotNorm: the refinement owns it
   MH_TRY(ws_get_t(ctx, kSlotIpiv, (size_t)(ipiv_stride(n) * chunk), &ipiv));
   MH_TRY(ws_get_t(ctx, kSlotInfo, (size_t)chunk, &info));
-  MH_TRY(ws_get_t(ctx, kSlotGrad, (size_t)((19 + 3 * n_dofs) * n), &grad));
+  MH_TRY(ws_get_t(ctx, kSlotGrad, (size_t)((19 + 3 * n_dofs) * n + static_adjoint_work(n)), &grad));
   void* oz_ws = nullptr;  // FP64 LU update on the tensor cores (MH_PREC_FP64_TC)
   int* oz_flag = nullptr;
   if (precision == MH_PREC_FP64_TC) {
@@ -226,7 +226,7 @@ int hydro_vjp_core(mh_context* ctx, mh_mesh* m, int64_t n_omega, const double* o
   }
   MH_CUDA(ctx, cudaMemcpyAsync(hF.data(), F, sizeof(double2) * hF.size(), cudaMemcpyDeviceToHost, st));
   if (nb) MH_CUDA(ctx, cudaMemcpyAsync(hFK.data(), FK, sizeof(double2) * hFK.size(), cudaMemcpyDeviceToHost, st));
-  if (stk) launch_static_adjoint(st, lc, pst, RS, RD, gc, gn, ga, gv);
+  if (stk) launch_static_adjoint(st, lc, pst, RS, RD, gc, gn, ga, gv, grad + (19 + 3 * n_dofs) * n);
   MH_TRY(check_launch(ctx, "static adjoint"));
   MH_TRY(sync(ctx, "forces"));
   if (oz_flag) {

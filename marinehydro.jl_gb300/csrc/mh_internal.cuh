@@ -264,8 +264,10 @@ void launch_forces(cudaStream_t st, LaunchCounter lc, const EpilogueGeom& g, int
                    double2* FK /*nw x n_inf x n_beta*/);
 
 // adjoint (mh_adjoint.cu)
+// (work: static_adjoint_work(n) doubles)
+int64_t static_adjoint_work(int64_t n);
 void launch_static_adjoint(cudaStream_t st, LaunchCounter lc, const AssemblyParams& p, const double* RS,
-                           const double* RD, double* gc, double* gn, double* ga, double* gv);
+                           const double* RD, double* gc, double* gn, double* ga, double* gv, double* work);
 // weights W^S = c lS rS^T, W^D = -c lD rD^T (n x nh each); egd_values: the packed exact
 // values of launch_egd_pair_values at k when p.gfs holds MH_GF_EXACT_DELHOMMEAU
 void launch_wave_adjoint(cudaStream_t st, LaunchCounter lc, const AssemblyParams& p, double k, const double2* lS,
