@@ -28,6 +28,7 @@
 #include <climits>
 #include <cmath>
 #include <initializer_list>
+#include <type_traits>
 
 #include "mh_fixpoint.cuh"
 #include "mh_internal.cuh"
@@ -183,16 +184,17 @@ constexpr int kPanelMaxCtas = 16;  // largest cluster (above 8 CTAs it is a non-
 // panel rows one CTA of a cluster of P holds in shared memory: 32 complex columns each, and the
 // candidate rows of two columns and P CTAs, below 227 KB
 template <typename T> __host__ __device__ constexpr int panel_rows(int P) {
-  return sizeof(T) == 8 ? (P <= 8 ? 430 : 414) : 864;
+  return sizeof(T) == 8 ? (P <= 8 ? 430 : 414) : 800;
 }
 // rows per CTA of a panel of m rows on P CTAs: a multiple of 32 where `cap` allows
 __host__ __device__ inline int panel_chunk(int64_t m, int P, int cap) {
   const int64_t c = ((m + P - 1) / P + 31) / 32 * 32;
   return (int)(c < cap ? c : cap);
 }
-// dynamic shared memory of the panel kernel: the chunk (odd leading dimension) and the slots
+// dynamic shared memory of the panel kernel: the chunk (odd leading dimension), the slots, and in
+// FP32 two copies of a column
 template <typename T> constexpr size_t panel_smem_bytes(int chunk, int width, int P) {
-  return 2 * sizeof(T) * ((size_t)(chunk | 1) * width + 2 * (size_t)P * kNB);
+  return 2 * sizeof(T) * ((size_t)(chunk | 1) * width + 2 * (size_t)P * kNB + (sizeof(T) == 8 ? 0 : 2 * (size_t)chunk));
 }
 
 // Pivot candidates compare |re| + |im| through the bit pattern of the (non-negative) value as
@@ -237,24 +239,35 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 // split into chunks of `chunk` rows (a multiple of 32, so that no warp of the update is left
 // part empty; CTA 0 holds the kb <= 32 diagonal rows), one per CTA, in its shared memory with
 // an odd leading dimension (a row's entries then sit in different banks).  Per column j:
-//   every CTA finds its best candidate and pushes it, with a copy of its row, into a slot of
-//   every CTA of the cluster (distributed shared memory stores); CTA 0 pushes row j;
-//   cluster barrier; warp 0 of every CTA picks the winner among the P slots, now local, and
-//   takes the pivot's reciprocal; CTA barrier
-//   a thread per row forms the multipliers l (the interchanged row's from the copy of row j);
-//   CTA barrier
-//   the rank-1 update, in items of 32 rows by a few columns dealt to all 16 warps, column
-//   j + 1 first, which is searched as it is updated.
-// What bounds it: for few rows the chain of barriers and reductions, for many the FP64 pipe
-// (124 FMAs per row at j = 0, two per clock and SM).  A warp issues to one of the SM's four
-// FP64 pipes, so the update goes by items and not by one thread per row (that left three pipes
-// idle for 32 rows, and a fifth of the time at 400); pushing saves the two remote reads of
-// the pull form, warp-wide integer reductions the shuffles.  Per 32-column panel on a GB300,
-// launch included: 200 rows 142 -> 82 us, five matrices of 1000 rows 165 -> 105 us, one of 3000
-// rows (16 CTAs instead of 8) 210 -> 146 us.
+//   warp q < P pushes this CTA's candidate (key, row number, reciprocal, a copy of its row) into
+//   CTA q's slot (distributed shared memory stores); CTA 0 pushes row j; cluster barrier; every
+//   warp picks the winner among the P slots, now local;
+//   FP64: a thread per row forms the multipliers l (the interchanged row's from the copy of
+//   row j); CTA barrier.  FP32: every item of the update forms its own, from a copy of the
+//   column;
+//   column j + 1 is updated and searched first, by warps 0 .. 14; then they take the rest of the
+//   rank-1 update in items of 32 rows by a few columns while warp 15 merges their candidates
+//   and takes the reciprocal of this CTA's; CTA barrier.
+// What bounds it: for few rows the chain of barriers, reductions and the reciprocal, for many
+// the FP64 pipe (124 FMAs per row at j = 0, two per clock and SM).  A warp issues to one of the
+// SM's four FP64 pipes, so the update goes by items and not by one thread per row (that left
+// three pipes idle for 32 rows, and a fifth of the time at 400).  Cycles per column, before -> now
+// (before: one warp pushed to all CTAs, 500 to 850; the reciprocal was taken on every CTA after
+// the barrier, 850 in FP64 and 330 in FP32, now under the update; FP32 scaled in a pass of its own,
+// 415; items of four and eight columns were too few for the warps, 2115 and 1190 for the update
+// of 32 rows): FP64 200 rows 5290 -> 4590, five matrices of 1000 7080 -> 6170, 3000 12080 -> 10350;
+// FP32 430 rows 3290 -> 2390, 1400 3890 -> 3160, 8000 5900 -> 5740.  Measured and dropped: fewer FP64
+// operations in the reciprocal, and fewer warps on the FP64 pipe beside it (4730 and 4890 at 200
+// rows: the reciprocal's chain is bound by its instructions' latency, not by the pipe).
 // Slots of parity j are written again at column j + 2, after the barrier of column j + 1, which
 // every CTA reaches only when it is done reading column j's.
-template <typename T> struct PanelItem { static constexpr int cols = sizeof(T) == 8 ? 4 : 8; };
+constexpr int kItemWarps = kPanelThreads / 32 - 1;  // the last warp merges and takes the reciprocal
+__device__ __forceinline__ void bar_arrive(int id, int threads) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void bar_sync(int id, int threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
 template <typename T>
 __global__ void __launch_bounds__(kPanelThreads) panel_cluster_kernel(BatchDesc d, typename cplx_t<T>::type* __restrict__ Aall,
                                                                      int32_t* __restrict__ ipiv_all,
@@ -262,7 +275,8 @@ __global__ void __launch_bounds__(kPanelThreads) panel_cluster_kernel(BatchDesc 
                                                                      int chunk_cap, int width) {
   using C = typename cplx_t<T>::type;
   using K = typename PivotKey<T>::type;
-  constexpr int kWarps = kPanelThreads / 32, GC = PanelItem<T>::cols;
+  constexpr int kWarps = kPanelThreads / 32;
+  constexpr bool kScaleApart = sizeof(T) == 8;  // multipliers formed once per row (FP64 work is dear)
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   extern __shared__ __align__(16) unsigned char panel_smem[];
@@ -271,12 +285,14 @@ __global__ void __launch_bounds__(kPanelThreads) panel_cluster_kernel(BatchDesc 
   __shared__ C pub_j[2][kNB];                          // row j
   __shared__ K cand_v[2][kPanelMaxCtas];
   __shared__ int cand_i[2][kPanelMaxCtas];
-  __shared__ C urow[kNB], jrow[kNB];
+  __shared__ C cand_inv[2][kPanelMaxCtas];
   __shared__ K red_v[kWarps];
   __shared__ int red_i[kWarps];
-  __shared__ int s_piv;
+  __shared__ K s_key;
+  __shared__ int s_row;
   __shared__ C s_inv;
   const int P = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  C* acol = slots + 2 * P * kNB;  // FP32: column j as the previous update left it [parity][chunk]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t bmat = blockIdx.y, n = d.order(bmat);
   if (k >= n) return;  // a grouped batch: this matrix is factored (the whole cluster leaves)
@@ -303,86 +319,128 @@ __global__ void __launch_bounds__(kPanelThreads) panel_cluster_kernel(BatchDesc 
     const int i = q * 32 + lane;
     if (i < rows) {
       const C a = sp[i];
+      if (!kScaleApart) acol[i] = a;
       argmax_merge(best, bi, PivotKey<T>::of(fabs(a.x) + fabs(a.y)), r0 + i);
     }
   }
+  warp_argmax(best, bi);
+  if (lane == 0) { red_v[warp] = best; red_i[warp] = bi; }
+  __syncthreads();
+  // warp 15: this CTA's candidate in column c, from the `w` warps that searched it
+  auto publish = [&](int c, int w) {
+    K v = lane < w ? red_v[lane] : (K)0;
+    int vi = lane < w ? red_i[lane] : INT_MAX;
+    warp_argmax(v, vi);
+    C inv = czero<C>();
+    if (v != 0) inv = crecip(sp[c * ld + (vi - r0)]);
+    if (lane == 0) { s_key = v; s_row = vi; s_inv = inv; }
+  };
+  if (warp == kItemWarps) publish(0, kWarps);
+  // the update's items: nrb of column j + 1, then (column group g, row block rb) in turn, item q
+  // to warp q % kItemWarps; this warp's first item past column j + 1, and its step
+  const int searchers = nrb < kItemWarps ? nrb : kItemWarps;
+  const int qb = nrb > 0 ? ((nrb - warp + kItemWarps - 1) / kItemWarps * kItemWarps + warp - nrb) : 0;
+  const int first = nrb > warp ? qb : warp - nrb;
+  const int g0 = nrb > 0 ? first / nrb : 0, rb0 = nrb > 0 ? first - g0 * nrb : 0;
+  const int dg = nrb > 0 ? kItemWarps / nrb : 0, drb = nrb > 0 ? kItemWarps - dg * nrb : 0;
   cluster_wait();
   for (int j = 0; j < kb; ++j) {
     const int par = j & 1;
-    warp_argmax(best, bi);
-    if (lane == 0) { red_v[warp] = best; red_i[warp] = bi; }
     __syncthreads();
-    if (warp == 0) {
-      best = lane < kWarps ? red_v[lane] : (K)0;
-      bi = lane < kWarps ? red_i[lane] : INT_MAX;
-      warp_argmax(best, bi);
-      const bool have = bi != INT_MAX;
-      C row = czero<C>(), rj = czero<C>();
-      if (have && lane < kb) row = sp[lane * ld + (bi - r0)];
-      if (rank == 0 && lane < kb) rj = sp[lane * ld + j];
+    if (warp < P) {
+      const int li = s_row - r0;
       C* slot = slots + (par * P + rank) * kNB + lane;
-      for (int q = 0; q < P; ++q) {
-        if (have && lane < kb) *cl.map_shared_rank(slot, (unsigned)q) = row;
-        if (rank == 0 && lane < kb) *cl.map_shared_rank(&pub_j[par][lane], (unsigned)q) = rj;
-      }
-      if (lane < P) {
-        *cl.map_shared_rank(&cand_v[par][rank], (unsigned)lane) = best;
-        *cl.map_shared_rank(&cand_i[par][rank], (unsigned)lane) = bi;
+      if (s_row != INT_MAX && lane < kb) *cl.map_shared_rank(slot, (unsigned)warp) = sp[lane * ld + li];
+      if (rank == 0 && lane < kb) *cl.map_shared_rank(&pub_j[par][lane], (unsigned)warp) = sp[lane * ld + j];
+      if (lane == 0) {
+        *cl.map_shared_rank(&cand_v[par][rank], (unsigned)warp) = s_key;
+        *cl.map_shared_rank(&cand_i[par][rank], (unsigned)warp) = s_row;
+        *cl.map_shared_rank(&cand_inv[par][rank], (unsigned)warp) = s_inv;
       }
     }
     cluster_arrive();
     cluster_wait();
-    if (warp == 0) {
-      K v = lane < P ? cand_v[par][lane] : (K)0;
-      int vi = lane < P ? cand_i[par][lane] : INT_MAX;
-      warp_argmax(v, vi);
-      const bool zero = v == 0;
-      const int p = zero ? j : vi;  // panel row of the pivot
-      if (lane < kb) {
-        const C rj = pub_j[par][lane];
-        const C u = (p == j) ? rj : slots[(par * P + p / chunk) * kNB + lane];
-        urow[lane] = u;
-        jrow[lane] = rj;
-        if (lane == j) s_inv = zero ? czero<C>() : crecip(u);
-      }
-      if (lane == 0) {
-        s_piv = p;
-        if (rank == 0) {
-          ipiv_all[bmat * ipiv_stride(d.n) + k + j] = (int32_t)(k + p);
-          if (zero && info_all[bmat] == 0) info_all[bmat] = (int32_t)(k + j + 1);
-        }
-      }
+    K v = lane < P ? cand_v[par][lane] : (K)0;
+    const int ci = lane < P ? cand_i[par][lane] : INT_MAX;
+    int p = ci;
+    warp_argmax(v, p);
+    const bool zero = v == 0;
+    const int win = zero ? 0 : __ffs(__ballot_sync(0xffffffffu, ci == p)) - 1;  // the CTA that holds the pivot
+    if (zero) p = j;                                                            // panel row of the pivot
+    const C* jrow = pub_j[par];
+    const C* urow = zero ? jrow : slots + (par * P + win) * kNB;
+    const C inv = zero ? czero<C>() : cand_inv[par][win];
+    const int lp = (p != j && rank == win) ? p - r0 : -1;  // this CTA's row that takes row j
+    if (kScaleApart) {
+      for (int i = tid; i < rows; i += kPanelThreads)
+        if (r0 + i > j) sp[j * ld + i] = cmul(i == lp ? jrow[j] : sp[j * ld + i], inv);
+      __syncthreads();
     }
-    __syncthreads();
-    const int p = s_piv;
-    const int lp = (p != j && rank == p / chunk) ? p - r0 : -1;  // this CTA's row that takes row j
-    const C inv = s_inv;
-    for (int i = tid; i < rows; i += kPanelThreads)
-      if (r0 + i > j) sp[j * ld + i] = cmul(i == lp ? jrow[j] : sp[j * ld + i], inv);
-    if (warp == kWarps - 1 && p != j) {  // the interchanged rows' entries that the update leaves alone
-      if (rank == 0 && lane < kb) sp[lane * ld + j] = urow[lane];
-      if (lp >= 0 && lane < j) sp[lane * ld + lp] = jrow[lane];
+    if (warp == kItemWarps) {
+      if (p != j) {  // the interchanged rows' entries that the update leaves alone
+        if (rank == 0 && lane < kb) sp[lane * ld + j] = urow[lane];
+        if (lp >= 0 && lane < j) sp[lane * ld + lp] = jrow[lane];
+      }
+      if (lane == 0 && rank == 0) {
+        ipiv_all[bmat * ipiv_stride(d.n) + k + j] = (int32_t)(k + p);
+        if (zero && info_all[bmat] == 0) info_all[bmat] = (int32_t)(k + j + 1);
+      }
+      if (j + 1 < kb) {
+        bar_sync(1, 32 * (searchers + 1));
+        publish(j + 1, searchers);
+      }
+      continue;
     }
-    __syncthreads();
+    // the multiplier of row i
+    auto multiplier = [&](int i) {
+      if (kScaleApart) return sp[j * ld + i];
+      return cmul(i == lp ? jrow[j] : acol[par * chunk + i], inv);
+    };
     best = 0;
     bi = INT_MAX;
-    const int items = nrb * ((kb - 1 - j + GC - 1) / GC);
-    for (int q = warp; q < items; q += kWarps) {
-      const int g = q / nrb, i = (q - g * nrb) * 32 + lane;
+    for (int rb = warp; rb < nrb; rb += kItemWarps) {
+      const int i = rb * 32 + lane;
       if (i >= rows || r0 + i <= j) continue;
-      const C l = sp[j * ld + i];
-      const int c0 = j + 1 + g * GC;
-      C v[GC];
+      const C l = multiplier(i);
+      if (!kScaleApart) sp[j * ld + i] = l;
+      if (j + 1 < kb) {
+        const C x = cfms(i == lp ? jrow[j + 1] : sp[(j + 1) * ld + i], l, urow[j + 1]);
+        sp[(j + 1) * ld + i] = x;
+        if (!kScaleApart) acol[(par ^ 1) * chunk + i] = x;
+        argmax_merge(best, bi, PivotKey<T>::of(fabs(x.x) + fabs(x.y)), r0 + i);
+      }
+    }
+    if (j + 1 < kb && warp < searchers) {
+      warp_argmax(best, bi);
+      if (lane == 0) { red_v[warp] = best; red_i[warp] = bi; }
+      __syncwarp();
+      bar_arrive(1, 32 * (searchers + 1));
+    }
+    auto rest = [&](auto width_of_item) {
+      constexpr int GC = decltype(width_of_item)::value;
+      int g = g0, rb = rb0;
+      while (j + 2 + g * GC < kb) {
+        const int i = rb * 32 + lane, c0 = j + 2 + g * GC;
+        if (i < rows && r0 + i > j) {
+          const C l = multiplier(i);
+          C x[GC];
 #pragma unroll
-      for (int t = 0; t < GC; ++t)
-        if (c0 + t < kb) v[t] = i == lp ? jrow[c0 + t] : sp[(c0 + t) * ld + i];
+          for (int t = 0; t < GC; ++t)
+            if (c0 + t < kb) x[t] = i == lp ? jrow[c0 + t] : sp[(c0 + t) * ld + i];
 #pragma unroll
-      for (int t = 0; t < GC; ++t)
-        if (c0 + t < kb) {
-          v[t] = cfms(v[t], l, urow[c0 + t]);
-          sp[(c0 + t) * ld + i] = v[t];
+          for (int t = 0; t < GC; ++t)
+            if (c0 + t < kb) sp[(c0 + t) * ld + i] = cfms(x[t], l, urow[c0 + t]);
         }
-      if (g == 0) argmax_merge(best, bi, PivotKey<T>::of(fabs(v[0].x) + fabs(v[0].y)), r0 + i);
+        g += dg;
+        rb += drb;
+        if (rb >= nrb) { rb -= nrb; ++g; }
+      }
+    };
+    if (nrb > 0) {
+      // as few columns per item as keep the multipliers' loads (FP32: and products) in the shade
+      if (nrb <= 2) rest(std::integral_constant<int, sizeof(T) == 8 ? 1 : 2>());
+      else if (sizeof(T) == 8 || nrb <= 6) rest(std::integral_constant<int, sizeof(T) == 8 ? 2 : 4>());
+      else rest(std::integral_constant<int, 8>());
     }
   }
   __syncthreads();

@@ -75,3 +75,17 @@ def test_ill_conditioned_backward_error(mh, ctx, precision, decades):
     x = mh.linsolve(A, b, precision=precision, ctx=ctx)
     r = np.abs(b - A @ x).max(axis=0)
     assert (r <= 20 * n * EPS * np.abs(A).sum(axis=1).max() * np.abs(x).max(axis=0)).all()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed", "fp64_tc"])
+@pytest.mark.parametrize("n", [97, 545, 1100])
+def test_pivots_from_other_ctas(mh, ctx, n, precision):
+    # the largest entry of column j sits n // 2 rows below (cyclically), so that every interchange
+    # of the first half takes a row held by another CTA or another row block
+    rng = np.random.default_rng(n)
+    A = 0.3 * (rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))) / np.sqrt(n)
+    A[(np.arange(n) + n // 2) % n, np.arange(n)] += 2.0 - 1.0j
+    b = rng.standard_normal((n, 2)) + 1j * rng.standard_normal((n, 2))
+    x = mh.linsolve(A, b, precision=precision, ctx=ctx)
+    r = np.abs(b - A @ x).max(axis=0)
+    assert (r <= 20 * n * EPS * (np.abs(A).sum(axis=1).max() * np.abs(x).max(axis=0) + np.abs(b).max(axis=0))).all()
