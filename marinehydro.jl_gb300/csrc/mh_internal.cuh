@@ -201,8 +201,9 @@ size_t ozaki_workspace_bytes(int64_t n, int64_t batch, int64_t extra = 0);
 // FP32 trailing update of the mixed-precision factors on the BF16 tensor cores, three-way
 // split (mh_bf16x3.cu); ws: bx3_workspace_bytes(n, batch) bytes
 size_t bx3_workspace_bytes(int64_t n, int64_t batch);
+bool bx3_deep(const BatchDesc& d, int64_t rest);
 void bx3_trailing_update(cudaStream_t st, LaunchCounter lc, const BatchDesc& d, float2* A, int64_t k, int kb,
-                         void* ws, int* timeout_flag);
+                         int64_t ccols, void* ws, int* timeout_flag);
 // kb: the panel's width (32; 16 for the update inside a two-level panel), cols: at most this
 // many columns right of the panel are updated
 void ozaki_trailing_update(cudaStream_t st, LaunchCounter lc, const BatchDesc& d, double2* A, int64_t k, int kb,

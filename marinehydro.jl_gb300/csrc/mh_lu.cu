@@ -608,6 +608,38 @@ __global__ void __launch_bounds__(128) trsm_kernel(BatchDesc d, typename cplx_t<
     if (r < kb) A[(k + r) + c * n] = x[r];
 }
 
+// U12 of the second of two panels taken together (rows k + 32 .. k + 63 of the columns right of
+// k + 64): L22^-1 (A - L21 Ua), Ua the first panel's U12 already in place; one thread per column.
+__global__ void __launch_bounds__(128) trsm_second_kernel(BatchDesc d, float2* __restrict__ Aall, int64_t k) {
+  __shared__ float2 sL[2 * kNB][kNB];  // rows k + 32 .. of columns k .. k + 63, by column
+  const int64_t n = d.n;
+  float2* A = Aall + d.offset(blockIdx.y);
+  for (int idx = threadIdx.x; idx < 2 * kNB * kNB; idx += blockDim.x) {
+    const int r = idx & (kNB - 1), q = idx / kNB;
+    sL[q][r] = A[(k + kNB + r) + (k + q) * n];
+  }
+  __syncthreads();
+  const int64_t c = k + 2 * kNB + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (c >= n) return;
+  float2* col = A + k + c * n;
+  float2 x[kNB];
+#pragma unroll
+  for (int r = 0; r < kNB; ++r) x[r] = col[kNB + r];
+#pragma unroll 8
+  for (int q = 0; q < kNB; ++q) {
+    const float2 u = col[q];
+#pragma unroll
+    for (int r = 0; r < kNB; ++r) x[r] = cfms(x[r], sL[q][r], u);
+  }
+#pragma unroll
+  for (int q = 0; q < kNB - 1; ++q) {
+#pragma unroll
+    for (int r = q + 1; r < kNB; ++r) x[r] = cfms(x[r], sL[kNB + q][r], x[q]);
+  }
+#pragma unroll
+  for (int r = 0; r < kNB; ++r) col[kNB + r] = x[r];
+}
+
 // FP64: eight lanes per column, lane r8 holding rows r8, r8 + 8, ..; the column-oriented
 // substitution broadcasts x_q within the eight and every lane updates its rows below q.  One
 // thread per column (trsm_kernel) runs 1984 FP64 FMAs in a row, each a 64-cycle issue of one of
@@ -1489,8 +1521,44 @@ int lu_factor_batched(cudaStream_t st, LaunchCounter lc, const BatchDesc& d, typ
     MH_LAUNCH(lc, st, sizeof(T) == 8 ? "lu_panel_f64" : "lu_panel_f32",
               cudaLaunchKernelEx(&cfg, panel_cluster_kernel<T>, d, A, ipiv, info, k0, chunk, width));
   };
+  // the full-width panel at k0 (on one CTA per matrix when no cluster holds it), and its row
+  // interchanges outside of it
+  auto full_panel = [&](int64_t k0) {
+    const int P = panel_cluster_size<T>(n - k0, d.batch, cap_ctas);
+    if (P > 0) {
+      cluster_panel(k0, kNB, P);
+    } else {
+      MH_LAUNCH(lc, st, sizeof(T) == 8 ? "lu_panel_f64" : "lu_panel_f32",
+                panel_kernel<T><<<(unsigned)d.batch, 512, 0, st>>>(d, A, ipiv, info, k0));
+    }
+  };
+  auto interchange = [&](int64_t k0, int64_t kb) {
+    if (n + d.extra - kb <= 0) return;
+    dim3 sg((unsigned)((n + d.extra - kb + kSwpCols - 1) / kSwpCols), (unsigned)d.batch);
+    MH_LAUNCH(lc, st, sizeof(T) == 8 ? "lu_laswp_f64" : "lu_laswp_f32",
+              laswp_kernel<T><<<sg, 256, 0, st>>>(d, A, ipiv, k0, (int)kb));
+  };
   for (int64_t k = 0; k < n; k += kNB) {
     const int64_t kb = (k + kNB < n) ? kNB : n - k;
+    if constexpr (sizeof(T) == 4) {
+      // two panels per pass over the trailing block: the first panel's update reaches only the
+      // second's columns, and both together the rest
+      if (emu_ws && bx3_deep(d, n - k - 2 * kNB)) {
+        full_panel(k);
+        interchange(k, kNB);
+        MH_LAUNCH(lc, st, "lu_trsm_f32",
+                  trsm_kernel<T><<<dim3((unsigned)((n - k - kNB + 127) / 128), (unsigned)d.batch), 128, 0, st>>>(d, A, k));
+        bx3_trailing_update(st, lc, d, A, k, kNB, kNB, emu_ws, emu_flag);
+        full_panel(k + kNB);
+        interchange(k + kNB, kNB);
+        MH_LAUNCH(lc, st, "lu_trsm_f32",
+                  trsm_second_kernel<<<dim3((unsigned)((n - k - 2 * kNB + 127) / 128), (unsigned)d.batch), 128, 0, st>>>(
+                      d, A, k));
+        bx3_trailing_update(st, lc, d, A, k, 2 * kNB, INT64_MAX, emu_ws, emu_flag);
+        k += kNB;
+        continue;
+      }
+    }
     // Two-level panel (FP64 with the tensor-core update, tall panels): two 16-column halves
     // on the CUDA cores, the left half's update of the right half (K = 16) on the tensor
     // cores -- half the panel's FP64 work, and half its shared memory per row
@@ -1513,19 +1581,9 @@ int lu_factor_batched(cudaStream_t st, LaunchCounter lc, const BatchDesc& d, typ
         MH_LAUNCH(lc, st, "lu_laswp_f64", laswp_cols_kernel<T><<<sg, 256, 0, st>>>(d, A, ipiv, k + H, H, k, k + H));
       }
     } else {
-      const int P = panel_cluster_size<T>(n - k, d.batch, cap_ctas);
-      if (P > 0) {
-        cluster_panel(k, kNB, P);
-      } else {
-        MH_LAUNCH(lc, st, sizeof(T) == 8 ? "lu_panel_f64" : "lu_panel_f32",
-                  panel_kernel<T><<<(unsigned)d.batch, 512, 0, st>>>(d, A, ipiv, info, k));
-      }
+      full_panel(k);
     }
-    if (n + d.extra - kb > 0) {
-      dim3 sg((unsigned)((n + d.extra - kb + kSwpCols - 1) / kSwpCols), (unsigned)d.batch);
-      MH_LAUNCH(lc, st, sizeof(T) == 8 ? "lu_laswp_f64" : "lu_laswp_f32",
-                laswp_kernel<T><<<sg, 256, 0, st>>>(d, A, ipiv, k, (int)kb));
-    }
+    interchange(k, kb);
     const int64_t rest = n - k - kb;              // trailing rows
     const int64_t rest_c = n + d.extra - k - kb;  // columns right of the panel
     if (rest_c <= 0) continue;
@@ -1550,7 +1608,7 @@ int lu_factor_batched(cudaStream_t st, LaunchCounter lc, const BatchDesc& d, typ
       if constexpr (sizeof(T) == 8) {  // FP64 update on the BF16 tensor cores (mh_ozaki.cu)
         ozaki_trailing_update(st, lc, d, A, k, (int)kb, emu_ws, emu_flag);
       } else {  // FP32 update on the BF16 tensor cores (mh_bf16x3.cu)
-        bx3_trailing_update(st, lc, d, A, k, (int)kb, emu_ws, emu_flag);
+        bx3_trailing_update(st, lc, d, A, k, (int)kb, INT64_MAX, emu_ws, emu_flag);
       }
       continue;
     }

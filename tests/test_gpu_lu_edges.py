@@ -89,3 +89,16 @@ def test_pivots_from_other_ctas(mh, ctx, n, precision):
     x = mh.linsolve(A, b, precision=precision, ctx=ctx)
     r = np.abs(b - A @ x).max(axis=0)
     assert (r <= 20 * n * EPS * (np.abs(A).sum(axis=1).max() * np.abs(x).max(axis=0) + np.abs(b).max(axis=0))).all()
+
+
+@pytest.mark.parametrize("n", [2900, 3001])
+def test_two_panels_per_update(mh, ctx, n):
+    # orders whose first trailing blocks have 8e6 entries or more: two FP32 panels per update, then one
+    # per update, whole and ragged tiles; with a residual of n^2 products, checked as above
+    rng = np.random.default_rng(n)
+    A = (rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))) / np.sqrt(n)
+    A[np.arange(n), np.arange(n)] += 1.5
+    b = rng.standard_normal((n, 1)) + 1j * rng.standard_normal((n, 1))
+    x = mh.linsolve(A, b, precision="mixed", ctx=ctx)
+    r = np.abs(b - A @ x).max(axis=0)
+    assert (r <= 20 * n * EPS * (np.abs(A).sum(axis=1).max() * np.abs(x).max(axis=0) + np.abs(b).max(axis=0))).all()
