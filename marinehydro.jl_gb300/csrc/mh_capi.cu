@@ -258,10 +258,7 @@ int refine_mixed(mh_context* ctx, const BatchDesc& d, const double2* Adev, const
   for (int it = 0; it <= 30; ++it) {
     if (adjoint) residual_batched(ctx->stream, ctx->lc(), d, Adev, X, B0, nrhs, xstride, R, work, true);
     else residual_tc_batched(ctx->stream, ctx->lc(), d, Adev, X, B0, nrhs, xstride, R, work, tcflag);
-    for (int64_t b = 0; b < d.batch; ++b) {
-      inf_norms_batched(ctx->stream, ctx->lc(), n, nrhs, R + b * xstride, norms + b * nrhs);
-      inf_norms_batched(ctx->stream, ctx->lc(), n, nrhs, X + b * xstride, norms + ncols + b * nrhs);
-    }
+    inf_norms_batched(ctx->stream, ctx->lc(), n, d.batch, nrhs, xstride, R, X, norms);
     MH_TRY(check_launch(ctx, "refinement"));
     MH_CUDA(ctx, cudaMemcpyAsync(hn, norms, sizeof(double) * (2 * ncols + d.batch), cudaMemcpyDeviceToHost,
                                  ctx->stream));

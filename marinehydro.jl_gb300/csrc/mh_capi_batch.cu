@@ -230,8 +230,7 @@ void enqueue_back(mh_context* ctx, LaunchCounter lc, cudaStream_t st, BodyPlan& 
     // the residual of the returned x, judged on the host after the graph
     const int64_t ncols = o.nrhs * nw;
     residual_tc_batched(st, lc, d, b.D, b.X, b.B0, o.nrhs, bstride, b.R, b.work, b.ozflag);
-    inf_norms_batched(st, lc, n, ncols, b.R, b.norms);
-    inf_norms_batched(st, lc, n, ncols, b.X, b.norms + ncols);
+    inf_norms_batched(st, lc, n, 1, ncols, 0, b.R, b.X, b.norms);
     cudaMemcpyAsync(b.hnorms, b.norms, sizeof(double) * 2 * ncols, cudaMemcpyDeviceToHost, st);
   }
   EpilogueGeom eg{n, b.m->n_hull, b.m->C, b.m->N, b.m->A, b.dofs};
@@ -295,8 +294,7 @@ int finish_body(mh_context* ctx, BatchCache& c, BodyPlan& b, const BatchOpts& o)
     lu_solve_batched<float>(st, lc, gb, c.LU32_all, ipiv_b, c.X32_all, o.nrhs, 0, false);
     ir_update(st, lc, bstride * nw, b.X, b.X32);
     residual_batched(st, lc, d, b.D, b.X, b.B0, o.nrhs, bstride, b.R, b.work, false);
-    inf_norms_batched(st, lc, n, ncols, b.R, b.norms);
-    inf_norms_batched(st, lc, n, ncols, b.X, b.norms + ncols);
+    inf_norms_batched(st, lc, n, 1, ncols, 0, b.R, b.X, b.norms);
     MH_CUDA(ctx, cudaMemcpyAsync(b.hnorms, b.norms, sizeof(double) * 2 * ncols, cudaMemcpyDeviceToHost, st));
     MH_TRY(sync(ctx, "batch refinement"));
     ok = converged();

@@ -244,8 +244,8 @@ void widen_c_to_z(cudaStream_t st, LaunchCounter lc, const float2* src, double2*
 // FP32 copy of each matrix (matrix stride stride32) and its |.|_inf norm into out[b], one pass over A
 void convert_with_norms(cudaStream_t st, LaunchCounter lc, const BatchDesc& d, const double2* A, float2* A32,
                         int64_t stride32, double* out);
-void inf_norms_batched(cudaStream_t st, LaunchCounter lc, int64_t n, int64_t ncols, const double2* X,
-                       double* out);
+void inf_norms_batched(cudaStream_t st, LaunchCounter lc, int64_t n, int64_t batch, int64_t nrhs, int64_t xstride,
+                       const double2* R, const double2* X, double* out);
 
 // epilogue (mh_epilogue.cu)
 struct EpilogueGeom {

@@ -1261,17 +1261,30 @@ __global__ void __launch_bounds__(kSolveThreads, 2) solve_cluster_kernel(BatchDe
 }
 
 // ------------------------------ Y = A X (FP64) --------------------------------
-constexpr int kGemvRows = 128;
+constexpr int kGemvRows = 32;     // outputs per CTA, one per lane
+constexpr int kGemvWarps = 8;     // each takes 8 of the kGemvCols terms of a step
+constexpr int kGemvCols = 8 * kGemvWarps;
 constexpr int kGemvNR = 8;
+constexpr int kGemvLd = 9;
+constexpr int kGemvMaxCtas = 4 * 152;
 
-// partial[js][b][r][i] = sum_{j in chunk js} A_b[i, j] X_b[j, r]  (ADJ: A^H)
+// partial[js][b][r][i] = sum_{j in chunk js} A_b[i, j] X_b[j, r]  (ADJ: A^H).  A CTA computes 32
+// outputs: per step of 64 terms each warp has its eight matrix entries per output in flight at
+// once (ADJ: read along the columns, 128 bytes at a time, and turned in shared memory), and the
+// warps' sums are added at the end.  Bound: the FP64 pipe for several right-hand sides, latency for
+// few (one warp instruction per 19 cycles and SM, 77 for a single warp).  A thread per output
+// that loaded one entry at a time, down a column for A^H, took 568 us for order 1400 (A^H, four
+// matrices for A 574), 93 us at 450 and 79 us at 200; now 151 (131), 11 and 9.
 template <bool ADJ>
-__global__ void __launch_bounds__(kGemvRows) zgemm_partial_kernel(BatchDesc d, const double2* __restrict__ Aall,
-                                                                  const double2* __restrict__ Xall, int64_t nrhs,
-                                                                  int64_t xstride, int64_t jchunk, int r0,
-                                                                  double2* __restrict__ part) {
+__global__ void __launch_bounds__(32 * kGemvWarps) zgemm_partial_kernel(BatchDesc d, const double2* __restrict__ Aall,
+                                                                       const double2* __restrict__ Xall, int64_t nrhs,
+                                                                       int64_t xstride, int64_t jchunk, int r0,
+                                                                       double2* __restrict__ part) {
+  __shared__ double2 sX[kGemvNR][kGemvCols];
+  __shared__ double2 sT[kGemvWarps][32 * kGemvLd];  // ADJ: entries [output][term]; at the end the warps' sums
   const int64_t n = d.n;
-  const int64_t i = blockIdx.x * (int64_t)kGemvRows + threadIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t i0 = blockIdx.x * (int64_t)kGemvRows, i = i0 + lane;
   const int64_t js = blockIdx.y;
   const int64_t b = blockIdx.z;
   const double2* A = Aall + b * d.stride;
@@ -1281,17 +1294,48 @@ __global__ void __launch_bounds__(kGemvRows) zgemm_partial_kernel(BatchDesc d, c
   double2 acc[kGemvNR];
 #pragma unroll
   for (int r = 0; r < kGemvNR; ++r) acc[r] = make_double2(0.0, 0.0);
-  if (i < n) {
-    for (int64_t j = ja; j < jbnd; ++j) {
-      double2 a = ADJ ? cconj(__ldg(A + j + i * n)) : __ldg(A + i + j * n);
+  double2* tile = sT[warp];
+  for (int64_t jb = ja; jb < jbnd; jb += kGemvCols) {
+    const int64_t j0 = jb + 8 * warp;
+    double2 a[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int64_t jj = ADJ ? j0 + (lane & 7) : j0 + q, ii = ADJ ? i0 + (lane >> 3) + 4 * q : i;
+      a[q] = (jj < jbnd && ii < n) ? __ldg(ADJ ? A + jj + ii * n : A + ii + jj * n) : make_double2(0.0, 0.0);
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < g * kGemvCols; e += 32 * kGemvWarps) {
+      const int r = e / kGemvCols, c = e & (kGemvCols - 1);
+      sX[r][c] = jb + c < jbnd ? X[jb + c + (r0 + r) * n] : make_double2(0.0, 0.0);
+    }
+    if (ADJ) {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) tile[((lane >> 3) + 4 * q) * kGemvLd + (lane & 7)] = cconj(a[q]);
+    }
+    __syncthreads();
+    if (ADJ) {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) a[q] = tile[lane * kGemvLd + q];
+    }
+    if (j0 < jbnd) {
 #pragma unroll
       for (int r = 0; r < kGemvNR; ++r)
-        if (r < g) acc[r] = cfma(acc[r], a, __ldg(X + j + (r0 + r) * n));
-    }
-    double2* P = part + ((js * d.batch + b) * nrhs) * n;
+        if (r < g) {
 #pragma unroll
-    for (int r = 0; r < kGemvNR; ++r)
-      if (r < g) P[(r0 + r) * n + i] = acc[r];
+          for (int q = 0; q < 8; ++q) acc[r] = cfma(acc[r], a[q], sX[r][8 * warp + q]);
+        }
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < kGemvNR; ++r)
+    if (r < g) tile[r * 32 + lane] = acc[r];
+  __syncthreads();
+  if (warp < g && i < n) {
+    double2 s = sT[0][warp * 32 + lane];
+#pragma unroll
+    for (int w = 1; w < kGemvWarps; ++w) s = cadd(s, sT[w][warp * 32 + lane]);
+    part[((js * d.batch + b) * nrhs + r0 + warp) * n + i] = s;
   }
 }
 
@@ -1316,13 +1360,11 @@ __global__ void zgemm_reduce_kernel(BatchDesc d, int64_t nrhs, int64_t nsplit, c
   Yall[b * ystride + e] = s;
 }
 
+// Splits of the sum: four CTAs per SM, each with at least half a step of terms
 int64_t gemm_split(int64_t n, int64_t batch) {
-  int64_t rows = (n + kGemvRows - 1) / kGemvRows;
-  int64_t want = (4 * 152 + rows * batch - 1) / (rows * batch);
-  int64_t maxs = (n + 63) / 64;
-  if (want < 1) want = 1;
-  if (want > maxs) want = maxs;
-  return want;
+  const int64_t rows = (n + kGemvRows - 1) / kGemvRows;
+  const int64_t want = kGemvMaxCtas / (rows * batch), most = (n + kGemvCols / 2 - 1) / (kGemvCols / 2);
+  return std::max<int64_t>(1, std::min(want, most));
 }
 
 __global__ void z_to_c_kernel(const double2* __restrict__ s, float2* __restrict__ d, int64_t count) {
@@ -1340,12 +1382,16 @@ __global__ void ir_update_kernel(double2* __restrict__ X, const float2* __restri
   if (q < count) { X[q].x += (double)Cc[q].x; X[q].y += (double)Cc[q].y; }
 }
 
-// out[col] = max_i |re| + |im|  over column col of an n x ncols array
-__global__ void col_inf_norm_kernel(int64_t n, const double2* __restrict__ X, double* __restrict__ out) {
-  const int64_t col = blockIdx.x;
+// out[col] = max_i |re| + |im| over column col of R, and out[ncols + col] of X (blockIdx.y 0, 1):
+// columns of n entries, nrhs per matrix, the matrices' xstride apart.  All columns in one launch:
+// two per matrix, 4.4 us each, were a tenth of a 12-frequency sweep of 430 panels.
+__global__ void col_inf_norm_kernel(int64_t n, int64_t nrhs, int64_t xstride, const double2* __restrict__ R,
+                                    const double2* __restrict__ Xs, double* __restrict__ out) {
+  const int64_t col = blockIdx.x + blockIdx.y * (int64_t)gridDim.x;
+  const double2* X = (blockIdx.y ? Xs : R) + blockIdx.x / nrhs * xstride + blockIdx.x % nrhs * n;
   double m = 0.0;
   for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
-    double2 v = X[i + col * n];
+    double2 v = X[i];
     double a = fabs(v.x) + fabs(v.y);
     m = a > m ? a : m;
   }
@@ -1771,7 +1817,9 @@ template void lu_solve_batched<float>(cudaStream_t, LaunchCounter, const BatchDe
                                       float2*, int64_t, int64_t, bool, bool);
 
 size_t zgemm_work_elems(int64_t n, int64_t nrhs, int64_t batch) {
-  const size_t fp64 = (size_t)gemm_split(n, batch) * (size_t)batch * (size_t)nrhs * (size_t)n;
+  // splits x matrices for this many matrices or fewer (gemm_split)
+  const int64_t sums = std::max<int64_t>(batch, kGemvMaxCtas / ((n + kGemvRows - 1) / kGemvRows));
+  const size_t fp64 = (size_t)sums * (size_t)nrhs * (size_t)n;
   const size_t tc = (tc_zgemv_workspace_bytes(n, batch) + sizeof(double2) - 1) / sizeof(double2);
   return fp64 > tc ? fp64 : tc;
 }
@@ -1796,8 +1844,8 @@ static void zgemm_impl(cudaStream_t st, LaunchCounter lc, const BatchDesc& d, co
   dim3 grid((unsigned)((n + kGemvRows - 1) / kGemvRows), (unsigned)ns, (unsigned)d.batch);
   for (int r0 = 0; r0 < nrhs; r0 += kGemvNR) {
     lc.pre(st);
-    if (adjoint) zgemm_partial_kernel<true><<<grid, kGemvRows, 0, st>>>(d, A, X, nrhs, xstride, jchunk, r0, work);
-    else zgemm_partial_kernel<false><<<grid, kGemvRows, 0, st>>>(d, A, X, nrhs, xstride, jchunk, r0, work);
+    if (adjoint) zgemm_partial_kernel<true><<<grid, 32 * kGemvWarps, 0, st>>>(d, A, X, nrhs, xstride, jchunk, r0, work);
+    else zgemm_partial_kernel<false><<<grid, 32 * kGemvWarps, 0, st>>>(d, A, X, nrhs, xstride, jchunk, r0, work);
     lc.post(st, "zgemm_rhs");
   }
   const int64_t tot = nrhs * n * d.batch;
@@ -1837,9 +1885,11 @@ void widen_c_to_z(cudaStream_t st, LaunchCounter lc, const float2* src, double2*
   MH_LAUNCH(lc, st, "convert", c_to_z_kernel<<<(unsigned)((count + 255) / 256), 256, 0, st>>>(src, dst, count));
 }
 
-void inf_norms_batched(cudaStream_t st, LaunchCounter lc, int64_t n, int64_t ncols, const double2* X, double* out) {
-  if (ncols <= 0) return;
-  MH_LAUNCH(lc, st, "ir_norms", col_inf_norm_kernel<<<(unsigned)ncols, 256, 0, st>>>(n, X, out));
+void inf_norms_batched(cudaStream_t st, LaunchCounter lc, int64_t n, int64_t batch, int64_t nrhs, int64_t xstride,
+                       const double2* R, const double2* X, double* out) {
+  if (batch <= 0 || nrhs <= 0) return;
+  MH_LAUNCH(lc, st, "ir_norms",
+            col_inf_norm_kernel<<<dim3((unsigned)(batch * nrhs), 2), 256, 0, st>>>(n, nrhs, xstride, R, X, out));
 }
 
 

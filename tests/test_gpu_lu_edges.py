@@ -102,3 +102,10 @@ def test_two_panels_per_update(mh, ctx, n):
     x = mh.linsolve(A, b, precision="mixed", ctx=ctx)
     r = np.abs(b - A @ x).max(axis=0)
     assert (r <= 20 * n * EPS * (np.abs(A).sum(axis=1).max() * np.abs(x).max(axis=0) + np.abs(b).max(axis=0))).all()
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 65, 200, 450, 1041])
+@pytest.mark.parametrize("rhs", [1, 8, 9])
+def test_fp64_residual_products(mh, ctx, n, rhs):
+    # A x and A^H x on the FP64 pipe: the adjoint solve's refinement uses them at every order
+    _solve_ok(mh, ctx, n, rhs, "mixed", adjoint=True)
