@@ -27,35 +27,11 @@ __device__ __forceinline__ int scale_of(int emax_biased) { return emax_biased > 
 __device__ __forceinline__ long long fixed55(double v, int emax_biased) {
   const long long bits = __double_as_longlong(v);
   const int ev = (int)((bits >> 52) & 0x7FF);
-  if (ev == 0) return 0;
-  const long long m = (bits & 0xFFFFFFFFFFFFFLL) | 0x10000000000000LL;
-  const int s = ev - emax_biased + 2;  // <= 2
-  long long X;
-  if (s >= 0) X = m << s;
-  else if (s > -63) X = (m + (1LL << (-s - 1))) >> (-s);
-  else X = 0;
+  const unsigned long long m4 = ev == 0 ? 0ull : ((unsigned long long)(bits & 0xFFFFFFFFFFFFFLL) | 0x10000000000000ull) << 2;
+  int s = emax_biased - ev;  // >= 0: m4 is the value at s = 0; from 56 on it rounds to 0
+  s = s < 63 ? s : 63;
+  const long long X = (long long)((m4 + ((1ull << s) >> 1)) >> s);
   return bits < 0 ? -X : X;
-}
-
-// the balanced digits of X, most significant first, with 32-bit arithmetic:
-// X = hi 2^28 + lo, lo in [0, 2^28) gives digits 7..4 and a carry, hi (|hi| < 2^27) 3..0
-__device__ __forceinline__ void digits(long long X, int (&d)[kDigits]) {
-  int lo = (int)(X & 0xFFFFFFF);
-  int hi = (int)(X >> 28);
-#pragma unroll
-  for (int p = kDigits - 1; p >= 4; --p) {
-    const int c = lo + 64;
-    d[p] = (c & 127) - 64;
-    lo = c >> 7;
-  }
-  hi += lo;
-#pragma unroll
-  for (int p = 3; p >= 1; --p) {
-    const int c = hi + 64;
-    d[p] = (c & 127) - 64;
-    hi = c >> 7;
-  }
-  d[0] = hi;
 }
 
 // two BF16 values of small integers (|d| <= 64) in one 32-bit word, the first in the low half
@@ -65,20 +41,30 @@ __device__ __forceinline__ uint32_t bf16x2(int d0, int d1) {
   return __byte_perm(__float_as_uint(f0), __float_as_uint(f1), 0x7632);
 }
 
-// Eight consecutive K values (one 16-byte row chunk of the canonical K-major layout) of one
-// row: their 16 digit planes (re/im x 8 digits) as packed BF16 pairs, pk[part][digit][0..3].
-__device__ __forceinline__ void split8(const double2 (&v)[8], int emax, uint32_t (&pk)[2][kDigits][4]) {
+// Four consecutive K values (half a 16-byte row chunk of the canonical K-major layout) of one
+// row: their 16 digit planes (re/im x 8 digits) as packed BF16 pairs, pk[part][digit][0..1].
+// With 64 added to every digit beforehand (one 64-bit addition, which does all the carries) digit p
+// is a bit field u_p = d_p + 64 in [0, 128] of the sum; two of them set into the mantissas of BF16
+// 128.0 and 192 subtracted from both in one packed operation are the digits: 45 instructions
+// per value, where digits peeled off one by one and converted through FP32 took about 100.
+__device__ __forceinline__ uint32_t digit_pair(uint32_t u0, uint32_t u1, uint32_t mask) {
+  const uint32_t t = (__byte_perm(u0, u1, 0x5410) & mask) | 0x43004300u;
+  uint32_t r;
+  asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(t), "r"(0x43404340u));
+  return r;
+}
+__device__ __forceinline__ void split4(const double2 (&v)[4], int emax, uint32_t (&pk)[2][kDigits][2]) {
+  constexpr long long kBias = 0x81020408102040ll;  // 64 in each of the eight base-128 digits
 #pragma unroll
-  for (int c = 0; c < 8; c += 2) {
-    int a0[kDigits], a1[kDigits], b0[kDigits], b1[kDigits];
-    digits(fixed55(v[c].x, emax), a0);
-    digits(fixed55(v[c + 1].x, emax), a1);
-    digits(fixed55(v[c].y, emax), b0);
-    digits(fixed55(v[c + 1].y, emax), b1);
+  for (int c = 0; c < 4; c += 2) {
 #pragma unroll
-    for (int p = 0; p < kDigits; ++p) {
-      pk[0][p][c >> 1] = bf16x2(a0[p], a1[p]);
-      pk[1][p][c >> 1] = bf16x2(b0[p], b1[p]);
+    for (int part = 0; part < 2; ++part) {
+      const unsigned long long x0 = (unsigned long long)(fixed55(part ? v[c].y : v[c].x, emax) + kBias);
+      const unsigned long long x1 = (unsigned long long)(fixed55(part ? v[c + 1].y : v[c + 1].x, emax) + kBias);
+#pragma unroll
+      for (int p = 0; p < kDigits; ++p)
+        pk[part][p][c >> 1] = digit_pair((uint32_t)(x0 >> (7 * (7 - p))), (uint32_t)(x1 >> (7 * (7 - p))),
+                                         p == 0 ? 0x00FF00FFu : 0x007F007Fu);
     }
   }
 }
@@ -106,7 +92,7 @@ __device__ __forceinline__ void digits7(long long X, int (&d)[kDigits7]) {
   d[0] = hi;
 }
 
-// split8 with seven base-256 digit planes
+// Eight consecutive K values (one 16-byte row chunk) of one row: their seven base-256 digit planes
 __device__ __forceinline__ void split7(const double2 (&v)[8], int emax, uint32_t (&pk)[2][kDigits7][4]) {
 #pragma unroll
   for (int c = 0; c < 8; c += 2) {

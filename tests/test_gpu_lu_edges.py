@@ -104,6 +104,24 @@ def test_two_panels_per_update(mh, ctx, n):
     assert (r <= 20 * n * EPS * (np.abs(A).sum(axis=1).max() * np.abs(x).max(axis=0) + np.abs(b).max(axis=0))).all()
 
 
+@pytest.mark.parametrize("n", [40, 200, 545, 1100, 2050])
+def test_refinement_settles_in_a_few_sweeps(mh, ctx, n):
+    # the tensor-core residual over split and ragged column blocks: were it off in a few rows, the
+    # refinement would go on to its 30th sweep (and the FP64 factorization hide it)
+    rng = np.random.default_rng(n)
+    A = (rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))) / np.sqrt(n)
+    A[np.arange(n), np.arange(n)] += 3.0
+    b = rng.standard_normal((n, 5)) + 1j * rng.standard_normal((n, 5))
+    mh.linsolve(A, b, precision="mixed", ctx=ctx)
+    before = ctx.launch_count()
+    x = mh.linsolve(A, b, precision="mixed", ctx=ctx)
+    # five launches per panel, eight sweeps of at most seven launches, a dozen around them
+    assert ctx.launch_count() - before <= 5 * ((n + 31) // 32) + 8 * 7 + 12
+    r = np.abs(b - A @ x).max(axis=0)
+    # the stopping rule sqrt(n) eps |A| |x| and the rounding of this check's own product
+    assert (r <= (2 * np.sqrt(n) + n) * 2 * EPS * np.abs(A).sum(axis=1).max() * np.abs(x).max(axis=0)).all()
+
+
 @pytest.mark.parametrize("n", [1, 31, 33, 65, 200, 450, 1041])
 @pytest.mark.parametrize("rhs", [1, 8, 9])
 def test_fp64_residual_products(mh, ctx, n, rhs):
