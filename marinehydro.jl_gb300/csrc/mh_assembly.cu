@@ -15,6 +15,8 @@
 // S = S_static + S_wave is the reference's own split, matrix_assembly.jl:183-208).
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include <algorithm>
 
 #include "mh_egd.cuh"
@@ -324,9 +326,9 @@ __device__ __forceinline__ WaveTerms egd_wave_terms(double r, double z, double k
 // WMODE bits: 1 = Wu, 2 = exact Delhommeau (the learned surrogate has its own kernel,
 // wave_kernel_tc).  kc[m] = -k^m / 4pi (m = 1, 2, 3), the pair-independent factors of the
 // terms: I = kc1 G, Gh dx_c = kc3 (1/hh) dx_c dG/dh, Gz = kc2 dG/dz (wu.jl:118-126).
-template <bool DIRECT, int WMODE>
+template <bool DIRECT, int WMODE, typename Step = NoStep>
 __device__ __forceinline__ void wave_terms(const AssemblyParams& p, const double ci[3], const double cj[3], double k,
-                                           const double kc[4], WaveTerms& w) {
+                                           const double kc[4], WaveTerms& w, Step step = Step()) {
   w.I = make_double2(0.0, 0.0);
   w.Gh = w.Gz = w.I;
   if (WMODE & 1) {  // _wu_sd (wu.jl:112-127)
@@ -334,7 +336,7 @@ __device__ __forceinline__ void wave_terms(const AssemblyParams& p, const double
     reduced_coords(ci, cj, k, hh, vv);
     double2 GF, Gh, Gv;
     double inv_hh;  // 1/hh, or 0 where the horizontal gradient is zeroed (hh <= 1e-6)
-    wu_wave_term_and_derivs(hh, vv, GF, Gh, Gv, &inv_hh);
+    wu_wave_term_and_derivs(hh, vv, GF, Gh, Gv, &inv_hh, step);
     const double a = kc[3] * inv_hh;
     w.I = make_double2(kc[1] * GF.x, kc[1] * GF.y);
     w.Gh = make_double2(a * Gh.x, a * Gh.y);
@@ -415,6 +417,17 @@ __device__ __forceinline__ void store_pair(const AssemblyParams& p, const WaveTe
   Db[mdx] = dm;
 }
 
+// The Wu term of one pair is some 4000 instructions with everything inlined and unrolled, more
+// than the instruction caches feed to warps that each run at a place of their own: half of the
+// time warps waited for instructions (the FP64 pipe 58 % busy, issue slots 24 %).  So what the
+// term does again and again is called (wu_fit, bessel_row, recip_call), and the CTA's warps walk
+// together, a barrier per column and between the term's parts; warps below the diagonal only
+// keep the count.  1750 panels 833 -> 635 us, thirty matrices of 2000 19.2 -> 15.7 ms; without the
+// barriers 5 % less; CTAs of 256 rows the same, of 512 15 % more (their tiles' last warps wait).
+struct CtaStep {
+  __device__ __forceinline__ void operator()() const { asm volatile("bar.sync 0;" ::: "memory"); }
+};
+constexpr int kWuSteps = 3;  // barriers inside wu_wave_term_and_derivs
 template <bool DIRECT, int WMODE>  // WMODE 1 = Wu only, 2 = exact Delhommeau, 3 = both
 __global__ void __launch_bounds__(kRowsPerCta) wave_kernel(AssemblyParams p, const double* SR, const double* DR,
                                                            const double* __restrict__ ks, double2* S, double2* D,
@@ -439,17 +452,24 @@ __global__ void __launch_bounds__(kRowsPerCta) wave_kernel(AssemblyParams p, con
   __syncthreads();
   for (int q = threadIdx.x; q < 3 * jmax; q += blockDim.x) san[q / 3][q % 3] = sp[q / 3].area * sp[q / 3].n[q % 3];
   __syncthreads();
-  if (i >= n) return;
+  const int64_t il = i < n ? i : n - 1;
   double ci[3], ni[3], ani[3];
-  for (int c = 0; c < 3; ++c) { ci[c] = __ldg(&p.P[i].c[c]); ni[c] = __ldg(&p.P[i].n[c]); }
-  const double ai = __ldg(&p.P[i].area);
+  for (int c = 0; c < 3; ++c) { ci[c] = __ldg(&p.P[il].c[c]); ni[c] = __ldg(&p.P[il].n[c]); }
+  const double ai = __ldg(&p.P[il].area);
+  using Step = typename std::conditional<(WMODE & 1) != 0, CtaStep, NoStep>::type;
   for (int c = 0; c < 3; ++c) ani[c] = ai * ni[c];
   for (int jj = 0; jj < jmax; ++jj) {
     const int64_t j = j0 + jj;
-    if (i > j) continue;
+    Step()();
+    const int64_t first = i - (threadIdx.x & 31);  // the warp's first row
+    if (first > j || first >= n) {
+      for (int q = 0; q < kWuSteps; ++q) Step()();
+      continue;
+    }
     const PanelRec& Pj = sp[jj];
     WaveTerms w;
-    wave_terms<DIRECT, WMODE>(p, ci, Pj.c, k, kc, w);
+    wave_terms<DIRECT, WMODE>(p, ci, Pj.c, k, kc, w, Step());
+    if (i > j || i >= n) continue;
     // (i, j) orientation: gradient w.r.t. the source (direct) or the field point (indirect)
     const double dx1 = DIRECT ? Pj.c[0] - ci[0] : ci[0] - Pj.c[0];
     const double dx2 = DIRECT ? Pj.c[1] - ci[1] : ci[1] - Pj.c[1];

@@ -45,6 +45,10 @@ __device__ __forceinline__ T horner_c(const T (&c)[N], T t) {
 // and z = 2 (x - q/2 - 1/4) as (X - q 2^59 - 2^58) 2^5 exactly; above 8 the Hankel
 // polynomials take z = (u - 1/2) / 2 from the FP64 u = (8/x)^2.  Absolute error below 1e-17
 // (the integer evaluation, emulated bit for bit by the generator, against mpmath).
+// one row of a table, called for the same reason as wu_fit (mh_greens.cuh)
+static __device__ __noinline__ double bessel_row(const long long* __restrict__ c, long long z) {
+  return fx::to_double(fx::horner_s_ld<bes::kLowTerms>(c, z), besq::kFrac);
+}
 __device__ __forceinline__ void bessel01(double x, double& J0, double& J1, double& Y0, double& Y1) {
   using namespace bes;
   if (x < 8.0) {
@@ -52,12 +56,12 @@ __device__ __forceinline__ void bessel01(double x, double& J0, double& J1, doubl
     X = X < 0 ? 0 : X;
     const int q = (int)(X >> 59);  // X < 2^63: q <= 15
     const long long z = (X - (((long long)q << 59) + (1ll << 58))) << 5;
-    J0 = fx::to_double(fx::horner_s_ld<kLowTerms>(besq::kJ0 + q * kLowTerms, z), besq::kFrac);
-    J1 = fx::to_double(fx::horner_s_ld<kLowTerms>(besq::kJ1 + q * kLowTerms, z), besq::kFrac);
+    J0 = bessel_row(besq::kJ0 + q * kLowTerms, z);
+    J1 = bessel_row(besq::kJ1 + q * kLowTerms, z);
     const int qy = q < 6 ? 0 : q - 6;
     const long long zy = q < 6 ? 0 : z;
-    Y0 = fx::to_double(fx::horner_s_ld<kLowTerms>(besq::kY0 + qy * kLowTerms, zy), besq::kFrac);
-    Y1 = fx::to_double(fx::horner_s_ld<kLowTerms>(besq::kY1 + qy * kLowTerms, zy), besq::kFrac);
+    Y0 = bessel_row(besq::kY0 + qy * kLowTerms, zy);
+    Y1 = bessel_row(besq::kY1 + qy * kLowTerms, zy);
   } else {
     const double f = rsqrt(3.14159265358979323846 * x);  // 1 / sqrt(pi x)
     const double s = 8.0 * 3.14159265358979323846 * f * f;  // 8 / x

@@ -121,6 +121,9 @@ __device__ __forceinline__ double recip(double x) {
   return __longlong_as_double((long long)(((unsigned long long)ex << 52) | (mant & 0x000FFFFFFFFFFFFFull)));
 }
 
+// recip as a call, where it is taken several times in a long loop body (wave_kernel)
+static __device__ __noinline__ double recip_call(double x) { return recip(x); }
+
 // e^x for x <= 0 on the integer pipe (0 for x <= -745.25 and where the result is below the
 // normal range).  y = x log2(e) from a 128-bit product of x 2^s (s = 60 for |x| < 8, else
 // 53: exact) and log2(e) 2^63, so y's fraction f carries 64 bits; 2^f = 2^(j/32) 2^(g/32)

@@ -187,35 +187,48 @@ struct WuFits {
   double A, B, C, D, dA, dB, dC;
 };
 
+constexpr int kWuFrac = 44;
+// A, B, C, D, dA, dB, dC, with zeros above their degrees
+static __device__ __constant__ const long long kWuFit[7][10] = {
+    {fx::q(1.21, kWuFrac), fx::q(-13.328, kWuFrac), fx::q(215.896, kWuFrac), fx::q(-1763.96, kWuFrac),
+     fx::q(8418.94, kWuFrac), fx::q(-24314.21, kWuFrac), fx::q(42002.57, kWuFrac), fx::q(-41592.9, kWuFrac),
+     fx::q(21859.0, kWuFrac), fx::q(-4838.6, kWuFrac)},
+    {fx::q(0.938, kWuFrac), fx::q(5.737, kWuFrac), fx::q(-67.92, kWuFrac), fx::q(796.534, kWuFrac),
+     fx::q(-4780.77, kWuFrac), fx::q(17137.74, kWuFrac), fx::q(-36618.81, kWuFrac), fx::q(44894.06, kWuFrac),
+     fx::q(-29030.24, kWuFrac), fx::q(7671.22, kWuFrac)},
+    {fx::q(1.268, kWuFrac), fx::q(-9.747, kWuFrac), fx::q(209.653, kWuFrac), fx::q(-1397.89, kWuFrac),
+     fx::q(5155.67, kWuFrac), fx::q(-9844.35, kWuFrac), fx::q(9136.4, kWuFrac), fx::q(-3272.62, kWuFrac), 0,
+     0},
+    {fx::q(0.632, kWuFrac), fx::q(-40.97, kWuFrac), fx::q(667.16, kWuFrac), fx::q(-6072.07, kWuFrac),
+     fx::q(31127.39, kWuFrac), fx::q(-96293.05, kWuFrac), fx::q(181856.75, kWuFrac), fx::q(-205690.43,
+     kWuFrac), fx::q(128170.2, kWuFrac), fx::q(-33744.6, kWuFrac)},
+    {fx::q(2.948, kWuFrac), fx::q(-24.53, kWuFrac), fx::q(249.69, kWuFrac), fx::q(-754.85, kWuFrac),
+     fx::q(-1187.71, kWuFrac), fx::q(16370.75, kWuFrac), fx::q(-48811.41, kWuFrac), fx::q(68220.87, kWuFrac),
+     fx::q(-46688.0, kWuFrac), fx::q(12622.25, kWuFrac)},
+    {fx::q(1.11, kWuFrac), fx::q(2.894, kWuFrac), fx::q(-76.765, kWuFrac), fx::q(1565.35, kWuFrac),
+     fx::q(-11336.19, kWuFrac), fx::q(44270.15, kWuFrac), fx::q(-97014.11, kWuFrac), fx::q(118879.26,
+     kWuFrac), fx::q(-76209.82, kWuFrac), fx::q(19923.28, kWuFrac)},
+    {fx::q(14.19, kWuFrac), fx::q(-148.24, kWuFrac), fx::q(847.8, kWuFrac), fx::q(-2318.58, kWuFrac),
+     fx::q(3168.35, kWuFrac), fx::q(-1590.27, kWuFrac), 0, 0, 0, 0}};
+
+// one function, called: inlined seven times the fits are 800 instructions, which the warps of an
+// SM fetch more slowly than they run (wave_kernel)
+static __device__ __noinline__ double wu_fit(int which, unsigned long long t) {
+  long long v = kWuFit[which][9];
+#pragma unroll
+  for (int i = 8; i >= 0; --i) v = kWuFit[which][i] + fx::mulhi_su(v, t);
+  return fx::to_double(v, kWuFrac);
+}
+
 __device__ __forceinline__ void wu_fits(double rho, WuFits& f) {
-  constexpr int F = 44;
-  constexpr long long kA[10] = {fx::q(1.21, F), fx::q(-13.328, F), fx::q(215.896, F), fx::q(-1763.96, F),
-                                fx::q(8418.94, F), fx::q(-24314.21, F), fx::q(42002.57, F), fx::q(-41592.9, F),
-                                fx::q(21859.0, F), fx::q(-4838.6, F)};
-  constexpr long long kB[10] = {fx::q(0.938, F), fx::q(5.737, F), fx::q(-67.92, F), fx::q(796.534, F),
-                                fx::q(-4780.77, F), fx::q(17137.74, F), fx::q(-36618.81, F), fx::q(44894.06, F),
-                                fx::q(-29030.24, F), fx::q(7671.22, F)};
-  constexpr long long kC[8] = {fx::q(1.268, F), fx::q(-9.747, F), fx::q(209.653, F), fx::q(-1397.89, F),
-                               fx::q(5155.67, F), fx::q(-9844.35, F), fx::q(9136.4, F), fx::q(-3272.62, F)};
-  constexpr long long kD[10] = {fx::q(0.632, F), fx::q(-40.97, F), fx::q(667.16, F), fx::q(-6072.07, F),
-                                fx::q(31127.39, F), fx::q(-96293.05, F), fx::q(181856.75, F), fx::q(-205690.43, F),
-                                fx::q(128170.2, F), fx::q(-33744.6, F)};
-  constexpr long long kdA[10] = {fx::q(2.948, F), fx::q(-24.53, F), fx::q(249.69, F), fx::q(-754.85, F),
-                                 fx::q(-1187.71, F), fx::q(16370.75, F), fx::q(-48811.41, F), fx::q(68220.87, F),
-                                 fx::q(-46688.0, F), fx::q(12622.25, F)};
-  constexpr long long kdB[10] = {fx::q(1.11, F), fx::q(2.894, F), fx::q(-76.765, F), fx::q(1565.35, F),
-                                 fx::q(-11336.19, F), fx::q(44270.15, F), fx::q(-97014.11, F), fx::q(118879.26, F),
-                                 fx::q(-76209.82, F), fx::q(19923.28, F)};
-  constexpr long long kdC[6] = {fx::q(14.19, F), fx::q(-148.24, F), fx::q(847.8, F), fx::q(-2318.58, F),
-                                fx::q(3168.35, F), fx::q(-1590.27, F)};
   const unsigned long long t = fx::unit_q64(rho);
-  f.A = fx::to_double(fx::horner_u(kA, t), F);
-  f.B = fx::to_double(fx::horner_u(kB, t), F);
-  f.C = fx::to_double(fx::horner_u(kC, t), F);
-  f.D = fx::to_double(fx::horner_u(kD, t), F);
-  f.dA = fx::to_double(fx::horner_u(kdA, t), F);
-  f.dB = fx::to_double(fx::horner_u(kdB, t), F);
-  f.dC = fx::to_double(fx::horner_u(kdC, t), F);
+  f.A = wu_fit(0, t);
+  f.B = wu_fit(1, t);
+  f.C = wu_fit(2, t);
+  f.D = wu_fit(3, t);
+  f.dA = wu_fit(4, t);
+  f.dB = wu_fit(5, t);
+  f.dC = wu_fit(6, t);
 }
 
 // StruveH0 and StruveH1 fits (wu.jl:368-435); also returns J0/J1.  The four Bessel
@@ -255,7 +268,7 @@ __device__ inline void struve_bessel(double xx, double inv_xx, double& H0, doubl
     const double c2 = kPi * xx * fx::to_double(fx::horner_u(kC2, t), G);
     const double d1 = fx::to_double(fx::horner_u(kD1, t), G);
     const double d2 = kPi * fx::to_double(fx::horner_u(kD2, t), G);
-    const double inv = fx::recip(c2 * d2);
+    const double inv = fx::recip_call(c2 * d2);
     H0 = c1 * d2 * inv + Y0;
     H1 = d1 * c2 * inv + Y1;
   }
@@ -268,8 +281,12 @@ __device__ inline void struve_bessel(double xx, double inv_xx, double& H0, doubl
 // and the square roots of the term, and are multiplied out (rho gets one residual
 // correction on top: an ulp of rho moves the fits A-D by up to 1e-13).  inv_hh: 1/hh for hh > 1e-6 (the only pairs
 // whose horizontal gradient factor k^2/hh is used, wu.jl:118-121), else 0.
-__device__ inline void wu_wave_term_and_derivs(double hh, double vv, double2& GF, double2& dGh, double2& dGv,
-                                               double* inv_hh = nullptr) {
+// `step` is called three times, by every thread: the wave assembly passes a CTA barrier that
+// keeps its warps on the same instructions.
+struct NoStep { __device__ __forceinline__ void operator()() const {} };
+template <typename Step = NoStep>
+__device__ __forceinline__ void wu_wave_term_and_derivs(double hh, double vv, double2& GF, double2& dGh, double2& dGv,
+                                                        double* inv_hh = nullptr, Step step = Step()) {
   double dd = fx::sqrt_pos(hh * hh + vv * vv);
   double dd2 = dd * dd, dd3 = dd * dd * dd;
   // 1/dd, 1/(dd - vv), 1/(1 + dd^3) and 1/hh from one division of their product (all
@@ -279,7 +296,7 @@ __device__ inline void wu_wave_term_and_derivs(double hh, double vv, double2& GF
   const bool has_h = fabs(hh) > 1e-6;
   const double hf = has_h ? hh : 1.0;
   const double prod3 = dd * dmv * opd3;
-  const double inv_all = fx::recip(prod3 * hf);
+  const double inv_all = fx::recip_call(prod3 * hf);
   const double inv_all3 = inv_all * hf;  // 1 / (dd dmv opd3)
   const double inv_dd = dmv * opd3 * inv_all3;
   const double inv_dmv = dd * opd3 * inv_all3;
@@ -291,20 +308,23 @@ __device__ inline void wu_wave_term_and_derivs(double hh, double vv, double2& GF
   // rho = dd / (1 + dd): the integer-pipe reciprocal and one residual correction, which
   // leaves rho within a rounding of the correctly rounded quotient
   const double opdd = 1 + dd;
-  const double r1 = fx::recip(opdd);
+  const double r1 = fx::recip_call(opdd);
   double rho = dd * r1;
   rho = fma(fma(-rho, opdd, dd), r1, rho);
   double omr = 1.0 - rho;
   double omr3 = omr * omr * omr;
   double ev = fx::exp_nonpos(vv);
   double H0, H1, J0, J1;
+  step();
   struve_bessel(hh, inv_h, H0, H1, J0, J1);
   // GF_Func_Lp
   WuFits fit;
+  step();
   wu_fits(rho, fit);
+  step();
   double RR = (1.0 - beta) * fit.A;
   RR -= beta * fit.B;
-  RR -= alpha * fit.C * fx::recip(1.0 + 6.0 * alpha * rho * (1.0 - rho));
+  RR -= alpha * fit.C * fx::recip_call(1.0 + 6.0 * alpha * rho * (1.0 - rho));
   RR += beta * (1.0 - beta) * fit.D;
   double Lp = rho * omr3 * RR;
   // GF_Func_L0
