@@ -424,9 +424,6 @@ __device__ __forceinline__ void store_pair(const AssemblyParams& p, const WaveTe
 // together, a barrier per column and between the term's parts; warps below the diagonal only
 // keep the count.  1750 panels 833 -> 635 us, thirty matrices of 2000 19.2 -> 15.7 ms; without the
 // barriers 5 % less; CTAs of 256 rows the same, of 512 15 % more (their tiles' last warps wait).
-struct CtaStep {
-  __device__ __forceinline__ void operator()() const { asm volatile("bar.sync 0;" ::: "memory"); }
-};
 constexpr int kWuSteps = 3;  // barriers inside wu_wave_term_and_derivs
 template <bool DIRECT, int WMODE>  // WMODE 1 = Wu only, 2 = exact Delhommeau, 3 = both
 __global__ void __launch_bounds__(kRowsPerCta) wave_kernel(AssemblyParams p, const double* SR, const double* DR,
@@ -885,7 +882,7 @@ void launch_panel_geometry(cudaStream_t st, LaunchCounter lc, int64_t n, const d
 // columns per CTA of the pair kernels: 8, fewer where the launch (`tiles` CTAs of one column each)
 // would not give every SM 16 CTAs (about four rounds of the resident ones, so that a last round
 // that is partly empty costs little)
-static int columns_per_cta(int64_t tiles) {
+int columns_per_cta(int64_t tiles) {
   return (int)std::max<int64_t>(1, std::min<int64_t>(kColsPerCta, tiles / (16 * 152)));
 }
 

@@ -73,7 +73,7 @@ template <int M> __device__ __forceinline__ Dn<M> operator*(const Dn<M>& a, cons
 // Divisions, square roots, exponentials and logarithms of the wave terms run on the integer pipe
 // (mh_fixpoint.cuh; every divisor and argument there is positive, every exponent <= 0), within
 // an ulp or two.  The panel frames' (birk_geometry_t) divisors take either sign: pos_recip.
-__device__ __forceinline__ double pos_recip(double x) { return x > 0.0 ? fx::recip(x) : 1.0 / x; }
+static __device__ __noinline__ double pos_recip(double x) { return x > 0.0 ? fx::recip(x) : 1.0 / x; }
 template <int M> __device__ __forceinline__ Dn<M> operator/(const Dn<M>& a, const Dn<M>& b) {
   const double inv = pos_recip(b.v), rv = a.v * inv;
   Dn<M> r(rv);
@@ -109,18 +109,4 @@ template <int M> __device__ __forceinline__ Dn<M> exp(const Dn<M>& a) {  // a <=
   const double e = fx::exp_nonpos(a.v);
   return chain1(a, e, e);
 }
-// J0, J1 (and Y0, Y1 for x >= 3) from one joint evaluation (mh_bessel01.cuh), with
-// J0' = -J1, J1' = J0 - J1/x (1/2 at 0), Y0' = -Y1, Y1' = Y0 - Y1/x
-template <int M>
-__device__ __forceinline__ void bessel01_t(const Dn<M>& a, Dn<M>& J0, Dn<M>& J1, Dn<M>& Y0, Dn<M>& Y1) {
-  const double x = a.v;
-  double j0v, j1v, y0v, y1v;
-  bessel01(x, j0v, j1v, y0v, y1v);
-  const double inv_x = x != 0.0 ? fx::recip(x) : 0.0;
-  J0 = chain1(a, j0v, -j1v);
-  J1 = chain1(a, j1v, x != 0.0 ? j0v - j1v * inv_x : 0.5);
-  Y0 = chain1(a, y0v, -y1v);
-  Y1 = chain1(a, y1v, y0v - y1v * inv_x);
-}
-
 }  // namespace mh

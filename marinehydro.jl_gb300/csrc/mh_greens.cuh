@@ -284,6 +284,9 @@ __device__ inline void struve_bessel(double xx, double inv_xx, double& H0, doubl
 // `step` is called three times, by every thread: the wave assembly passes a CTA barrier that
 // keeps its warps on the same instructions.
 struct NoStep { __device__ __forceinline__ void operator()() const {} };
+struct CtaStep {
+  __device__ __forceinline__ void operator()() const { asm volatile("bar.sync 0;" ::: "memory"); }
+};
 template <typename Step = NoStep>
 __device__ __forceinline__ void wu_wave_term_and_derivs(double hh, double vv, double2& GF, double2& dGh, double2& dGv,
                                                         double* inv_hh = nullptr, Step step = Step()) {

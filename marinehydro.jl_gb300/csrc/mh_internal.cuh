@@ -116,6 +116,7 @@ struct AssemblyParams {
 
 // Static (wavenumber-independent) part into real n x n arrays SR, DR (identity included when asked).
 // step 2 (Birk kinds only): into the real parts of complex arrays, the imaginary parts zeroed
+int columns_per_cta(int64_t tiles);
 void launch_assemble_static(cudaStream_t st, LaunchCounter lc, const AssemblyParams& p, double* SR, double* DR,
                             int step = 1);
 // S = SR + S_wave(k), D = DR + D_wave(k) (complex); SR/DR may be null (no static part).

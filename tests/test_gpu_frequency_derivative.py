@@ -44,6 +44,20 @@ def test_derivative_matches_central_differences(mh, ctx, direct):
             assert close(res["d_" + k], fd[k], 1e-6), (om, k)
 
 
+@pytest.mark.parametrize("direct", [True, False])
+@pytest.mark.parametrize("rings, around", [(3, 11), (5, 26), (4, 33), (7, 37)])
+def test_derivative_across_row_tiles(mh, ctx, rings, around, direct):
+    # 33, 130, 132 and 259 panels: one and several 128-row tiles, a last warp of one to four rows
+    body = mh.FloatingBody(mh.hemisphere_mesh(1.0, rings, around), ["Surge", "Heave"])
+    F = mh.DirectBEM() if direct else mh.IndirectBEM()
+    params = {"wave_frequencies": [1.7], "radiating_dofs": ["Surge", "Heave"], "wave_directions": [0.3]}
+    res = mh.hydrodynamic_coefficients_derivative(body, params, F, ctx=ctx, rho=1025.0)
+    fd = _fd(lambda w: mh.hydrodynamic_coefficients(body, dict(params, wave_frequencies=[w]), F, ctx=ctx, rho=1025.0),
+             1.7, 1.7e-5)
+    for k in KEYS:
+        assert close(res["d_" + k], fd[k], 1e-6), k
+
+
 def test_derivative_with_lid_and_several_frequencies(mh, ctx):
     hull = mh.vertical_cylinder_mesh(1.0, 1.0, n_theta=20, n_z=6, n_r=4)
     lid = mh.disc_lid_mesh(1.0, -0.15, n_theta=20, n_r=4)
