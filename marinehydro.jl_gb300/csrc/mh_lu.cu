@@ -16,7 +16,7 @@
 //                  tall for the cluster's shared memory
 //   laswp_kernel   the panel's row interchanges applied to every column outside it,
 //                  as one permutation of at most 64 rows (a warp per column)
-//   trsm8_kernel, trsm_kernel   U12 = L11^-1 A12 with L11 in shared memory: eight lanes
+//   trsm_lanes_kernel, trsm_kernel   U12 = L11^-1 A12 with L11 in shared memory: 8 or 32 lanes
 //                  per column in FP64, one thread per column in FP32
 //   gemm3m_kernel, gemm_kernel  A22 -= L21 U12 on the CUDA cores (FP64, FP32)
 // Templated on the real type: double (the plain FP64 path) and float (the factor
@@ -640,43 +640,48 @@ __global__ void __launch_bounds__(128) trsm_second_kernel(BatchDesc d, float2* _
   for (int r = 0; r < kNB; ++r) col[kNB + r] = x[r];
 }
 
-// FP64: eight lanes per column, lane r8 holding rows r8, r8 + 8, ..; the column-oriented
-// substitution broadcasts x_q within the eight and every lane updates its rows below q.  One
-// thread per column (trsm_kernel) runs 1984 FP64 FMAs in a row, each a 64-cycle issue of one of
-// the SM's four FP64 pipes, on a few warps in all: 74 us whatever the width; here the same
-// columns spread over eight times the warps with 320 FMAs each: 25 us at up to five matrices
-// of order 1000.
-constexpr int kTrsmCols = 32;  // columns per CTA of 256 threads
-__global__ void __launch_bounds__(8 * kTrsmCols) trsm8_kernel(BatchDesc d, double2* __restrict__ Aall, int64_t k) {
+// FP64: LANES (8 or 32) lanes per column, lane l holding rows l, l + LANES, ..; the column-oriented
+// substitution broadcasts x_q within them and every lane updates its rows below q.  A warp gets
+// one FP64 instruction per 77 cycles and an SM one per 19, so with few columns the chain counts:
+// one thread per column (trsm_kernel) runs 1984 FMAs in a row, 74 us whatever the width, eight lanes
+// 320 in 23 us, 32 lanes 124 in 12 us while every SM has one CTA of eight columns and in 20 us while it
+// has two.  With more columns the pipe counts, and eight lanes waste less of it (four columns share
+// a warp's instruction): 2400 columns in all 23.5 us with eight lanes against 28.6 with 32.
+constexpr int kTrsmThreads = 256;
+constexpr int64_t kTrsmFewColumns = 2 * 152 * (kTrsmThreads / 32);
+template <int LANES>
+__global__ void __launch_bounds__(kTrsmThreads) trsm_lanes_kernel(BatchDesc d, double2* __restrict__ Aall, int64_t k) {
+  constexpr int kRowsPer = kNB / LANES, kCols = kTrsmThreads / LANES;
   __shared__ double2 sL[kNB][kNB + 1];
   const int64_t n = d.order(blockIdx.y), ncols = n + d.extra;
   if (k >= n) return;  // this matrix is factored (grouped batches)
   double2* A = Aall + d.offset(blockIdx.y);
   const int kb = (int)((k + kNB < n) ? kNB : n - k);
-  if (k + kb >= ncols) return;  // nothing right of the panel
+  if (k + kb + blockIdx.x * (int64_t)kCols >= ncols) return;  // nothing right of the panel here
   for (int idx = threadIdx.x; idx < kNB * kNB; idx += blockDim.x) {
     const int r = idx & (kNB - 1), q = idx / kNB;
     sL[r][q] = (r < kb && q < kb) ? A[(k + r) + (k + q) * n] : make_double2(0.0, 0.0);
   }
   __syncthreads();
-  const int64_t c = k + kb + blockIdx.x * (int64_t)kTrsmCols + (threadIdx.x >> 3);
+  const int64_t c = k + kb + blockIdx.x * (int64_t)kCols + threadIdx.x / LANES;
   const bool live = c < ncols;
-  const int r8 = threadIdx.x & 7, base = threadIdx.x & 24;  // first lane of this column's eight
-  double2 x[4];
+  const int l = threadIdx.x & (LANES - 1), base = threadIdx.x & 31 & ~(LANES - 1);  // first lane of this column
+  double2 x[kRowsPer];
 #pragma unroll
-  for (int t = 0; t < 4; ++t) x[t] = (live && r8 + 8 * t < kb) ? A[(k + r8 + 8 * t) + c * n] : make_double2(0.0, 0.0);
+  for (int t = 0; t < kRowsPer; ++t)
+    x[t] = (live && l + LANES * t < kb) ? A[(k + l + LANES * t) + c * n] : make_double2(0.0, 0.0);
 #pragma unroll
   for (int q = 0; q < kNB - 1; ++q) {
-    const double2 xq = shfl_c(x[q >> 3], base | (q & 7));
+    const double2 xq = shfl_c(x[q / LANES], base | (q & (LANES - 1)));
 #pragma unroll
-    for (int t = q >> 3; t < 4; ++t) {
-      const int r = r8 + 8 * t;
+    for (int t = q / LANES; t < kRowsPer; ++t) {
+      const int r = l + LANES * t;
       if (r > q) x[t] = cfms(x[t], sL[r][q], xq);
     }
   }
 #pragma unroll
-  for (int t = 0; t < 4; ++t)
-    if (live && r8 + 8 * t < kb) A[(k + r8 + 8 * t) + c * n] = x[t];
+  for (int t = 0; t < kRowsPer; ++t)
+    if (live && l + LANES * t < kb) A[(k + l + LANES * t) + c * n] = x[t];
 }
 
 // ------------------------------ trailing update -------------------------------
@@ -1642,8 +1647,11 @@ int lu_factor_batched(cudaStream_t st, LaunchCounter lc, const BatchDesc& d, typ
     }
     if (!trsm_done) {
       if constexpr (sizeof(T) == 8) {
-        dim3 tg((unsigned)((rest_c + kTrsmCols - 1) / kTrsmCols), (unsigned)d.batch);
-        MH_LAUNCH(lc, st, "lu_trsm_f64", trsm8_kernel<<<tg, 8 * kTrsmCols, 0, st>>>(d, A, k));
+        const bool few = rest_c * d.batch <= kTrsmFewColumns;
+        const int64_t cols = kTrsmThreads / (few ? 32 : 8);
+        dim3 tg((unsigned)((rest_c + cols - 1) / cols), (unsigned)d.batch);
+        if (few) MH_LAUNCH(lc, st, "lu_trsm_f64", trsm_lanes_kernel<32><<<tg, kTrsmThreads, 0, st>>>(d, A, k));
+        else MH_LAUNCH(lc, st, "lu_trsm_f64", trsm_lanes_kernel<8><<<tg, kTrsmThreads, 0, st>>>(d, A, k));
       } else {
         dim3 tg((unsigned)((rest_c + 127) / 128), (unsigned)d.batch);
         MH_LAUNCH(lc, st, "lu_trsm_f32", trsm_kernel<T><<<tg, 128, 0, st>>>(d, A, k));
