@@ -21,7 +21,7 @@ import numpy as np
 from . import _device, _lib
 from .bodies import FloatingBody, evaluate_gradient_of_motion
 from .formulations import BEMFormulation, DirectBEM, SurrogateDelhommeau, bem_formulation, gf_flags, is_direct
-from .meshes import StaticArraysMesh, face_fields, face_fields_jacobian
+from .meshes import StaticArraysMesh, face_fields, face_fields_pullback
 from .problems import (DiffractionProblem, DiffractionResult, RadiationProblem, RadiationResult, SETTINGS,
                        added_mass, compute_wavenumber, make_result, radiation_damping)
 
@@ -504,9 +504,7 @@ def _vertex_gradient(body, gc, gn, ga, gv, gd_by_name):
             e = np.zeros(3)
             e[ax] = 1.0
             gc[p0:p1] += np.cross(gdn[p0:p1], e)
-    dC, dN, dA = face_fields_jacobian(mesh.panel_vertices)
-    corner = (np.einsum("ik,ikq->iq", gc, dC) + np.einsum("ik,ikq->iq", gn, dN) + ga[:, None] * dA
-              + gv.reshape(-1, 12))
+    corner = face_fields_pullback(mesh.panel_vertices, gc, gn, ga) + gv.reshape(-1, 12)
     grad = np.zeros_like(mesh.vertices)
     faces0 = mesh.faces - 1
     for q in range(4):

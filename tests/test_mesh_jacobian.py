@@ -36,3 +36,18 @@ def test_rotation_metadata_follows_combination(mh):
     c = a + b
     na = a.mesh.nfaces
     assert c.rotations == {"a__Pitch": (1, (0.0, 0.0, -1.0), 0, na), "b__Yaw": (2, (0.0, 0.0, 0.0), na, c.mesh.nfaces)}
+
+
+def test_pullback_contracts_the_jacobians(mh):
+    # quads, warped quads and the triangles of an apex; the contraction has 12 * 7 terms of order one,
+    # and both sides are exact to rounding
+    rng = np.random.default_rng(5)
+    mesh = mh.hemisphere_mesh(1.0, 5, 9)
+    V = mesh.panel_vertices.copy()
+    quads = ~np.all(V[:, 2] == V[:, 3], axis=1)
+    V[quads] += 0.02 * rng.standard_normal(V[quads].shape)
+    gc, gn, ga = rng.standard_normal((len(V), 3)), rng.standard_normal((len(V), 3)), rng.standard_normal(len(V))
+    dC, dN, dA = mh.face_fields_jacobian(V)
+    ref = np.einsum("ik,ikq->iq", gc, dC) + np.einsum("ik,ikq->iq", gn, dN) + ga[:, None] * dA
+    got = mh.meshes.face_fields_pullback(V, gc, gn, ga)
+    assert not quads.all() and np.abs(got - ref).max() <= 1e-13 * np.abs(ref).max()
