@@ -612,7 +612,8 @@ __global__ void __launch_bounds__(128) trsm_kernel(BatchDesc d, typename cplx_t<
 // k + 64): L22^-1 (A - L21 Ua), Ua the first panel's U12 already in place; one thread per column.
 __global__ void __launch_bounds__(128) trsm_second_kernel(BatchDesc d, float2* __restrict__ Aall, int64_t k) {
   __shared__ float2 sL[2 * kNB][kNB];  // rows k + 32 .. of columns k .. k + 63, by column
-  const int64_t n = d.n;
+  const int64_t n = d.order(blockIdx.y);
+  if (k + 2 * kNB >= n) return;  // a grouped batch: no column of this matrix is right of both panels
   float2* A = Aall + d.offset(blockIdx.y);
   for (int idx = threadIdx.x; idx < 2 * kNB * kNB; idx += blockDim.x) {
     const int r = idx & (kNB - 1), q = idx / kNB;

@@ -107,3 +107,18 @@ def test_batch_after_a_mesh_is_destroyed(mh, ctx):
         for h in list(body.mesh._handles.values()):
             h.close()
         body.mesh._handles.clear()
+
+
+@pytest.mark.parametrize("direct", [True, False])
+def test_batch_with_two_panels_per_update(mh, ctx, direct):
+    # one class of orders 1230, 1261 and 1300 with 8 frequencies each: the first updates take two
+    # panels at once, and the smaller matrices' trailing blocks are ragged against the largest's
+    bodies = [mh.FloatingBody(mh.hemisphere_mesh(1.0, r, c), ["Heave", "Pitch"], rotation_center=(0.0, 0.0, 0.0),
+                              body_name=f"h{r}") for r, c in ((30, 41), (13, 97), (26, 50))]
+    F = (mh.DirectBEM if direct else mh.IndirectBEM)(precision="mixed")
+    p = {"wave_frequencies": np.linspace(0.5, 2.4, 8), "radiating_dofs": ["Heave", "Pitch"],
+         "influenced_dofs": ["Heave", "Pitch"], "wave_directions": [0.3]}
+    out = mh.batch_hydrodynamic_coefficients(bodies, [p] * 3, F, ctx=ctx, rho=1025.0)
+    for body, res in zip(bodies, out):
+        _check(res, mh.hydrodynamic_coefficients(body, p, mh.DirectBEM(precision="fp64_tc") if direct else
+                                                 mh.IndirectBEM(precision="fp64_tc"), ctx=ctx, rho=1025.0))
