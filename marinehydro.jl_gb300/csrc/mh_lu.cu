@@ -1532,19 +1532,13 @@ int panel_cluster_size(int64_t m, int64_t batch, int cap_ctas, int width = kNB) 
   return p;
 }
 
-// Whether the FP64 tensor-core path factors the panel of m rows in two halves of 16 columns: when
-// its clusters do not run for all `batch` matrices at once (its rows then run in waves), or when
-// each CTA has so many rows that half of the panel's FP64 work (the FP64 pipe's 124 FMAs per row
-// at the first column) is worth more than the five small launches in between.  Thirty matrices of 2000
-// in all 60.8 ms without the rule, 60.2 / 60.0 / 59.95 / 60.0 / 60.1 from 300 / 220 / 160 / 110 / 80 rows
-// on; one of 4000 32.3, and 32.3 / 31.8 / 31.4 / 31.5 / 31.8; one of 1500 7.66, from 80 rows on 7.90.
-constexpr int kHalvesRows = 160;
+// true when the full-width panel of m rows runs its clusters for all `batch` matrices at once
+// (its rows need at most as many CTAs per matrix as fit every cluster on the GPU); a panel that
+// does not fit runs in waves, and the FP64 tensor-core path factors it in two halves instead
 template <typename T>
-bool panel_in_halves(int64_t m, int64_t batch, int cap_ctas) {
+bool panel_fits_one_wave(int64_t m, int64_t batch) {
   const int need = panel_least_ctas<T>(m);
-  if (need <= 0 || panel_residency<T>(kNB)[need] < batch) return true;
-  const int P = panel_cluster_size<T>(m, batch, cap_ctas);
-  return P > 0 && m >= (int64_t)P * kHalvesRows;
+  return need > 0 && panel_residency<T>(kNB)[need] >= batch;
 }
 
 template <typename T>
@@ -1622,7 +1616,7 @@ int lu_factor_batched(cudaStream_t st, LaunchCounter lc, const BatchDesc& d, typ
     // cores -- half the panel's FP64 work, and half its shared memory per row
     int Pl = 0, P16 = 0;
     if constexpr (sizeof(T) == 8) {
-      if (emu_ws && kb == kNB && !d.orders && panel_in_halves<T>(n - k, d.batch, cap_ctas)) {
+      if (emu_ws && kb == kNB && !d.orders && !panel_fits_one_wave<T>(n - k, d.batch)) {
         Pl = panel_cluster_size<T>(n - k, d.batch, cap_ctas, kNB / 2);
         P16 = panel_cluster_size<T>(n - k - kNB / 2, d.batch, cap_ctas, kNB / 2);
       }
