@@ -53,44 +53,46 @@ template <typename R> struct CR { R x, y; };
 // multiples of the fixed-point ones: as doubles (7 * 205690.43 ..) they would round by up to
 // 1e-10, the same way in every pair, and the added mass' frequency derivative would be off by
 // 2e-14 instead of 8e-15.
-static __device__ __constant__ const long long kWuDual[14][8] = {
-    {fx::q(215.896, 47), fx::q(-1763.96, 47), fx::q(8418.94, 47), fx::q(-24314.21, 47), fx::q(42002.57, 47),
-     fx::q(-41592.9, 47), fx::q(21859.0, 47), fx::q(-4838.6, 47)},
-    {fx::q(-67.92, 47), fx::q(796.534, 47), fx::q(-4780.77, 47), fx::q(17137.74, 47), fx::q(-36618.81, 47),
-     fx::q(44894.06, 47), fx::q(-29030.24, 47), fx::q(7671.22, 47)},
-    {fx::q(209.653, 49), fx::q(-1397.89, 49), fx::q(5155.67, 49), fx::q(-9844.35, 49), fx::q(9136.4, 49),
-     fx::q(-3272.62, 49) - 1, 0, 0},
-    {fx::q(667.16, 45), fx::q(-6072.07, 45), fx::q(31127.39, 45), fx::q(-96293.05, 45), fx::q(181856.75, 45),
-     fx::q(-205690.43, 45), fx::q(128170.2, 45), fx::q(-33744.6, 45)},
-    {fx::q(249.69, 46), fx::q(-754.85, 46), fx::q(-1187.71, 46), fx::q(16370.75, 46), fx::q(-48811.41, 46),
-     fx::q(68220.87, 46), fx::q(-46688.0, 46), fx::q(12622.25, 46)},
-    {fx::q(-76.765, 46), fx::q(1565.35, 46), fx::q(-11336.19, 46), fx::q(44270.15, 46), fx::q(-97014.11, 46),
-     fx::q(118879.26, 46), fx::q(-76209.82, 46), fx::q(19923.28, 46)},
-    {fx::q(847.8, 51), fx::q(-2318.58, 51), fx::q(3168.35, 51), fx::q(-1590.27, 51) - 1, 0, -1, 0, 0},
-    {3 * fx::q(-1763.96, 44), 4 * fx::q(8418.94, 44), 5 * fx::q(-24314.21, 44), 6 * fx::q(42002.57, 44),
-     7 * fx::q(-41592.9, 44), 8 * fx::q(21859.0, 44), 9 * fx::q(-4838.6, 44), 0},
-    {3 * fx::q(796.534, 44), 4 * fx::q(-4780.77, 44), 5 * fx::q(17137.74, 44), 6 * fx::q(-36618.81, 44),
-     7 * fx::q(44894.06, 44), 8 * fx::q(-29030.24, 44), 9 * fx::q(7671.22, 44), 0},
-    {3 * fx::q(-1397.89, 47), 4 * fx::q(5155.67, 47), 5 * fx::q(-9844.35, 47), 6 * fx::q(9136.4, 47),
-     7 * fx::q(-3272.62, 47), -1, 0, 0},
-    {3 * fx::q(-6072.07, 42), 4 * fx::q(31127.39, 42), 5 * fx::q(-96293.05, 42), 6 * fx::q(181856.75, 42),
-     7 * fx::q(-205690.43, 42), 8 * fx::q(128170.2, 42), 9 * fx::q(-33744.6, 42), 0},
-    {3 * fx::q(-754.85, 44), 4 * fx::q(-1187.71, 44), 5 * fx::q(16370.75, 44), 6 * fx::q(-48811.41, 44),
-     7 * fx::q(68220.87, 44), 8 * fx::q(-46688.0, 44), 9 * fx::q(12622.25, 44), 0},
-    {3 * fx::q(1565.35, 43), 4 * fx::q(-11336.19, 43), 5 * fx::q(44270.15, 43), 6 * fx::q(-97014.11, 43),
-     7 * fx::q(118879.26, 43), 8 * fx::q(-76209.82, 43), 9 * fx::q(19923.28, 43), 0},
-    {3 * fx::q(-2318.58, 49), 4 * fx::q(3168.35, 49), 5 * fx::q(-1590.27, 49), -1, 0, -1, 0, 0}};
-static __device__ __constant__ const double kWuDualLow[14][2] = {
-    {1.21, -13.328}, {0.938, 5.737}, {1.268, -9.747}, {0.632, -40.97}, {2.948, -24.53}, {1.11, 2.894}, {14.19, -148.24}, {-13.328, 2 * 215.896}, {5.737, 2 * -67.92}, {-9.747, 2 * 209.653}, {-40.97, 2 * 667.16}, {-24.53, 2 * 249.69}, {2.894, 2 * -76.765}, {-148.24, 2 * 847.8}};
-static __device__ __constant__ const int kWuDualFrac[14] = {47, 47, 49, 45, 46, 46, 51, 44, 44, 47, 42, 44, 43, 49};
+constexpr double kWuCoef[7][10] = {
+    {1.21, -13.328, 215.896, -1763.96, 8418.94, -24314.21, 42002.57, -41592.9, 21859.0, -4838.6},        // A
+    {0.938, 5.737, -67.92, 796.534, -4780.77, 17137.74, -36618.81, 44894.06, -29030.24, 7671.22},        // B
+    {1.268, -9.747, 209.653, -1397.89, 5155.67, -9844.35, 9136.4, -3272.62},                             // C
+    {0.632, -40.97, 667.16, -6072.07, 31127.39, -96293.05, 181856.75, -205690.43, 128170.2, -33744.6},   // D
+    {2.948, -24.53, 249.69, -754.85, -1187.71, 16370.75, -48811.41, 68220.87, -46688.0, 12622.25},       // dA
+    {1.11, 2.894, -76.765, 1565.35, -11336.19, 44270.15, -97014.11, 118879.26, -76209.82, 19923.28},     // dB
+    {14.19, -148.24, 847.8, -2318.58, 3168.35, -1590.27}};                                               // dC
+struct WuDualTable {
+  long long c[14][8];  // the seven fits', then their derivatives', coefficients from rho^2 up
+  double low[14][2];
+  int frac[14];
+};
+constexpr WuDualTable make_wu_dual_table() {
+  constexpr int degree[7] = {9, 9, 7, 9, 9, 9, 5};
+  constexpr int frac[14] = {47, 47, 49, 45, 46, 46, 51, 44, 44, 47, 42, 44, 43, 49};
+  WuDualTable t{};
+  for (int w = 0; w < 14; ++w) {
+    const int der = w >= 7, top = degree[w % 7] - 2 - der;
+    const double* c = kWuCoef[w % 7];
+    t.frac[w] = frac[w];
+    t.low[w][0] = c[der];
+    t.low[w][1] = (1 + der) * c[1 + der];
+    for (int i = 0; i <= top; ++i) t.c[w][i] = (der ? i + 3 : 1) * fx::q(c[i + 2 + der], frac[w]);
+    // a shorter fit starts from zeros: what the half units of horner_u_mid would add to them (every
+    // odd coefficient but the first of all) is taken off again
+    for (int i = top < 7 ? top : 7; i < 7; ++i)
+      if (i & 1) t.c[w][i] -= 1;
+  }
+  return t;
+}
+static __device__ __constant__ const WuDualTable kWuDual = make_wu_dual_table();
 
 // called fourteen times (inlined, the fits outgrow the instruction caches; see wu_fit in
 // mh_greens.cuh)
 static __device__ __noinline__ double wu_dual_fit(int which, double rho, unsigned long long t) {
-  long long v = kWuDual[which][7];
+  long long v = kWuDual.c[which][7];
 #pragma unroll
-  for (int i = 6; i >= 0; --i) v = kWuDual[which][i] + (i & 1) + fx::mulhi_su(v, t);
-  return fma(fma(fx::to_double(v, kWuDualFrac[which]), rho, kWuDualLow[which][1]), rho, kWuDualLow[which][0]);
+  for (int i = 6; i >= 0; --i) v = kWuDual.c[which][i] + (i & 1) + fx::mulhi_su(v, t);
+  return fma(fma(fx::to_double(v, kWuDual.frac[which]), rho, kWuDual.low[which][1]), rho, kWuDual.low[which][0]);
 }
 __device__ __forceinline__ void wu_fits_and_derivatives(double rho, WuFits& f, WuFits& d) {
   const unsigned long long t = fx::unit_q64(rho);
@@ -110,6 +112,29 @@ __device__ __forceinline__ void wu_fits_and_derivatives(double rho, WuFits& f, W
   d.dC = wu_dual_fit(13, rho, t);
 }
 
+// sum c_i t^i, its derivative, and the derivative of t times it
+template <int N>
+__device__ __forceinline__ double poly(const double (&c)[N], double t) {
+  double v = c[N - 1];
+#pragma unroll
+  for (int i = N - 2; i >= 0; --i) v = fma(v, t, c[i]);
+  return v;
+}
+template <int N>
+__device__ __forceinline__ double poly_d(const double (&c)[N], double t) {
+  double v = (N - 1) * c[N - 1];
+#pragma unroll
+  for (int i = N - 2; i >= 1; --i) v = fma(v, t, i * c[i]);
+  return v;
+}
+template <int N>
+__device__ __forceinline__ double poly_td(const double (&c)[N], double t) {
+  double v = N * c[N - 1];
+#pragma unroll
+  for (int i = N - 2; i >= 0; --i) v = fma(v, t, (i + 1) * c[i]);
+  return v;
+}
+
 // StruveH0 and StruveH1 fits (wu.jl:368-435) and J0, J1 of one argument: the values and the
 // derivatives as plain numbers, the dual's directions multiplied on at the end (J0' = -J1, J1' =
 // J0 - J1/x, Y0' = -Y1, Y1' = Y0 - Y1/x)
@@ -122,27 +147,22 @@ __device__ __forceinline__ void struve_bessel_t(const R& hh, R& H0, R& H1, R& J0
   J0 = chain1(hh, j0, -j1);
   J1 = chain1(hh, j1, x != 0.0 ? fma(-j1, inv_x, j0) : 0.5);
   if (x <= 3.0) {
+    constexpr double kP[6] = {1.909859164, -1.909855001, 0.687514637, -0.126164557, 0.013828813, -0.000876918};
+    constexpr double kQ[6] = {1.909859286, -1.145914713, 0.294656958, -0.042070508, 0.003785727, -0.000207183};
     const double x3 = x * (1.0 / 3.0), yy = x3 * x3;
-    const double p = fma(fma(fma(fma(fma(-0.000876918, yy, 0.013828813), yy, -0.126164557), yy, 0.687514637), yy,
-                             -1.909855001), yy, 1.909859164);
-    const double dp = fma(fma(fma(fma(5 * -0.000876918, yy, 4 * 0.013828813), yy, 3 * -0.126164557), yy,
-                              2 * 0.687514637), yy, -1.909855001);
-    const double q = fma(fma(fma(fma(fma(-0.000207183, yy, 0.003785727), yy, -0.042070508), yy, 0.294656958), yy,
-                             -1.145914713), yy, 1.909859286);
-    const double dq = fma(fma(fma(fma(6 * -0.000207183, yy, 5 * 0.003785727), yy, 4 * -0.042070508), yy,
-                              3 * 0.294656958), yy, 2 * -1.145914713);  // (q yy)' = q0 + dq yy
+    const double p = poly(kP, yy), dp = poly_d(kP, yy), q = poly(kQ, yy);
     H0 = chain1(hh, p * x3, fma(2.0 * yy, dp, p) * (1.0 / 3.0));
-    H1 = chain1(hh, q * yy, fma(dq, yy, 1.909859286) * (2.0 / 3.0) * x3);
+    H1 = chain1(hh, q * yy, poly_td(kQ, yy) * (2.0 / 3.0) * x3);
   } else {
+    constexpr double kA[4] = {0.99999906, 4.77228920, 3.85542044, 0.32303607};
+    constexpr double kB[3] = {4.88331068, 4.28957333, 0.52120508};  // after 1
+    constexpr double kC[4] = {1.00000004, 3.92205313, 2.64893033, 0.27450895};
+    constexpr double kD[3] = {3.81095112, 2.26216956, 0.10885141};
     const double t3 = 3.0 * inv_x, yy = t3 * t3, dy = -2.0 * yy * inv_x;
-    const double c1 = 2.0 * fma(fma(fma(0.32303607, yy, 3.85542044), yy, 4.77228920), yy, 0.99999906);
-    const double dc1 = 2.0 * fma(fma(3 * 0.32303607, yy, 2 * 3.85542044), yy, 4.77228920) * dy;
-    const double e2 = kPi * fma(fma(fma(0.52120508, yy, 4.28957333), yy, 4.88331068), yy, 1.0);
-    const double de2 = kPi * fma(fma(3 * 0.52120508, yy, 2 * 4.28957333), yy, 4.88331068) * dy;
-    const double d1 = 2.0 * fma(fma(fma(0.27450895, yy, 2.64893033), yy, 3.92205313), yy, 1.00000004);
-    const double dd1 = 2.0 * fma(fma(3 * 0.27450895, yy, 2 * 2.64893033), yy, 3.92205313) * dy;
-    const double d2 = kPi * fma(fma(fma(0.10885141, yy, 2.26216956), yy, 3.81095112), yy, 1.0);
-    const double dd2 = kPi * fma(fma(3 * 0.10885141, yy, 2 * 2.26216956), yy, 3.81095112) * dy;
+    const double c1 = 2.0 * poly(kA, yy), dc1 = 2.0 * poly_d(kA, yy) * dy;
+    const double e2 = kPi * fma(poly(kB, yy), yy, 1.0), de2 = kPi * poly_td(kB, yy) * dy;
+    const double d1 = 2.0 * poly(kC, yy), dd1 = 2.0 * poly_d(kC, yy) * dy;
+    const double d2 = kPi * fma(poly(kD, yy), yy, 1.0), dd2 = kPi * poly_td(kD, yy) * dy;
     // c2 = x e2
     const double inv_c2 = fx::recip_call(e2) * inv_x, inv_d2 = fx::recip_call(d2);
     const double r = c1 * inv_c2, s = d1 * inv_d2;
