@@ -77,8 +77,8 @@ constexpr WuDualTable make_wu_dual_table() {
     t.low[w][0] = c[der];
     t.low[w][1] = (1 + der) * c[1 + der];
     for (int i = 0; i <= top; ++i) t.c[w][i] = (der ? i + 3 : 1) * fx::q(c[i + 2 + der], frac[w]);
-    // a shorter fit starts from zeros: what the half units of horner_u_mid would add to them (every
-    // odd coefficient but the first of all) is taken off again
+    // a shorter fit starts from zeros: what wu_dual_fit's half units add to them (every odd
+    // coefficient) is taken off again
     for (int i = top < 7 ? top : 7; i < 7; ++i)
       if (i & 1) t.c[w][i] -= 1;
   }
@@ -86,8 +86,10 @@ constexpr WuDualTable make_wu_dual_table() {
 }
 static __device__ __constant__ const WuDualTable kWuDual = make_wu_dual_table();
 
-// called fourteen times (inlined, the fits outgrow the instruction caches; see wu_fit in
-// mh_greens.cuh)
+// Horner's scheme without the bias of fx::horner_u: every step rounds down by half a unit on average,
+// which every other coefficient makes up for with one unit.  A sum over many pairs would not
+// average the bias out, as it does the rounding itself.  Called fourteen times (inlined, the fits
+// outgrow the instruction caches; see wu_fit in mh_greens.cuh).
 static __device__ __noinline__ double wu_dual_fit(int which, double rho, unsigned long long t) {
   long long v = kWuDual.c[which][7];
 #pragma unroll

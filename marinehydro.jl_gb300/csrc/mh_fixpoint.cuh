@@ -282,17 +282,6 @@ __device__ __forceinline__ long long horner_u(const long long (&c)[N], unsigned 
   return v;
 }
 
-// horner_u without its bias: every step rounds down by half a unit on average, which every other
-// coefficient makes up for with one unit (the constants fold at compile time).  A sum over many
-// pairs would not average the bias out, as it does the rounding itself.
-template <int N>
-__device__ __forceinline__ long long horner_u_mid(const long long (&c)[N], unsigned long long t) {
-  long long v = c[N - 1];
-#pragma unroll
-  for (int i = N - 2; i >= 0; --i) v = c[i] + (i & 1) + mulhi_su(v, t);
-  return v;
-}
-
 // sum_i c[i] z^i for z in [-1/2, 1/2) given as z 2^64 (coefficients in a constant bank or
 // registers)
 template <int N>

@@ -25,8 +25,8 @@
 //   zgemv_reduce_kernel: the splits' sums, in order.
 // Bound: the integer pipe that cuts the digits (45 instructions per value) and the epilogue; the
 // products run under the cutting of the next half.  Four matrices of order 8000 with four
-// right-hand sides 4.03 -> 2.45 ms (6.6 of the 8.1 us per block were the cutting and the wait for
-// the products in turn; splits alone fill the last wave: 3.19), four of 1400 365 -> 92 us and
+// right-hand sides 4.03 -> 2.45 ms (8.1 us per block with the cutting and the products in turn; splits
+// and the shorter cutting alone 3.19), four of 1400 365 -> 92 us and
 // twelve of 430 122 -> 37 us (44 and 48 CTAs became 132 and 144), five of 640 167 -> 20 us.
 // Every wait is bounded; on timeout the kernel raises the caller's flag, drains (bounded)
 // and frees its tensor memory.
