@@ -250,7 +250,7 @@ NCU = {
                       "dram_bytes_per_trailing_entry": 30.0,
                       "capture": "one launch of the 8-frequency sweep (trailing block 1328 x 1328, 8 matrices, "
                                  "persistent grid of 152 CTAs); C read and written plus the digit tiles"},
-    "assemble_wave_wu": {"fp64_pipe_active": 0.686, "alu_pipe_active": 0.288,
+    "assemble_wave_wu": {"fp64_pipe_active": 0.739, "alu_pipe_active": 0.305,
                          "dram_bytes_per_unordered_pair": 398e6 / 4.0e6},
     "lu_gemm_f64": {"fp64_pipe_active": 0.977, "dram_bytes_per_launch": 1.236e9},
 }

@@ -422,7 +422,7 @@ __device__ __forceinline__ void store_pair(const AssemblyParams& p, const WaveTe
 // time warps waited for instructions (the FP64 pipe 58 % busy, issue slots 24 %).  So what the
 // term does again and again is called (wu_fit, bessel_row, recip_call), and the CTA's warps walk
 // together, a barrier per column and between the term's parts; warps below the diagonal only
-// keep the count.  1750 panels 833 -> 635 us, thirty matrices of 2000 19.2 -> 15.7 ms; without the
+// keep the count.  1750 panels 833 -> 635 us (the FP64 pipe 74 % busy), thirty matrices of 2000 19.2 -> 15.7 ms; without the
 // barriers 5 % less; CTAs of 256 rows the same, of 512 15 % more (their tiles' last warps wait).
 constexpr int kWuSteps = 3;  // barriers inside wu_wave_term_and_derivs
 template <bool DIRECT, int WMODE>  // WMODE 1 = Wu only, 2 = exact Delhommeau, 3 = both
