@@ -417,13 +417,15 @@ __device__ __forceinline__ void store_pair(const AssemblyParams& p, const WaveTe
   Db[mdx] = dm;
 }
 
-// The Wu term of one pair is some 4000 instructions with everything inlined and unrolled, more
+// The Wu term of one pair is some 5000 instructions with everything inlined and unrolled, more
 // than the instruction caches feed to warps that each run at a place of their own: half of the
 // time warps waited for instructions (the FP64 pipe 58 % busy, issue slots 24 %).  So what the
 // term does again and again is called (wu_fit, bessel_row, recip_call), and the CTA's warps walk
 // together, a barrier per column and between the term's parts; warps below the diagonal only
-// keep the count.  1750 panels 833 -> 635 us (the FP64 pipe 74 % busy), thirty matrices of 2000 19.2 -> 15.7 ms; without the
-// barriers 5 % less; CTAs of 256 rows the same, of 512 15 % more (their tiles' last warps wait).
+// keep the count.  1750 panels 833 -> 635 us (the FP64 pipe 74 % busy), thirty matrices of 2000 19.2
+// -> 15.8 ms.  An assembly of 1750 panels with its static part: neither 1.16 ms, barriers alone 1.05,
+// calls alone 1.03, both 0.96; barriers with CTAs of 256 rows 1.04 but the larger cases slower, of
+// 512 rows 1.18 (the last warps of their tiles wait).
 constexpr int kWuSteps = 3;  // barriers inside wu_wave_term_and_derivs
 template <bool DIRECT, int WMODE>  // WMODE 1 = Wu only, 2 = exact Delhommeau, 3 = both
 __global__ void __launch_bounds__(kRowsPerCta) wave_kernel(AssemblyParams p, const double* SR, const double* DR,
