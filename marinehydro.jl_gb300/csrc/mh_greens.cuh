@@ -56,7 +56,10 @@ __device__ inline void birk_phi_and_velocity(double x, double y, double z, const
     h[k] = sx[k] * sy[k];
   }
   const bool inplane = fabs(z) <= kBirkZTol;  // _inplane_atan (:49-54)
-  double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+  // 0, or NaN for a point or panel that is not finite (a collapsed panel's frame among them): the
+  // integer functions give a number whatever they are given, so every sum starts from it
+  const double nan_or_0 = 0.0 * fabs(x + y + z);
+  double s0 = nan_or_0, s1 = nan_or_0, s2 = nan_or_0, s3 = nan_or_0;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     const int kn = (k + 1) & 3;

@@ -46,3 +46,33 @@ def test_noalloc_equals_allocating(mh, ctx, n_lat, n_lon, direct, fixed):
         torch.cuda.synchronize()
         S0, D0 = mh.assemble_matrices(greens, mesh, 0.8, direct=direct, all_normals=fixed, ctx=ctx)
         assert np.array_equal(S.cpu().numpy().T, S0) and np.array_equal(D.cpu().numpy().T, D0)
+
+
+@pytest.mark.parametrize("field, entry", [("centers", (5, 0)), ("centers", (5, 2)), ("panel_vertices", (5, 1, 1))])
+@pytest.mark.parametrize("gfs", [1, 3, 5, 35])
+@pytest.mark.parametrize("direct", [True, False])
+def test_nan_geometry_stays_nan(mh, field, entry, gfs, direct):
+    # device buffers are not checked for NaN (host meshes are): what a NaN enters has to come out as
+    # NaN, never as a number
+    torch = pytest.importorskip("torch")
+    mesh = mh.hemisphere_mesh(1.0, 6, 12)
+    n, L = mesh.nfaces, mh.load_library()
+    arrays = {f: np.array(getattr(mesh, f), dtype=np.float64)
+              for f in ("panel_vertices", "centers", "normals", "areas", "radii")}
+    arrays[field][entry] = np.nan
+    dev = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in arrays.values()]
+    S = torch.zeros((n, n), dtype=torch.complex128, device="cuda")
+    D = torch.zeros_like(S)
+    rc = L.mh_assemble_matrices_noalloc(torch.cuda.current_stream().cuda_stream, n, *[t.data_ptr() for t in dev], 0.8,
+                                        gfs, int(direct), 1, None, S.data_ptr(), D.data_ptr())
+    assert rc == 0
+    torch.cuda.synchronize()
+    S, D = S.cpu().numpy().T, D.cpu().numpy().T
+    # panel 5 as the source: the near integral takes its corners, the wave term its centre; as the
+    # field point: every term takes its centre
+    if field == "panel_vertices" or gfs & 32:
+        assert np.isnan(S[:, 5]).all() and np.isnan(D[:, 5]).all()
+    if field == "centers":
+        assert np.isnan(S[5]).all() and np.isnan(D[5]).all()
+    keep = np.arange(n) != 5
+    assert np.isfinite(S[np.ix_(keep, keep)]).all() and np.isfinite(D[np.ix_(keep, keep)]).all()
