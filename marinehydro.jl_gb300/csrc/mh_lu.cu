@@ -200,14 +200,18 @@ template <typename T> constexpr size_t panel_smem_bytes(int chunk, int width, in
 // Pivot candidates compare |re| + |im| through the bit pattern of the (non-negative) value as
 // an unsigned integer, which orders like the value (and puts a NaN above every number): FP64
 // comparisons run on GB300's narrow FP64 pipe, integer ones do not.  "No candidate" is key 0
-// with row INT_MAX, which loses against any row (a zero column is recognised by the key 0).
+// with row INT_MAX, which loses against any row (a zero column is recognised by the key 0).  A NaN
+// that wins leaves nothing but NaN; in FP64 it is reported like a zero pivot, so that a matrix that is
+// not finite is refused (in FP32 the refinement fails and the FP64 factorization decides).
 template <typename T> struct PivotKey;
 template <> struct PivotKey<double> {
   using type = unsigned long long;
+  static constexpr type kInf = 0x7FF0000000000000ull;
   __device__ static __forceinline__ type of(double v) { return (type)__double_as_longlong(v); }
 };
 template <> struct PivotKey<float> {
   using type = unsigned;
+  static constexpr type kInf = 0xFFFFFFFFu;  // no key is above it
   __device__ static __forceinline__ type of(float v) { return __float_as_uint(v); }
 };
 
@@ -383,7 +387,7 @@ __global__ void __launch_bounds__(kPanelThreads) panel_cluster_kernel(BatchDesc 
       }
       if (lane == 0 && rank == 0) {
         ipiv_all[bmat * ipiv_stride(d.n) + k + j] = (int32_t)(k + p);
-        if (zero && info_all[bmat] == 0) info_all[bmat] = (int32_t)(k + j + 1);
+        if ((zero || v > PivotKey<T>::kInf) && info_all[bmat] == 0) info_all[bmat] = (int32_t)(k + j + 1);
       }
       if (j + 1 < kb) {
         bar_sync(1, 32 * (searchers + 1));

@@ -127,3 +127,28 @@ def test_refinement_settles_in_a_few_sweeps(mh, ctx, n):
 def test_fp64_residual_products(mh, ctx, n, rhs):
     # A x and A^H x on the FP64 pipe: the adjoint solve's refinement uses them at every order
     _solve_ok(mh, ctx, n, rhs, "mixed", adjoint=True)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed", "fp64_tc"])
+@pytest.mark.parametrize("n", [1, 8, 40, 300, 1100])
+@pytest.mark.parametrize("adjoint", [False, True])
+def test_nan_matrix_is_refused(mh, ctx, n, precision, adjoint):
+    # a NaN in the pivot search has the status of a zero pivot
+    rng = np.random.default_rng(n)
+    b = rng.standard_normal((n, 2)) + 0j
+    for row, col in {(0, 0), (n // 2, n // 3), (n - 1, n - 1)}:
+        A = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+        A[row, col] = np.nan
+        with pytest.raises(np.linalg.LinAlgError):
+            (mh.linsolve_adjoint if adjoint else mh.linsolve)(A, b, precision=precision, ctx=ctx)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp64_tc"])
+@pytest.mark.parametrize("value", [np.inf, -np.inf, complex(np.inf, np.inf), complex(1, np.inf)])
+def test_infinite_matrix_is_refused(mh, ctx, precision, value):
+    for n in (8, 40, 300):
+        rng = np.random.default_rng(n)
+        A = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+        A[3, 5] = value
+        with pytest.raises(np.linalg.LinAlgError):
+            mh.linsolve(A, rng.standard_normal((n, 2)) + 0j, precision=precision, ctx=ctx)
