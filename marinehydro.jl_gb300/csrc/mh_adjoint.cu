@@ -21,6 +21,7 @@
 //   gc[n][3] centre, gn[n][3] normal, ga[n] area, gv[n][12] Birk corner vertices.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "mh_dual.cuh"
@@ -841,10 +842,32 @@ __global__ void __launch_bounds__(kEgdThreads) egd_pair_values_kernel(AssemblyPa
   const int64_t i = q - j * (j + 1) / 2;
   double r, z;
   reduced_coords(p.P[i].c, p.P[j].c, k, r, z);
-  double2 G, Gr;
-  egd_values(r, z, p.quad_rtol, p.quad_atol, G, Gr);
-  out[2 * q] = G;
-  out[2 * q + 1] = Gr;
+  if (!egd_takes_quadrature(r, z)) egd_values(r, z, out[2 * q], out[2 * q + 1]);
+}
+
+// the same for the pairs above the surface, a warp each (wave_quadrature_kernel, mh_assembly.cu)
+__global__ void __launch_bounds__(kEgdThreads) egd_pair_quadrature_kernel(AssemblyParams p, double k,
+                                                                          double2* __restrict__ out) {
+  __shared__ double sw[kEgdThreads / 32][8 * kGKWarpStack];
+  const int64_t n = p.n;
+  if (!egd_any_quadrature(p, k)) return;
+  for_items_by_warp(
+      n * n,
+      [&](int64_t t) {
+        const int64_t j = t / n, i = t - j * n;
+        return i <= j && egd_pair_takes_quadrature(p.P[i].c, p.P[j].c, k);
+      },
+      [&](int64_t t) {
+        const int64_t j = t / n, i = t - j * n, pair = packed_pair(i, j);
+        double r, z;
+        reduced_coords(p.P[i].c, p.P[j].c, k, r, z);
+        double2 G, Gr;
+        egd_pair_quadrature(r, z, p.quad_rtol, p.quad_atol, sw[threadIdx.x >> 5], &G, &Gr);
+        if ((threadIdx.x & 31) == 0) {
+          out[2 * pair] = G;
+          out[2 * pair + 1] = Gr;
+        }
+      });
 }
 
 // dS/dk and dD/dk of the exact term from the packed values: S = sc a k G(k dis, k Z) and
@@ -1181,6 +1204,9 @@ void launch_egd_pair_values(cudaStream_t st, LaunchCounter lc, const AssemblyPar
   if (m <= 0) return;
   MH_LAUNCH(lc, st, "egd_pair_values",
             egd_pair_values_kernel<<<(unsigned)((m + kEgdThreads - 1) / kEgdThreads), kEgdThreads, 0, st>>>(p, k, m, out));
+  MH_LAUNCH(lc, st, "egd_pair_values",
+            egd_pair_quadrature_kernel<<<(unsigned)std::min<int64_t>((p.n * p.n + 3) / 4, 16 * 152), kEgdThreads, 0,
+                                         st>>>(p, k, out));
 }
 
 void launch_egd_dk(cudaStream_t st, LaunchCounter lc, const AssemblyParams& p, double k, const double2* values,

@@ -40,7 +40,7 @@ constexpr uint32_t kDelhKinds = MH_GF_DELHOMMEAU_RANKINE | MH_GF_DELHOMMEAU_RANK
 // mesh's own center / normal / area / radius.
 __global__ void panel_geometry_kernel(int64_t n, const double* __restrict__ V, const double* __restrict__ C,
                                       const double* __restrict__ N, const double* __restrict__ A,
-                                      const double* __restrict__ R, PanelRec* __restrict__ out) {
+                                      const double* __restrict__ R, PanelRec* __restrict__ out, int* above) {
   int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (j >= n) return;
   const double* v = V + 12 * j;
@@ -101,6 +101,7 @@ __global__ void panel_geometry_kernel(int64_t n, const double* __restrict__ V, c
     P.edge[k] = hypot(P.lc[2 * kn] - P.lc[2 * k], P.lc[2 * kn + 1] - P.lc[2 * k + 1]);
   }
   out[j] = P;
+  if (above && !(P.c[2] < kBelowSurface)) atomicOr(above, 1);
 }
 
 __device__ __forceinline__ void stage_panels(PanelRec* sp, const PanelRec* __restrict__ P, int64_t j0, int64_t n) {
@@ -326,8 +327,9 @@ __device__ __forceinline__ WaveTerms egd_wave_terms(double r, double z, double k
 // WMODE bits: 1 = Wu, 2 = exact Delhommeau (the learned surrogate has its own kernel,
 // wave_kernel_tc).  kc[m] = -k^m / 4pi (m = 1, 2, 3), the pair-independent factors of the
 // terms: I = kc1 G, Gh dx_c = kc3 (1/hh) dx_c dG/dh, Gz = kc2 dG/dz (wu.jl:118-126).
+// False for a pair that the exact term leaves to wave_quadrature_kernel.
 template <bool DIRECT, int WMODE, typename Step = NoStep>
-__device__ __forceinline__ void wave_terms(const AssemblyParams& p, const double ci[3], const double cj[3], double k,
+__device__ __forceinline__ bool wave_terms(const AssemblyParams& p, const double ci[3], const double cj[3], double k,
                                            const double kc[4], WaveTerms& w, Step step = Step()) {
   w.I = make_double2(0.0, 0.0);
   w.Gh = w.Gz = w.I;
@@ -345,13 +347,15 @@ __device__ __forceinline__ void wave_terms(const AssemblyParams& p, const double
   if (WMODE & 2) {  // both_greens_and_gradient_greens(::ExactGuevelDelhommeau)
     double r, z;
     reduced_coords(ci, cj, k, r, z);
+    if (egd_takes_quadrature(r, z)) return false;
     double2 G, Gr;
-    egd_values(r, z, p.quad_rtol, p.quad_atol, G, Gr);
+    egd_values(r, z, G, Gr);
     const WaveTerms e = egd_wave_terms(r, z, k, G, Gr);
     w.I = zadd(w.I, e.I);
     w.Gh = zadd(w.Gh, e.Gh);
     w.Gz = zadd(w.Gz, e.Gz);
   }
+  return true;
 }
 
 // S and D entries (before adding the static part) from the wave terms: `sgn` = -1 gives the
@@ -467,13 +471,72 @@ __global__ void __launch_bounds__(kRowsPerCta) wave_kernel(AssemblyParams p, con
     }
     const PanelRec& Pj = sp[jj];
     WaveTerms w;
-    wave_terms<DIRECT, WMODE>(p, ci, Pj.c, k, kc, w, Step());
-    if (i > j || i >= n) continue;
+    if (!wave_terms<DIRECT, WMODE>(p, ci, Pj.c, k, kc, w, Step()) || i > j || i >= n) continue;
     // (i, j) orientation: gradient w.r.t. the source (direct) or the field point (indirect)
     const double dx1 = DIRECT ? Pj.c[0] - ci[0] : ci[0] - Pj.c[0];
     const double dx2 = DIRECT ? Pj.c[1] - ci[1] : ci[1] - Pj.c[1];
     store_pair<DIRECT>(p, w, i, j, ni, ai, ani, Pj, san[jj], dx1, dx2, SR, DR, Sb, Db, wave_identity, step);
   }
+}
+
+constexpr int kPairThreads = 128;  // threads per CTA of the kernels with one thread or warp per pair or point
+
+// writes the entries of the pair (i, j) and its mirror image from the exact term's G and dG/dr at
+// (r, z), added to the Wu term where WMODE asks for it
+template <bool DIRECT, int WMODE>
+__device__ __forceinline__ void store_exact_pair(const AssemblyParams& p, int64_t i, int64_t j, double k, double r,
+                                                 double z, double2 G, double2 Gr, const double* SR, const double* DR,
+                                                 double2* Sb, double2* Db, int wave_identity, int step) {
+  const PanelRec& Pi = p.P[i];
+  const PanelRec& Pj = p.P[j];
+  const double ci[3] = {Pi.c[0], Pi.c[1], Pi.c[2]};
+  // both_greens_and_gradient_greens + with_reduced_coordinates_derivative, as wave_terms<., 2>
+  const double dx1 = DIRECT ? Pj.c[0] - ci[0] : ci[0] - Pj.c[0];
+  const double dx2 = DIRECT ? Pj.c[1] - ci[1] : ci[1] - Pj.c[1];
+  WaveTerms w = egd_wave_terms(r, z, k, G, Gr);
+  if (WMODE & 1) {
+    const double kc[4] = {0.0, kMinusInv4Pi * k, kMinusInv4Pi * k * k, kMinusInv4Pi * k * k * k};
+    WaveTerms u;
+    wave_terms<DIRECT, 1>(p, ci, Pj.c, k, kc, u);
+    w.I = zadd(u.I, w.I);
+    w.Gh = zadd(u.Gh, w.Gh);
+    w.Gz = zadd(u.Gz, w.Gz);
+  }
+  const double ni[3] = {Pi.n[0], Pi.n[1], Pi.n[2]};
+  const double ani[3] = {Pi.area * ni[0], Pi.area * ni[1], Pi.area * ni[2]};
+  const double anj[3] = {Pj.area * Pj.n[0], Pj.area * Pj.n[1], Pj.area * Pj.n[2]};
+  store_pair<DIRECT>(p, w, i, j, ni, Pi.area, ani, Pj, anj, dx1, dx2, SR, DR, Sb, Db, wave_identity, step);
+}
+
+// The pairs that wave_kernel leaves to the exact term's quadrature (centres above the surface), a
+// warp each; blockIdx.y = wavenumber.
+template <bool DIRECT, int WMODE>
+__global__ void __launch_bounds__(kPairThreads) wave_quadrature_kernel(AssemblyParams p, const double* SR,
+                                                                      const double* DR, const double* __restrict__ ks,
+                                                                      double2* S, double2* D, int64_t sstride,
+                                                                      int wave_identity, int step) {
+  __shared__ double sw[kPairThreads / 32][8 * kGKWarpStack];
+  const int64_t n = p.n;
+  const double k = ks ? ks[blockIdx.y] : p.k;
+  double2* Sb = S + blockIdx.y * sstride;
+  double2* Db = D + blockIdx.y * sstride;
+  if (!egd_any_quadrature(p, k)) return;
+  auto column = [&](int64_t q) { return n < 65536 ? (int64_t)((unsigned)q / (unsigned)n) : q / n; };
+  for_items_by_warp(
+      n * n,
+      [&](int64_t q) {
+        const int64_t j = column(q), i = q - j * n;
+        return i <= j && egd_pair_takes_quadrature(p.P[i].c, p.P[j].c, k);
+      },
+      [&](int64_t q) {
+        const int64_t j = column(q), i = q - j * n;
+        double r, z;
+        reduced_coords(p.P[i].c, p.P[j].c, k, r, z);
+        double2 G, Gr;
+        egd_pair_quadrature(r, z, p.quad_rtol, p.quad_atol, sw[threadIdx.x >> 5], &G, &Gr);
+        if ((threadIdx.x & 31) == 0)
+          store_exact_pair<DIRECT, WMODE>(p, i, j, k, r, z, G, Gr, SR, DR, Sb, Db, wave_identity, step);
+      });
 }
 
 // ---------------------------------------------------------------------------------------
@@ -727,9 +790,8 @@ __global__ void __launch_bounds__(kTcRows) wave_kernel_tc(AssemblyParams p, cons
   if (warp == 0) tc::tmem_dealloc(tmem, kTcCols);
 }
 
-constexpr int kPairThreads = 128;  // threads per CTA of the kernels with one thread per pair or point
-
-// Exact Delhommeau terms for the pairs the surrogate queued (one thread per pair).
+// Exact Delhommeau terms for the pairs the surrogate queued: one thread per pair, one warp per pair
+// that takes the quadrature.
 template <bool DIRECT>
 __global__ void __launch_bounds__(kPairThreads) surrogate_fallback_kernel(AssemblyParams p,
                                                                           const double* __restrict__ SR,
@@ -738,29 +800,36 @@ __global__ void __launch_bounds__(kPairThreads) surrogate_fallback_kernel(Assemb
                                                                           double2* __restrict__ S,
                                                                           double2* __restrict__ D,
                                                                           int64_t sstride, int wave_identity) {
+  __shared__ double sw[kPairThreads / 32][8 * kGKWarpStack];
   const unsigned long long queued = p.fb_state[0];
   if (blockIdx.x == 0 && threadIdx.x == 0 && (int64_t)queued > p.fb_cap) p.fb_state[1] = 1ull;  // sticky overflow
   const int64_t count = (int64_t)queued < p.fb_cap ? (int64_t)queued : p.fb_cap;
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < count; q += (int64_t)gridDim.x * blockDim.x) {
     const int4 e = p.fb_list[q];
-    const PanelRec& Pi = p.P[e.x];
-    const PanelRec& Pj = p.P[e.y];
-    const double k = ks[e.z];
-    const double ci[3] = {Pi.c[0], Pi.c[1], Pi.c[2]};
     double r, z;
-    reduced_coords(ci, Pj.c, k, r, z);
+    reduced_coords(p.P[e.x].c, p.P[e.y].c, ks[e.z], r, z);
+    if (egd_takes_quadrature(r, z)) continue;
     double2 G, Gr;
-    egd_values(r, z, p.quad_rtol, p.quad_atol, G, Gr);
-    // both_greens_and_gradient_greens + with_reduced_coordinates_derivative, as wave_terms<., 2>
-    const double dx1 = DIRECT ? Pj.c[0] - ci[0] : ci[0] - Pj.c[0];
-    const double dx2 = DIRECT ? Pj.c[1] - ci[1] : ci[1] - Pj.c[1];
-    const WaveTerms w = egd_wave_terms(r, z, k, G, Gr);
-    const double ni[3] = {Pi.n[0], Pi.n[1], Pi.n[2]};
-    const double ani[3] = {Pi.area * ni[0], Pi.area * ni[1], Pi.area * ni[2]};
-    const double anj[3] = {Pj.area * Pj.n[0], Pj.area * Pj.n[1], Pj.area * Pj.n[2]};
-    store_pair<DIRECT>(p, w, e.x, e.y, ni, Pi.area, ani, Pj, anj, dx1, dx2, SR, DR, S + e.z * sstride,
-                       D + e.z * sstride, wave_identity);
+    egd_values(r, z, G, Gr);
+    store_exact_pair<DIRECT, 2>(p, e.x, e.y, ks[e.z], r, z, G, Gr, SR, DR, S + e.z * sstride, D + e.z * sstride,
+                                wave_identity, 1);
   }
+  for_items_by_warp(
+      count,
+      [&](int64_t q) {
+        const int4 e = p.fb_list[q];
+        return egd_pair_takes_quadrature(p.P[e.x].c, p.P[e.y].c, ks[e.z]);
+      },
+      [&](int64_t q) {
+        const int4 e = p.fb_list[q];
+        double r, z;
+        reduced_coords(p.P[e.x].c, p.P[e.y].c, ks[e.z], r, z);
+        double2 G, Gr;
+        egd_pair_quadrature(r, z, p.quad_rtol, p.quad_atol, sw[threadIdx.x >> 5], &G, &Gr);
+        if ((threadIdx.x & 31) == 0)
+          store_exact_pair<DIRECT, 2>(p, e.x, e.y, ks[e.z], r, z, G, Gr, SR, DR, S + e.z * sstride, D + e.z * sstride,
+                                      wave_identity, 1);
+      });
 }
 
 __global__ void static_only_kernel(int64_t count, const double* __restrict__ SR, const double* __restrict__ DR,
@@ -804,19 +873,28 @@ __global__ void bessel01_points_kernel(int64_t m, const double* __restrict__ x, 
   out[4 * q + 3] = y_defined ? Y1 : __longlong_as_double(0x7FF8000000000000LL);
 }
 
+// G and dG/dr at m points: a thread each for the closed form, a warp each for the others
 __global__ void __launch_bounds__(kPairThreads) exact_points_kernel(int64_t m, const double* __restrict__ r,
                                                                     const double* __restrict__ z, double rtol,
                                                                     double atol, double2* __restrict__ out) {
+  __shared__ double sw[kPairThreads / 32][8 * kGKWarpStack];
   const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (q >= m) return;
-  double2 G, Gr;
-  egd_values(r[q], z[q], rtol, atol, G, Gr);
-  out[2 * q] = G;
-  out[2 * q + 1] = Gr;
+  if (q < m && !egd_takes_quadrature(r[q], z[q])) egd_values(r[q], z[q], out[2 * q], out[2 * q + 1]);
+  for_items_by_warp(
+      m, [&](int64_t t) { return egd_takes_quadrature(r[t], z[t]); },
+      [&](int64_t t) {
+        double2 G, Gr;
+        egd_warp(r[t], z[t], rtol, atol, sw[threadIdx.x >> 5], G, Gr);
+        if ((threadIdx.x & 31) == 0) {
+          out[2 * t] = G;
+          out[2 * t + 1] = Gr;
+        }
+      });
 }
 
 // The exact path's check of a surrogate-assembled matrix (the learned term approximates
-// exact_Guevel_Delhommeau.jl:15-46): one thread per sampled ordered pair (i, j), drawn from a
+// exact_Guevel_Delhommeau.jl:15-46): one thread (or warp, for the quadrature) per sampled ordered
+// pair (i, j), drawn from a
 // counter-based SplitMix64 stream of (seed, matrix, sample), recomputes the pair's S and D
 // entries with the exact term, adds the static part as the assembly does, and accumulates the
 // squared differences to the assembled entries and the squared assembled entries per matrix:
@@ -833,52 +911,75 @@ __global__ void __launch_bounds__(kPairThreads) surrogate_judge_kernel(
     AssemblyParams p, const double* __restrict__ SR, const double* __restrict__ DR, const double* __restrict__ ks,
     const double2* __restrict__ S, const double2* __restrict__ D, int64_t sstride, int64_t n_samples, uint64_t seed,
     int64_t first_matrix, int wave_identity, double* __restrict__ acc) {
-  const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  __shared__ double sw[kPairThreads / 32][8 * kGKWarpStack];
   const int b = blockIdx.y;
-  if (q >= n_samples) return;
   const int64_t n = p.n;
-  const uint64_t h = judge_mix(seed ^ judge_mix(((uint64_t)(first_matrix + b) << 32) ^ (uint64_t)q));
-  const int64_t i = (int64_t)((h & 0xFFFFFFFFULL) % (uint64_t)n);
-  const int64_t j = (int64_t)((h >> 32) % (uint64_t)n);
   const double k = ks[b];
-  const PanelRec& Pi = p.P[i];
-  const PanelRec& Pj = p.P[j];
-  const double ci[3] = {Pi.c[0], Pi.c[1], Pi.c[2]};
+  auto sample = [&](int64_t q, int64_t& i, int64_t& j) {
+    const uint64_t h = judge_mix(seed ^ judge_mix(((uint64_t)(first_matrix + b) << 32) ^ (uint64_t)q));
+    i = (int64_t)((h & 0xFFFFFFFFULL) % (uint64_t)n);
+    j = (int64_t)((h >> 32) % (uint64_t)n);
+  };
+  auto account = [&](int64_t i, int64_t j, double r, double z, double2 GF, double2 dGdr) {
+    const PanelRec& Pi = p.P[i];
+    const PanelRec& Pj = p.P[j];
+    const double ci[3] = {Pi.c[0], Pi.c[1], Pi.c[2]};
+    // the (i, j) entries as store_pair forms them
+    const double dx1 = DIRECT ? Pj.c[0] - ci[0] : ci[0] - Pj.c[0];
+    const double dx2 = DIRECT ? Pj.c[1] - ci[1] : ci[1] - Pj.c[1];
+    const WaveTerms w = egd_wave_terms(r, z, k, GF, dGdr);
+    const double ni[3] = {Pi.n[0], Pi.n[1], Pi.n[2]};
+    double nv[3];
+    pick_normal<DIRECT>(p, Pj, ni, nv);
+    const double an[3] = {Pj.area * nv[0], Pj.area * nv[1], Pj.area * nv[2]};
+    double2 sv, dv;
+    wave_entry(w, dx1, dx2, 1.0, Pj.area, an, sv, dv);
+    if (wave_identity && i == j) dv.x += identity_jump(p, ni);
+    const int64_t idx = i + j * n;
+    if (SR) {
+      sv.x = SR[idx] + sv.x;
+      dv.x = DR[idx] + dv.x;
+    }
+    const double2 sa = S[b * sstride + idx], da = D[b * sstride + idx];
+    const double e2 = (sa.x - sv.x) * (sa.x - sv.x) + (sa.y - sv.y) * (sa.y - sv.y) + (da.x - dv.x) * (da.x - dv.x) +
+                      (da.y - dv.y) * (da.y - dv.y);
+    const double t2 = sa.x * sa.x + sa.y * sa.y + da.x * da.x + da.y * da.y;
+    atomicAdd(acc + 2 * b, e2);
+    atomicAdd(acc + 2 * b + 1, t2);
+  };
+  int64_t i, j;
   double r, z;
-  reduced_coords(ci, Pj.c, k, r, z);
-  double2 GF, dGdr;
-  egd_values(r, z, p.quad_rtol, p.quad_atol, GF, dGdr);
-  // the (i, j) entries as store_pair forms them
-  const double dx1 = DIRECT ? Pj.c[0] - ci[0] : ci[0] - Pj.c[0];
-  const double dx2 = DIRECT ? Pj.c[1] - ci[1] : ci[1] - Pj.c[1];
-  const WaveTerms w = egd_wave_terms(r, z, k, GF, dGdr);
-  const double ni[3] = {Pi.n[0], Pi.n[1], Pi.n[2]};
-  double nv[3];
-  pick_normal<DIRECT>(p, Pj, ni, nv);
-  const double an[3] = {Pj.area * nv[0], Pj.area * nv[1], Pj.area * nv[2]};
-  double2 sv, dv;
-  wave_entry(w, dx1, dx2, 1.0, Pj.area, an, sv, dv);
-  if (wave_identity && i == j) dv.x += identity_jump(p, ni);
-  const int64_t idx = i + j * n;
-  if (SR) {
-    sv.x = SR[idx] + sv.x;
-    dv.x = DR[idx] + dv.x;
+  double2 G, Gr;
+  const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (q < n_samples) {
+    sample(q, i, j);
+    reduced_coords(p.P[i].c, p.P[j].c, k, r, z);
+    if (!egd_takes_quadrature(r, z)) {
+      egd_values(r, z, G, Gr);
+      account(i, j, r, z, G, Gr);
+    }
   }
-  const double2 sa = S[b * sstride + idx], da = D[b * sstride + idx];
-  const double e2 = (sa.x - sv.x) * (sa.x - sv.x) + (sa.y - sv.y) * (sa.y - sv.y) + (da.x - dv.x) * (da.x - dv.x) +
-                    (da.y - dv.y) * (da.y - dv.y);
-  const double t2 = sa.x * sa.x + sa.y * sa.y + da.x * da.x + da.y * da.y;
-  atomicAdd(acc + 2 * b, e2);
-  atomicAdd(acc + 2 * b + 1, t2);
+  for_items_by_warp(
+      n_samples,
+      [&](int64_t t) {
+        sample(t, i, j);
+        return egd_pair_takes_quadrature(p.P[i].c, p.P[j].c, k);
+      },
+      [&](int64_t t) {
+        sample(t, i, j);
+        reduced_coords(p.P[i].c, p.P[j].c, k, r, z);
+        egd_pair_quadrature(r, z, p.quad_rtol, p.quad_atol, sw[threadIdx.x >> 5], &G, &Gr);
+        if ((threadIdx.x & 31) == 0) account(i, j, r, z, G, Gr);
+      });
 }
 
 }  // namespace
 
 void launch_panel_geometry(cudaStream_t st, LaunchCounter lc, int64_t n, const double* V, const double* C,
-                           const double* N, const double* A, const double* R, PanelRec* out) {
+                           const double* N, const double* A, const double* R, PanelRec* out, int* above) {
   if (n <= 0) return;
   MH_LAUNCH(lc, st, "panel_geometry",
-            panel_geometry_kernel<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(n, V, C, N, A, R, out));
+            panel_geometry_kernel<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(n, V, C, N, A, R, out, above));
 }
 
 // columns per CTA of the pair kernels: 8, fewer where the launch (`tiles` CTAs of one column each)
@@ -962,6 +1063,18 @@ void launch_assemble_wave(cudaStream_t st, LaunchCounter lc, const AssemblyParam
   }
 #undef MH_WAVE
   lc.post(st, mode == 1 ? "assemble_wave_wu" : "assemble_wave_exact");
+  if (mode == 1 || (p.below && !ks_dev && p.k > 1e-100)) return;  // as egd_any_quadrature finds (5 us)
+  lc.pre(st);
+  const dim3 qg((unsigned)std::min<int64_t>((p.n * p.n + 3) / 4, 16 * 152), (unsigned)nk);
+#define MH_WAVE(DIR, MODE) \
+  wave_quadrature_kernel<DIR, MODE><<<qg, kPairThreads, 0, st>>>(p, SR, DR, ks_dev, S, D, sstride, wave_identity, step)
+  if (p.direct) {
+    if (mode == 2) MH_WAVE(true, 2); else MH_WAVE(true, 3);
+  } else {
+    if (mode == 2) MH_WAVE(false, 2); else MH_WAVE(false, 3);
+  }
+#undef MH_WAVE
+  lc.post(st, "assemble_wave_exact");
 }
 
 void launch_surrogate_judge(cudaStream_t st, LaunchCounter lc, const AssemblyParams& p, const double* SR,
@@ -996,9 +1109,10 @@ void launch_wu_points(cudaStream_t st, LaunchCounter lc, int64_t m, const double
 void launch_exact_points(cudaStream_t st, LaunchCounter lc, int64_t m, const double* r, const double* z, double rtol,
                          double atol, double2* out) {
   if (m <= 0) return;
+  // few points: as many warps as points, for those that take the quadrature
+  const int64_t ctas = std::max((m + kPairThreads - 1) / kPairThreads, std::min<int64_t>((m + 3) / 4, 8 * 152));
   MH_LAUNCH(lc, st, "exact_points",
-            exact_points_kernel<<<(unsigned)((m + kPairThreads - 1) / kPairThreads), kPairThreads, 0, st>>>(
-                m, r, z, rtol, atol, out));
+            exact_points_kernel<<<(unsigned)ctas, kPairThreads, 0, st>>>(m, r, z, rtol, atol, out));
 }
 
 }  // namespace mh

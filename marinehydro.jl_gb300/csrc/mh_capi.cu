@@ -103,6 +103,8 @@ AssemblyParams make_params(mh_context* ctx, const mh_mesh* m, uint32_t gfs, int 
   AssemblyParams p;
   p.n = m->n;
   p.P = m->P;
+  p.above = m->above;
+  p.below = m->below;
   p.V = m->V;
   p.gfs = gfs;
   p.direct = direct ? 1 : 0;
@@ -474,9 +476,9 @@ int mh_mesh_create(mh_context* ctx, int64_t n, const double* vertices, const dou
   m->n = n;
   m->n_hull = n;
   const size_t nb = (size_t)n * sizeof(double);
-  // one allocation: V | C | N | A | R | P
+  // one allocation: V | C | N | A | R | P | above
   char* base = nullptr;
-  size_t bytes = nb * 20 + (size_t)n * sizeof(PanelRec) + 256;
+  size_t bytes = nb * 20 + (size_t)n * sizeof(PanelRec) + 256 + sizeof(int);
   cudaError_t e = cudaMallocAsync((void**)&base, bytes, ctx->stream);
   if (e != cudaSuccess) {
     delete m;
@@ -488,13 +490,19 @@ int mh_mesh_create(mh_context* ctx, int64_t n, const double* vertices, const dou
   m->A = m->N + 3 * n;
   m->R = m->A + n;
   m->P = (PanelRec*)(((uintptr_t)(m->R + n) + 255) & ~(uintptr_t)255);
+  m->above = (int*)(m->P + n);
+  if (mem == MH_MEM_HOST) {
+    m->below = true;
+    for (int64_t i = 0; i < n; ++i) m->below = m->below && centers[3 * i + 2] < kBelowSurface;
+  }
   int rc = copy_in(ctx, m->V, vertices, nb * 12, mem);
   if (!rc) rc = copy_in(ctx, m->C, centers, nb * 3, mem);
   if (!rc) rc = copy_in(ctx, m->N, normals, nb * 3, mem);
   if (!rc) rc = copy_in(ctx, m->A, areas, nb, mem);
   if (!rc) rc = copy_in(ctx, m->R, radii, nb, mem);
   if (!rc) {
-    launch_panel_geometry(ctx->stream, ctx->lc(), n, m->V, m->C, m->N, m->A, m->R, m->P);
+    cudaMemsetAsync(m->above, 0, sizeof(int), ctx->stream);
+    launch_panel_geometry(ctx->stream, ctx->lc(), n, m->V, m->C, m->N, m->A, m->R, m->P, m->above);
     rc = check_launch(ctx, "panel geometry");
   }
   if (rc) {

@@ -126,6 +126,8 @@ struct mh_mesh {
   double* A = nullptr;  // n
   double* R = nullptr;  // n
   PanelRec* P = nullptr;
+  int* above = nullptr;  // AssemblyParams::above and below
+  bool below = false;
   // cached wavenumber-independent part
   double* SR = nullptr;
   double* DR = nullptr;

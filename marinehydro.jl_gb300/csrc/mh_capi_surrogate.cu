@@ -147,17 +147,15 @@ int mh_surrogate_train(mh_context* ctx, int64_t n_samples, uint64_t seed, int ep
     cudaEvent_t a, b, c;
     ~EvGuard() { cudaEventDestroy(a); cudaEventDestroy(b); cudaEventDestroy(c); }
   } evg{e0, e1, e2};
-  // training and validation samples (exact kernel at the context's quadrature tolerances)
+  // training and validation samples
   MH_CUDA(ctx, cudaEventRecord(e0, st));
-  // targets are FP32: quadrature to 1e-10 relative is ample for them
-  const double srtol = std::max(ctx->quad_rtol, 1e-10), satol = std::max(ctx->quad_atol, 1e-13);
   const int64_t chunk = (int64_t)1 << 18;
   for (int64_t off = 0; off < M; off += chunk) {
-    launch_surrogate_samples(st, lc, seed, M, off, std::min(chunk, M - off), srtol, satol, X, Y8, nullptr);
+    launch_surrogate_samples(st, lc, seed, M, off, std::min(chunk, M - off), X, Y8, nullptr);
     MH_TRY(check_launch(ctx, "surrogate samples"));
   }
   const uint64_t vseed = seed ^ 0x5DEECE66Dull;
-  launch_surrogate_samples(st, lc, vseed, n_val, 0, n_val, srtol, satol, Xv, Yv, Rv);
+  launch_surrogate_samples(st, lc, vseed, n_val, 0, n_val, Xv, Yv, Rv);
   MH_TRY(check_launch(ctx, "surrogate validation samples"));
   MH_CUDA(ctx, cudaEventRecord(e1, st));
   // Glorot-uniform initialisation from a seeded 64-bit Mersenne twister (raw bits -> [0, 1))

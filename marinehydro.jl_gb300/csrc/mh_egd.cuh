@@ -28,9 +28,12 @@
 // * J0, J1 and the entire parts F0, F1 of pi (H0 + Y0), pi (H0' + Y0') from half-unit tables
 //   below r = 8 (namespace egdq); above, Hankel's forms and H - Y as polynomials in (8/r)^2.
 //
-// Points the closed form does not cover (z > 0, the free surface's own r = z = 0, non-finite
-// input) take the adaptive quadrature at the caller's tolerances, which the closed form
-// undercuts everywhere else.
+// Points above the surface (z > 0) and the surface's own r = z = 0 take the adaptive quadrature at
+// the caller's tolerances, which the closed form undercuts everywhere else.  It runs one warp per
+// point (egd_warp): the kernels go over their points twice, thread by thread for the closed form
+// and warp by warp for the others, few or none as a rule.  (One thread per point with a refinement
+// stack of its own made 8192 points above the surface 295 ms instead of 15.7, and reserved 300 MB of
+// local memory for every kernel of the exact term.)
 #pragma once
 
 #include <cuda_runtime.h>
@@ -57,18 +60,67 @@ __device__ __forceinline__ void egd_gauss(const double (&rule)[N][2], double Y, 
   }
 }
 
-// G and dG/dr by the adaptive quadrature (a call, so that its stack stays out of the kernels
-// that practically never take it)
-__device__ static __noinline__ void egd_quadrature(double r, double z, double rtol, double atol, double2* G,
-                                                   double2* Gr) {
-  *G = egd_adaptive<false>(r, z, rtol, atol);
-  *Gr = egd_adaptive<true>(r, z, rtol, atol);
+constexpr double kDoubleMax = 1.7976931348623157e308;
+
+// finite points that the closed form does not cover
+__device__ __forceinline__ bool egd_takes_quadrature(double r, double z) {
+  if (z <= 0.0 && r >= 0.0 && r - z > 1e-140) return false;
+  return fabs(r) <= kDoubleMax && fabs(z) <= kDoubleMax;
 }
 
-__device__ inline void egd_values(double r, double z, double rtol, double atol, double2& G, double2& Gr) {
+// G and dG/dr at a point (r, z) of that kind for a pair of panels, by the whole warp (the same r and
+// z on every lane; sw: 8 kGKWarpStack doubles of shared memory of this warp).  Vertically stacked
+// centres: the integrand does not depend on theta (zeta = z), so 4 times its integral over
+// [0, pi/2] is 2 pi times its value; the r-derivative is not needed (the horizontal gradient
+// vanishes for r <= 1e-6).
+__device__ static __noinline__ void egd_pair_quadrature(double r, double z, double rtol, double atol, double* sw,
+                                                        double2* G, double2* Gr) {
+  if (r == 0.0) {
+    double f[4];
+    egd_integrands(0.0, 0.0, z, f);
+    *G = make_double2(2.0 * kPi * f[0], 2.0 * kPi * f[1]);
+    *Gr = make_double2(0.0, 0.0);
+    return;
+  }
+  egd_warp(r, z, rtol, atol, sw, *G, *Gr);
+}
+
+// work(q) by the whole warp for those q of [0, m) with need(q); the warps of the grid's x direction
+// share the range, at most 32 neighbours per warp and turn
+template <typename Need, typename Work>
+__device__ __forceinline__ void for_items_by_warp(int64_t m, Need need, Work work) {
+  const int lane = threadIdx.x & 31;
+  const int64_t per_cta = blockDim.x >> 5, warps = gridDim.x * per_cta;
+  const int64_t each = (m + warps - 1) / warps, group = each < 32 ? each : 32;
+  for (int64_t q0 = (blockIdx.x * per_cta + (threadIdx.x >> 5)) * group; q0 < m; q0 += warps * group) {
+    unsigned todo = __ballot_sync(0xffffffffu, lane < group && q0 + lane < m && need(q0 + lane));
+    while (todo) {
+      const int src = __ffs(todo) - 1;
+      todo &= todo - 1;
+      work(q0 + src);
+      __syncwarp();
+    }
+  }
+}
+
+__device__ __forceinline__ bool egd_pair_takes_quadrature(const double* x, const double* xi, double k) {
+  double r, z;
+  reduced_coords(x, xi, k, r, z);
+  return egd_takes_quadrature(r, z);
+}
+
+// false where no pair of the mesh takes the quadrature, as a rule: every centre below kBelowSurface
+__device__ __forceinline__ bool egd_any_quadrature(const AssemblyParams& p, double k) {
+  return !p.above || *p.above != 0 || !(k > 1e-100);
+}
+
+// G and dG/dr in closed form (NaN where r or z is not finite); for every point but those of
+// egd_takes_quadrature
+__device__ inline void egd_values(double r, double z, double2& G, double2& Gr) {
   const double Y = -z;
-  if (!(Y >= 0.0 && r >= 0.0 && r + Y > 1e-140 && r + Y < 1e140)) {
-    egd_quadrature(r, z, rtol, atol, &G, &Gr);
+  if (!(fabs(r) + fabs(z) <= kDoubleMax)) {
+    const double nan = __longlong_as_double(0x7FF8000000000000LL);
+    G = Gr = make_double2(nan, nan);
     return;
   }
   const double r2 = r * r;

@@ -427,25 +427,6 @@ __device__ inline double2 exp_e1(double2 z, double2 ez) {
   }
   return rdivz(1.0, f);
 }
-__device__ inline double2 exp_e1(double2 z) { return exp_e1(z, zexp(z)); }
-
-// integrands of _dimless_wave_term / _d_dimless_wave_term_dr
-// (exact_Guevel_Delhommeau.jl:16-23, 36-43)
-template <bool DR>
-__device__ __forceinline__ double2 egd_integrand(double theta, double r, double z) {
-  double ct = cos(theta);
-  double2 zeta = make_double2(z, r * ct);
-  double2 ez = zexp(zeta);
-  double2 g = exp_e1(zeta, ez);
-  // j = e^zeta (E1(zeta)/pi + i) = g/pi + i e^zeta
-  const double inv_pi = 1.0 / kPi;
-  double2 j = make_double2(g.x * inv_pi - ez.y, g.y * inv_pi + ez.x);
-  if (!DR) return make_double2(j.x, ez.x);
-  double2 inv = rdivz(inv_pi, zeta);  // 1 / (pi zeta); |zeta| >= -z > 0 below the free surface
-  double2 w = make_double2(j.x - inv.x, j.y - inv.y);
-  // Re(i ct w) = -ct Im(w); Re(i ct e^zeta) = -ct Im(e^zeta)
-  return make_double2(-ct * w.y, -ct * ez.y);
-}
 
 __constant__ static const double kGKx[8] = {0.991455371120812639206854697526329, 0.949107912342758524526189684047851,
                                            0.864864423359769072789712788640926, 0.741531185599394439863864773280788,
@@ -458,88 +439,166 @@ __constant__ static const double kGKwk[8] = {0.022935322010529224963732008058970
 __constant__ static const double kGKwg[4] = {0.129484966168869693270611432679082, 0.279705391489276667901467771423780,
                                             0.381830050505118944950369775488975, 0.417959183673469387755102040816327};
 
-template <bool DR>
-__device__ inline void gk15(double a, double b, double r, double z, double2& val, double& err) {
-  double c = 0.5 * (a + b), h = 0.5 * (b - a);
-  double2 fc = egd_integrand<DR>(c, r, z);
-  double2 Ik = zscale(kGKwk[7], fc), Ig = zscale(kGKwg[3], fc);
-#pragma unroll 1
-  for (int j = 0; j < 7; ++j) {
-    double dx = h * kGKx[j];
-    double2 f1 = egd_integrand<DR>(c - dx, r, z), f2 = egd_integrand<DR>(c + dx, r, z);
-    double2 fs = zadd(f1, f2);
-    Ik = zadd(Ik, zscale(kGKwk[j], fs));
-    if (j & 1) Ig = zadd(Ig, zscale(kGKwg[j >> 1], fs));
-  }
-  val = zscale(h, Ik);
-  double2 dif = zsub(Ik, Ig);
-  err = hypot(dif.x * h, dif.y * h);
+// Adaptive GK(7,15) over [0, pi/2], times 4 (exact_Guevel_Delhommeau.jl:8-13, 25, 45), by a whole
+// warp: the 15 Kronrod nodes of two segments run on 30 lanes, G and dG/dr come from the same
+// exp(zeta), E1(zeta) evaluation at each node, and the depth-first refinement stack lives in
+// shared memory, written by lane 0 and read by the whole warp.
+constexpr int kGKWarpStack = 48;   // entries of 8 doubles: a, b, G (2), dG/dr (2), err G, err dG/dr
+constexpr int kGKMaxEvals = 8192;  // evaluations of two segments, a hard bound
+
+// both integrands at theta (exact_Guevel_Delhommeau.jl:16-23, 36-43), from one E1
+__device__ __forceinline__ void egd_integrands(double theta, double r, double z, double f[4]) {
+  const double ct = cos(theta);
+  const double2 zeta = make_double2(z, r * ct);
+  const double2 ez = zexp(zeta);
+  const double2 g = exp_e1(zeta, ez);
+  const double inv_pi = 1.0 / kPi;
+  // j = e^zeta (E1(zeta)/pi + i) = g/pi + i e^zeta
+  const double2 j = make_double2(g.x * inv_pi - ez.y, g.y * inv_pi + ez.x);
+  f[0] = j.x;
+  f[1] = ez.x;
+  const double2 inv = rdivz(inv_pi, zeta);  // 1 / (pi zeta); |zeta| >= -z > 0 below the free surface
+  const double2 w = make_double2(j.x - inv.x, j.y - inv.y);
+  // Re(i ct w) = -ct Im(w); Re(i ct e^zeta) = -ct Im(e^zeta)
+  f[2] = -ct * w.y;
+  f[3] = -ct * ez.y;
 }
 
-constexpr int kGKStack = 48;        // depth-first refinement stack (segments)
-constexpr int kGKMaxEvals = 8192;   // GK15 evaluations per integral, a hard bound
+// Kronrod node, Kronrod weight and Gauss weight of this lane (lanes 15 and 31 idle)
+__device__ __forceinline__ void gk_lane_node(int lane, double& t, double& wk, double& wg) {
+  const int j = lane & 15;
+  t = 0.0; wk = 0.0; wg = 0.0;
+  if (j == 15) return;
+  if (j < 7) {
+    t = -kGKx[j]; wk = kGKwk[j]; wg = (j & 1) ? kGKwg[j >> 1] : 0.0;
+  } else if (j == 7) {
+    wk = kGKwk[7]; wg = kGKwg[3];
+  } else {
+    const int m = 14 - j;
+    t = kGKx[m]; wk = kGKwk[m]; wg = (m & 1) ? kGKwg[m >> 1] : 0.0;
+  }
+}
 
-// 4 * adaptive GK(7,15) over [0, pi/2] (exact_Guevel_Delhommeau.jl:8-13, 25, 45) to a
-// total error estimate <= max(atol, rtol |I|).  The phase r cos(theta) of the integrand
-// turns through r radians over the interval, so the interval is first cut into
-// ceil(r / 4) equal segments (at most 1024, about 2/3 of an oscillation each); each is
-// then refined depth-first by bisection until its GK error estimate is below its
-// share of the tolerance, tol * length / (pi/2), with tol from a first pass over the
-// initial segments.  The per-thread state is a short stack, so large r costs time,
-// not memory.
-template <bool DR>
-__device__ inline double2 egd_adaptive(double r, double z, double rtol, double atol) {
+// GK(7,15) of both integrands over [aA, bA] (lanes 0-15) and [aB, bB] (lanes 16-31);
+// every lane returns both results
+__device__ __forceinline__ void gk15_pair_warp(double aA, double bA, double aB, double bB, double r, double z,
+                                               double vA[4], double& eGA, double& eRA, double vB[4], double& eGB,
+                                               double& eRB) {
+  const int lane = threadIdx.x & 31;
+  double t, wk, wg;
+  gk_lane_node(lane, t, wk, wg);
+  const double a = lane < 16 ? aA : aB, b = lane < 16 ? bA : bB;
+  const double c = 0.5 * (a + b), h = 0.5 * (b - a);
+  double f[4];
+  egd_integrands(c + h * t, r, z, f);
+  double K[4], Gs[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) { K[q] = wk * f[q]; Gs[q] = wg * f[q]; }
+#pragma unroll
+  for (int off = 8; off > 0; off >>= 1) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      K[q] += __shfl_xor_sync(0xffffffffu, K[q], off);
+      Gs[q] += __shfl_xor_sync(0xffffffffu, Gs[q], off);
+    }
+  }
+  double KA[4], GA[4], KB[4], GB[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    KA[q] = __shfl_sync(0xffffffffu, K[q], 0);
+    GA[q] = __shfl_sync(0xffffffffu, Gs[q], 0);
+    KB[q] = __shfl_sync(0xffffffffu, K[q], 16);
+    GB[q] = __shfl_sync(0xffffffffu, Gs[q], 16);
+  }
+  const double hA = 0.5 * (bA - aA), hB = 0.5 * (bB - aB);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) { vA[q] = hA * KA[q]; vB[q] = hB * KB[q]; }
+  eGA = hypot(hA * (KA[0] - GA[0]), hA * (KA[1] - GA[1]));
+  eRA = hypot(hA * (KA[2] - GA[2]), hA * (KA[3] - GA[3]));
+  eGB = hypot(hB * (KB[0] - GB[0]), hB * (KB[1] - GB[1]));
+  eRB = hypot(hB * (KB[2] - GB[2]), hB * (KB[3] - GB[3]));
+}
+
+// G = _dimless_wave_term(r, z) and dG/dr = _d_dimless_wave_term_dr(r, z) by the whole warp
+// (all 32 lanes call it with the same r, z; `sw` is this warp's 8 * kGKWarpStack doubles of
+// shared memory), to a total error estimate <= max(atol, rtol |I|) of each integral.  The phase
+// r cos(theta) of the integrand turns through r radians over the interval, so the interval is
+// first cut into ceil(r / 4) equal segments (at most 1024, about 2/3 of an oscillation each); each
+// is then refined depth-first by bisection until both error estimates are below its share of the
+// tolerances, tol * length / (pi/2), with tol from a first pass over the initial segments.  Large r
+// costs time, not memory.
+__device__ inline void egd_warp(double r, double z, double rtol, double atol, double* sw, double2& G, double2& Gr) {
+  const int lane = threadIdx.x & 31;
   const double L = kPi / 2;
   const int m0 = (int)fmin(1024.0, fmax(1.0, ceil(r / 4.0)));
   const double h0 = L / m0;
-  // first pass: the integral and the tolerance it implies
-  double2 coarse = make_double2(0.0, 0.0);
-  double v0e = 0.0;
-  double2 v0 = make_double2(0.0, 0.0);
-  for (int s = 0; s < m0; ++s) {
-    double2 v;
-    double e;
-    gk15<DR>(s * h0, s == m0 - 1 ? L : (s + 1) * h0, r, z, v, e);
-    coarse = zadd(coarse, v);
-    if (s == 0) { v0 = v; v0e = e; }
-  }
-  int evals = m0;
-  const double tol = fmax(atol, rtol * hypot(coarse.x, coarse.y));
-  double2 total = make_double2(0.0, 0.0);
-  double sa[kGKStack], sb[kGKStack], se[kGKStack];
-  double2 sv[kGKStack];
-  for (int s = 0; s < m0; ++s) {
-    int top = 0;
-    sa[0] = s * h0;
-    sb[0] = s == m0 - 1 ? L : (s + 1) * h0;
-    if (m0 == 1) {
-      sv[0] = v0;
-      se[0] = v0e;
-    } else {
-      gk15<DR>(sa[0], sb[0], r, z, sv[0], se[0]);
-      ++evals;
+  // first pass: the integrals over the initial segments and the tolerances they imply
+  double cg[4] = {0.0, 0.0, 0.0, 0.0};
+  double v1[4] = {0.0, 0.0, 0.0, 0.0}, e1G = 0.0, e1R = 0.0;
+  int evals = 0;
+  for (int s = 0; s < m0; s += 2) {
+    const int s2 = s + 1 < m0 ? s + 1 : s;
+    double vA[4], vB[4], eGA, eRA, eGB, eRB;
+    gk15_pair_warp(s * h0, s == m0 - 1 ? L : (s + 1) * h0, s2 * h0, s2 == m0 - 1 ? L : (s2 + 1) * h0, r, z, vA, eGA,
+                   eRA, vB, eGB, eRB);
+    ++evals;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) cg[q] += vA[q] + (s2 != s ? vB[q] : 0.0);
+    if (s == 0) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) v1[q] = vA[q];
+      e1G = eGA;
+      e1R = eRA;
     }
-    top = 1;
+  }
+  const double tolG = fmax(atol, rtol * hypot(cg[0], cg[1]));
+  const double tolR = fmax(atol, rtol * hypot(cg[2], cg[3]));
+  double tot[4] = {0.0, 0.0, 0.0, 0.0};
+  int top = 0;
+  auto push = [&](double a, double b, const double v[4], double eG, double eR) {
+    if (lane == 0) {
+      double* e = sw + 8 * top;
+      e[0] = a; e[1] = b; e[2] = v[0]; e[3] = v[1]; e[4] = v[2]; e[5] = v[3]; e[6] = eG; e[7] = eR;
+    }
+    ++top;
+  };
+  for (int s = 0; s < m0; s += 2) {
+    const int s2 = s + 1 < m0 ? s + 1 : s;
+    if (m0 == 1) {
+      push(0.0, L, v1, e1G, e1R);
+    } else {
+      double vA[4], vB[4], eGA, eRA, eGB, eRB;
+      const double aA = s * h0, bA = s == m0 - 1 ? L : (s + 1) * h0;
+      const double aB = s2 * h0, bB = s2 == m0 - 1 ? L : (s2 + 1) * h0;
+      gk15_pair_warp(aA, bA, aB, bB, r, z, vA, eGA, eRA, vB, eGB, eRB);
+      ++evals;
+      if (s2 != s) push(aB, bB, vB, eGB, eRB);
+      push(aA, bA, vA, eGA, eRA);
+    }
+    __syncwarp();
     while (top > 0) {
       --top;
-      const double a = sa[top], b = sb[top];
-      const double2 v = sv[top];
-      const double e = se[top];
-      if (e <= tol * (b - a) / L || top + 2 > kGKStack || evals + 2 > kGKMaxEvals) {
-        total = zadd(total, v);
+      const double* e = sw + 8 * top;
+      const double a = e[0], b = e[1], eG = e[6], eR = e[7];
+      const double v[4] = {e[2], e[3], e[4], e[5]};
+      __syncwarp();  // every lane has read the entry before it can be overwritten
+      const double frac = (b - a) / L;
+      if ((eG <= tolG * frac && eR <= tolR * frac) || top + 2 > kGKWarpStack || evals + 1 > kGKMaxEvals) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) tot[q] += v[q];
         continue;
       }
       const double mid = 0.5 * (a + b);
-      double2 v1, v2;
-      double e1, e2;
-      gk15<DR>(a, mid, r, z, v1, e1);
-      gk15<DR>(mid, b, r, z, v2, e2);
-      evals += 2;
-      sa[top] = mid; sb[top] = b; sv[top] = v2; se[top] = e2; ++top;
-      sa[top] = a; sb[top] = mid; sv[top] = v1; se[top] = e1; ++top;
+      double vA[4], vB[4], eGA, eRA, eGB, eRB;
+      gk15_pair_warp(a, mid, mid, b, r, z, vA, eGA, eRA, vB, eGB, eRB);
+      ++evals;
+      push(mid, b, vB, eGB, eRB);
+      push(a, mid, vA, eGA, eRA);  // the left half is refined first
+      __syncwarp();
     }
   }
-  return zscale(4.0, total);
+  G = make_double2(4.0 * tot[0], 4.0 * tot[1]);
+  Gr = make_double2(4.0 * tot[2], 4.0 * tot[3]);
 }
 
 }  // namespace mh

@@ -88,8 +88,10 @@ struct LaunchCounter {
   } while (0)
 
 // assembly (mh_assembly.cu)
+constexpr double kBelowSurface = -1e-30;
+// above (may be null, zeroed by the caller): set when a centre's z is not below kBelowSurface
 void launch_panel_geometry(cudaStream_t st, LaunchCounter lc, int64_t n, const double* V, const double* C,
-                           const double* N, const double* A, const double* R, PanelRec* out);
+                           const double* N, const double* A, const double* R, PanelRec* out, int* above);
 // loads the panel-geometry, Birk and Wu kernels on the current device now (lazy loading would do
 // it at their first launch)
 cudaError_t load_pair_kernels();
@@ -97,6 +99,8 @@ cudaError_t load_pair_kernels();
 struct AssemblyParams {
   int64_t n;
   const PanelRec* P;
+  const int* above;       // 0: every centre's z is below kBelowSurface (null: not known)
+  bool below;             // the same, where the host knows it
   const double* V;        // n x 12 raw vertices (Delhommeau Rankine near field)
   uint32_t gfs;
   int direct;
@@ -138,7 +142,7 @@ void launch_surrogate_points(cudaStream_t st, LaunchCounter lc, const float* mlp
 // training samples [offset, offset + count) of the M samples of `seed`: inputs X (u, v),
 // scaled targets Y8 (8 floats per sample, 6 used), optionally (r, z) in FP64 into R2
 void launch_surrogate_samples(cudaStream_t st, LaunchCounter lc, uint64_t seed, int64_t M, int64_t offset,
-                              int64_t count, double rtol, double atol, float2* X, float* Y8, double* R2);
+                              int64_t count, float2* X, float* Y8, double* R2);
 // floats of the per-step activation buffer for a batch of B samples
 int64_t mlp_act_floats(int B);
 // one Adam step (t >= 1) over samples ((base + b) mod M) * prime mod M, b < B; the mean

@@ -121,7 +121,7 @@ extern "C" int mh_assemble_matrices_noalloc(void* stream, int64_t n_panels, cons
   if (rc != MH_OK) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const LaunchCounter none{nullptr, nullptr};
-  launch_panel_geometry(st, none, n_panels, vertices, centers, normals, areas, radii, panels);
+  launch_panel_geometry(st, none, n_panels, vertices, centers, normals, areas, radii, panels, nullptr);
   AssemblyParams p = {};
   p.n = n_panels;
   p.P = panels;

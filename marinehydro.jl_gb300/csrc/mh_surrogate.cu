@@ -57,7 +57,6 @@ constexpr int kPointThreads = 128;
 // one thread per sample
 __global__ void __launch_bounds__(kPointThreads) surrogate_samples_kernel(uint64_t seed, int64_t M,
                                                                           int64_t offset, int64_t count,
-                                                                          double rtol, double atol,
                                                                           float2* __restrict__ X,
                                                                           float* __restrict__ Y8,
                                                                           double* __restrict__ R2) {
@@ -67,7 +66,7 @@ __global__ void __launch_bounds__(kPointThreads) surrogate_samples_kernel(uint64
   double r, z;
   sample_point(seed, (uint64_t)q, (uint64_t)M, r, z);
   double2 G, Gr;
-  egd_values(r, z, rtol, atol, G, Gr);
+  egd_values(r, z, G, Gr);  // z <= 0 < r: never the quadrature
   double2 GF, Gh, Gv;
   wu_wave_term_and_derivs(r, z, GF, Gh, Gv);
   const double d = sqrt(r * r + z * z);
@@ -284,18 +283,31 @@ __global__ void round_bf16_kernel(const float* __restrict__ in, float* __restric
 }
 
 // surrogate GF, Gh, Gv at points (r, z) (the layout of the Wu point evaluator), one thread per
-// point; points outside the training box take the exact term, as in assembly, inside it the
-// Wu terms and the network
+// point (a warp where the exact term's quadrature is needed); points outside the training box take
+// the exact term, as in assembly, inside it the Wu terms and the network
 __global__ void __launch_bounds__(kPointThreads) surrogate_points_kernel(const float* __restrict__ mlp, int64_t m,
                                                                               const double* __restrict__ r,
                                                                               const double* __restrict__ z,
                                                                               double rtol, double atol,
                                                                               double2* __restrict__ out) {
   extern __shared__ float4 spp4[];
+  __shared__ double sw[kPointThreads / 32][8 * kGKWarpStack];
   load_params(spp4, mlp);
   __syncthreads();
+  auto by_quadrature = [&](int64_t t) {
+    return !surrogate_in_box((float)r[t], (float)z[t]) && egd_takes_quadrature(r[t], z[t]);
+  };
+  for_items_by_warp(m, by_quadrature, [&](int64_t t) {
+    double2 GF, Gh;
+    egd_warp(r[t], z[t], rtol, atol, sw[threadIdx.x >> 5], GF, Gh);
+    if ((threadIdx.x & 31) == 0) {
+      out[3 * t] = GF;
+      out[3 * t + 1] = Gh;
+      out[3 * t + 2] = make_double2(GF.x + 2.0 / hypot(r[t], z[t]), GF.y);
+    }
+  });
   const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (q >= m) return;
+  if (q >= m || by_quadrature(q)) return;
   const double rq = r[q], zq = z[q];
   double2 GF, Gh, Gv;
   if (surrogate_in_box((float)rq, (float)zq)) {
@@ -308,7 +320,7 @@ __global__ void __launch_bounds__(kPointThreads) surrogate_points_kernel(const f
     Gh = make_double2(gh.x + dGr.x, gh.y + dGr.y);
     Gv = make_double2(gv.x + dGz.x, gv.y + dGz.y);
   } else {
-    egd_values(rq, zq, rtol, atol, GF, Gh);
+    egd_values(rq, zq, GF, Gh);
     Gv = make_double2(GF.x + 2.0 / hypot(rq, zq), GF.y);
   }
   out[3 * q] = GF;
@@ -321,10 +333,11 @@ __global__ void __launch_bounds__(kPointThreads) surrogate_points_kernel(const f
 int64_t mlp_act_floats(int B) { return (int64_t)kActRows * B; }
 
 void launch_surrogate_samples(cudaStream_t st, LaunchCounter lc, uint64_t seed, int64_t M, int64_t offset,
-                              int64_t count, double rtol, double atol, float2* X, float* Y8, double* R2) {
+                              int64_t count, float2* X, float* Y8, double* R2) {
   if (count <= 0) return;
   MH_LAUNCH(lc, st, "surrogate_samples",
-            surrogate_samples_kernel<<<(unsigned)((count + kPointThreads - 1) / kPointThreads), kPointThreads, 0, st>>>(seed, M, offset, count, rtol, atol, X, Y8, R2));
+            surrogate_samples_kernel<<<(unsigned)((count + kPointThreads - 1) / kPointThreads), kPointThreads, 0, st>>>(
+                seed, M, offset, count, X, Y8, R2));
 }
 
 void launch_mlp_loss_grad(cudaStream_t st, LaunchCounter lc, const float* qparams, const float2* X, const float* Y8,
