@@ -56,10 +56,7 @@ __device__ inline void birk_phi_and_velocity(double x, double y, double z, const
     h[k] = sx[k] * sy[k];
   }
   const bool inplane = fabs(z) <= kBirkZTol;  // _inplane_atan (:49-54)
-  // 0, or NaN for a point or panel that is not finite (a collapsed panel's frame among them): the
-  // integer functions give a number whatever they are given, so every sum starts from it
-  const double nan_or_0 = 0.0 * fabs(x + y + z);
-  double s0 = nan_or_0, s1 = nan_or_0, s2 = nan_or_0, s3 = nan_or_0;
+  double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     const int kn = (k + 1) & 3;
@@ -86,6 +83,9 @@ __device__ inline void birk_phi_and_velocity(double x, double y, double z, const
     s2 -= dx * lt_dk;
   }
   s0 += z * s3;
+  // a point or panel that is not finite (a collapsed panel's frame among them) shows in z; the integer
+  // functions give a number whatever they are given
+  if ((__double2hiint(z) & 0x7FF00000) == 0x7FF00000) s0 = s1 = s2 = s3 = z - z;
   phi = kMinusInv4Pi * s0;
   v[0] = kMinusInv4Pi * s1;
   v[1] = kMinusInv4Pi * s2;
