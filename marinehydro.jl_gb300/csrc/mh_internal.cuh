@@ -166,6 +166,12 @@ void launch_exact_points(cudaStream_t st, LaunchCounter lc, int64_t m, const dou
                          double atol, double2* out);
 
 // dense linear algebra (mh_lu.cu)
+inline int current_device() {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  return dev;
+}
+int sm_count();  // of the current device
 // int32 entries per matrix of order n in the pivot array: the pivots (after the factorization
 // the row permutation), then one flag word per 32 x 32 diagonal block (lu_finish_kernel)
 __host__ __device__ inline int64_t ipiv_stride(int64_t n) { return n + (n + 31) / 32; }

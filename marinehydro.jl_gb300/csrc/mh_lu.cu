@@ -32,6 +32,7 @@
 
 #include "mh_fixpoint.cuh"
 #include "mh_internal.cuh"
+#include "mh_per_device.h"
 
 namespace mh {
 
@@ -1462,9 +1463,20 @@ void convert_with_norms(cudaStream_t st, LaunchCounter lc, const BatchDesc& d, c
 }
 
 
+int sm_count() {
+  static PerDevice<int> counts;
+  const int dev = current_device();
+  return counts.get(dev, [dev] {
+    int v = 152;
+    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+    return v;
+  });
+}
+
 // Clusters of p CTAs of the panel kernel resident on the GPU at once, by p (clusters are placed
 // within one GPC, so this is the occupancy query's answer, not the SM count's); `width` 32 at the
-// largest chunk (a full-width panel fills one SM's shared memory), 16 half of it.
+// largest chunk (a full-width panel fills one SM's shared memory), 16 half of it.  The first call on
+// a device also sets the kernel's attributes there.
 template <typename T>
 const int* panel_residency(int width) {
   struct Table { int resident[kPanelMaxCtas + 1]; };
@@ -1496,9 +1508,8 @@ const int* panel_residency(int width) {
     }
     return t;
   };
-  static const Table tab_full = make_table(kNB);
-  static const Table tab_half = make_table(kNB / 2);
-  return width < kNB ? tab_half.resident : tab_full.resident;
+  static PerDevice<Table> full, half;
+  return (width < kNB ? half : full).get(current_device(), [&] { return make_table(width < kNB ? kNB / 2 : kNB); }).resident;
 }
 
 // the fewest CTAs whose shared memory holds a panel of m rows (0: no cluster does)
@@ -1517,12 +1528,7 @@ int panel_least_ctas(int64_t m) {
 // largest cluster the GPU can schedule (panel_kernel then runs).
 template <typename T>
 int panel_cluster_size(int64_t m, int64_t batch, int cap_ctas, int width = kNB) {
-  static const int sms = [] {
-    int dev = 0, v = 152;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-    return v;
-  }();
+  const int sms = sm_count();
   const int* resident = panel_residency<T>(width);
   const int need = panel_least_ctas<T>(m);
   if (need == 0 || resident[need] <= 0) return 0;
@@ -1702,8 +1708,10 @@ struct SolveShape { int P, g; };
 template <typename T>
 SolveShape solve_shape(int64_t n, int64_t nrhs, int64_t batch, bool upper_only) {
   struct Table { int one[kSolveMaxCtas + 1]; };
-  // clusters of P CTAs resident at once with one CTA per SM; also sets the kernels' attributes
-  static const Table tab = [] {
+  // clusters of P CTAs resident at once with one CTA per SM; also sets the kernels' attributes on
+  // the device
+  static PerDevice<Table> tables;
+  const Table& tab = tables.get(current_device(), [] {
     Table t{};
     for (const void* fn : {(const void*)solve_cluster_kernel<T, false>, (const void*)solve_cluster_kernel<T, true>}) {
       cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolveMaxSmem);
@@ -1729,7 +1737,7 @@ SolveShape solve_shape(int64_t n, int64_t nrhs, int64_t batch, bool upper_only) 
       t.one[p] = num;
     }
     return t;
-  }();
+  });
   const int64_t nblk = (n + 31) / 32;
   const double steps = (double)(upper_only ? nblk : 2 * nblk);
   SolveShape best{0, 0};

@@ -679,14 +679,8 @@ static int64_t oz_col_tiles(const BatchDesc& d) { return (d.n + d.extra + kOzCol
 // the persistent GEMM kernel's grid: one CTA per SM (at most one per tile)
 template <bool TRSM>
 static unsigned oz_grid(int64_t ntiles) {
-  static const int sms = [] {
-    int dev = 0, v = 152;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-    return v;
-  }();
   cudaFuncSetAttribute(ozaki_gemm_kernel<TRSM>, cudaFuncAttributeMaxDynamicSharedMemorySize, kOzSmem);
-  return (unsigned)std::max<int64_t>(1, std::min<int64_t>(ntiles, sms));
+  return (unsigned)std::max<int64_t>(1, std::min<int64_t>(ntiles, sm_count()));
 }
 
 size_t ozaki_workspace_bytes(int64_t n, int64_t batch, int64_t extra) {
