@@ -300,7 +300,7 @@ int finish_body(mh_context* ctx, BatchCache& c, BodyPlan& b, const BatchOpts& o)
     ok = converged();
   }
   if (!ok) {
-    // FP64 factors of this body's matrices (a uniform batch of its own, pivots at stride n
+    // FP64 factors of this body's matrices (a uniform batch of its own, its pivots
     // inside its slice of the grouped pivot array)
     MH_CUDA(ctx, cudaMemcpyAsync(b.X, b.B0, sizeof(double2) * bstride * nw, cudaMemcpyDeviceToDevice, st));
     lu_factor_batched<double>(st, lc, d, b.D, ipiv_b, b.info);
