@@ -60,7 +60,7 @@ __device__ __forceinline__ unsigned long long unit_q63(double x) {
   return sh >= 0 ? (m << sh) : (sh > -64 ? (m >> -sh) : 0ull);
 }
 
-// trunc(x 2^s) as a signed integer, for |x| 2^s < 2^62 (0 below 2^-1022)
+// trunc(x 2^s) as a signed integer, for -2^63 <= x 2^s < 2^63 (0 below 2^-1022)
 __device__ __forceinline__ long long to_q(double x, int s) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(x);
   const int e = (int)((b >> 52) & 0x7FF);
@@ -68,7 +68,7 @@ __device__ __forceinline__ long long to_q(double x, int s) {
   const unsigned long long m = (b & 0x000FFFFFFFFFFFFFull) | (1ull << 52);
   const int sh = e - 1075 + s;
   const unsigned long long a = sh >= 0 ? (m << sh) : (sh > -64 ? (m >> -sh) : 0ull);
-  return (b >> 63) ? -(long long)a : (long long)a;
+  return (long long)((b >> 63) ? 0ull - a : a);
 }
 
 // v 2^-frac as a double, rounded to nearest (ties away from zero); |v| < 2^63, results
