@@ -39,16 +39,17 @@ __device__ __forceinline__ T horner_c(const T (&c)[N], T t) {
 
 }  // namespace bes
 
+// one row of a table, called for the same reason as wu_fit (mh_greens.cuh)
+static __device__ __noinline__ double bessel_row(const long long* __restrict__ c, long long z) {
+  return fx::to_double(fx::horner_s_ld<bes::kLowTerms>(c, z), besq::kFrac);
+}
+
 // J0(x), J1(x) for x >= 0; Y0(x), Y1(x) for x >= 3 (below 3 the Y outputs are not defined
 // and must not be used).  The polynomials run in 64-bit fixed point on the integer pipe
 // (mh_fixpoint.cuh, tables besq): below 8, X = floor(x 2^60) gives the interval q = X >> 59
 // and z = 2 (x - q/2 - 1/4) as (X - q 2^59 - 2^58) 2^5 exactly; above 8 the Hankel
 // polynomials take z = (u - 1/2) / 2 from the FP64 u = (8/x)^2.  Absolute error below 1e-17
 // (the integer evaluation, emulated bit for bit by the generator, against mpmath).
-// one row of a table, called for the same reason as wu_fit (mh_greens.cuh)
-static __device__ __noinline__ double bessel_row(const long long* __restrict__ c, long long z) {
-  return fx::to_double(fx::horner_s_ld<bes::kLowTerms>(c, z), besq::kFrac);
-}
 __device__ __forceinline__ void bessel01(double x, double& J0, double& J1, double& Y0, double& Y1) {
   using namespace bes;
   if (x < 8.0) {

@@ -34,7 +34,7 @@ __device__ __forceinline__ long long fixed55(double v, int emax_biased) {
   return bits < 0 ? -X : X;
 }
 
-// two BF16 values of small integers (|d| <= 64) in one 32-bit word, the first in the low half
+// two BF16 values of small integers (|d| <= 128, eight significant bits) in one 32-bit word, the first in the low half
 __device__ __forceinline__ uint32_t bf16x2(int d0, int d1) {
   const float f0 = __int_as_float(0x4B400000 + d0) - 12582912.0f;
   const float f1 = __int_as_float(0x4B400000 + d1) - 12582912.0f;

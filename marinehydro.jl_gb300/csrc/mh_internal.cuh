@@ -56,8 +56,8 @@ struct Profiler;
 struct TileChoice {
   int oz_group = 8;     // reserved: the Ozaki (FP64 tensor-core) update is a persistent kernel
   int bx_group = 4;     // 128-column tiles per CTA of the BF16x3 (FP32) update, 1..8
-  int cluster_f64 = 8;  // largest thread-block cluster of the FP64 LU panel, 1..8
-  int cluster_f32 = 8;  // largest thread-block cluster of the FP32 LU panel, 1..8
+  int cluster_f64 = 8;  // largest thread-block cluster of the FP64 LU panel, 1..7; 8: up to 16 CTAs
+  int cluster_f32 = 8;  // the same for the FP32 panel
 };
 constexpr int kMaxTileEntries = 16;
 struct TileTable {

@@ -18,7 +18,8 @@
 //                  as one permutation of at most 64 rows (a warp per column)
 //   trsm_lanes_kernel, trsm_kernel   U12 = L11^-1 A12 with L11 in shared memory: 8 or 32 lanes
 //                  per column in FP64, one thread per column in FP32
-//   gemm3m_kernel, gemm_kernel  A22 -= L21 U12 on the CUDA cores (FP64, FP32)
+//   gemm3m_kernel  A22 -= L21 U12 on the CUDA cores (FP64); the tensor cores' updates are in
+//                  mh_ozaki.cu (FP64) and mh_bf16x3.cu (FP32, always)
 // Templated on the real type: double (the plain FP64 path) and float (the factor
 // used by mixed-precision iterative refinement).
 #include <cooperative_groups.h>
@@ -691,80 +692,6 @@ __global__ void __launch_bounds__(kTrsmThreads) trsm_lanes_kernel(BatchDesc d, d
 }
 
 // ------------------------------ trailing update -------------------------------
-// Tile shapes per precision: FP64 is FP64-pipe bound already with 64x64 CTA tiles
-// and 4x4 complex outputs per thread; FP32 needs 8x8 outputs per thread (128x128
-// CTA tiles) so that the shared-memory loads keep up with the FP32 FMA rate.
-template <typename T> struct GemmTile;
-template <> struct GemmTile<double> { static constexpr int RM = 4, TM = 64, KC = 16; };
-template <> struct GemmTile<float> { static constexpr int RM = 8, TM = 128, KC = 32; };  // whole panel depth
-
-template <typename T>
-__global__ void __launch_bounds__(256) gemm_kernel(BatchDesc d, typename cplx_t<T>::type* __restrict__ Aall,
-                                                   int64_t k) {
-  using C = typename cplx_t<T>::type;
-  constexpr int RM = GemmTile<T>::RM, TM = GemmTile<T>::TM, KC = GemmTile<T>::KC;
-  extern __shared__ unsigned char gemm_smem[];
-  C (*sA)[TM + 1] = reinterpret_cast<C (*)[TM + 1]>(gemm_smem);
-  C (*sB)[TM + 1] = reinterpret_cast<C (*)[TM + 1]>(gemm_smem + sizeof(C) * KC * (TM + 1));
-  const int64_t n = d.order(blockIdx.z);
-  if (k + kNB >= n) return;  // no trailing block for this matrix (grouped batches)
-  C* A = Aall + d.offset(blockIdx.z);
-  const int kb = (int)((k + kNB < n) ? kNB : n - k);
-  const int64_t base = k + kb;
-  const int64_t row0 = base + blockIdx.x * (int64_t)TM;
-  const int64_t col0 = base + blockIdx.y * (int64_t)TM;
-  if (row0 >= n || col0 >= n) return;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  C acc[RM][RM];
-#pragma unroll
-  for (int r = 0; r < RM; ++r)
-#pragma unroll
-    for (int c = 0; c < RM; ++c) acc[r][c] = czero<C>();
-  for (int k0 = 0; k0 < kb; k0 += KC) {
-    for (int idx = threadIdx.x; idx < KC * TM; idx += 256) {
-      int r = idx % TM, q = idx / TM;
-      int64_t gi = row0 + r;
-      int kk = k0 + q;
-      sA[q][r] = (gi < n && kk < kb) ? A[gi + (k + kk) * n] : czero<C>();
-    }
-    for (int idx = threadIdx.x; idx < KC * TM; idx += 256) {
-      int q = idx % KC, c = idx / KC;
-      int64_t gc = col0 + c;
-      int kk = k0 + q;
-      sB[q][c] = (gc < n && kk < kb) ? A[(k + kk) + gc * n] : czero<C>();
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < KC; ++q) {
-      C a[RM], b[RM];
-#pragma unroll
-      for (int r = 0; r < RM; ++r) a[r] = sA[q][tx + 16 * r];
-#pragma unroll
-      for (int c = 0; c < RM; ++c) b[c] = sB[q][ty + 16 * c];
-#pragma unroll
-      for (int r = 0; r < RM; ++r)
-#pragma unroll
-        for (int c = 0; c < RM; ++c) acc[r][c] = cfma(acc[r][c], a[r], b[c]);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int c = 0; c < RM; ++c) {
-    int64_t gc = col0 + ty + 16 * c;
-    if (gc >= n) continue;
-#pragma unroll
-    for (int r = 0; r < RM; ++r) {
-      int64_t gi = row0 + tx + 16 * r;
-      if (gi < n) {
-        C v = A[gi + gc * n];
-        v.x -= acc[r][c].x;
-        v.y -= acc[r][c].y;
-        A[gi + gc * n] = v;
-      }
-    }
-  }
-}
-
 // A22 -= L21 U12 in FP64 with Gauss's three-multiplication complex product (the ZGEMM3M
 // scheme): per complex multiply-add P1 += ar br, P2 += ai bi, P3 += (ar + ai)(br + bi), and
 // at the end Re = P1 - P2, Im = P3 - P1 - P2 -- three FP64 FMAs instead of four.  The sums
@@ -1556,14 +1483,11 @@ int lu_factor_batched(cudaStream_t st, LaunchCounter lc, const BatchDesc& d, typ
                       int32_t* ipiv, int32_t* info, void* emu_ws, int* emu_flag) {
   const int64_t n = d.n;
   if (n <= 0 || d.batch <= 0) return 0;
-  // appended right-hand sides need the rectangular trailing update of the FP64 tensor-core path
+  // appended right-hand sides need the rectangular trailing update of the FP64 tensor-core path;
+  // the FP32 update has no other path than the tensor cores'
   if (d.extra > 0 && (sizeof(T) != 8 || !emu_ws || d.orders)) return -1;
+  if (sizeof(T) == 4 && !emu_ws) return -1;
   cudaMemsetAsync(info, 0, sizeof(int32_t) * d.batch, st);
-  {
-    constexpr int TM = GemmTile<T>::TM;
-    constexpr size_t gsmem = 2 * sizeof(typename cplx_t<T>::type) * GemmTile<T>::KC * (TM + 1);
-    cudaFuncSetAttribute(gemm_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gsmem);
-  }
   const int cap_ctas = sizeof(T) == 8 ? lc.tile(n).cluster_f64 : lc.tile(n).cluster_f32;
   // the panel at k0 of `width` columns on a cluster of P CTAs
   auto cluster_panel = [&](int64_t k0, int width, int P) {
@@ -1683,11 +1607,6 @@ int lu_factor_batched(cudaStream_t st, LaunchCounter lc, const BatchDesc& d, typ
       dim3 gg((unsigned)(wide ? t2 : t1), (unsigned)(wide ? t2 : t1), (unsigned)d.batch);
       if (wide) MH_LAUNCH(lc, st, "lu_gemm_f64", gemm3m_kernel<2><<<gg, 256, 0, st>>>(d, A, k));
       else MH_LAUNCH(lc, st, "lu_gemm_f64", gemm3m_kernel<1><<<gg, 256, 0, st>>>(d, A, k));
-    } else {
-      constexpr int TM = GemmTile<T>::TM;
-      dim3 gg((unsigned)((rest + TM - 1) / TM), (unsigned)((rest + TM - 1) / TM), (unsigned)d.batch);
-      constexpr size_t gsmem = 2 * sizeof(typename cplx_t<T>::type) * GemmTile<T>::KC * (TM + 1);
-      MH_LAUNCH(lc, st, "lu_gemm_f32", gemm_kernel<T><<<gg, 256, gsmem, st>>>(d, A, k));
     }
   }
   const int nblk = (int)((n + kNB - 1) / kNB);

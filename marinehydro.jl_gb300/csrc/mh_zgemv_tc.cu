@@ -81,8 +81,6 @@ __device__ __forceinline__ int scale_exp(double maxabs) {
   return e;
 }
 
-__device__ __forceinline__ double pow2i(int s) { return __longlong_as_double((long long)(s + 1023) << 52); }
-
 // X columns r0 .. r0+g-1 of matrix b -> per block the operand tile and the column exponents
 __global__ void __launch_bounds__(256) zgemv_xsplit_kernel(BatchDesc d, const double2* __restrict__ Xall,
                                                            int64_t xstride, int r0, int g, int64_t nkb,
