@@ -1453,10 +1453,9 @@ int panel_least_ctas(int64_t m) {
 // more), up to `cap_ctas` beyond the minimum (the launch-shape table's cluster bound; its
 // largest value, 8, stands for the largest cluster of 16); 0 when the panel does not fit the
 // largest cluster the GPU can schedule (panel_kernel then runs).
+// (resident: panel_residency of the panel's width; sms: of the device.)
 template <typename T>
-int panel_cluster_size(int64_t m, int64_t batch, int cap_ctas, int width = kNB) {
-  const int sms = sm_count();
-  const int* resident = panel_residency<T>(width);
+int panel_cluster_size(int64_t m, int64_t batch, int cap_ctas, const int* resident, int sms) {
   const int need = panel_least_ctas<T>(m);
   if (need == 0 || resident[need] <= 0) return 0;
   const int most = cap_ctas >= 8 ? kPanelMaxCtas : cap_ctas;
@@ -1473,9 +1472,9 @@ int panel_cluster_size(int64_t m, int64_t batch, int cap_ctas, int width = kNB) 
 // (its rows need at most as many CTAs per matrix as fit every cluster on the GPU); a panel that
 // does not fit runs in waves, and the FP64 tensor-core path factors it in two halves instead
 template <typename T>
-bool panel_fits_one_wave(int64_t m, int64_t batch) {
+bool panel_fits_one_wave(int64_t m, int64_t batch, const int* resident) {
   const int need = panel_least_ctas<T>(m);
-  return need > 0 && panel_residency<T>(kNB)[need] >= batch;
+  return need > 0 && resident[need] >= batch;
 }
 
 template <typename T>
@@ -1488,6 +1487,8 @@ int lu_factor_batched(cudaStream_t st, LaunchCounter lc, const BatchDesc& d, typ
   if (d.extra > 0 && (sizeof(T) != 8 || !emu_ws || d.orders)) return -1;
   if (sizeof(T) == 4 && !emu_ws) return -1;
   cudaMemsetAsync(info, 0, sizeof(int32_t) * d.batch, st);
+  const int sms = sm_count();
+  const int *resident = panel_residency<T>(kNB), *resident_half = panel_residency<T>(kNB / 2);
   const int cap_ctas = sizeof(T) == 8 ? lc.tile(n).cluster_f64 : lc.tile(n).cluster_f32;
   // the panel at k0 of `width` columns on a cluster of P CTAs
   auto cluster_panel = [&](int64_t k0, int width, int P) {
@@ -1510,7 +1511,7 @@ int lu_factor_batched(cudaStream_t st, LaunchCounter lc, const BatchDesc& d, typ
   // the full-width panel at k0 (on one CTA per matrix when no cluster holds it), and its row
   // interchanges outside of it
   auto full_panel = [&](int64_t k0) {
-    const int P = panel_cluster_size<T>(n - k0, d.batch, cap_ctas);
+    const int P = panel_cluster_size<T>(n - k0, d.batch, cap_ctas, resident, sms);
     if (P > 0) {
       cluster_panel(k0, kNB, P);
     } else {
@@ -1550,9 +1551,9 @@ int lu_factor_batched(cudaStream_t st, LaunchCounter lc, const BatchDesc& d, typ
     // cores -- half the panel's FP64 work, and half its shared memory per row
     int Pl = 0, P16 = 0;
     if constexpr (sizeof(T) == 8) {
-      if (emu_ws && kb == kNB && !d.orders && !panel_fits_one_wave<T>(n - k, d.batch)) {
-        Pl = panel_cluster_size<T>(n - k, d.batch, cap_ctas, kNB / 2);
-        P16 = panel_cluster_size<T>(n - k - kNB / 2, d.batch, cap_ctas, kNB / 2);
+      if (emu_ws && kb == kNB && !d.orders && !panel_fits_one_wave<T>(n - k, d.batch, resident)) {
+        Pl = panel_cluster_size<T>(n - k, d.batch, cap_ctas, resident_half, sms);
+        P16 = panel_cluster_size<T>(n - k - kNB / 2, d.batch, cap_ctas, resident_half, sms);
       }
     }
     if (Pl > 0 && P16 > 0) {
