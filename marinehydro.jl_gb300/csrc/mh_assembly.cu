@@ -1065,7 +1065,9 @@ void launch_assemble_wave(cudaStream_t st, LaunchCounter lc, const AssemblyParam
   lc.post(st, mode == 1 ? "assemble_wave_wu" : "assemble_wave_exact");
   if (mode == 1 || (p.below && !ks_dev && p.k > 1e-100)) return;  // as egd_any_quadrature finds (5 us)
   lc.pre(st);
-  const dim3 qg((unsigned)std::min<int64_t>((p.n * p.n + 3) / 4, 16 * 152), (unsigned)nk);
+  // as many CTAs as are resident, over all wavenumbers
+  const int64_t most = std::max<int64_t>(1, 16 * 152 / nk);
+  const dim3 qg((unsigned)std::min<int64_t>((p.n * p.n + 3) / 4, most), (unsigned)nk);
 #define MH_WAVE(DIR, MODE) \
   wave_quadrature_kernel<DIR, MODE><<<qg, kPairThreads, 0, st>>>(p, SR, DR, ks_dev, S, D, sstride, wave_identity, step)
   if (p.direct) {
