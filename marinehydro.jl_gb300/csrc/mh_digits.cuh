@@ -70,26 +70,20 @@ __device__ __forceinline__ void split4(const double2 (&v)[4], int emax, uint32_t
 }
 
 // Seven balanced base-256 digits in [-128, 128] of the same X (|X| < 2^55), most significant
-// first: X = sum_p d_p 256^(6 - p).  X = hi 2^24 + lo, lo in [0, 2^24) gives digits 6..4 and
-// a carry, hi (|hi| < 2^31) digits 3..0.  Each is exact in BF16 (eight significant bits).
+// first: X = sum_p d_p 256^(6 - p).  With 128 added to every digit beforehand (one 64-bit addition,
+// which does all the carries, for X up to 2^55 into the 57th bit) they are the sum's bytes, the top one
+// with what is above it.  Each is exact in BF16 (eight significant bits).
 constexpr int kDigits7 = 7;
 __device__ __forceinline__ void digits7(long long X, int (&d)[kDigits7]) {
-  int lo = (int)(X & 0xFFFFFF);
-  int hi = (int)(X >> 24);
-#pragma unroll
-  for (int p = kDigits7 - 1; p >= 4; --p) {
-    const int c = lo + 128;
-    d[p] = (c & 255) - 128;
-    lo = c >> 8;
-  }
-  hi += lo;
-#pragma unroll
-  for (int p = 3; p >= 1; --p) {
-    const int c = hi + 128;
-    d[p] = (c & 255) - 128;
-    hi = c >> 8;
-  }
-  d[0] = hi;
+  const unsigned long long u = (unsigned long long)(X + 0x80808080808080ll);
+  const unsigned int lo = (unsigned int)u, hi = (unsigned int)(u >> 32);
+  d[6] = (int)(lo & 255u) - 128;
+  d[5] = (int)((lo >> 8) & 255u) - 128;
+  d[4] = (int)((lo >> 16) & 255u) - 128;
+  d[3] = (int)(lo >> 24) - 128;
+  d[2] = (int)(hi & 255u) - 128;
+  d[1] = (int)((hi >> 8) & 255u) - 128;
+  d[0] = (int)(hi >> 16) - 128;
 }
 
 // Eight consecutive K values (one 16-byte row chunk) of one row: their seven base-256 digit planes

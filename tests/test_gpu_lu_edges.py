@@ -152,3 +152,23 @@ def test_infinite_matrix_is_refused(mh, ctx, precision, value):
         A[3, 5] = value
         with pytest.raises(np.linalg.LinAlgError):
             mh.linsolve(A, rng.standard_normal((n, 2)) + 0j, precision=precision, ctx=ctx)
+
+
+@pytest.mark.parametrize("bits", [23, 24, 25, 31, 40, 52, 53])
+@pytest.mark.parametrize("unit", [1.0, -1.0, 1j, -1j])
+def test_entries_just_below_a_power_of_two(mh, ctx, bits, unit):
+    # multipliers and rows of U just below one, the largest fixed-point numbers of the exact digits:
+    # symmetric meshes have such multipliers
+    n = 200
+    rng = np.random.default_rng(bits)
+    A = 0.2 * (rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))) / np.sqrt(n) + 2.0 * np.eye(n)
+    near = 1.0 - 2.0 ** -bits
+    A[0, 0] = 1.0
+    A[40:80, 0] = unit * near
+    A[0, 100:140] = near
+    A[64, 64] = 4.0
+    A[150:160, 64] = 4.0 * unit * near
+    b = rng.standard_normal((n, 2)) + 0j
+    x = mh.linsolve(A, b, precision="fp64_tc", ctx=ctx)
+    r = np.abs(b - A @ x).max(axis=0)
+    assert (r <= 20 * n * EPS * (np.abs(A).sum(axis=1).max() * np.abs(x).max(axis=0) + np.abs(b).max(axis=0))).all()
