@@ -290,8 +290,8 @@ int mh_autotune(mh_context* ctx, int precision, int64_t n_sizes, const int64_t* 
                 MH_GF_EXACT_DELHOMMEAU (not both).  The exact term's second
                 derivatives come from its value and r-derivative at each pair
                 (dG/dz = G + 2/d, exact_Guevel_Delhommeau.jl:52-59, and Laplace's
-                equation in (r, z)); its quadrature runs once per pair and frequency
-                at the context's tolerance, as in the primal
+                equation in (r, z)), evaluated once per pair and frequency, as in
+                the primal
      direct:    1 DirectBEM (phi = D^-1 S bc), 0 IndirectBEM (sigma = K^-1 bc,
                 phi = S sigma): solve(D, S, bc; direct), matrix_assembly.jl:436-449
      dofs:      n_dofs x n x 3 dof fields, held fixed
@@ -361,14 +361,13 @@ int mh_solve_pullback(mh_context* ctx, int64_t n, int64_t nrhs, const double* D,
    b3, W4[6][64], b4 (mh_surrogate_param_count() floats). */
 int mh_surrogate_param_count(void);
 /* Trains on the device: n_samples points drawn with `seed` (r log-uniform, z uniform
-   in the box), targets from the exact kernel at the context's quadrature
-   tolerances; Adam with cosine-decayed learning rate from lr, `epochs` passes in
-   batches of `batch`, BF16-rounded forward weights.  Installs the result on the
-   context and writes it to params_out (may be NULL).  report (may be NULL), 10
-   doubles: final mean squared error; RMS and max relative error of G over held-out
-   points for the surrogate, then for the Wu fits; max relative error of dG/dr,
-   surrogate then Wu; seconds of sample generation; seconds of training; number of
-   held-out points. */
+   in the box), targets from the exact kernel; Adam with cosine-decayed learning rate
+   from lr, `epochs` passes in batches of `batch`, BF16-rounded forward weights.
+   Installs the result on the context and writes it to params_out (may be NULL).
+   report (may be NULL), 10 doubles: final mean squared error; RMS and max relative
+   error of G over held-out points for the surrogate, then for the Wu fits; max relative
+   error of dG/dr, surrogate then Wu; seconds of sample generation; seconds of training;
+   number of held-out points. */
 int mh_surrogate_train(mh_context* ctx, int64_t n_samples, uint64_t seed, int epochs, int batch, double lr,
                        float* params_out, double* report);
 /* Installs parameters (rounded to BF16) on the context. */
@@ -386,9 +385,9 @@ int mh_surrogate_loss_grad(mh_context* ctx, const float* params, int64_t m, cons
    surrogate approximates exact_Guevel_Delhommeau.jl:15-46).  With n_samples > 0, every
    sweep (mh_hydrodynamic_coefficients) and batch that assembles with MH_GF_SURROGATE has
    each frequency's S and D checked against the exact term on n_samples ordered panel
-   pairs drawn from `seed` (the adaptive quadrature at the context's tolerance): the
-   estimate is the relative error sqrt(sum |S - S_exact|^2 + |D - D_exact|^2) /
-   sqrt(sum |S|^2 + |D|^2) over the sampled entries.  A frequency whose estimate exceeds
+   pairs drawn from `seed`: the estimate is the relative error
+   sqrt(sum |S - S_exact|^2 + |D - D_exact|^2) / sqrt(sum |S|^2 + |D|^2) over the
+   sampled entries.  A frequency whose estimate exceeds
    `tolerance` is solved with the exact term instead (the sweep assembles that matrix
    again before its factorization; the batch re-runs those frequency-solves after its
    graph).  n_samples = 0 turns the check off (the default). */
@@ -407,7 +406,8 @@ int mh_wu_wave_terms(mh_context* ctx, int64_t m, const double* hh, const double*
    for m points: out 2 complex per point; rtol/atol: adaptive Gauss-Kronrod
    tolerances (the reference's Integrals.jl call uses its defaults), used at points
    with z > 0 (or r = z = 0); at and below the surface the integrals are evaluated in
-   closed form up to a smooth finite integral, to rounding. */
+   closed form up to a smooth finite integral, to rounding.  A point that is not finite
+   gives NaN. */
 int mh_exact_wave_terms(mh_context* ctx, int64_t m, const double* r, const double* z, double rtol, double atol,
                         double* out, int mem);
 /* J0, J1, Y0, Y1 at m points x >= 0, as the Wu kernels evaluate them: out 4 doubles

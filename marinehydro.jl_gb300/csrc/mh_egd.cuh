@@ -12,7 +12,7 @@
 // some 5000 FP64 instructions for each) becomes one thread per pair with at most ~550 FP64
 // instructions, its exponentials, square roots, logarithms and Bessel polynomials on the integer
 // pipe (mh_fixpoint.cuh).  The kernels stay bound by the FP64 pipe (two lanes per SM and clock).  S and
-// D of a 900-panel hemisphere into device buffers: 44.8 ms with the quadrature, 0.52 ms so.
+// D of a 900-panel hemisphere into device buffers: 44.8 ms with the quadrature, 0.37 ms so.
 //
 // * I over [a, Y] by Gauss-Legendre: e^(t - Y) makes everything below Y - 38 vanish, so the
 //   interval is at most 38 long; 18 nodes up to a length of 22, 24 above (the integrand's

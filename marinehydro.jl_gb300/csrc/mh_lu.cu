@@ -443,7 +443,11 @@ __global__ void __launch_bounds__(kPanelThreads) panel_cluster_kernel(BatchDesc 
       }
     };
     if (nrb > 0) {
-      // as few columns per item as keep the multipliers' loads (FP32: and products) in the shade
+      // As few columns per item as keep the multipliers' loads (FP32: and products) in the shade.
+      // All panels of one factorization, ms, this rule against 1, 2, 4 and 8 columns throughout: FP64
+      // order 200 0.437 (0.440 0.451 0.442 0.544), 900 2.30 (2.31 2.37 2.37 2.75), 4500 20.4 (20.0 20.5
+      // 21.3 23.8); FP32 200 0.238 (0.240 0.237 0.246 0.276), 900 1.26 (1.27 1.25 1.27 1.41), 4500 8.52
+      // (8.81 8.49 8.29 8.73).
       if (nrb <= 2) rest(std::integral_constant<int, sizeof(T) == 8 ? 1 : 2>());
       else if (sizeof(T) == 8 || nrb <= 6) rest(std::integral_constant<int, sizeof(T) == 8 ? 2 : 4>());
       else rest(std::integral_constant<int, 8>());
@@ -1623,7 +1627,12 @@ int lu_factor_batched(cudaStream_t st, LaunchCounter lc, const BatchDesc& d, typ
 // time in SM cycles.  A step's chain is two 32 x 32 products by the g vectors on one SM (2300 g
 // cycles each on the FP64 pipes; latency in FP32) and a cluster barrier; its bulk the update of
 // half the rows, by the cluster's SMs.  More CTAs shorten the bulk, fewer vectors per cluster
-// both, as long as the clusters stay resident and have SMs of their own.
+// both, as long as the clusters stay resident and have SMs of their own.  The constants are
+// measured phase times; the shape that they pick against the fastest of 42 (P of 1 to 16, g of 1 to
+// 8), us: FP64 order 200, 2 vectors 64 (57 at P 6 g 1; the slowest 188), 2999, 9 vectors 1701 (1916 P 16
+// g 1; 34 ms), 1000, 40 vectors 618 (614 P 6 g 1; 10.7 ms), five of 1000, 7 vectors 516 (504 P 8 g 1; 8.1
+// ms), one of 1000 311 (272 P 16 g 1; 8.1 ms); FP32 twelve of 450, 7 vectors 79 (80 P 4 g 3; 229), four of
+// 1400 228 (226 P 12 g 2; 1.2 ms), 4500, 4 vectors 748 (748 P 16 g 1; 8.5 ms).
 struct SolveShape { int P, g; };
 template <typename T>
 SolveShape solve_shape(int64_t n, int64_t nrhs, int64_t batch, bool upper_only) {

@@ -42,9 +42,8 @@ __device__ __forceinline__ uint64_t splitmix64(uint64_t x) {
 
 __device__ __forceinline__ double u01(uint64_t h) { return (double)(h >> 11) * (1.0 / 9007199254740992.0); }
 
-// sample q of M for `seed`: log10(r) stratified (one jittered point per 1/M of
-// [-3, 3], so neighbouring threads get similar r and similar quadrature work),
-// z uniform in [-50, 0]
+// sample q of M for `seed`: log10(r) stratified (one jittered point per 1/M of [-3, 3], so that
+// neighbouring threads get similar r and mostly the same branches), z uniform in [-50, 0]
 __device__ __forceinline__ void sample_point(uint64_t seed, uint64_t q, uint64_t M, double& r, double& z) {
   const uint64_t h1 = splitmix64(seed ^ splitmix64(q));
   const uint64_t h2 = splitmix64(h1);

@@ -61,7 +61,7 @@ class GFWu(GreensFunction):
 
 
 class ExactGuevelDelhommeau(GreensFunction):
-    """Exact Guevel-Delhommeau wave term by adaptive quadrature (exact_Guevel_Delhommeau.jl:3)."""
+    """Exact Guevel-Delhommeau wave term (exact_Guevel_Delhommeau.jl:3)."""
     flag = _lib.GF_EXACT_DELHOMMEAU
 
 
